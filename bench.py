@@ -1186,7 +1186,7 @@ def main():
     B, H, N, D, order, causal, dtype_name, scale = WORKLOADS[args.workload]
     dtype = torch.bfloat16 if dtype_name == "bf16" else torch.float32
     inv_temp = 1.0 / (8.0 * math.sqrt(D))
-    flags = _lib.FLAG_NO_TENSOR_CORES if args.no_tensor_cores else 0
+    flags = _lib.FLAG_NO_TENSOR_CORES if args.no_tensor_cores else _lib.FLAG_PAIRWISE   # what the Python operators ask for
     gen = torch.Generator(device=dev).manual_seed(1234 + rank)
     q, k, v, do = ((torch.randn(B, H, N, D, device=dev, generator=gen) * scale).to(dtype) for _ in range(4))
     lib = _lib.load()
@@ -1253,9 +1253,17 @@ def main():
     m_full = 1 + D + (D * D if order == 2 else 0)
     ratio_exec = executed_units(D, order) / m_full
 
+    # The pairwise kernels report under the same kinds; their products per visible pair: forward 4 d, dq 6 d, dk and dv 8 d
+    # from one launch (listed under both kinds).  The scans are told apart by the transposed copies they read.
+    pairwise = bool(flags & _lib.FLAG_PAIRWISE) and dtype_name == "bf16" and "tc_transpose" not in kernels
+    visible = B * H * (N * (N + 1) / 2 if causal else N * N)
+    pair_flops = {"tc_scan_fwd": 4.0, "tc_scan_bwd_q": 6.0, "tc_scan_bwd_kv": 4.0, "tc_scan_bwd_dv": 4.0}
+
     def counted_flops(name):
         """min(algorithmic, executed) flops of one launch: never credits more than the hardware did."""
         alg = units_alg.get(name, 0.0) * U
+        if pairwise:
+            return min(alg, pair_flops.get(name, 0.0) * D * visible), alg
         ex = units_exec.get(name, units_alg.get(name, 0.0)) * U * (ratio_exec if name.startswith("tc_") else 1.0)
         return min(alg, ex), alg
 
@@ -1271,12 +1279,14 @@ def main():
             "kernel": dominant, "bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak, "peak_source": pk["_source"] + " (sustained cuBLAS bf16: kernel timed inside a long step)",
             "full_d2_equivalent": alg * per_launch / dur_s / 1e12,
-            "note": "achieved = min(algorithmic, executed) flops of the launch / its CUDA-event time: executed counts the "
-                    "block-symmetric feature rows (0.569 of D^2+D+1) the kernel contracts over, twice (state rebuild + "
-                    "apply or dphi); full_d2_equivalent is the rate the reference's D^2 formulation would need",
-            "traffic": DRAM_TRAFFIC.get(dominant, {}).get("bytes_per_launch") and
+            "note": "achieved = min(algorithmic, executed) flops of the launch / its CUDA-event time: " +
+                    ("executed counts the products of visible token pairs" if pairwise else
+                     "executed counts the block-symmetric feature rows (0.569 of D^2+D+1) the kernel contracts over, twice "
+                     "(state rebuild + apply or dphi)") +
+                    "; full_d2_equivalent is the rate the reference's D^2 formulation would need",
+            "traffic": None if pairwise else DRAM_TRAFFIC.get(dominant, {}).get("bytes_per_launch") and
                        DRAM_TRAFFIC[dominant]["bytes_per_launch"] * (B * H * N) / DRAM_TRAFFIC[dominant]["head_tokens"],
-            "traffic_source": DRAM_TRAFFIC.get(dominant, {}).get("source"),
+            "traffic_source": None if pairwise else DRAM_TRAFFIC.get(dominant, {}).get("source"),
         }
     if order == 1:   # 33 flop per byte: bound by HBM; the whole call against its algorithmic bytes
         esz = 2 if dtype_name == "bf16" else 4

@@ -68,6 +68,9 @@ typedef struct {
 
 enum {
   FASTMAX_FLAG_NO_TENSOR_CORES = 1, /* force the CUDA-core kernels even where a tcgen05 kernel exists */
+  FASTMAX_FLAG_PAIRWISE = 4,        /* let the library evaluate the scores pair by pair (quadratic in the length) where  */
+                                    /* that is the faster form; without it every call runs on the moment engines, whose  */
+                                    /* time and scratch are linear in the length.  The Python operators set it.          */
   FASTMAX_FLAG_SINGLE_STREAM = 2    /* keep every launch on the caller's stream.  By default the tensor-core path runs  */
                                     /* its independent scans side by side on up to three internal streams (created once */
                                     /* per device on first use, forked from and joined back into the caller's stream    */

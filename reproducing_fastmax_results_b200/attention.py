@@ -139,8 +139,8 @@ class FastMax(torch.autograd.Function):
         cast = qc is not q
         # the fourth entry: per-segment key moments when the call computed some (long sequences with few heads on the
         # CUDA-core engine); the backward reads them instead of passing over k and v again
-        o, g, _, kmom = ext.forward(qc, kc, vc, bool(mask), inv_t, float(a0), float(a1), float(a2), int(p), None, False, True, 0,
-                                    None, None, True)
+        o, g, _, kmom = ext.forward(qc, kc, vc, bool(mask), inv_t, float(a0), float(a1), float(a2), int(p), None, False, True,
+                                    ext.PAIRWISE, None, None, True)
         noise = None
         out = o
         if noise_dropout and float(dropout) != 0.0:
@@ -172,8 +172,8 @@ class FastMax(torch.autograd.Function):
             grad_output = grad_output.to(o.dtype)
         if noise_scale != 0.0:     # out = o * (1 + s * noise)  ->  d o = d out * (1 + s * noise)
             grad_output = ext.output_noise(grad_output, ctx.saved_tensors[-1], noise_scale)
-        dq, dk, dv, _ = ext.backward(q, k, v, o, g, grad_output, mask, inv_t, a0, a1, a2, p, None, None, False, True, 0,
-                                     None, ctx.key_moments)
+        dq, dk, dv, _ = ext.backward(q, k, v, o, g, grad_output, mask, inv_t, a0, a1, a2, p, None, None, False, True,
+                                     ext.PAIRWISE, None, ctx.key_moments)
         if ctx.cast:
             dq, dk, dv = dq.float(), dk.float(), dv.float()
         if k_scale != 1.0:         # the operator saw k / temperature + rpe rows

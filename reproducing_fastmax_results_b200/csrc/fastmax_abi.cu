@@ -10,6 +10,7 @@
 #include "../../include/fastmax_b200.h"
 #include "aux_kernels.cuh"
 #include "launchers.cuh"
+#include "pair_launchers.cuh"
 #include "tc_launchers.cuh"
 
 namespace fm {
@@ -19,7 +20,7 @@ static thread_local int g_last_cuda_error = 0;
 
 // ---- optional per-kernel timing -----------------------------------------------------------------
 struct ProfRec {
-  int kind;
+  int kind, also;
   cudaEvent_t a, b;
 };
 static std::atomic<int> g_prof_on{0};
@@ -37,14 +38,14 @@ void launch_begin(int kind, cudaStream_t st) {
   cudaEventRecord(a, st);
   g_prof_open = a;
 }
-void launch_end(int kind, cudaStream_t st) {
+void launch_end(int kind, cudaStream_t st, int also) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (g_prof_open == nullptr) return;
   cudaEvent_t b = nullptr;
   if (cudaEventCreate(&b) == cudaSuccess) {
     cudaEventRecord(b, st);
     std::lock_guard<std::mutex> lk(g_prof_mu);
-    g_prof_recs.push_back(ProfRec{kind, g_prof_open, b});
+    g_prof_recs.push_back(ProfRec{kind, also, g_prof_open, b});
   } else {
     cudaEventDestroy(g_prof_open);
   }
@@ -409,8 +410,13 @@ int32_t fastmax_profile_collect(double* ms, uint64_t* count, int32_t nkinds) {
       g_last_cuda_error = (int)e;
       rc = FASTMAX_ERR_CUDA;
     } else if (r.kind >= 0 && r.kind < nkinds) {
-      ms[r.kind] += t;
+      const bool both = r.also >= 0 && r.also < nkinds;
+      ms[r.kind] += both ? 0.5 * t : t;
       count[r.kind] += 1;
+      if (both) {
+        ms[r.also] += 0.5 * t;
+        count[r.also] += 1;
+      }
     }
     cudaEventDestroy(r.a);
     cudaEventDestroy(r.b);
@@ -438,6 +444,7 @@ static int fwd_layout(const fastmax_problem* pb, const fastmax_forward_args* a, 
 size_t fastmax_forward_workspace(const fastmax_problem* pb, const fastmax_forward_args* args) {
   Plan pl;
   if (!args || make_plan(pb, pl) != FASTMAX_OK) return 0;
+  if (pair_takes_forward(pb, args)) return 0;
   FwdLayout L;
   fwd_layout(pb, args, pl, L);
   size_t tc = tc_forward_workspace(pb, args);
@@ -453,6 +460,7 @@ int32_t fastmax_forward_engine(const fastmax_problem* pb, const fastmax_forward_
 size_t fastmax_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_args* args) {
   Plan pl;
   if (!args || make_plan(pb, pl) != FASTMAX_OK || pb->nk == 0) return 0;
+  if (pair_takes_forward(pb, args)) return 0;
   if (const size_t t = tc_key_moments_bytes(pb, args)) return t;   // a long sequence cut into segments for the tensor-memory kernels
   if (tc_takes_forward(pb, args)) return 0;   // the tensor-memory kernels take this call whole: no segment sums
   FwdLayout L;
@@ -483,6 +491,7 @@ int32_t fastmax_forward(const fastmax_problem* pb, const fastmax_forward_args* a
   if (ws_bytes < fastmax_forward_workspace(pb, a) || (ws_bytes && (!ws || ((uintptr_t)ws % 256))))
     return FASTMAX_ERR_WORKSPACE;
 
+  if (want_o && pair_takes_forward(pb, a)) return pair_forward(pb, a, st);
   int tcrc = tc_forward(pb, a, ws, ws_bytes, st);
   if (tcrc != FASTMAX_TC_NOT_HANDLED) return tcrc;
 
@@ -563,6 +572,7 @@ static void bwd_layout(const fastmax_problem* pb, const fastmax_backward_args* a
 size_t fastmax_backward_workspace(const fastmax_problem* pb, const fastmax_backward_args* args) {
   Plan pl;
   if (!args || make_plan(pb, pl, true) != FASTMAX_OK) return 0;
+  if (pair_takes_backward(pb, args)) return pair_backward_workspace(pb) + 256;
   BwdLayout L;
   bwd_layout(pb, args, pl, L);
   size_t tc = tc_backward_workspace(pb, args);
@@ -572,6 +582,7 @@ size_t fastmax_backward_workspace(const fastmax_problem* pb, const fastmax_backw
 size_t fastmax_grad_moments_bytes(const fastmax_problem* pb, const fastmax_backward_args* args) {
   Plan pl;
   if (!args || make_plan(pb, pl, true) != FASTMAX_OK) return 0;
+  if (pair_takes_backward(pb, args)) return 0;
   if (const size_t t = tc_grad_moments_bytes(pb, args)) return t;
   if (tc_takes_backward(pb, args)) return 0;   // the tensor-memory kernels take this call whole: no segment sums
   BwdLayout L;
@@ -624,6 +635,7 @@ int32_t fastmax_backward(const fastmax_problem* pb, const fastmax_backward_args*
     return FASTMAX_OK;
   }
 
+  if (pair_takes_backward(pb, a)) return pair_backward(pb, a, ws, st);
   int tcrc = tc_backward(pb, a, ws, ws_bytes, st);
   if (tcrc != FASTMAX_TC_NOT_HANDLED) return tcrc;
 

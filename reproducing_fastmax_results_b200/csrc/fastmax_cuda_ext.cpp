@@ -113,6 +113,7 @@ torch::Tensor forwardpass(torch::Tensor q, torch::Tensor k, torch::Tensor v, tor
     fastmax_forward_args ab = a;
     ab.q = view_nbd(qb); ab.k = view_nbd(kb); ab.v = view_nbd(vb); ab.o = view_nbd(ob);
     if (fastmax_forward_engine(&pbb, &ab) == 1) {
+      pbb.flags |= FASTMAX_FLAG_PAIRWISE;
       size_t need = fastmax_forward_workspace(&pbb, &ab);
       auto ws = workspace(need, q);
       check_status(fastmax_forward(&pbb, &ab, aligned(ws), need, stream), "fastmax forwardpass (bfloat16 compute)");
@@ -159,6 +160,7 @@ std::vector<torch::Tensor> backwardpass(torch::Tensor q, torch::Tensor k, torch:
       fastmax_backward_args ab = a;
       ab.q = fb.q; ab.k = fb.k; ab.v = fb.v; ab.o = fb.o; ab.d_out = view_nbd(gb);
       ab.dq = view_nbd(dqb); ab.dk = view_nbd(dkb); ab.dv = view_nbd(dvb);
+      pbb.flags |= FASTMAX_FLAG_PAIRWISE;
       size_t need = fastmax_backward_workspace(&pbb, &ab);
       auto ws = workspace(need, q);
       check_status(fastmax_backward(&pbb, &ab, aligned(ws), need, stream), "fastmax backwardpass (bfloat16 compute)");
@@ -415,6 +417,7 @@ PYBIND11_MODULE(fastmax_cuda, m) {
         py::arg("rpe") = py::none(), release());
   m.def("output_noise", &output_noise, "x * (1 + scale * noise)", release());
   m.def("forward_engine", &forward_engine, "1: tensor-memory kernels, 0: CUDA-core engine, for a forward call on these tensors");
+  m.attr("PAIRWISE") = (int)FASTMAX_FLAG_PAIRWISE;
   m.def("launch_count", &launch_count, "kernel launches issued by the library so far");
   m.def("version", []() { return std::string(fastmax_version()); });
 }

@@ -25,12 +25,14 @@ enum KernelKind {
 };
 bool profiling_on();   // per-kernel timing is enabled: launch sequences then stay on one stream so the times do not overlap
 void launch_begin(int kind, cudaStream_t st);
-void launch_end(int kind, cudaStream_t st);
+void launch_end(int kind, cudaStream_t st, int also);
+// also: a second kind the same launch does the work of (dk and dv from one kernel): it is listed under both, with half of
+// its time each, and counts as one launch.
 struct LaunchScope {
-  int kind;
+  int kind, also;
   cudaStream_t st;
-  LaunchScope(int k, cudaStream_t s) : kind(k), st(s) { launch_begin(k, s); }
-  ~LaunchScope() { launch_end(kind, st); }
+  LaunchScope(int k, cudaStream_t s, int a = -1) : kind(k), also(a), st(s) { launch_begin(k, s); }
+  ~LaunchScope() { launch_end(kind, st, also); }
 };
 
 }  // namespace fm

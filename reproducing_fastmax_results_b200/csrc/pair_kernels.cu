@@ -1,0 +1,922 @@
+// Pairwise tcgen05 / TMEM kernels: the scores are evaluated tile by tile and nothing is carried between tiles, so
+//     forward   S = Q K^T,             P = f(S),                                  O' = P V,  g = row sums of P
+//     dq        S = Q K^T, dP = dO' V^T, dS = f'(S) (dP - delta),                 dq = dS K
+//     dk, dv    the transposes with a key tile held:                              dv = P^T dO',  dk = dS^T Q
+// where dO' = dO / g and delta = (dO . o) / g.  Cost is quadratic in the length, 14 d products per visible pair against
+// 2145 x 65 products per token and moment pass at d = 64: below several thousand tokens this is the smaller number, every
+// thread block is independent (no scan over the sequence, no partial sums in memory), and each result is written once,
+// in its own type.  pair_takes_* hold the rule that chooses between this and the moment scans.
+//
+// A work item holds 128 rows (256 in the forward: two tiles that take turns on the tensor pipe; keys for dk / dv, queries
+// otherwise) and streams 128-row tiles of the other side through a TMA ring.  Scores land in TMEM as [held x streamed];
+// the element-wise warps turn them into the bf16 A operand of the second product in place, and the streamed tile is read
+// from shared memory K-major by the first product and MN-major by the second: nothing is transposed or copied.
+//
+// One thread block per SM works through items.  A block asks the hardware scheduler for its next item (cluster launch
+// control: it takes over a block that has not started), so the items' lengths may differ by any factor; the loads and
+// first products of the next item run under the last tiles and the stores of the current one.
+#include <cuda.h>
+#include <cuda_bf16.h>
+
+#include <atomic>
+#include <cmath>
+#include <cstring>
+
+#include "common.cuh"
+#include "launchers.cuh"
+#include "pair_launchers.cuh"
+#include "tc_launchers.cuh"
+#include "tc_ptx.cuh"
+
+namespace fm {
+namespace pair {
+
+using namespace tc;
+
+__device__ int g_status = 0;
+__device__ int g_wait_hist[256];
+
+constexpr long long WAIT_CYCLES = 4000000000ll;   // ~2 s at 2 GHz
+constexpr int R = 128;                  // held rows of one accumulator (the TMEM lanes)
+constexpr int T = 128;                  // streamed rows per tile
+constexpr int EW = 8;                   // element-wise warps: two per TMEM lane quarter (FWD: one per held tile; else 64-column halves)
+constexpr int W_SCORE = 0, W_ACC = 1, W_LOAD = 2, W_EW = 4;   // warp roles: two issuers, loader, (spare), element-wise warps
+constexpr int ROLES = EW + 3;           // warps that follow the items
+constexpr int THREADS = (W_EW + EW) * 32;
+constexpr int X_BYTES = T * 128;        // operand tile: 128-byte rows whatever the head dim (narrow heads zero-filled by the copy engine)
+constexpr int STAGES = 4;               // ring of streamed tile pairs
+enum Kind { FWD = 0, DQ = 1, DKV = 2 };
+
+struct Params {
+  View out0, out1;            // FWD: o, g; DQ: dq; DKV: dk, dv
+  const float* ndelta;        // [batch*heads][nd_ld]: -delta per query, zero from nq on
+  int nd_ld;
+  int heads, nr, nx;          // held rows, streamed rows per head
+  int off, causal;            // query l sees the keys up to l + off
+  int ntiles;                 // items per head
+  uint32_t mul_t, mul_h;      // quotients by ntiles and heads without a division: (n * mul) >> shift
+  int sh_t, sh_h;
+  int vec0, vec1;             // rows of out0 / out1 start on 16-byte boundaries: written by the copy engine
+  float c0, c1, c2;
+  float k, w0, w1;            // completed square (see SQ): c0 / c2 - h^2; factors of out0 and out1
+  uint32_t h01, h2;           // h = c1 / (2 c2) as the sum of three bf16 numbers
+};
+
+// ---- two-lane float32 arithmetic -------------------------------------------------------------------------
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t pack2u(uint32_t a, uint32_t b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
+  __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&r);
+}
+__device__ __forceinline__ uint32_t bf16x2(uint64_t v) {
+  float a, b;
+  unpack2(v, a, b);
+  return bf16x2(a, b);
+}
+
+__device__ __noinline__ void fail_record(int code, volatile int* abort_flag) {
+  if (*abort_flag == 0) atomicAdd(&g_wait_hist[code & 255], 1);
+  *abort_flag = 1;
+  atomicExch(&g_status, code);
+}
+__device__ __noinline__ void wait_slow(uint64_t* bar, uint32_t parity, int code, volatile int* abort_flag) {
+  if (*abort_flag == 0 && !mbar_wait_abortable(bar, parity, WAIT_CYCLES, abort_flag)) fail_record(code, abort_flag);
+}
+// Waits for the phase of parity `parity`.  Returns in any case: when the wait runs out the abort flag is up, every later
+// wait of the block falls through at once and the roles run out of items (next_item).  No caller branches on the outcome,
+// which keeps the issuer's control flow warp-uniform and its operands in uniform registers.
+__device__ __forceinline__ void wait_fast(uint64_t* bar, uint32_t parity, int code, volatile int* abort_flag) {
+  if (!mbar_try_wait(bar, parity)) wait_slow(bar, parity, code, abort_flag);
+}
+
+// N consecutive TMEM columns of this thread's lane
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&r)[N]) {
+  if constexpr (N == 32) tmem_ld32(addr, r);
+  else if constexpr (N == 16) tmem_ld16(addr, r);
+  else tmem_ld8(addr, r);
+}
+template <int N>
+__device__ __forceinline__ void tmem_st(uint32_t addr, const uint32_t (&r)[N]) {
+  if constexpr (N == 32) tmem_st32(addr, r);
+  else if constexpr (N == 16) tmem_st16(addr, r);
+  else tmem_st8(addr, r);
+}
+
+// ---- cluster launch control: the next block of the grid that has not started, or none ---------------------
+__device__ __forceinline__ void clc_try_cancel(void* smem16, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(smem_u32(smem16)), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ int clc_read(const void* smem16) {   // block index, or -1
+  uint32_t ok, x;
+  asm volatile(
+      "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\t"
+      "ld.shared.b128 h, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t"
+      "mov.b32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+      : "=r"(ok), "=r"(x)
+      : "r"(smem_u32(smem16))
+      : "memory");
+  return ok ? (int)x : -1;
+}
+
+constexpr int OFF_HELD = 0;                              // two sets of two held tiles
+constexpr int OFF_X = 4 * X_BYTES;
+constexpr int STAGE = 2 * X_BYTES;
+constexpr int OFF_ND = OFF_X + STAGES * STAGE;           // DKV: -delta of the streamed queries, T floats per stage
+constexpr int OFF_H = OFF_ND + STAGES * T * 4;              // SQ: two constant 128 x 16 operands whose product is h everywhere
+constexpr int OFF_CLC = OFF_H + 2 * R * 32;         // ring of 16-byte answers of the scheduler
+constexpr int CLC = 4;
+constexpr int OFF_BAR = OFF_CLC + 16 * CLC;
+constexpr int SMEM_BYTES = OFF_BAR + 512 + 1024;
+static_assert(SMEM_BYTES <= 232448, "shared memory budget");
+// barrier slots
+constexpr int B_FULL = 0, B_EMPTY = 4, B_HFULL = 8, B_HEMPTY = 10, B_S = 12, B_READS = 14, B_READD = 16, B_P = 17, B_SFREE = 19, B_ACC = 21,
+              B_AFREE = 23, B_CFULL = 25, B_CEMPTY = B_CFULL + CLC, B_DRAIN = B_CEMPTY + CLC, B_COUNT = B_DRAIN + 2;
+static_assert(B_COUNT * 8 <= 384, "barriers and flags share 512 bytes");
+// TMEM columns.  FWD: O' of the two held tiles, their scores, their bf16 tiles P.  DQ: dq, dS, two score buffers, dP.
+// DKV: dv, dk, scores, dP, P, dS.  The bf16 tiles have columns of their own: scores and dP are free as soon as the
+// element-wise warps have READ them, so the next tile's first products run under this tile's arithmetic.
+constexpr uint32_t C_ACC = 0, C_ACC1 = 64, C_S = 128;
+template <int KIND>
+struct Cols {
+  static constexpr uint32_t DP = KIND == DQ ? 384 : 256;
+  static constexpr uint32_t P = 384;                         // FWD: + 64 for the second held tile
+  static constexpr uint32_t DS = KIND == DQ ? 64 : 448;
+};
+
+struct Item {
+  int head, b, h;
+  int r0;          // first held row
+  int t0;          // first streamed tile
+  int n0, n1;      // streamed tiles of the held tile(s); n1: the second tile of a forward item
+};
+template <int KIND>
+__device__ __forceinline__ Item decode(int idx, const Params& P) {
+  // Head-major, the longest item of a head first: the blocks at work share a few heads' streamed tiles in L2, and the
+  // last items are short.
+  Item it;
+  it.head = (int)(((uint64_t)(uint32_t)idx * P.mul_t) >> P.sh_t);
+  const int ti = idx - it.head * P.ntiles;
+  it.b = (int)(((uint64_t)(uint32_t)it.head * P.mul_h) >> P.sh_h);
+  it.h = it.head - it.b * P.heads;
+  it.t0 = 0;
+  it.n1 = 0;
+  const int all = (P.nx + T - 1) / T;
+  if (KIND == DKV) {
+    it.r0 = ti * R;
+    const int first = it.r0 - P.off;                 // first query that sees key r0
+    if (P.causal && first > 0) it.t0 = first / T;
+    it.n0 = all - it.t0;
+  } else {
+    it.r0 = (P.ntiles - 1 - ti) * (KIND == FWD ? 2 * R : R);
+    it.n0 = P.causal ? min(all, (it.r0 + R - 1 + P.off) / T + 1) : all;
+    if (KIND == FWD && it.r0 + R < P.nr) it.n1 = P.causal ? min(all, (it.r0 + 2 * R - 1 + P.off) / T + 1) : all;
+  }
+  return it;
+}
+
+// SQ: the square completed.  f(s) / c2 = u^2 + k and f'(s) / (2 c2) = u with u = s + h, h = c1 / (2 c2): the first product
+// itself adds h (one more K = 16 step with constant operands, 65 clocks of the tensor pipe), so f costs one multiply-add
+// instead of two and f' nothing; the factors go into the epilogues.  The element-wise warps are bound by the FMA pipe (a
+// packed instruction takes 2.2 clocks per warp), which makes every instruction per element worth 140 clocks per tile.
+struct Maps {
+  CUtensorMap x, y;     // streamed tiles
+  CUtensorMap a, b;     // held tiles
+  CUtensorMap o0, o1;   // outputs, 32-row boxes
+};
+
+template <int D, int KIND, bool SQ>
+__global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant__ Maps M, const Params P) {
+  constexpr int KS = D / 16;                    // K steps of the first products
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  uint8_t* sm = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + OFF_BAR);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + OFF_BAR + 384);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + OFF_BAR + 392);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int w = __shfl_sync(0xffffffffu, tid >> 5, 0);   // warp-uniform for the compiler too
+
+  if (tid == 0) {
+    for (int i = 0; i < B_COUNT; ++i) {
+      uint32_t n = 1;
+      if (i >= B_READS && i < B_SFREE) n = KIND == FWD ? EW / 2 : EW;                          // READS, READD, P
+      if (i == B_AFREE || i == B_AFREE + 1) n = KIND == DKV ? EW : EW / 2;
+      if (i == B_HEMPTY || i == B_HEMPTY + 1) n = 1 + EW;                       // products done, output rows staged there copied
+      if (i >= B_CEMPTY && i < B_CEMPTY + CLC) n = ROLES;                       // every role has read the answer
+      mbar_init(&bars[i], n);
+    }
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (SQ && tid < 2 * R) {   // K-major without swizzle: 8 x 8 core matrices of 128 bytes, two along K
+    uint8_t* dst = sm + OFF_H + (tid >> 7) * (R * 32) + ((tid & 127) >> 3) * 256 + (tid & 7) * 16;
+    *reinterpret_cast<uint4*>(dst) = tid < R ? make_uint4(P.h01, P.h2, 0u, 0u) : make_uint4(0x3F803F80u, 0x00003F80u, 0u, 0u);
+    *reinterpret_cast<uint4*>(dst + 128) = make_uint4(0u, 0u, 0u, 0u);
+    fence_proxy_async_smem();
+  }
+  if (w == W_ACC) tmem_alloc(tmem_slot, 512);
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  auto WAIT = [&](int bar, uint32_t phase, int code) { wait_fast(&bars[bar], phase & 1u, code, abort_flag); };
+  // item n + 1 of this block, for every role: -1 at the end (or when a wait ran out)
+  auto next_item = [&](int n) -> int {
+    const int c = n & (CLC - 1);
+    WAIT(B_CFULL + c, (uint32_t)(n / CLC), 76);
+    int idx = *abort_flag != 0 ? -1 : clc_read(sm + OFF_CLC + 16 * c);
+    fence_proxy_async_smem();   // the slot is written again by the copy engine's side
+    idx = __shfl_sync(0xffffffffu, idx, 0);
+    if (lane == 0) mbar_arrive(&bars[B_CEMPTY + c]);
+    return idx;
+  };
+
+  int issued = 0;   // streamed tiles the loader has asked for
+  int helds = 0;    // held sets it has asked for
+  int asked = 0;    // items it has asked for
+  if (w == W_LOAD) {
+    // ================= loader and item scheduler =================
+    int idx = blockIdx.x;
+    for (int n = 0; idx >= 0; ++n) {
+      const int c = n & (CLC - 1);
+      if (n >= CLC) WAIT(B_CEMPTY + c, (uint32_t)(n / CLC) - 1u, 77);
+      if (*abort_flag != 0) break;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&bars[B_CFULL + c], 16);
+        clc_try_cancel(sm + OFF_CLC + 16 * c, &bars[B_CFULL + c]);
+      }
+      asked = n + 1;
+      const Item it = decode<KIND>(idx, P);
+      const int tiles = it.n0 > it.n1 ? it.n0 : it.n1;
+      if (n >= 2) WAIT(B_HEMPTY + (n & 1), (uint32_t)(n >> 1) - 1u, 78);
+      if (*abort_flag != 0) break;
+      if (lane == 0) {
+        uint8_t* hs = sm + OFF_HELD + (n & 1) * STAGE;
+        uint64_t* bar = &bars[B_HFULL + (n & 1)];
+        const bool two = KIND != FWD || it.n1 > 0;
+        mbar_arrive_expect_tx(bar, two ? 2 * X_BYTES : X_BYTES);
+        tma_load_4d(hs, &M.a, bar, 0, it.r0, it.h, it.b);
+        if (KIND == FWD && two) tma_load_4d(hs + X_BYTES, &M.a, bar, 0, it.r0 + R, it.h, it.b);
+        if (KIND == DQ) tma_load_4d(hs + X_BYTES, &M.b, bar, 0, it.r0, it.head, 0);   // dO': a dense array over all heads
+        if (KIND == DKV) tma_load_4d(hs + X_BYTES, &M.b, bar, 0, it.r0, it.h, it.b);
+      }
+      helds = n + 1;
+      for (int i = 0; i < tiles; ++i) {
+        const int s = issued & (STAGES - 1);
+        if (issued >= STAGES) WAIT(B_EMPTY + s, (uint32_t)(issued / STAGES) - 1u, 70);
+        if (*abort_flag != 0) break;
+        if (lane == 0) {
+          uint8_t* x = sm + OFF_X + s * STAGE;
+          const int row = (it.t0 + i) * T;
+          mbar_arrive_expect_tx(&bars[B_FULL + s], 2 * X_BYTES + (KIND == DKV ? T * 4 : 0));
+          tma_load_4d(x, &M.x, &bars[B_FULL + s], 0, row, it.h, it.b);
+          if (KIND == DKV) {
+            tma_load_4d(x + X_BYTES, &M.y, &bars[B_FULL + s], 0, row, it.head, 0);
+            bulk_load(sm + OFF_ND + s * T * 4, P.ndelta + (long long)it.head * P.nd_ld + row, T * 4, &bars[B_FULL + s]);
+          } else {
+            tma_load_4d(x + X_BYTES, &M.y, &bars[B_FULL + s], 0, row, it.h, it.b);
+          }
+        }
+        ++issued;
+      }
+      idx = next_item(n);
+    }
+  } else if (w == W_SCORE) {
+    // ================= issuer of the first products =================
+    // Two issuers, because a wait costs an issuing warp 150 clocks and a tile has up to four of them: one warp's serial
+    // chain (1010 clocks per tile in the forward) was twice the tensor pipe's time.
+    constexpr uint32_t ID_S = make_idesc_bf16(R, T, 0, 0);
+    const uint64_t dHeld = make_smem_desc(smem_u32(sm + OFF_HELD), 16, 1024, 2);
+    const uint64_t dXk = make_smem_desc(smem_u32(sm + OFF_X), 16, 1024, 2);          // streamed tile, K-major
+    const uint64_t dHa = make_smem_desc(smem_u32(sm + OFF_H), 128, 256, 0), dHb = make_smem_desc(smem_u32(sm + OFF_H + R * 32), 128, 256, 0);
+    uint32_t cnt[2] = {0, 0};     // tiles so far (FWD: of each held tile)
+    uint32_t tile = 0;            // streamed tiles so far
+    int idx = blockIdx.x;
+    for (int n = 0; idx >= 0; ++n) {
+      const Item it = decode<KIND>(idx, P);
+      const int tiles = it.n0 > it.n1 ? it.n0 : it.n1;
+      WAIT(B_HFULL + (n & 1), (uint32_t)(n >> 1), 71);
+      const uint64_t dH = dHeld + (uint64_t)((n & 1) * (STAGE >> 4));
+      for (int i = 0; i < tiles; ++i) {
+        const uint32_t s = tile & (STAGES - 1);
+        WAIT(B_FULL + s, tile / STAGES, 73);
+        const uint64_t dX = dXk + (uint64_t)(s * (STAGE >> 4)), dY = dX + (X_BYTES >> 4);
+#pragma unroll
+        for (int m = 0; m < (KIND == FWD ? 2 : 1); ++m) {
+          if (i < (m ? it.n1 : it.n0)) {
+            const uint32_t k = cnt[m];
+            const uint32_t buf = KIND == FWD ? (uint32_t)m : KIND == DQ ? (k & 1u) : 0u;
+            if (KIND == DQ) { if (k >= 2) WAIT(B_READS + buf, (k >> 1) - 1u, 80); }   // the buffer's last scores have been read
+            else if (k > 0) WAIT(B_READS + buf, k - 1u, 80);
+            tc_fence_after_sync();
+            if (SQ) mma_ss_elect(tmem + C_S + buf * 128u, dHa, dHb, ID_S, 0u);
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks)
+              mma_ss_elect(tmem + C_S + buf * 128u, dH + (uint64_t)(m * (X_BYTES >> 4) + 2 * ks), dX + (uint64_t)(2 * ks), ID_S, SQ || ks > 0);
+            if (KIND != FWD) {
+              if (k > 0) WAIT(B_READD, k - 1u, 82);
+              tc_fence_after_sync();
+#pragma unroll
+              for (int ks = 0; ks < KS; ++ks)
+                mma_ss_elect(tmem + Cols<KIND>::DP, dH + (uint64_t)((X_BYTES >> 4) + 2 * ks), dY + (uint64_t)(2 * ks), ID_S, ks > 0);
+            }
+            mma_commit_elect(&bars[B_S + buf]);
+            cnt[m] = k + 1;
+          }
+        }
+        ++tile;
+      }
+      mma_commit_elect(&bars[B_HEMPTY + (n & 1)]);
+      idx = next_item(n);
+    }
+    if (*abort_flag != 0) {   // a wait ran out: leave only after the products in flight
+      mma_commit_elect(&bars[B_DRAIN]);
+      mbar_wait_bounded(&bars[B_DRAIN], 0, WAIT_CYCLES);
+    }
+  } else if (w == W_ACC) {
+    // ================= issuer of the second products =================
+    constexpr uint32_t ID_ACC = make_idesc_bf16(R, D, 0, 1);
+    const uint64_t dXm = make_smem_desc(smem_u32(sm + OFF_X), X_BYTES, 1024, 2);     // streamed tile, MN-major
+    uint32_t cnt[2] = {0, 0}, tile = 0;
+    uint32_t nfree[2] = {0, 0};   // items that have started on each accumulator
+    int idx = blockIdx.x;
+    for (int n = 0; idx >= 0; ++n) {
+      const Item it = decode<KIND>(idx, P);
+      const int tiles = it.n0 > it.n1 ? it.n0 : it.n1;
+      for (int i = 0; i < tiles; ++i) {
+        const uint32_t s = tile & (STAGES - 1);
+        const uint64_t dX = dXm + (uint64_t)(s * (STAGE >> 4)), dY = dX + (X_BYTES >> 4);
+#pragma unroll
+        for (int m = 0; m < (KIND == FWD ? 2 : 1); ++m) {
+          const int nm = m ? it.n1 : it.n0;
+          if (i < nm) {
+            if (i == 0) {   // the accumulator's previous rows have been read
+              if (nfree[m] > 0) WAIT(B_AFREE + m, nfree[m] - 1u, 79);
+              nfree[m]++;
+            }
+            WAIT(B_P + m, cnt[m]++, 72);   // the bf16 tiles of the element-wise warps
+            tc_fence_after_sync();
+            const uint32_t keep = i > 0 ? 1u : 0u;
+            const uint32_t a = tmem + (KIND == DQ ? Cols<KIND>::DS : Cols<KIND>::P + 64u * m);
+#pragma unroll
+            for (int kk = 0; kk < T / 16; ++kk)
+              mma_ts_elect(tmem + C_ACC + 64u * m, a + 8u * kk, (KIND == DQ ? dX : dY) + (uint64_t)(128 * kk), ID_ACC, kk > 0 ? 1u : keep);
+            if (KIND == DKV) {
+#pragma unroll
+              for (int kk = 0; kk < T / 16; ++kk)
+                mma_ts_elect(tmem + C_ACC1, tmem + Cols<KIND>::DS + 8u * kk, dX + (uint64_t)(128 * kk), ID_ACC, kk > 0 ? 1u : keep);
+            }
+            mma_commit_elect(&bars[B_SFREE + m]);
+            if (KIND != FWD || m == 1 || i >= it.n1) mma_commit_elect(&bars[B_EMPTY + s]);
+            if (i == nm - 1) mma_commit_elect(&bars[B_ACC + m]);
+          }
+        }
+        ++tile;
+      }
+      idx = next_item(n);
+    }
+    if (*abort_flag != 0) {
+      mma_commit_elect(&bars[B_DRAIN + 1]);
+      mbar_wait_bounded(&bars[B_DRAIN + 1], 0, WAIT_CYCLES);
+    }
+  } else if (w >= W_EW) {
+    // ================= element-wise warps =================
+    const int we = w - W_EW, quarter = w & 3;
+    const int grp = KIND == FWD ? we >> 2 : 0;    // FWD: held tile
+    const int half = KIND == FWD ? 0 : we >> 2;   // else: 64-column half of the tile
+    constexpr int W = KIND == FWD ? 128 : 64;     // columns of a warp
+    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+    const uint64_t C0 = pack2(P.c0, P.c0), C1 = pack2(P.c1, P.c1), C2 = pack2(P.c2, P.c2), C22 = pack2(2.f * P.c2, 2.f * P.c2),
+                   K = pack2(P.k, P.k);   // what a mode does not use is not computed
+    // which rows this warp writes out: FWD O' of its tile, DKV dv (half 0) and dk (half 1), DQ dq (half 0)
+    const bool writes = KIND != DQ || half == 0;
+    uint64_t sum[4] = {0ull, 0ull, 0ull, 0ull};   // FWD: four chains, one would serialise the additions
+    uint64_t ND = 0ull;                           // DQ: -delta of this row
+    uint32_t k = 0;          // tiles of this warp's group so far
+    uint32_t done = 0;       // items whose results this warp has written
+    // Results of an item are written after the next item's first tile, whose products run meanwhile.
+    auto results = [&](int n, const Item& it, float total) {
+      const int row = it.r0 + grp * R + quarter * 32 + lane;
+      WAIT(B_ACC + grp, done, 75);
+      ++done;
+      if (!writes) return;
+      tc_fence_after_sync();
+      constexpr int CH = D < 32 ? D : 32;
+      uint32_t r[D / CH][CH];
+#pragma unroll
+      for (int c = 0; c < D / CH; ++c) tmem_ld<CH>(lane_addr + (KIND == FWD ? 64u * grp : 64u * half) + (uint32_t)(CH * c), r[c]);
+      tmem_ld_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[B_AFREE + grp]);
+      const bool second = KIND == DKV && half == 0;   // dv
+      float wgt = second ? P.w1 : P.w0;
+      if (KIND == FWD) {
+        wgt = 1.f / total;   // the sum and the products carry the same factor
+        if (row < P.nr)
+          reinterpret_cast<float*>(const_cast<void*>(P.out1.ptr))[(long long)it.b * P.out1.sb + (long long)it.h * P.out1.sh + (long long)row * P.out1.sn] = total * P.w1;
+      }
+      if (second ? P.vec1 : P.vec0) {
+        // rows -> the item's held set (its products are done), 128-byte swizzle -> the copy engine, which writes whole lines
+        // and clips what lies outside; stored by the threads, 32 lines per instruction, this took 1200 to 3000 clocks
+        uint8_t* stage = sm + OFF_HELD + (n & 1) * STAGE + (KIND == FWD ? grp : half) * X_BYTES + quarter * 4096;
+#pragma unroll
+        for (int c = 0; c < D / 8; ++c) {
+          const uint32_t(&x)[CH] = r[8 * c / CH];
+          const int o = 8 * c % CH;
+          uint4 v;
+          v.x = bf16x2(__uint_as_float(x[o]) * wgt, __uint_as_float(x[o + 1]) * wgt);
+          v.y = bf16x2(__uint_as_float(x[o + 2]) * wgt, __uint_as_float(x[o + 3]) * wgt);
+          v.z = bf16x2(__uint_as_float(x[o + 4]) * wgt, __uint_as_float(x[o + 5]) * wgt);
+          v.w = bf16x2(__uint_as_float(x[o + 6]) * wgt, __uint_as_float(x[o + 7]) * wgt);
+          *reinterpret_cast<uint4*>(stage + lane * 128 + ((c ^ (lane & 7)) << 4)) = v;
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && row < P.nr) {
+          tma_store_4d(second ? &M.o1 : &M.o0, stage, 0, row, it.h, it.b);
+          bulk_commit_group();
+        }
+      } else if (row < P.nr) {
+        const View& out = second ? P.out1 : P.out0;
+        __nv_bfloat16* p = reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(out.ptr)) + (long long)it.b * out.sb + (long long)it.h * out.sh + (long long)row * out.sn;
+#pragma unroll
+        for (int c = 0; c < D; ++c) p[c] = __float2bfloat16(__uint_as_float(r[c / CH][c % CH]) * wgt);
+      }
+    };
+    // the held set of item n has been read by the copy engine
+    auto give_back = [&](int n) {
+      if (lane == 0) {
+        bulk_wait_read_all();
+        mbar_arrive(&bars[B_HEMPTY + (n & 1)]);
+      }
+    };
+    bool pend = false;   // the last item's results are still to be written
+    Item last{};
+    int idx = blockIdx.x, n = 0;
+    for (; idx >= 0; ++n) {
+      const Item it = decode<KIND>(idx, P);
+      const int nt = (KIND == FWD && grp) ? it.n1 : it.n0;
+      const int row = it.r0 + grp * R + quarter * 32 + lane;
+      float total = 0.f;
+      if (KIND == FWD) {
+        float a, b;
+        unpack2(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])), a, b);
+        total = a + b;
+        sum[0] = sum[1] = sum[2] = sum[3] = 0ull;
+      }
+      if (KIND == DQ) {
+        const float nd = row < P.nr ? __ldg(P.ndelta + (long long)it.head * P.nd_ld + row) : 0.f;
+        ND = pack2(nd, nd);
+      }
+      for (int i = 0; i < nt; ++i) {
+        const int buf = KIND == FWD ? grp : KIND == DQ ? (int)(k & 1u) : 0;
+        WAIT(B_S + buf, KIND == DQ ? k >> 1 : k, 74);
+        if (KIND == DKV) WAIT(B_FULL + (int)(k & (STAGES - 1)), k / STAGES, 81);
+        tc_fence_after_sync();
+        const int x0 = (it.t0 + i) * T + half * W;   // streamed row of this warp's first column
+        // columns [lo, hi) of this row are visible
+        int lo = 0, hi = W;
+        if (KIND == DKV) {
+          if (P.causal) lo = row - P.off - x0;
+        } else {
+          if (P.causal) hi = row + P.off - x0 + 1;
+          if (KIND == FWD && P.nx - x0 < hi) hi = P.nx - x0;   // rows past the last key would count f(0) in the sum
+        }
+        const bool whole = __all_sync(0xffffffffu, lo <= 0 && hi >= W);
+        const uint32_t sa = lane_addr + C_S + (uint32_t)(buf * 128 + W * half);
+        if (KIND == FWD) {
+          uint32_t s[4][32];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tmem_ld32(sa + 32u * c, s[c]);
+          tmem_ld_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars[B_READS + grp]);
+          if (k > 0) WAIT(B_SFREE + grp, k - 1u, 83);   // the last tile's second product has read P
+          tc_fence_after_sync();
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t pr[16];
+            if (whole) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const uint64_t x = pack2u(s[c][2 * j], s[c][2 * j + 1]);
+                const uint64_t p = SQ ? fma2(x, x, K) : fma2(fma2(C2, x, C1), x, C0);
+                sum[j & 3] = add2(sum[j & 3], p);
+                pr[j] = bf16x2(p);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const uint64_t x = pack2u(s[c][2 * j], s[c][2 * j + 1]);
+                float p0, p1;
+                unpack2(SQ ? fma2(x, x, K) : fma2(fma2(C2, x, C1), x, C0), p0, p1);
+                if (32 * c + 2 * j >= hi) p0 = 0.f;
+                if (32 * c + 2 * j + 1 >= hi) p1 = 0.f;
+                sum[j & 3] = add2(sum[j & 3], pack2(p0, p1));
+                pr[j] = bf16x2(p0, p1);
+              }
+            }
+            tmem_st16(lane_addr + Cols<KIND>::P + 64u * grp + 16u * c, pr);
+          }
+        } else {
+          uint32_t d[2][32], s[2][32], pr[2][16], dr[2][16];
+          tmem_ld32(lane_addr + Cols<KIND>::DP + 64u * half, d[0]);
+          tmem_ld32(lane_addr + Cols<KIND>::DP + 64u * half + 32u, d[1]);
+          tmem_ld32(sa, s[0]);
+          tmem_ld32(sa + 32u, s[1]);
+          tmem_ld_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(&bars[B_READS + buf]);
+            mbar_arrive(&bars[B_READD]);
+          }
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const ulonglong2* ndp = reinterpret_cast<const ulonglong2*>(sm + OFF_ND + (k & (STAGES - 1)) * T * 4 + half * 256 + c * 128);
+#pragma unroll
+            for (int j2 = 0; j2 < 8; ++j2) {
+              ulonglong2 n2;
+              n2.x = n2.y = ND;
+              if (KIND == DKV) n2 = ndp[j2];
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const int j = 2 * j2 + e;
+                const uint64_t x = pack2u(s[c][2 * j], s[c][2 * j + 1]);
+                const uint64_t dp = add2(pack2u(d[c][2 * j], d[c][2 * j + 1]), e ? n2.y : n2.x);
+                if (KIND == DQ || SQ) {
+                  const uint64_t u = SQ ? x : fma2(C22, x, C1);
+                  dr[c][j] = bf16x2(mul2(u, dp));
+                  if (KIND == DKV) pr[c][j] = bf16x2(fma2(u, u, K));
+                } else {
+                  const uint64_t t = fma2(C2, x, C1);
+                  pr[c][j] = bf16x2(fma2(t, x, C0));
+                  dr[c][j] = bf16x2(mul2(fma2(C2, x, t), dp));
+                }
+              }
+            }
+          }
+          if (!whole) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const uint32_t keep = ((2 * j >= lo && 2 * j < hi) ? 0x0000ffffu : 0u) | ((2 * j + 1 >= lo && 2 * j + 1 < hi) ? 0xffff0000u : 0u);
+              dr[j >> 4][j & 15] &= keep;
+              if (KIND == DKV) pr[j >> 4][j & 15] &= keep;
+            }
+          }
+          if (k > 0) WAIT(B_SFREE, k - 1u, 83);   // the last tile's second products have read theirs
+          tc_fence_after_sync();
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            if (KIND == DKV) tmem_st16(lane_addr + Cols<KIND>::P + 32u * half + 16u * c, pr[c]);
+            tmem_st16(lane_addr + Cols<KIND>::DS + 32u * half + 16u * c, dr[c]);
+          }
+        }
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[B_P + grp]);
+        ++k;
+        if (i == 0 && pend) results(n - 1, last, total);
+        if (i == 1 && pend) give_back(n - 1);
+      }
+      if (nt == 0) {   // FWD, second tile absent: the last item's results now, nothing to stage for this one
+        if (pend) {
+          results(n - 1, last, total);
+          give_back(n - 1);
+        }
+        WAIT(B_HFULL + (n & 1), (uint32_t)(n >> 1), 84);   // (not before the set's last phase is over)
+        if (lane == 0) mbar_arrive(&bars[B_HEMPTY + (n & 1)]);
+      } else if (nt == 1 && pend) {
+        give_back(n - 1);
+      }
+      pend = nt > 0;
+      last = it;
+      idx = next_item(n);
+    }
+    if (pend) {
+      float a, b;
+      unpack2(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])), a, b);
+      results(n - 1, last, a + b);
+    }
+    if (lane == 0) bulk_wait_read_all();   // before the block's shared memory goes
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag != 0) {   // a wait ran out: copies in flight still land in this block's shared memory
+    if (w == W_LOAD) {
+      for (int i = issued > STAGES ? issued - STAGES : 0; i < issued; ++i)
+        mbar_wait_bounded(&bars[B_FULL + (i & (STAGES - 1))], (uint32_t)(i / STAGES) & 1u, WAIT_CYCLES);
+      for (int i = helds > 2 ? helds - 2 : 0; i < helds; ++i) mbar_wait_bounded(&bars[B_HFULL + (i & 1)], (uint32_t)(i >> 1) & 1u, WAIT_CYCLES);
+      for (int i = asked > CLC ? asked - CLC : 0; i < asked; ++i)
+        mbar_wait_bounded(&bars[B_CFULL + (i & (CLC - 1))], (uint32_t)(i / CLC) & 1u, WAIT_CYCLES);
+    }
+    __syncthreads();
+  }
+  if (w == W_ACC) tmem_dealloc(tmem, 512);
+}
+
+// dO' = dO / g in bf16 (dense [batch*heads][nq][D]) and -delta = -(dO . o) / g (zero from nq on).  D / 8 threads per row,
+// 16-byte accesses (VEC) or element by element for views that do not allow them.
+template <int D, bool VEC>
+__global__ void __launch_bounds__(256) prologue_kernel(View dout, View o, View g, __nv_bfloat16* __restrict__ dop, float* __restrict__ ndelta,
+                                                       int nq, int nd_ld, int heads) {
+  constexpr int TPR = D / 8;
+  const int head = blockIdx.y, b = head / heads, h = head - b * heads;
+  const int row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, c = (threadIdx.x % TPR) * 8;
+  float dv[8], dot = 0.f;
+  float inv = 0.f;
+  if (row < nq) {
+    const __nv_bfloat16* pd = reinterpret_cast<const __nv_bfloat16*>(dout.ptr) + (long long)b * dout.sb + (long long)h * dout.sh + (long long)row * dout.sn + c;
+    const __nv_bfloat16* po = reinterpret_cast<const __nv_bfloat16*>(o.ptr) + (long long)b * o.sb + (long long)h * o.sh + (long long)row * o.sn + c;
+    inv = 1.f / reinterpret_cast<const float*>(g.ptr)[(long long)b * g.sb + (long long)h * g.sh + (long long)row * g.sn];
+    __nv_bfloat16 xd[8], xo[8];
+    if (VEC) {
+      *reinterpret_cast<uint4*>(xd) = *reinterpret_cast<const uint4*>(pd);
+      *reinterpret_cast<uint4*>(xo) = *reinterpret_cast<const uint4*>(po);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { xd[i] = pd[i]; xo[i] = po[i]; }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      dv[i] = __bfloat162float(xd[i]) * inv;
+      dot += dv[i] * __bfloat162float(xo[i]);
+    }
+  }
+#pragma unroll
+  for (int m = TPR / 2; m > 0; m >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, m);
+  if (row < nq) {
+    uint4 r;
+    r.x = bf16x2(dv[0], dv[1]); r.y = bf16x2(dv[2], dv[3]); r.z = bf16x2(dv[4], dv[5]); r.w = bf16x2(dv[6], dv[7]);
+    *reinterpret_cast<uint4*>(dop + ((long long)head * nq + row) * D + c) = r;
+  }
+  if (c == 0 && row < nd_ld) ndelta[(long long)head * nd_ld + row] = row < nq ? -dot : 0.f;
+}
+
+}  // namespace pair
+
+// ------------------------------------------------------------------------------------------------------
+// host side
+// ------------------------------------------------------------------------------------------------------
+namespace {
+
+// n / d = (n * mul) >> shift for every n < 2^31
+void quotient(int d, uint32_t& mul, int& shift) {
+  int log = 0;
+  while ((1ll << log) < d) ++log;
+  shift = 31 + log;
+  mul = (uint32_t)(((1ull << shift) + d - 1) / d);
+}
+
+template <int D, int KIND, bool SQ>
+cudaError_t launch(const pair::Maps& M, const pair::Params& P, int bh, cudaStream_t st) {
+  auto kernel = pair::pair_kernel<D, KIND, SQ>;
+  static std::atomic<bool> done[64];   // the attribute sticks to the kernel on its device
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64 || !done[dev].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+  }
+  kernel<<<dim3((unsigned)(P.ntiles * bh)), pair::THREADS, pair::SMEM_BYTES, st>>>(M, P);
+  return cudaGetLastError();
+}
+template <int KIND, bool SQ>
+cudaError_t launch_d(int d, const pair::Maps& M, pair::Params& P, int bh, cudaStream_t st) {
+  quotient(P.ntiles, P.mul_t, P.sh_t);
+  quotient(P.heads, P.mul_h, P.sh_h);
+  switch (d) {
+    case 16: return launch<16, KIND, SQ>(M, P, bh, st);
+    case 32: return launch<32, KIND, SQ>(M, P, bh, st);
+    default: return launch<64, KIND, SQ>(M, P, bh, st);
+  }
+}
+
+View view_of(const fastmax_tensor& t) { return View{t.ptr, t.stride_b, t.stride_h, t.stride_n}; }
+bool rows16(const fastmax_tensor& t) {   // every row of a bf16 view starts on a 16-byte boundary
+  return ((uintptr_t)t.ptr & 15) == 0 && (t.stride_b & 7) == 0 && (t.stride_h & 7) == 0 && (t.stride_n & 7) == 0;
+}
+int tiles(int n, int rows = pair::R) { return (n + rows - 1) / rows; }
+int nd_ld(int n) { return (n + pair::T - 1) / pair::T * pair::T; }
+size_t up256(size_t x) { return (x + 255) / 256 * 256; }
+
+// a view the copy engine can read (a stride of a size-1 dimension is never used)
+bool mappable(const fastmax_tensor& t, const fastmax_problem* pb, int n) {
+  const int64_t big = (int64_t)1 << 39;
+  auto ok = [&](int64_t s, int extent) { return extent == 1 || (s > 0 && s < big && (s & 7) == 0); };
+  return t.ptr && ((uintptr_t)t.ptr & 15) == 0 && ok(t.stride_n, n) && ok(t.stride_h, pb->heads) && ok(t.stride_b, pb->batch);
+}
+
+// The pairwise kernels cost pairs x ~2.1e-7 us forward and ~7e-7 us backward (d = 64; narrower heads are bound by the
+// element-wise warps and cost the same), the moment scans tokens x ~1.2e-3 and ~4e-3 us at order 2: equal where a query sees
+// about 6000 keys.  At order 1 the scans run over one feature tile of nineteen: 5e-4 and 1.1e-3 us per token, equal at 2000
+// and 1300; without a mask and with at least 64 heads the order-1 forward is one pass over the tensors and always cheaper.
+// Measured crossings (causal, B x H x N, bf16): order 2 d = 64 32 heads 12000 tokens 1.30x / 1.08x for the pairs, 16 heads
+// 16384 tokens 0.85x / 0.88x; order 1 128 heads 2048 tokens 1.33x / 1.10x, 4096 tokens 0.96x / 0.67x.
+bool chosen(const fastmax_problem* pb, bool backward) {
+  if (!(pb->flags & FASTMAX_FLAG_PAIRWISE) || (pb->flags & FASTMAX_FLAG_NO_TENSOR_CORES)) return false;
+  if (pb->dtype != FASTMAX_BF16 || pb->nq <= 0 || pb->nk <= 0) return false;
+  if ((long long)tiles(pb->nq > pb->nk ? pb->nq : pb->nk) * pb->batch * pb->heads >= (1ll << 31)) return false;
+  const double nq = pb->nq, nk = pb->nk;
+  const double pairs = pb->causal ? nq * (nk - 0.5 * (nq - 1.0)) : nq * nk;
+  const double per_token = pairs / (0.5 * (nq + nk));
+  if (pb->order == 2) return per_token <= 6500.0;
+  if (!backward && !pb->causal && pb->d == 64 && (long long)pb->batch * pb->heads >= 64) return false;
+  return per_token <= (backward ? 1300.0 : 2000.0);
+}
+uint32_t bf16_bits(float x) {
+  const __nv_bfloat16 v = __float2bfloat16(x);
+  return *reinterpret_cast<const uint16_t*>(&v);
+}
+// Returns whether the kernels run with the square completed (SQ): order 2 with 64 a0 a2 >= a1^2, i.e. h^2 at most sixteen
+// times c0 / c2, so that u^2 + k keeps its accuracy (the reference's coefficients: h^2 half of c0 / c2).
+bool fill(const fastmax_problem* pb, pair::Params& P) {
+  P.heads = pb->heads;
+  P.causal = pb->causal;
+  P.off = pb->causal ? pb->nk - pb->nq : 0;
+  P.c0 = pb->a0;
+  P.c1 = pb->a1 * pb->inv_temperature;
+  P.c2 = pb->order == 2 ? pb->a2 * pb->inv_temperature * pb->inv_temperature : 0.f;
+  P.w0 = P.w1 = 1.f;
+  if (pb->order != 2 || !(fabsf(P.c2) >= 1e-30f) || !(64.0 * pb->a0 * pb->a2 >= (double)pb->a1 * pb->a1)) return false;
+  const double h = (double)P.c1 / (2.0 * P.c2);
+  if (!(fabs(h) < 1e15)) return false;
+  double rest = h, sum = 0.0;
+  uint32_t piece[3];
+  for (int i = 0; i < 3; ++i) {
+    piece[i] = bf16_bits((float)rest);
+    const uint32_t bits = piece[i] << 16;
+    float back;
+    memcpy(&back, &bits, 4);
+    sum += back;
+    rest -= back;
+  }
+  P.h01 = piece[0] | piece[1] << 16;
+  P.h2 = piece[2];
+  P.k = (float)((double)P.c0 / P.c2 - sum * sum);
+  return true;
+}
+
+}  // namespace
+
+bool pair_takes_forward(const fastmax_problem* pb, const fastmax_forward_args* a) {
+  return chosen(pb, false) && a->o.ptr && a->g.ptr && !a->state_in && !a->state_out && mappable(a->q, pb, pb->nq) &&
+         mappable(a->k, pb, pb->nk) && mappable(a->v, pb, pb->nk);
+}
+bool pair_takes_backward(const fastmax_problem* pb, const fastmax_backward_args* a) {
+  return chosen(pb, true) && a->dq.ptr && a->dk.ptr && a->dv.ptr && !a->state_in && !a->dstate_in && !a->dstate_out &&
+         mappable(a->q, pb, pb->nq) && mappable(a->k, pb, pb->nk) && mappable(a->v, pb, pb->nk);
+}
+
+size_t pair_backward_workspace(const fastmax_problem* pb) {
+  const size_t bh = (size_t)pb->batch * pb->heads;
+  return up256(bh * pb->nq * pb->d * 2) + up256(bh * nd_ld(pb->nq) * sizeof(float));
+}
+
+// 32-row boxes of an output view, one per warp; views the copy engine cannot write are stored element by element
+static int out_map(CUtensorMap* m, const fastmax_tensor& t, const fastmax_problem* pb, int n) {
+  return rows16(t) && tc_make_map(m, t, pb->batch, pb->heads, n, 64, 32, true, pb->d) ? 1 : 0;
+}
+
+int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, cudaStream_t st) {
+  pair::Maps M;
+  if (!tc_make_map(&M.a, a->q, pb->batch, pb->heads, pb->nq, 64, pair::R, true, pb->d) ||
+      !tc_make_map(&M.x, a->k, pb->batch, pb->heads, pb->nk, 64, pair::T, true, pb->d) ||
+      !tc_make_map(&M.y, a->v, pb->batch, pb->heads, pb->nk, 64, pair::T, true, pb->d))
+    return FASTMAX_ERR_UNSUPPORTED;
+  M.b = M.o0 = M.o1 = M.a;
+  pair::Params P{};
+  const bool sq = fill(pb, P);
+  P.out0 = view_of(a->o);
+  P.out1 = view_of(a->g);
+  P.nr = pb->nq;
+  P.nx = pb->nk;
+  P.ntiles = tiles(pb->nq, 2 * pair::R);
+  P.vec0 = out_map(&M.o0, a->o, pb, pb->nq);
+  if (sq) P.w1 = P.c2;
+  const int bh = pb->batch * pb->heads;
+  LaunchScope ls(KK_TC_FWD, st);
+  const cudaError_t e = sq ? launch_d<pair::FWD, true>(pb->d, M, P, bh, st) : launch_d<pair::FWD, false>(pb->d, M, P, bh, st);
+  return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
+}
+
+template <int D>
+static void launch_prologue(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, cudaStream_t st) {
+  const int ld = nd_ld(pb->nq), rows = 256 / (D / 8);
+  const dim3 grid((unsigned)((ld + rows - 1) / rows), (unsigned)(pb->batch * pb->heads));
+  if (rows16(a->o) && rows16(a->d_out))
+    pair::prologue_kernel<D, true><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads);
+  else
+    pair::prologue_kernel<D, false><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads);
+}
+
+int pair_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
+  const int bh = pb->batch * pb->heads;
+  __nv_bfloat16* dop = (__nv_bfloat16*)ws;
+  float* nd = (float*)((char*)ws + up256((size_t)bh * pb->nq * pb->d * 2));
+  const fastmax_tensor dopt{dop, (int64_t)bh * pb->nq * pb->d, (int64_t)pb->nq * pb->d, pb->d};   // one batch of bh heads
+  pair::Maps M;   // dq: held q, dO', streamed k, v
+  if (!tc_make_map(&M.x, a->k, pb->batch, pb->heads, pb->nk, 64, pair::T, true, pb->d) ||
+      !tc_make_map(&M.y, a->v, pb->batch, pb->heads, pb->nk, 64, pair::T, true, pb->d) ||
+      !tc_make_map(&M.a, a->q, pb->batch, pb->heads, pb->nq, 64, pair::R, true, pb->d) ||
+      !tc_make_map(&M.b, dopt, 1, bh, pb->nq, 64, pair::R, true, pb->d))
+    return FASTMAX_ERR_UNSUPPORTED;
+  M.o0 = M.o1 = M.a;
+  pair::Maps N;   // dk, dv: the other way round (held and streamed tiles have the same 128-row box)
+  N.x = M.a; N.y = M.b; N.a = M.x; N.b = M.y; N.o0 = N.o1 = M.a;
+  {
+    LaunchScope ls(KK_PROLOGUE, st, pb->d < 64 ? KK_TC_PAD : -1);
+    switch (pb->d) {
+      case 16: launch_prologue<16>(pb, a, dop, nd, st); break;
+      case 32: launch_prologue<32>(pb, a, dop, nd, st); break;
+      default: launch_prologue<64>(pb, a, dop, nd, st); break;
+    }
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return report_cuda_error(e);
+  pair::Params P{};
+  const bool sq = fill(pb, P);
+  P.ndelta = nd;
+  P.nd_ld = nd_ld(pb->nq);
+  pair::Params K = P;
+  K.out0 = view_of(a->dk);
+  K.out1 = view_of(a->dv);
+  K.nr = pb->nk;
+  K.nx = pb->nq;
+  K.ntiles = tiles(pb->nk);
+  K.vec0 = out_map(&N.o0, a->dk, pb, pb->nk);
+  K.vec1 = out_map(&N.o1, a->dv, pb, pb->nk);
+  if (sq) { K.w0 = 2.f * K.c2; K.w1 = K.c2; }
+  {
+    LaunchScope ls(KK_TC_BWD_KV, st, KK_TC_BWD_DV);
+    e = sq ? launch_d<pair::DKV, true>(pb->d, N, K, bh, st) : launch_d<pair::DKV, false>(pb->d, N, K, bh, st);
+  }
+  if (e != cudaSuccess) return report_cuda_error(e);
+  P.out0 = P.out1 = view_of(a->dq);
+  P.nr = pb->nq;
+  P.nx = pb->nk;
+  P.ntiles = tiles(pb->nq);
+  P.vec0 = out_map(&M.o0, a->dq, pb, pb->nq);
+  if (sq) P.w0 = 2.f * P.c2;
+  {
+    LaunchScope ls(KK_TC_BWD_Q, st);
+    e = sq ? launch_d<pair::DQ, true>(pb->d, M, P, bh, st) : launch_d<pair::DQ, false>(pb->d, M, P, bh, st);
+  }
+  return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
+}
+
+int pair_status(int* out) {
+  cudaError_t e = cudaMemcpyFromSymbol(out, pair::g_status, sizeof(int), 0, cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return report_cuda_error(e);
+  if (*out != 0) {
+    const int zero = 0;
+    cudaMemcpyToSymbol(pair::g_status, &zero, sizeof(int), 0, cudaMemcpyHostToDevice);
+  }
+  return FASTMAX_OK;
+}
+int pair_wait_histogram(int* out, int n) {   // adds to out
+  int h[256];
+  cudaError_t e = cudaMemcpyFromSymbol(h, pair::g_wait_hist, sizeof(h), 0, cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return report_cuda_error(e);
+  for (int i = 0; i < n && i < 256; ++i) out[i] += h[i];
+  static const int zeros[256] = {0};
+  cudaMemcpyToSymbol(pair::g_wait_hist, zeros, sizeof(zeros), 0, cudaMemcpyHostToDevice);
+  return FASTMAX_OK;
+}
+
+}  // namespace fm

@@ -20,6 +20,7 @@
 
 #include "common.cuh"
 #include "launchers.cuh"
+#include "pair_launchers.cuh"
 #include "tc_launchers.cuh"
 #include "tc_ptx.cuh"
 
@@ -325,16 +326,18 @@ static EncodeTiledFn encode_fn() {
 }
 
 // bf16 (batch, head, token, cols) view -> 4-D tensor map with a [box_rows x box_cols] box.
-static bool make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int heads, int n, int box_cols, int box_rows,
-                     bool swizzle128, int cols = 64) {
+bool tc_make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int heads, int n, int box_cols, int box_rows,
+                     bool swizzle128, int cols) {
   EncodeTiledFn fn = encode_fn();
   if (!fn || n <= 0) return false;
   const cuuint64_t dims[4] = {(cuuint64_t)cols, (cuuint64_t)n, (cuuint64_t)heads, (cuuint64_t)batch};
-  // a stride of a size-1 dimension is never used for addressing; any legal value will do
+  // a stride of a size-1 dimension is never used for addressing; any legal value will do.  A zero stride of a longer one
+  // (a tensor expanded over tokens, heads or the batch) is left to the CUDA-core engine.
   cuuint64_t sn = (cuuint64_t)t.stride_n * 2, sh = (cuuint64_t)t.stride_h * 2, sbb = (cuuint64_t)t.stride_b * 2;
-  if (n == 1 || sn == 0) sn = 128;
-  if (heads == 1 || sh == 0) sh = sn * (cuuint64_t)n;
-  if (batch == 1 || sbb == 0) sbb = 128;
+  if ((n > 1 && sn == 0) || (heads > 1 && sh == 0) || (batch > 1 && sbb == 0)) return false;
+  if (n == 1) sn = 128;
+  if (heads == 1) sh = sn * (cuuint64_t)n;
+  if (batch == 1) sbb = 128;
   const cuuint64_t strides[3] = {sn, sh, sbb};
   for (int i = 0; i < 3; ++i)
     if (strides[i] % 16 || strides[i] >= (1ull << 40)) return false;
@@ -344,6 +347,11 @@ static bool make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int hea
                   swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
+}
+
+static bool make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int heads, int n, int box_cols, int box_rows,
+                     bool swizzle128, int cols = 64) {
+  return tc_make_map(m, t, batch, heads, n, box_cols, box_rows, swizzle128, cols);
 }
 
 // Transposed bf16 copy xt [batch*heads][64][ntp] -> 3-D tensor map (tokens, 64 dims, batch*heads), box 72 x 64, no swizzle.
@@ -1322,10 +1330,10 @@ int tc_wait_histogram(int* out, int n) {
   int h[256];
   cudaError_t e = cudaMemcpyFromSymbol(h, g_tc_wait_hist, sizeof(h), 0, cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return report_cuda_error(e);
-  for (int i = 0; i < n && i < 256; ++i) out[i] = h[i];
+  for (int i = 0; i < n; ++i) out[i] = i < 256 ? h[i] : 0;
   static const int zeros[256] = {0};
   cudaMemcpyToSymbol(g_tc_wait_hist, zeros, sizeof(zeros), 0, cudaMemcpyHostToDevice);
-  return FASTMAX_OK;
+  return pair_wait_histogram(out, n);
 }
 
 int tc_device_status(int* out) {
@@ -1337,6 +1345,10 @@ int tc_device_status(int* out) {
     int zero = 0;
     cudaMemcpyToSymbol(g_tc_status, &zero, sizeof(int), 0, cudaMemcpyHostToDevice);
   }
+  int p = 0;
+  const int rc = pair_status(&p);
+  if (rc != FASTMAX_OK) return rc;
+  if (v == 0) *out = p;
   return FASTMAX_OK;
 }
 

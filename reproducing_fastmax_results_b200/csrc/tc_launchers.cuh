@@ -1,6 +1,7 @@
 // Entry points of the tcgen05 / TMA kernels.  Each returns FASTMAX_TC_NOT_HANDLED when the problem is
 // outside what the tensor-core kernels cover, and the caller then runs the CUDA-core engine.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 
@@ -25,6 +26,11 @@ int tc_device_status(int* out);
 int tc_wait_histogram(int* out, int n);
 // Launches the test-only kernel that lets a bounded wait of `cycles` SM clocks run out and records wait site `code`.
 int tc_wait_selftest(long long cycles, int code, cudaStream_t st);
+
+// bf16 (batch, head, token, cols) view -> 4-D tensor map with a [box_rows x box_cols] box (columns past `cols` read as
+// zero); false when the copy engine cannot describe the view
+bool tc_make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int heads, int n, int box_cols, int box_rows, bool swizzle128,
+                 int cols);
 
 // shared with the C-ABI translation unit
 int report_cuda_error(cudaError_t e);  // remembers e for fastmax_last_cuda_error(), returns FASTMAX_ERR_CUDA

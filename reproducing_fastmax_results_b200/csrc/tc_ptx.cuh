@@ -101,6 +101,12 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tensor_m
       : "memory");
 }
 
+// Untiled bulk copy global -> shared of `bytes` (both 16-byte aligned, bytes a multiple of 16), counted on an mbarrier.
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
 // Bulk asynchronous reduce-add of `bytes` of float32 from shared memory into global memory (both 16-byte aligned,
 // bytes a multiple of 16), executed by the copy engine; tracked with bulk async-groups of the issuing thread.
 __device__ __forceinline__ void bulk_reduce_add_f32(float* gdst, const void* smem_src, uint32_t bytes) {

@@ -68,9 +68,10 @@ class HostFastmax:
                 ready = torch.cuda.Event()
                 ready.record(self._s_in)
             cur.wait_event(ready)
-            o, g, _ = _lib.forward(dq_[sl], dk_[sl], dv_[sl], self.mask, self.inv_temperature, self.a0, self.a1, self.a2, self.p)
+            o, g, _ = _lib.forward(dq_[sl], dk_[sl], dv_[sl], self.mask, self.inv_temperature, self.a0, self.a1, self.a2, self.p,
+                                    flags=_lib.FLAG_PAIRWISE)
             gq, gk, gv, _ = _lib.backward(dq_[sl], dk_[sl], dv_[sl], o, g, ddo[sl], self.mask, self.inv_temperature, self.a0,
-                                          self.a1, self.a2, self.p)
+                                          self.a1, self.a2, self.p, flags=_lib.FLAG_PAIRWISE)
             done = torch.cuda.Event()
             done.record(cur)
             keep.append((o, g, gq, gk, gv))

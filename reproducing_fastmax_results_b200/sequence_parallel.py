@@ -102,9 +102,9 @@ class CudaEngine:
         if cast:
             q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
         if moments is None:
-            o, g, _ = self.ext.forward(q, k, v, True, it, a0, a1, a2, p, state_in, False, True, 0)
+            o, g, _ = self.ext.forward(q, k, v, True, it, a0, a1, a2, p, state_in, False, True, self.ext.PAIRWISE)
             return (o.float() if cast else o), g
-        res = self.ext.forward(q, k, v, True, it, a0, a1, a2, p, state_in, False, True, 0, None, moments.buf, True)
+        res = self.ext.forward(q, k, v, True, it, a0, a1, a2, p, state_in, False, True, self.ext.PAIRWISE, None, moments.buf, True)
         moments.buf = res[3]
         return (res[0].float() if cast else res[0]), res[1]
 
@@ -125,7 +125,7 @@ class CudaEngine:
         if cast:
             q, k, v, o, do = q.bfloat16(), k.bfloat16(), v.bfloat16(), o.bfloat16(), do.bfloat16()
         km, gm = (None, None) if moments is None else (moments.buf, moments.grad_buf)
-        grads = self.ext.backward(q, k, v, o, g, do, True, it, a0, a1, a2, p, state_in, dstate_in, False, True, 0,
+        grads = self.ext.backward(q, k, v, o, g, do, True, it, a0, a1, a2, p, state_in, dstate_in, False, True, self.ext.PAIRWISE,
                                   None, km, gm, False)[:3]
         return tuple(t.float() for t in grads) if cast else tuple(grads)
 

@@ -1,0 +1,94 @@
+"""The pairwise tcgen05 kernels (FASTMAX_FLAG_PAIRWISE) against the CPU oracle at the sizes where they can go wrong: one row,
+the edges of the 128-row tiles and of the 256-row forward items, one item per block and many, an absent second tile, keys
+without queries, both forms of the polynomial (square completed or not), outputs the copy engine cannot write."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import fastmax_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def host(t):
+    return t.detach().float().cpu().numpy().astype(np.float64)
+
+
+CASES = [  # B, H, nq, nk, D, causal, order
+    (1, 2, 1, 1, 64, False, 2),
+    (1, 2, 2, 5, 16, True, 2),
+    (2, 2, 127, 127, 32, True, 2),
+    (1, 2, 128, 128, 64, True, 2),
+    (1, 2, 129, 129, 64, True, 1),
+    (1, 2, 256, 257, 64, True, 2),
+    (1, 2, 257, 129, 64, False, 2),
+    (1, 3, 385, 640, 32, True, 2),
+    (1, 2, 640, 64, 16, False, 1),
+    (4, 40, 200, 200, 64, True, 2),    # more items than SMs, second tile ragged
+    (10, 40, 100, 100, 32, False, 2),  # items of one tile, several per block
+    (2, 2, 1100, 1100, 64, True, 2),
+]
+
+
+@pytest.mark.parametrize("poly", [(1.0, 1.0, 0.5), (0.3, 1.7, 0.1)])   # square completed; general form
+@pytest.mark.parametrize("case", CASES)
+def test_pairwise_kernels_match_oracle(case, poly):
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    B, H, nq, nk, D, causal, order = case
+    g = torch.Generator(device="cuda").manual_seed(nq + nk + D)
+    # head-split views of (b, n, h*d) buffers
+    mk = lambda n: torch.randn(B, n, H, D, device="cuda", generator=g).bfloat16().transpose(1, 2)
+    q, do, k, v = mk(nq), mk(nq), mk(nk), mk(nk)
+    p = orc.Poly(*poly, 1.0 / (3.0 * math.sqrt(D)), order)
+    args = (causal, p.inv_temp, p.a0, p.a1, p.a2, order)
+    o, gg, _ = L.forward(q, k, v, *args, flags=L.FLAG_PAIRWISE)
+    dq, dk, dv, _ = L.backward(q, k, v, o, gg, do, *args, flags=L.FLAG_PAIRWISE)
+    L.check_status()
+    assert L.wait_histogram() == {}
+    for b, h in {(0, 0), (B - 1, H - 1)}:
+        a = [host(t[b, h]) for t in (q, k, v, do)]
+        o_ref, g_ref = orc.fastmax_naive(a[0], a[1], a[2], causal, p)
+        refs = (o_ref, g_ref) + tuple(orc.fastmax_naive_grads(a[0], a[1], a[2], a[3], causal, p))
+        for name, x, r, tol in zip(("o", "g", "dq", "dk", "dv"), (o, gg, dq, dk, dv), refs, (2e-2, 1e-5, 2e-2, 2e-2, 2e-2)):
+            if np.abs(r).max() > 1e-9:   # dq and dk of a single visible key are analytically zero
+                assert orc.max_norm_err(host(x[b, h]), r) < tol, (name, b, h)
+
+
+def test_pairwise_outputs_in_rows_the_copy_engine_cannot_write():
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    B, H, N, D = 1, 3, 300, 64
+    g = torch.Generator(device="cuda").manual_seed(4)
+    q, k, v, do = (torch.randn(B, H, N, D, device="cuda", generator=g).bfloat16() for _ in range(4))
+    odd = lambda: torch.zeros(B, H, N, D + 1, device="cuda", dtype=torch.bfloat16)
+    bufs = [odd() for _ in range(4)]
+    views = [t[..., :D] for t in bufs]
+    o, gg, _ = L.forward(q, k, v, True, 0.05, order=2, flags=L.FLAG_PAIRWISE)
+    grads = L.backward(q, k, v, o, gg, do, True, 0.05, order=2, flags=L.FLAG_PAIRWISE)[:3]
+    o2, g2, _ = L.forward(q, k, v, True, 0.05, order=2, flags=L.FLAG_PAIRWISE, out=views[0])
+    grads2 = L.backward(q, k, v, o, gg, do, True, 0.05, order=2, flags=L.FLAG_PAIRWISE, grads_out=tuple(views[1:]))[:3]
+    L.check_status()
+    assert torch.equal(gg, g2)
+    for a, b in zip((o,) + tuple(grads), (o2,) + tuple(grads2)):
+        assert torch.equal(a, b)
+    assert all(float(t[..., D].abs().max()) == 0.0 for t in bufs)   # the column beside the rows is untouched
+
+
+def test_pairwise_form_is_left_to_the_moment_engines_where_it_does_not_apply():
+    """Carried states, and tensors expanded with a zero stride, run as without the flag."""
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    B, H, N, D = 1, 16, 256, 64
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (torch.randn(B, H, N, D, device="cuda", generator=g).bfloat16() for _ in range(3))
+    o, _, state = L.forward(q, k, v, True, 0.05, order=2, want_state=True, flags=L.FLAG_PAIRWISE)
+    o_ref, _, state_ref = L.forward(q, k, v, True, 0.05, order=2, want_state=True)
+    shared = k[:, :1].expand(B, H, N, D)   # one key head for all query heads
+    oe, ge, _ = L.forward(q, shared, v, True, 0.05, order=2, flags=L.FLAG_PAIRWISE)
+    oc, gc, _ = L.forward(q, shared.contiguous(), v, True, 0.05, order=2, flags=L.FLAG_PAIRWISE)
+    L.check_status()
+    for a, b, tol in ((o, o_ref, 2e-3), (state, state_ref, 1e-5), (oe, oc, 1e-2), (ge, gc, 1e-3)):
+        assert orc.max_norm_err(host(a), host(b)) < tol
