@@ -444,7 +444,7 @@ static int fwd_layout(const fastmax_problem* pb, const fastmax_forward_args* a, 
 size_t fastmax_forward_workspace(const fastmax_problem* pb, const fastmax_forward_args* args) {
   Plan pl;
   if (!args || make_plan(pb, pl) != FASTMAX_OK) return 0;
-  if (pair_takes_forward(pb, args)) return 0;
+  if (pair_takes_forward(pb, args)) return pair_forward_workspace(pb) + 256;
   FwdLayout L;
   fwd_layout(pb, args, pl, L);
   size_t tc = tc_forward_workspace(pb, args);
@@ -491,7 +491,7 @@ int32_t fastmax_forward(const fastmax_problem* pb, const fastmax_forward_args* a
   if (ws_bytes < fastmax_forward_workspace(pb, a) || (ws_bytes && (!ws || ((uintptr_t)ws % 256))))
     return FASTMAX_ERR_WORKSPACE;
 
-  if (want_o && pair_takes_forward(pb, a)) return pair_forward(pb, a, st);
+  if (want_o && pair_takes_forward(pb, a)) return pair_forward(pb, a, ws, st);
   int tcrc = tc_forward(pb, a, ws, ws_bytes, st);
   if (tcrc != FASTMAX_TC_NOT_HANDLED) return tcrc;
 

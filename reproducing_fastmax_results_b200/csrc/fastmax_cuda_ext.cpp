@@ -99,6 +99,7 @@ torch::Tensor forwardpass(torch::Tensor q, torch::Tensor k, torch::Tensor v, tor
   fastmax_problem pb{};
   pb.batch = 1; pb.heads = bh; pb.nq = nq; pb.nk = nk; pb.d = d; pb.order = p; pb.causal = mask ? 1 : 0;
   pb.dtype = FASTMAX_F32; pb.a0 = a0; pb.a1 = a1; pb.a2 = a2; pb.inv_temperature = 1.0f;
+  pb.flags = FASTMAX_FLAG_PAIRWISE;
   fastmax_forward_args a{};
   a.q = view_nbd(q); a.k = view_nbd(k); a.v = view_nbd(v);
   a.o = fastmax_tensor{o.data_ptr(), 0, o.stride(1), o.stride(0)};
@@ -110,6 +111,7 @@ torch::Tensor forwardpass(torch::Tensor q, torch::Tensor k, torch::Tensor v, tor
     auto ob = torch::empty({nq, bh, d}, qb.options());
     fastmax_problem pbb = pb;
     pbb.dtype = FASTMAX_BF16;
+    pbb.flags = 0;   // the question is which moment engine the call would go to
     fastmax_forward_args ab = a;
     ab.q = view_nbd(qb); ab.k = view_nbd(kb); ab.v = view_nbd(vb); ab.o = view_nbd(ob);
     if (fastmax_forward_engine(&pbb, &ab) == 1) {
@@ -142,6 +144,7 @@ std::vector<torch::Tensor> backwardpass(torch::Tensor q, torch::Tensor k, torch:
   fastmax_problem pb{};
   pb.batch = 1; pb.heads = bh; pb.nq = nq; pb.nk = nk; pb.d = d; pb.order = p; pb.causal = mask ? 1 : 0;
   pb.dtype = FASTMAX_F32; pb.a0 = a0; pb.a1 = a1; pb.a2 = a2; pb.inv_temperature = 1.0f;
+  pb.flags = FASTMAX_FLAG_PAIRWISE;
   fastmax_backward_args a{};
   a.q = view_nbd(q); a.k = view_nbd(k); a.v = view_nbd(v);
   a.o = fastmax_tensor{o.data_ptr(), 0, o.stride(1), o.stride(0)};
@@ -153,6 +156,7 @@ std::vector<torch::Tensor> backwardpass(torch::Tensor q, torch::Tensor k, torch:
     auto ob = o.narrow(2, 0, d).to(torch::kBFloat16), gb = grad_output.to(torch::kBFloat16);   // contiguous (nq, bh, d) copies
     fastmax_problem pbb = pb;
     pbb.dtype = FASTMAX_BF16;
+    pbb.flags = 0;   // the question is which moment engine the call would go to
     fastmax_forward_args fb{};   // which engine the bfloat16 form of the forward call goes to decides for the pair
     fb.q = view_nbd(qb); fb.k = view_nbd(kb); fb.v = view_nbd(vb); fb.o = view_nbd(ob); fb.g = a.g;
     if (fastmax_forward_engine(&pbb, &fb) == 1) {

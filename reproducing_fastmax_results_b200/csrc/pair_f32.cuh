@@ -1,0 +1,515 @@
+// Pairwise kernels for float32 tensors.  Included by pair_kernels.cu inside fm::pair.
+//
+// Every float32 operand is the exact sum of three bf16 numbers (8 + 8 + 8 bits), so a product is the sum of the six piece
+// products that reach 2^-24 of the largest: hi hi, hi mid, mid hi, mid mid, hi lo, lo hi.  q, k, v and dO' are split once, by
+// a pass over memory; P and dS are split in registers.  Six bf16 products run at 1/6 of the bf16 rate, still four times the
+// FFMA pipe's.
+//
+// The tensor pipe adds into its float32 accumulator with truncation: 1e-7 of the value per addition when the terms have one
+// sign (measured: 3e-7 after 16 additions, 8e-5 after 1024).  So a chain is kept short: the second products start from zero
+// for every streamed tile (64 rows: four additions of hi hi behind the twenty small ones, which go first) and the
+// element-wise warps add the tile's result to float32 totals in registers, rounding to nearest.
+//
+// Roles and hand-offs are those of the bf16 kernels; the streamed pair's two tiles have barriers of their own, because with
+// three pieces each only two or three stages fit and each tile can be let go at a different time.
+#pragma once
+
+namespace f32 {
+
+constexpr int TF = 64;                       // streamed rows per tile
+constexpr int XF = TF * 128;                 // one piece of a streamed tile
+constexpr int AF = R * 128;                  // one piece of a held tile
+template <int KIND>
+struct Lay {
+  static constexpr int STAGES = KIND == FWD ? 3 : 2;
+  static constexpr int HELD = (KIND == FWD ? 3 : 6) * AF;
+  static constexpr int STAGE = 6 * XF;       // X pieces, then Y pieces
+  static constexpr int OFF_X = HELD;
+  static constexpr int OFF_OUT = OFF_X + STAGES * STAGE;   // 4 KB of output staging per element-wise warp
+  static constexpr int OFF_ND = OFF_OUT + EW * 4096;       // DKV: -delta of the streamed queries per stage; FWD: row sums of the halves
+  static constexpr int OFF_CLC = OFF_ND + 1024;
+  static constexpr int OFF_BAR = OFF_CLC + 16 * CLC;
+  static constexpr int BYTES = OFF_BAR + 512 + 1024;
+};
+static_assert(Lay<FWD>::BYTES <= 232448 && Lay<DKV>::BYTES <= 232448, "shared memory budget");
+constexpr int B_FX = 0, B_FY = 3, B_EX = 6, B_EY = 9, B_HFULL = 12, B_HEMPTY = 13, B_S = 14, B_READ = 15, B_P = 16, B_ACC = 17, B_AFREE = 18,
+              B_CFULL = 19, B_CEMPTY = B_CFULL + CLC, B_DRAIN = B_CEMPTY + CLC, B_COUNT = B_DRAIN + 2;
+// TMEM columns: accumulators (dv, dk / dq / O'), scores, dP, pieces of P and of dS (32 columns each)
+constexpr uint32_t C_ACC = 0, C_ACC1 = 64, C_S = 128, C_DP = 192, C_P = 256, C_DS = 352;
+// dk / dv: a warpgroup of its own adds up the accumulators (128 totals per thread: beside a tile they do not fit into the
+// element-wise warps' registers; spilled, the kernel took four times as long).  Registers are moved between the warpgroups.
+constexpr int W_SUM = W_EW + EW;
+template <int KIND>
+constexpr int THREADS_F = KIND == DKV ? (W_SUM + 4) * 32 : THREADS;
+constexpr int REG_LAUNCH = 128, REG_REST = 48, REG_EW = 136, REG_SUM = 192;
+static_assert(REG_REST * W_EW + REG_EW * EW + REG_SUM * 4 <= REG_LAUNCH * (W_SUM + 4), "setmaxnreg.inc waits for registers the block does not have");
+
+// two float32 numbers -> their three bf16 pieces
+__device__ __forceinline__ void split3(uint64_t x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const uint64_t minus = 0xBF800000BF800000ull;
+  hi = bf16x2(x);
+  const uint64_t r = fma2(pack2u(hi << 16, hi & 0xffff0000u), minus, x);   // exact
+  mid = bf16x2(r);
+  lo = bf16x2(fma2(pack2u(mid << 16, mid & 0xffff0000u), minus, r));
+}
+
+// waits without an out-of-line call (ptxas cannot allocate a callee under mixed register allowances)
+__device__ __forceinline__ void wait_inline(uint64_t* bar, uint32_t parity, int code, volatile int* abort_flag) {
+  if (mbar_try_wait(bar, parity)) return;
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (*abort_flag != 0) return;
+    if (clock64() - t0 > WAIT_CYCLES) {
+      if (*abort_flag == 0) atomicAdd(&g_wait_hist[code & 255], 1);
+      *abort_flag = 1;
+      atomicExch(&g_status, code);
+      return;
+    }
+  }
+}
+
+template <int D, int KIND>
+__global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __grid_constant__ Maps M, const Params P) {
+  using L = Lay<KIND>;
+  constexpr int KS = D / 16, STAGES = L::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = smem_u32(smem_raw);
+  uint8_t* sm = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + L::OFF_BAR);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + L::OFF_BAR + 384);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + L::OFF_BAR + 392);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int w = __shfl_sync(0xffffffffu, tid >> 5, 0);
+
+  if (tid == 0) {
+    for (int i = 0; i < B_COUNT; ++i) {
+      uint32_t n = 1;
+      if (i == B_READ || i == B_P) n = EW;
+      if (i == B_AFREE) n = KIND == DKV ? 4 : EW;
+      if (i >= B_CEMPTY && i < B_CEMPTY + CLC) n = KIND == DKV ? ROLES + 4 : ROLES;
+      mbar_init(&bars[i], n);
+    }
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (w == W_ACC) tmem_alloc(tmem_slot, 512);
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  auto WAIT = [&](int bar, uint32_t phase, int code) { wait_inline(&bars[bar], phase & 1u, code, abort_flag); };
+  auto next_item = [&](int n) -> int {
+    const int c = n & (CLC - 1);
+    WAIT(B_CFULL + c, (uint32_t)(n / CLC), 76);
+    int idx = *abort_flag != 0 ? -1 : clc_read(sm + L::OFF_CLC + 16 * c);
+    fence_proxy_async_smem();
+    idx = __shfl_sync(0xffffffffu, idx, 0);
+    if (lane == 0) mbar_arrive(&bars[B_CEMPTY + c]);
+    return idx;
+  };
+  // DKV: the role branches move registers (inside each branch: past a join of branches ptxas assumes the smaller allowance)
+#define FM_REG_DEC() if (KIND == DKV) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REG_REST))
+#define FM_REG_INC(n_) if (KIND == DKV) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(n_))
+  int issued_x = 0, issued_y = 0, helds = 0, asked = 0;   // what the loader has asked for
+  if (w == W_LOAD) {
+    FM_REG_DEC();
+    // ================= loader and item scheduler =================
+    // tile i of the item: the three pieces of one operand
+    auto load_tile = [&](const Item& it, int i, bool y) {
+      int& issued = y ? issued_y : issued_x;
+      const int s = issued % STAGES;
+      if (issued >= STAGES) WAIT((y ? B_EY : B_EX) + s, (uint32_t)(issued / STAGES) - 1u, y ? 71 : 70);
+      if (*abort_flag != 0) return;
+      if (lane == 0) {
+        uint8_t* x = sm + L::OFF_X + s * L::STAGE + (y ? 3 * XF : 0);
+        uint64_t* bar = &bars[(y ? B_FY : B_FX) + s];
+        const int row = (it.t0 + i) * TF;
+        const bool nd = KIND == DKV && y;
+        mbar_arrive_expect_tx(bar, 3 * XF + (nd ? TF * 4 : 0));
+#pragma unroll
+        for (int p = 0; p < 3; ++p) tma_load_4d(x + p * XF, y ? &M.y : &M.x, bar, 0, row, it.head, p);
+        if (nd) bulk_load(sm + L::OFF_ND + s * TF * 4, P.ndelta + (long long)it.head * P.nd_ld + row, TF * 4, bar);
+      }
+      ++issued;
+    };
+    int idx = blockIdx.x;
+    for (int n = 0; idx >= 0; ++n) {
+      const int c = n & (CLC - 1);
+      if (n >= CLC) WAIT(B_CEMPTY + c, (uint32_t)(n / CLC) - 1u, 77);
+      if (*abort_flag != 0) break;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&bars[B_CFULL + c], 16);
+        clc_try_cancel(sm + L::OFF_CLC + 16 * c, &bars[B_CFULL + c]);
+      }
+      asked = n + 1;
+      const Item it = decode<KIND, TF, R>(idx, P);
+      if (n >= 1) WAIT(B_HEMPTY, (uint32_t)n - 1u, 78);
+      if (*abort_flag != 0) break;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&bars[B_HFULL], L::HELD);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          tma_load_4d(sm + p * AF, &M.a, &bars[B_HFULL], 0, it.r0, it.head, p);
+          if (KIND != FWD) tma_load_4d(sm + (3 + p) * AF, &M.b, &bars[B_HFULL], 0, it.r0, it.head, p);
+        }
+      }
+      helds = n + 1;
+      for (int i = 0; i < it.n0 && *abort_flag == 0; ++i) {   // in the order in which the tiles are used
+        load_tile(it, i, KIND == DQ);
+        load_tile(it, i, KIND != DQ);
+      }
+      idx = next_item(n);
+    }
+  } else if (w == W_SCORE) {
+    FM_REG_DEC();
+    // ================= issuer of the first products =================
+    constexpr uint32_t ID_S = make_idesc_bf16(R, TF, 0, 0);
+    const uint64_t dH = make_smem_desc(smem_u32(sm), 16, 1024, 2);
+    const uint64_t dX0 = make_smem_desc(smem_u32(sm + L::OFF_X), 16, 1024, 2);
+    // sum over the piece products, the smallest first
+    auto product = [&](uint32_t acc, uint64_t a, uint64_t b) {
+#pragma unroll
+      for (int t = 0; t < 6; ++t) {
+        constexpr int PA[6] = {0, 2, 1, 0, 1, 0}, PB[6] = {2, 0, 1, 1, 0, 0};
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+          mma_ss_elect(acc, a + (uint64_t)(PA[t] * (AF >> 4) + 2 * ks), b + (uint64_t)(PB[t] * (XF >> 4) + 2 * ks), ID_S, t > 0 || ks > 0);
+      }
+    };
+    uint32_t k = 0;
+    int idx = blockIdx.x;
+    for (int n = 0; idx >= 0; ++n) {
+      const Item it = decode<KIND, TF, R>(idx, P);
+      WAIT(B_HFULL, (uint32_t)n, 72);
+      for (int i = 0; i < it.n0; ++i) {
+        const uint32_t s = k % STAGES;
+        const uint64_t dX = dX0 + (uint64_t)(s * (L::STAGE >> 4)), dY = dX + (uint64_t)(3 * XF >> 4);
+        if (k > 0) WAIT(B_READ, k - 1u, 80);   // the last tile's scores and dP have been read
+        if (KIND == DQ) {   // v is needed here only: it can go before k, which the second product reads too
+          WAIT(B_FY + (int)s, k / STAGES, 74);
+          tc_fence_after_sync();
+          product(tmem + C_DP, dH + (uint64_t)(3 * AF >> 4), dY);
+          mma_commit_elect(&bars[B_EY + s]);
+        }
+        WAIT(B_FX + (int)s, k / STAGES, 73);
+        tc_fence_after_sync();
+        product(tmem + C_S, dH, dX);
+        if (KIND == FWD) mma_commit_elect(&bars[B_EX + s]);
+        if (KIND == DKV) {
+          WAIT(B_FY + (int)s, k / STAGES, 74);
+          tc_fence_after_sync();
+          product(tmem + C_DP, dH + (uint64_t)(3 * AF >> 4), dY);
+        }
+        mma_commit_elect(&bars[B_S]);
+        ++k;
+      }
+      mma_commit_elect(&bars[B_HEMPTY]);
+      idx = next_item(n);
+    }
+    if (*abort_flag != 0) {
+      mma_commit_elect(&bars[B_DRAIN]);
+      mbar_wait_bounded(&bars[B_DRAIN], 0, WAIT_CYCLES);
+    }
+  } else if (w == W_ACC) {
+    FM_REG_DEC();
+    // ================= issuer of the second products =================
+    constexpr uint32_t ID_ACC = make_idesc_bf16(R, D, 0, 1);
+    const uint64_t dX0 = make_smem_desc(smem_u32(sm + L::OFF_X), XF, 1024, 2);
+    auto product = [&](uint32_t acc, uint32_t a, uint64_t b) {
+#pragma unroll
+      for (int t = 0; t < 6; ++t) {
+        constexpr int PA[6] = {0, 2, 1, 0, 1, 0}, PB[6] = {2, 0, 1, 1, 0, 0};
+#pragma unroll
+        for (int kk = 0; kk < TF / 16; ++kk)
+          mma_ts_elect(acc, a + 32u * PA[t] + 8u * kk, b + (uint64_t)(PB[t] * (XF >> 4) + 128 * kk), ID_ACC, t > 0 || kk > 0);
+      }
+    };
+    uint32_t k = 0;
+    int idx = blockIdx.x;
+    for (int n = 0; idx >= 0; ++n) {
+      const Item it = decode<KIND, TF, R>(idx, P);
+      for (int i = 0; i < it.n0; ++i) {
+        const uint32_t s = k % STAGES;
+        const uint64_t dX = dX0 + (uint64_t)(s * (L::STAGE >> 4)), dY = dX + (uint64_t)(3 * XF >> 4);
+        if (KIND == FWD) WAIT(B_FY + (int)s, k / STAGES, 75);
+        WAIT(B_P, k, 79);
+        if (k > 0) WAIT(B_AFREE, k - 1u, 82);   // the last tile's results are in the totals
+        tc_fence_after_sync();
+        if (KIND != FWD) {
+          product(tmem + (KIND == DKV ? C_ACC1 : C_ACC), tmem + C_DS, dX);
+          mma_commit_elect(&bars[B_EX + s]);
+        }
+        if (KIND != DQ) {
+          product(tmem + C_ACC, tmem + C_P, dY);
+          mma_commit_elect(&bars[B_EY + s]);
+        }
+        mma_commit_elect(&bars[B_ACC]);
+        ++k;
+      }
+      idx = next_item(n);
+    }
+    if (*abort_flag != 0) {
+      mma_commit_elect(&bars[B_DRAIN + 1]);
+      mbar_wait_bounded(&bars[B_DRAIN + 1], 0, WAIT_CYCLES);
+    }
+  } else if (w < W_EW) {   // spare
+    FM_REG_DEC();
+  } else {
+    // ================= element-wise warps: TMEM lane quarter x 32-column half of the tile; DKV: + the warps that add up =================
+    const int quarter = w & 3, half = (w - W_EW) >> 2;   // half == 2: adding up (DKV)
+    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+    // Totals of this warp: half a row of dq or O'; dv and dk (two rows of D) in the warps that add up
+    constexpr int NA = KIND == DKV ? 2 * D : D / 2;
+    constexpr int CH = KIND == DKV ? (D < 32 ? D : 32) : (NA < 32 ? NA : 32);
+    auto clear = [&](uint64_t (&tot)[NA / 2]) {
+#pragma unroll
+      for (int j = 0; j < NA / 2; ++j) tot[j] = 0ull;
+    };
+    auto drain = [&](uint64_t (&tot)[NA / 2], uint32_t tile) {   // adds the results of a tile's second products
+      WAIT(B_ACC, tile, 83);
+      tc_fence_after_sync();
+#pragma unroll
+      for (int c = 0; c < NA / CH; ++c) {
+        uint32_t r[CH];
+        // DKV: chunks of dv, then of dk
+        tmem_ld<CH>(lane_addr + (KIND == DKV ? (uint32_t)(64 * (c * CH / D) + c * CH % D) : (uint32_t)(half * NA + CH * c)), r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < CH / 2; ++j) tot[c * (CH / 2) + j] = add2(tot[c * (CH / 2) + j], pack2u(r[2 * j], r[2 * j + 1]));
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars[B_AFREE]);
+    };
+    // rows -> shared memory (column xor row: no bank conflicts either way) -> one row per store instruction, any strides
+    auto write_rows = [&](const Item& it, const uint64_t (&tot)[NA / 2], float wgt) {
+      float* stage = reinterpret_cast<float*>(sm + L::OFF_OUT + (KIND == DKV ? quarter : w - W_EW) * 4096);
+#pragma unroll
+      for (int c = 0; c < NA / CH; ++c) {
+        const View& out = KIND == DKV && c * CH < D ? P.out1 : P.out0;
+        float* base = reinterpret_cast<float*>(const_cast<void*>(out.ptr)) + (long long)it.b * out.sb + (long long)it.h * out.sh +
+                      (KIND == DKV ? c * CH % D : half * NA + CH * c);
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < CH / 2; ++j) {
+          float a, b;
+          unpack2(tot[c * (CH / 2) + j], a, b);
+          stage[lane * 32 + ((2 * j) ^ lane)] = a * wgt;
+          stage[lane * 32 + ((2 * j + 1) ^ lane)] = b * wgt;
+        }
+        __syncwarp();
+        constexpr int RP = 32 / CH;   // rows per instruction
+        const int rr = lane / CH, cc = lane % CH;
+#pragma unroll 4
+        for (int r = 0; r < 32; r += RP) {
+          const int g = it.r0 + quarter * 32 + r + rr;
+          const float v = stage[(r + rr) * 32 + (cc ^ (r + rr))];
+          if (g < P.nr) base[(long long)g * out.sn + cc] = v;
+        }
+      }
+    };
+    uint32_t k = 0;
+    int idx = blockIdx.x;
+    if (KIND == DKV && w >= W_SUM) {
+      FM_REG_INC(REG_SUM);
+      for (int n = 0; idx >= 0; ++n) {
+        const Item it = decode<KIND, TF, R>(idx, P);
+        uint64_t tot[NA / 2];
+        clear(tot);
+        for (int i = 0; i < it.n0; ++i) drain(tot, k++);
+        write_rows(it, tot, 1.f);
+        idx = next_item(n);
+      }
+    } else {
+      FM_REG_INC(REG_EW);
+      const uint64_t C0 = pack2(P.c0, P.c0), C1 = pack2(P.c1, P.c1), C2 = pack2(P.c2, P.c2);
+      for (int n = 0; idx >= 0; ++n) {
+        const Item it = decode<KIND, TF, R>(idx, P);
+        const int row = it.r0 + quarter * 32 + lane;
+        uint64_t ND = 0ull;
+        if (KIND == DQ) {
+          const float nd = row < P.nr ? __ldg(P.ndelta + (long long)it.head * P.nd_ld + row) : 0.f;
+          ND = pack2(nd, nd);
+        }
+        uint64_t tot[NA / 2];
+        if (KIND != DKV) clear(tot);
+        float total = 0.f;
+        for (int i = 0; i < it.n0; ++i) {
+          WAIT(B_S, k, 84);
+          const int s_ = (int)(k % STAGES);
+          if (KIND == DKV) WAIT(B_FY + s_, k / STAGES, 81);
+          tc_fence_after_sync();
+          const int x0 = (it.t0 + i) * TF + half * 32;
+          int lo = 0, hi = 32;
+          if (KIND == DKV) {
+            if (P.causal) lo = row - P.off - x0;
+          } else {
+            if (P.causal) hi = row + P.off - x0 + 1;
+            if (KIND == FWD && P.nx - x0 < hi) hi = P.nx - x0;
+          }
+          const bool whole = __all_sync(0xffffffffu, lo <= 0 && hi >= 32);
+          uint32_t s[32], d[32];
+          tmem_ld32(lane_addr + C_S + 32u * half, s);
+          if (KIND != FWD) tmem_ld32(lane_addr + C_DP + 32u * half, d);
+          tmem_ld_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars[B_READ]);
+          // the last tile's second products are done: P and dS may be overwritten, and their results are added up
+          if (KIND == DKV) {
+            if (k > 0) WAIT(B_ACC, k - 1u, 85);
+            tc_fence_after_sync();
+          } else if (i > 0) {
+            drain(tot, k - 1u);
+          }
+          const ulonglong2* ndp = reinterpret_cast<const ulonglong2*>(sm + L::OFF_ND + s_ * TF * 4 + half * 128);
+          uint64_t sum = 0ull;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t pp[3][4], dd[3][4];
+#pragma unroll
+            for (int j2 = 0; j2 < 2; ++j2) {
+              ulonglong2 n2;
+              n2.x = n2.y = ND;
+              if (KIND == DKV) n2 = ndp[2 * c + j2];
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const int j = 2 * j2 + e, col = 8 * c + 2 * j;
+                const bool v0 = whole || (col >= lo && col < hi), v1 = whole || (col + 1 >= lo && col + 1 < hi);
+                const uint64_t x = pack2u(s[col], s[col + 1]);
+                const uint64_t t = fma2(C2, x, C1);
+                if (KIND != DQ) {
+                  uint64_t p = fma2(t, x, C0);
+                  if (!whole) {
+                    float a, b;
+                    unpack2(p, a, b);
+                    p = pack2(v0 ? a : 0.f, v1 ? b : 0.f);
+                  }
+                  if (KIND == FWD) sum = add2(sum, p);
+                  split3(p, pp[0][j], pp[1][j], pp[2][j]);
+                }
+                if (KIND != FWD) {
+                  uint64_t ds = mul2(fma2(C2, x, t), add2(pack2u(d[col], d[col + 1]), e ? n2.y : n2.x));
+                  if (!whole) {
+                    float a, b;
+                    unpack2(ds, a, b);
+                    ds = pack2(v0 ? a : 0.f, v1 ? b : 0.f);
+                  }
+                  split3(ds, dd[0][j], dd[1][j], dd[2][j]);
+                }
+              }
+            }
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+              if (KIND != DQ) tmem_st4(lane_addr + C_P + 32u * p + 16u * half + 4u * c, pp[p]);
+              if (KIND != FWD) tmem_st4(lane_addr + C_DS + 32u * p + 16u * half + 4u * c, dd[p]);
+            }
+          }
+          tmem_st_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars[B_P]);
+          if (KIND == FWD) {
+            float a, b;
+            unpack2(sum, a, b);
+            total += a + b;
+          }
+          ++k;
+        }
+        if (KIND != DKV) {
+          drain(tot, k - 1u);
+          float wgt = 1.f;
+          if (KIND == FWD) {   // the two halves' row sums
+            float* sums = reinterpret_cast<float*>(sm + L::OFF_ND);
+            sums[half * R + quarter * 32 + lane] = total;
+            named_bar_sync(1 + quarter, 64);
+            const float g = sums[quarter * 32 + lane] + sums[R + quarter * 32 + lane];
+            named_bar_sync(1 + quarter, 64);
+            wgt = 1.f / g;
+            if (half == 0 && row < P.nr)
+              reinterpret_cast<float*>(const_cast<void*>(P.out1.ptr))[(long long)it.b * P.out1.sb + (long long)it.h * P.out1.sh + (long long)row * P.out1.sn] = g;
+          }
+          write_rows(it, tot, wgt);
+        }
+        idx = next_item(n);
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag != 0) {
+    if (w == W_LOAD) {
+      for (int i = issued_x > STAGES ? issued_x - STAGES : 0; i < issued_x; ++i)
+        mbar_wait_bounded(&bars[B_FX + i % STAGES], (uint32_t)(i / STAGES) & 1u, WAIT_CYCLES);
+      for (int i = issued_y > STAGES ? issued_y - STAGES : 0; i < issued_y; ++i)
+        mbar_wait_bounded(&bars[B_FY + i % STAGES], (uint32_t)(i / STAGES) & 1u, WAIT_CYCLES);
+      if (helds > 0) mbar_wait_bounded(&bars[B_HFULL], (uint32_t)(helds - 1) & 1u, WAIT_CYCLES);
+      for (int i = asked > CLC ? asked - CLC : 0; i < asked; ++i)
+        mbar_wait_bounded(&bars[B_CFULL + (i & (CLC - 1))], (uint32_t)(i / CLC) & 1u, WAIT_CYCLES);
+    }
+    __syncthreads();
+  }
+  if (w == W_ACC) tmem_dealloc(tmem, 512);
+}
+
+// Splits float32 views into bf16 pieces: out[piece][batch*heads][n][D].  A thread takes eight columns; blockIdx.z picks the tensor.
+struct SplitArgs {
+  View x[3];
+  __nv_bfloat16* out[3];
+  int n[3];
+};
+__device__ __forceinline__ void store_pieces(__nv_bfloat16* out, long long plane, long long at, const float (&v)[8]) {
+  uint32_t r[3][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) split3(pack2(v[2 * i], v[2 * i + 1]), r[0][i], r[1][i], r[2][i]);
+#pragma unroll
+  for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(out + p * plane + at) = make_uint4(r[p][0], r[p][1], r[p][2], r[p][3]);
+}
+template <int D>
+__global__ void __launch_bounds__(256) split_kernel(const SplitArgs A, int heads) {
+  constexpr int TPR = D / 8;
+  const int t = blockIdx.z, head = blockIdx.y, b = head / heads, h = head - b * heads;
+  const int row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, c = (threadIdx.x % TPR) * 8;
+  if (row >= A.n[t]) return;
+  const float4* p = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(A.x[t].ptr) + (long long)b * A.x[t].sb + (long long)h * A.x[t].sh +
+                                                    (long long)row * A.x[t].sn + c);
+  const float4 u = p[0], w = p[1];
+  const float v[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+  store_pieces(A.out[t], (long long)gridDim.y * A.n[t] * D, ((long long)head * A.n[t] + row) * D + c, v);
+}
+
+// dO' = dO / g in pieces and -delta = -(dO . o) / g
+template <int D, bool VEC>
+__global__ void __launch_bounds__(256) prologue_f32_kernel(View dout, View o, View g, __nv_bfloat16* __restrict__ dop, float* __restrict__ ndelta,
+                                                           int nq, int nd_ld, int heads) {
+  constexpr int TPR = D / 8;
+  const int head = blockIdx.y, b = head / heads, h = head - b * heads;
+  const int row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, c = (threadIdx.x % TPR) * 8;
+  float v[8], dot = 0.f;
+  if (row < nq) {
+    const float* pd = reinterpret_cast<const float*>(dout.ptr) + (long long)b * dout.sb + (long long)h * dout.sh + (long long)row * dout.sn + c;
+    const float* po = reinterpret_cast<const float*>(o.ptr) + (long long)b * o.sb + (long long)h * o.sh + (long long)row * o.sn + c;
+    const float inv = 1.f / reinterpret_cast<const float*>(g.ptr)[(long long)b * g.sb + (long long)h * g.sh + (long long)row * g.sn];
+    float x[8];
+    if (VEC) {
+      *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(pd);
+      *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(pd + 4);
+      *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(po);
+      *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(po + 4);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { v[i] = pd[i]; x[i] = po[i]; }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[i] *= inv;
+      dot += v[i] * x[i];
+    }
+  }
+#pragma unroll
+  for (int m = TPR / 2; m > 0; m >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, m);
+  if (row < nq) store_pieces(dop, (long long)gridDim.y * nq * D, ((long long)head * nq + row) * D + c, v);
+  if (c == 0 && row < nd_ld) ndelta[(long long)head * nd_ld + row] = row < nq ? -dot : 0.f;
+}
+
+}  // namespace f32

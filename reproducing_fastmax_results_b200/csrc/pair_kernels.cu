@@ -179,7 +179,8 @@ struct Item {
   int t0;          // first streamed tile
   int n0, n1;      // streamed tiles of the held tile(s); n1: the second tile of a forward item
 };
-template <int KIND>
+// TILE: streamed rows per tile, HELD: rows of an item
+template <int KIND, int TILE, int HELD>
 __device__ __forceinline__ Item decode(int idx, const Params& P) {
   // Head-major, the longest item of a head first: the blocks at work share a few heads' streamed tiles in L2, and the
   // last items are short.
@@ -190,24 +191,20 @@ __device__ __forceinline__ Item decode(int idx, const Params& P) {
   it.h = it.head - it.b * P.heads;
   it.t0 = 0;
   it.n1 = 0;
-  const int all = (P.nx + T - 1) / T;
+  const int all = (P.nx + TILE - 1) / TILE;
   if (KIND == DKV) {
-    it.r0 = ti * R;
+    it.r0 = ti * HELD;
     const int first = it.r0 - P.off;                 // first query that sees key r0
-    if (P.causal && first > 0) it.t0 = first / T;
+    if (P.causal && first > 0) it.t0 = first / TILE;
     it.n0 = all - it.t0;
   } else {
-    it.r0 = (P.ntiles - 1 - ti) * (KIND == FWD ? 2 * R : R);
-    it.n0 = P.causal ? min(all, (it.r0 + R - 1 + P.off) / T + 1) : all;
-    if (KIND == FWD && it.r0 + R < P.nr) it.n1 = P.causal ? min(all, (it.r0 + 2 * R - 1 + P.off) / T + 1) : all;
+    it.r0 = (P.ntiles - 1 - ti) * HELD;
+    it.n0 = P.causal ? min(all, (it.r0 + R - 1 + P.off) / TILE + 1) : all;
+    if (HELD > R && it.r0 + R < P.nr) it.n1 = P.causal ? min(all, (it.r0 + 2 * R - 1 + P.off) / TILE + 1) : all;
   }
   return it;
 }
 
-// SQ: the square completed.  f(s) / c2 = u^2 + k and f'(s) / (2 c2) = u with u = s + h, h = c1 / (2 c2): the first product
-// itself adds h (one more K = 16 step with constant operands, 65 clocks of the tensor pipe), so f costs one multiply-add
-// instead of two and f' nothing; the factors go into the epilogues.  The element-wise warps are bound by the FMA pipe (a
-// packed instruction takes 2.2 clocks per warp), which makes every instruction per element worth 140 clocks per tile.
 struct Maps {
   CUtensorMap x, y;     // streamed tiles
   CUtensorMap a, b;     // held tiles
@@ -217,6 +214,7 @@ struct Maps {
 template <int D, int KIND, bool SQ>
 __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant__ Maps M, const Params P) {
   constexpr int KS = D / 16;                    // K steps of the first products
+  constexpr int HELD_ROWS = KIND == FWD ? 2 * R : R;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* sm = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
@@ -276,7 +274,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
         clc_try_cancel(sm + OFF_CLC + 16 * c, &bars[B_CFULL + c]);
       }
       asked = n + 1;
-      const Item it = decode<KIND>(idx, P);
+      const Item it = decode<KIND, T, HELD_ROWS>(idx, P);
       const int tiles = it.n0 > it.n1 ? it.n0 : it.n1;
       if (n >= 2) WAIT(B_HEMPTY + (n & 1), (uint32_t)(n >> 1) - 1u, 78);
       if (*abort_flag != 0) break;
@@ -323,7 +321,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
     uint32_t tile = 0;            // streamed tiles so far
     int idx = blockIdx.x;
     for (int n = 0; idx >= 0; ++n) {
-      const Item it = decode<KIND>(idx, P);
+      const Item it = decode<KIND, T, HELD_ROWS>(idx, P);
       const int tiles = it.n0 > it.n1 ? it.n0 : it.n1;
       WAIT(B_HFULL + (n & 1), (uint32_t)(n >> 1), 71);
       const uint64_t dH = dHeld + (uint64_t)((n & 1) * (STAGE >> 4));
@@ -371,7 +369,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
     uint32_t nfree[2] = {0, 0};   // items that have started on each accumulator
     int idx = blockIdx.x;
     for (int n = 0; idx >= 0; ++n) {
-      const Item it = decode<KIND>(idx, P);
+      const Item it = decode<KIND, T, HELD_ROWS>(idx, P);
       const int tiles = it.n0 > it.n1 ? it.n0 : it.n1;
       for (int i = 0; i < tiles; ++i) {
         const uint32_t s = tile & (STAGES - 1);
@@ -485,7 +483,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
     Item last{};
     int idx = blockIdx.x, n = 0;
     for (; idx >= 0; ++n) {
-      const Item it = decode<KIND>(idx, P);
+      const Item it = decode<KIND, T, HELD_ROWS>(idx, P);
       const int nt = (KIND == FWD && grp) ? it.n1 : it.n0;
       const int row = it.r0 + grp * R + quarter * 32 + lane;
       float total = 0.f;
@@ -686,6 +684,8 @@ __global__ void __launch_bounds__(256) prologue_kernel(View dout, View o, View g
   if (c == 0 && row < nd_ld) ndelta[(long long)head * nd_ld + row] = row < nq ? -dot : 0.f;
 }
 
+#include "pair_f32.cuh"
+
 }  // namespace pair
 
 // ------------------------------------------------------------------------------------------------------
@@ -735,8 +735,12 @@ int tiles(int n, int rows = pair::R) { return (n + rows - 1) / rows; }
 int nd_ld(int n) { return (n + pair::T - 1) / pair::T * pair::T; }
 size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 
+}  // namespace
+bool f32_registers_ok();
+namespace {
 // a view the copy engine can read (a stride of a size-1 dimension is never used)
 bool mappable(const fastmax_tensor& t, const fastmax_problem* pb, int n) {
+  if (pb->dtype == FASTMAX_F32) return t.ptr != nullptr;   // split by ordinary loads
   const int64_t big = (int64_t)1 << 39;
   auto ok = [&](int64_t s, int extent) { return extent == 1 || (s > 0 && s < big && (s & 7) == 0); };
   return t.ptr && ((uintptr_t)t.ptr & 15) == 0 && ok(t.stride_n, n) && ok(t.stride_h, pb->heads) && ok(t.stride_b, pb->batch);
@@ -750,11 +754,21 @@ bool mappable(const fastmax_tensor& t, const fastmax_problem* pb, int n) {
 // 16384 tokens 0.85x / 0.88x; order 1 128 heads 2048 tokens 1.33x / 1.10x, 4096 tokens 0.96x / 0.67x.
 bool chosen(const fastmax_problem* pb, bool backward) {
   if (!(pb->flags & FASTMAX_FLAG_PAIRWISE) || (pb->flags & FASTMAX_FLAG_NO_TENSOR_CORES)) return false;
-  if (pb->dtype != FASTMAX_BF16 || pb->nq <= 0 || pb->nk <= 0) return false;
+  if (pb->nq <= 0 || pb->nk <= 0) return false;
   if ((long long)tiles(pb->nq > pb->nk ? pb->nq : pb->nk) * pb->batch * pb->heads >= (1ll << 31)) return false;
   const double nq = pb->nq, nk = pb->nk;
   const double pairs = pb->causal ? nq * (nk - 0.5 * (nq - 1.0)) : nq * nk;
   const double per_token = pairs / (0.5 * (nq + nk));
+  if (pb->dtype == FASTMAX_F32) {
+    // against the CUDA-core engine, whose cost per token goes with d^3 (order 2) or d^2, while six piece products on half-empty
+    // tiles hardly get cheaper for narrow heads.  Measured ratios near the line (x = pairs faster, forward / backward):
+    // order 2: d = 64 12000 keys 2.0 / 1.9, d = 32 4096 keys 1.2-1.45 / 1.3-1.4, d = 16 2048 keys 1.05 / 1.2;
+    // order 1, mask: d = 64 2048 keys 1.2 / 1.2, d = 32 1024 keys 1.0 / 1.2; no mask: d = 64 1024 keys 1.3 / 1.3.
+    const double most = pb->order == 2 ? (pb->d == 64 ? 16000.0 : pb->d == 32 ? 5000.0 : 2000.0)
+                        : pb->causal   ? (pb->d == 64 ? 2300.0 : pb->d == 32 ? 1050.0 : 900.0)
+                                       : (pb->d == 64 ? 1300.0 : pb->d == 32 ? 800.0 : 600.0);
+    return per_token <= most && f32_registers_ok();
+  }
   if (pb->order == 2) return per_token <= 6500.0;
   if (!backward && !pb->causal && pb->d == 64 && (long long)pb->batch * pb->heads >= 64) return false;
   return per_token <= (backward ? 1300.0 : 2000.0);
@@ -803,17 +817,168 @@ bool pair_takes_backward(const fastmax_problem* pb, const fastmax_backward_args*
          mappable(a->q, pb, pb->nq) && mappable(a->k, pb, pb->nk) && mappable(a->v, pb, pb->nk);
 }
 
+// ---- float32 ------------------------------------------------------------------------------------------------------------
+// bf16 pieces [3][batch*heads][n][d] as a tensor map: piece = batch index, head = batch*heads
+static size_t pieces_bytes(const fastmax_problem* pb, int n) { return up256((size_t)3 * pb->batch * pb->heads * n * pb->d * 2); }
+size_t pair_forward_workspace(const fastmax_problem* pb) {
+  return pb->dtype == FASTMAX_F32 ? pieces_bytes(pb, pb->nq) + 2 * pieces_bytes(pb, pb->nk) : 0;
+}
 size_t pair_backward_workspace(const fastmax_problem* pb) {
+  if (pb->dtype == FASTMAX_F32)
+    return 2 * pieces_bytes(pb, pb->nq) + 2 * pieces_bytes(pb, pb->nk) + up256((size_t)pb->batch * pb->heads * nd_ld(pb->nq) * sizeof(float));
   const size_t bh = (size_t)pb->batch * pb->heads;
   return up256(bh * pb->nq * pb->d * 2) + up256(bh * nd_ld(pb->nq) * sizeof(float));
 }
 
+static bool pieces_map(CUtensorMap* m, void* p, const fastmax_problem* pb, int n, int rows) {
+  const int64_t bh = (int64_t)pb->batch * pb->heads;
+  return tc_make_map(m, fastmax_tensor{p, bh * n * pb->d, (int64_t)n * pb->d, pb->d}, 3, (int)bh, n, 64, rows, true, pb->d);
+}
+static void launch_split(const fastmax_problem* pb, const pair::f32::SplitArgs& A, int count, cudaStream_t st) {
+  int n = A.n[0];
+  for (int i = 1; i < count; ++i) n = A.n[i] > n ? A.n[i] : n;
+  const int rows = 256 / (pb->d / 8);
+  const dim3 grid((unsigned)((n + rows - 1) / rows), (unsigned)(pb->batch * pb->heads), (unsigned)count);
+  LaunchScope ls(KK_CAST, st);
+  switch (pb->d) {
+    case 16: pair::f32::split_kernel<16><<<grid, 256, 0, st>>>(A, pb->heads); break;
+    case 32: pair::f32::split_kernel<32><<<grid, 256, 0, st>>>(A, pb->heads); break;
+    default: pair::f32::split_kernel<64><<<grid, 256, 0, st>>>(A, pb->heads); break;
+  }
+}
+template <int D, int KIND>
+static cudaError_t launch_f32(const pair::Maps& M, const pair::Params& P, int bh, cudaStream_t st) {
+  auto kernel = pair::f32::pair_f32_kernel<D, KIND>;
+  constexpr int bytes = pair::f32::Lay<KIND>::BYTES;
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64 || !done[dev].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+  }
+  kernel<<<dim3((unsigned)(P.ntiles * bh)), pair::f32::THREADS_F<KIND>, bytes, st>>>(M, P);
+  return cudaGetLastError();
+}
+template <int KIND>
+static cudaError_t launch_f32_d(int d, const pair::Maps& M, pair::Params& P, int bh, cudaStream_t st) {
+  quotient(P.ntiles, P.mul_t, P.sh_t);
+  quotient(P.heads, P.mul_h, P.sh_h);
+  switch (d) {
+    case 16: return launch_f32<16, KIND>(M, P, bh, st);
+    case 32: return launch_f32<32, KIND>(M, P, bh, st);
+    default: return launch_f32<64, KIND>(M, P, bh, st);
+  }
+}
+// dk / dv move registers between their warps (setmaxnreg), which only ends if the blocks are launched with what the budget
+// in pair_f32.cuh assumes
+bool f32_registers_ok() {
+  static const bool ok = [] {
+    cudaFuncAttributes a{}, b{}, c{};
+    return cudaFuncGetAttributes(&a, pair::f32::pair_f32_kernel<16, pair::DKV>) == cudaSuccess && a.numRegs == pair::f32::REG_LAUNCH &&
+           cudaFuncGetAttributes(&b, pair::f32::pair_f32_kernel<32, pair::DKV>) == cudaSuccess && b.numRegs == pair::f32::REG_LAUNCH &&
+           cudaFuncGetAttributes(&c, pair::f32::pair_f32_kernel<64, pair::DKV>) == cudaSuccess && c.numRegs == pair::f32::REG_LAUNCH;
+  }();
+  return ok;
+}
+
+static int pair_f32_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st) {
+  char* base = (char*)ws;
+  void *qp = base, *kp = base + pieces_bytes(pb, pb->nq), *vp = base + pieces_bytes(pb, pb->nq) + pieces_bytes(pb, pb->nk);
+  pair::Maps M;
+  if (!pieces_map(&M.a, qp, pb, pb->nq, pair::R) || !pieces_map(&M.x, kp, pb, pb->nk, pair::f32::TF) || !pieces_map(&M.y, vp, pb, pb->nk, pair::f32::TF))
+    return FASTMAX_ERR_UNSUPPORTED;
+  M.b = M.o0 = M.o1 = M.a;
+  launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
+                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {pb->nq, pb->nk, pb->nk}}, 3, st);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return report_cuda_error(e);
+  pair::Params P{};
+  fill(pb, P);
+  P.out0 = view_of(a->o);
+  P.out1 = view_of(a->g);
+  P.nr = pb->nq;
+  P.nx = pb->nk;
+  P.ntiles = tiles(pb->nq);
+  LaunchScope ls(KK_SCAN_FWD, st);
+  e = launch_f32_d<pair::FWD>(pb->d, M, P, pb->batch * pb->heads, st);
+  return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
+}
+
+template <int D>
+static void launch_prologue_f32(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, cudaStream_t st) {
+  const int ld = nd_ld(pb->nq), rows = 256 / (D / 8);
+  const dim3 grid((unsigned)((ld + rows - 1) / rows), (unsigned)(pb->batch * pb->heads));
+  auto vec = [](const fastmax_tensor& t) {
+    return ((uintptr_t)t.ptr & 15) == 0 && (t.stride_b & 3) == 0 && (t.stride_h & 3) == 0 && (t.stride_n & 3) == 0;
+  };
+  if (vec(a->o) && vec(a->d_out))
+    pair::f32::prologue_f32_kernel<D, true><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads);
+  else
+    pair::f32::prologue_f32_kernel<D, false><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads);
+}
+
+static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
+  const int bh = pb->batch * pb->heads;
+  const size_t nqb = pieces_bytes(pb, pb->nq), nkb = pieces_bytes(pb, pb->nk);
+  char* base = (char*)ws;
+  void *qp = base, *dp = base + nqb, *kp = base + 2 * nqb, *vp = base + 2 * nqb + nkb;
+  float* nd = (float*)(base + 2 * nqb + 2 * nkb);
+  pair::Maps M, N;   // M: dq, N: dk and dv
+  if (!pieces_map(&M.a, qp, pb, pb->nq, pair::R) || !pieces_map(&M.b, dp, pb, pb->nq, pair::R) ||
+      !pieces_map(&M.x, kp, pb, pb->nk, pair::f32::TF) || !pieces_map(&M.y, vp, pb, pb->nk, pair::f32::TF) ||
+      !pieces_map(&N.a, kp, pb, pb->nk, pair::R) || !pieces_map(&N.b, vp, pb, pb->nk, pair::R) ||
+      !pieces_map(&N.x, qp, pb, pb->nq, pair::f32::TF) || !pieces_map(&N.y, dp, pb, pb->nq, pair::f32::TF))
+    return FASTMAX_ERR_UNSUPPORTED;
+  M.o0 = M.o1 = N.o0 = N.o1 = M.a;
+  launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
+                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {pb->nq, pb->nk, pb->nk}}, 3, st);
+  {
+    LaunchScope ls(KK_PROLOGUE, st);
+    switch (pb->d) {
+      case 16: launch_prologue_f32<16>(pb, a, (__nv_bfloat16*)dp, nd, st); break;
+      case 32: launch_prologue_f32<32>(pb, a, (__nv_bfloat16*)dp, nd, st); break;
+      default: launch_prologue_f32<64>(pb, a, (__nv_bfloat16*)dp, nd, st); break;
+    }
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return report_cuda_error(e);
+  pair::Params P{};
+  fill(pb, P);
+  P.ndelta = nd;
+  P.nd_ld = nd_ld(pb->nq);
+  pair::Params K = P;
+  K.out0 = view_of(a->dk);
+  K.out1 = view_of(a->dv);
+  K.nr = pb->nk;
+  K.nx = pb->nq;
+  K.ntiles = tiles(pb->nk);
+  {
+    LaunchScope ls(KK_SCAN_BWD_KV, st);
+    e = launch_f32_d<pair::DKV>(pb->d, N, K, bh, st);
+  }
+  if (e != cudaSuccess) return report_cuda_error(e);
+  P.out0 = P.out1 = view_of(a->dq);
+  P.nr = pb->nq;
+  P.nx = pb->nk;
+  P.ntiles = tiles(pb->nq);
+  {
+    LaunchScope ls(KK_SCAN_BWD_Q, st);
+    e = launch_f32_d<pair::DQ>(pb->d, M, P, bh, st);
+  }
+  return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
+}
+
+// ---- bf16 ---------------------------------------------------------------------------------------------------------------
 // 32-row boxes of an output view, one per warp; views the copy engine cannot write are stored element by element
 static int out_map(CUtensorMap* m, const fastmax_tensor& t, const fastmax_problem* pb, int n) {
   return rows16(t) && tc_make_map(m, t, pb->batch, pb->heads, n, 64, 32, true, pb->d) ? 1 : 0;
 }
 
-int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, cudaStream_t st) {
+int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st) {
+  if (pb->dtype == FASTMAX_F32) return pair_f32_forward(pb, a, ws, st);
   pair::Maps M;
   if (!tc_make_map(&M.a, a->q, pb->batch, pb->heads, pb->nq, 64, pair::R, true, pb->d) ||
       !tc_make_map(&M.x, a->k, pb->batch, pb->heads, pb->nk, 64, pair::T, true, pb->d) ||
@@ -846,6 +1011,7 @@ static void launch_prologue(const fastmax_problem* pb, const fastmax_backward_ar
 }
 
 int pair_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
+  if (pb->dtype == FASTMAX_F32) return pair_f32_backward(pb, a, ws, st);
   const int bh = pb->batch * pb->heads;
   __nv_bfloat16* dop = (__nv_bfloat16*)ws;
   float* nd = (float*)((char*)ws + up256((size_t)bh * pb->nq * pb->d * 2));
