@@ -15,10 +15,16 @@ import math
 import torch
 
 
-def _ext():
-    from . import load_extension
+_extension = None
 
-    return load_extension()
+
+def _ext():
+    global _extension
+    if _extension is None:
+        from . import load_extension
+
+        _extension = load_extension()
+    return _extension
 
 
 def _alert_not_deterministic(what):
@@ -39,8 +45,29 @@ def _alert_not_deterministic(what):
         raise RuntimeError(msg)
 
 
+def _float32_in_bfloat16(q):
+    """float32 tensors under torch.set_float32_matmul_precision("medium"): the bfloat16 form of the call may run instead."""
+    return q.dtype == torch.float32 and torch.get_float32_matmul_precision() == "medium"
+
+
 class FASTMultiHeadAttention_Function(torch.autograd.Function):
-    """Behavioural twin of transformer/model.py:14-74 on top of the new `fastmax_cuda` extension."""
+    """Behavioural twin of transformer/model.py:14-74.  float32 CUDA tensors go through the extension's native autograd node,
+    which reads them where they are (no (n, b*h, d) copies; same values, same gradients, contiguous results); what that node
+    does not cover goes through forwardpass / backwardpass on top of the `fastmax_cuda` extension, as in the reference."""
+
+    @classmethod
+    def apply(cls, q, k, v, drop_noise, rpe_matrix=None, mask=False, dropout=0.0, normalize=False,
+              temperature=1.0, a0=1.0, a1=1.0, a2=0.5, lim=1.0, p=2):
+        if (rpe_matrix is None or q.dim() not in (3, 4) or not q.is_cuda or q.dtype != torch.float32 or k.dtype != torch.float32
+                or v.dtype != torch.float32 or _float32_in_bfloat16(q)):
+            return super().apply(q, k, v, drop_noise, rpe_matrix, mask, dropout, normalize, temperature, a0, a1, a2, lim, p)
+        _alert_not_deterministic("FASTMultiHeadAttention_Function")
+        three_d = q.dim() == 3
+        if three_d:
+            q, k, v = q.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0)
+        # exact_norm_grad False: the reference's backward ignores the normalisation
+        o = _ext().fastmax(q, k, v, mask, normalize, False, True, 1.0 / temperature, a0, a1, a2, lim, p)
+        return o.squeeze(0) if three_d else o
 
     @staticmethod
     def forward(ctx, q, k, v, drop_noise, rpe_matrix=None, mask=False, dropout=0.0, normalize=False,
@@ -103,7 +130,19 @@ class FastMax(torch.autograd.Function):
     reference's apply_dropout, :340-349, which it launches with scale 0).  With `normalize` the op computes
     lim * (x - mean_d x) / max_token ||x - mean_d x|| for q and k (fastattention_einops.py:327-334) and its
     exact gradient.  Scores are (q . k) / temperature.
+
+    Calls without the optional steps run as one native autograd node of the extension (apply below); the Python node that
+    follows covers the rest.
     """
+
+    @classmethod
+    def apply(cls, q, k, v, drop_noise=None, rpe_matrix=None, mask=False, dropout=0.0, normalize=False,
+              temperature=1.0, a0=1.0, a1=1.0, a2=0.5, lim=1.0, p=2, apply_rpe=False, noise_dropout=False):
+        if apply_rpe or noise_dropout or q.dim() != 4 or _float32_in_bfloat16(q):
+            return super().apply(q, k, v, drop_noise, rpe_matrix, mask, dropout, normalize, temperature, a0, a1, a2, lim, p,
+                                 apply_rpe, noise_dropout)
+        _alert_not_deterministic("FastMax (fastmax_custom)")
+        return _ext().fastmax(q, k, v, mask, normalize, True, False, 1.0 / temperature, a0, a1, a2, lim, p)
 
     @staticmethod
     def forward(ctx, q, k, v, drop_noise=None, rpe_matrix=None, mask=False, dropout=0.0, normalize=False,

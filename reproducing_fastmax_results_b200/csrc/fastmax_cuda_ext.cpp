@@ -394,6 +394,96 @@ int64_t forward_engine(torch::Tensor q, torch::Tensor k, torch::Tensor v, bool c
   return fastmax_forward_engine(&pb, &a);
 }
 
+// ---- the operator as one native autograd node --------------------------------------------------------------------------
+// FastMax (attention.py) without its optional steps, and FASTMultiHeadAttention_Function for float32 tensors: the same
+// launches as the Python Functions, without their per-call interpreter time (a training call of a few hundred tokens spent
+// 115 us on the host and 50 us on the GPU).
+// what the kernels take of a (b, h, n, d) tensor: unit stride on d, rows on 16-byte boundaries
+torch::Tensor readable(const torch::Tensor& t) {
+  const int64_t unit = 16 / t.element_size();
+  bool ok = (t.size(3) == 1 || t.stride(3) == 1) && (uintptr_t)t.data_ptr() % 16 == 0;
+  for (int i = 0; i < 3; ++i) ok = ok && (t.size(i) == 1 || t.stride(i) % unit == 0);
+  return ok ? t : t.contiguous();
+}
+
+struct FastmaxNode : public torch::autograd::Function<FastmaxNode> {
+  static torch::Tensor forward(torch::autograd::AutogradContext* ctx, torch::Tensor q, torch::Tensor k, torch::Tensor v, bool mask,
+                               bool normalize, bool exact_norm_grad, bool contiguous, double inv_t, double a0, double a1, double a2,
+                               double lim, int64_t p) {
+    torch::Tensor stats_q, stats_k;
+    if (contiguous) {   // the reference's wrapper takes tensors of any layout
+      q = readable(q); k = readable(k); v = readable(v);
+    }
+    if (normalize) {
+      auto nq = normalize_forward(q, lim);
+      auto nk = normalize_forward(k, lim);
+      q = nq[0]; stats_q = nq[1];
+      k = nk[0]; stats_k = nk[1];
+    }
+    c10::optional<torch::Tensor> out;
+    if (contiguous) out = torch::empty(q.sizes(), q.options());
+    auto res = ::forward(q, k, v, mask, inv_t, a0, a1, a2, p, c10::nullopt, false, true, FASTMAX_FLAG_PAIRWISE, out, c10::nullopt, true);
+    ctx->save_for_backward({q, k, v, res[0], res[1], stats_q, stats_k, res[3]});
+    auto& d = ctx->saved_data;
+    d["mask"] = mask; d["normalize"] = normalize && exact_norm_grad; d["contiguous"] = contiguous;
+    d["inv_t"] = inv_t; d["a0"] = a0; d["a1"] = a1; d["a2"] = a2; d["lim"] = lim; d["p"] = p;
+    return res[0];
+  }
+  static torch::autograd::tensor_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::tensor_list grads) {
+    auto saved = ctx->get_saved_variables();
+    auto& d = ctx->saved_data;
+    auto go = grads[0];
+    if (d["contiguous"].toBool()) go = go.contiguous();
+    else if (go.stride(-1) != 1) go = go.contiguous();
+    c10::optional<std::vector<torch::Tensor>> outs;
+    if (d["contiguous"].toBool())
+      outs = std::vector<torch::Tensor>{torch::empty(saved[0].sizes(), saved[0].options()), torch::empty(saved[1].sizes(), saved[1].options()),
+                                        torch::empty(saved[2].sizes(), saved[2].options())};
+    c10::optional<torch::Tensor> km;
+    if (saved[7].defined()) km = saved[7];
+    auto res = ::backward(saved[0], saved[1], saved[2], saved[3], saved[4], go, d["mask"].toBool(), d["inv_t"].toDouble(), d["a0"].toDouble(),
+                          d["a1"].toDouble(), d["a2"].toDouble(), d["p"].toInt(), c10::nullopt, c10::nullopt, false, true,
+                          FASTMAX_FLAG_PAIRWISE, outs, km, c10::nullopt, false);
+    if (d["normalize"].toBool()) {
+      res[0] = normalize_backward(saved[0], res[0], saved[5], d["lim"].toDouble());
+      res[1] = normalize_backward(saved[1], res[1], saved[6], d["lim"].toDouble());
+    }
+    torch::Tensor none;
+    return {res[0], res[1], res[2], none, none, none, none, none, none, none, none, none, none};
+  }
+};
+
+torch::Tensor fastmax_op(torch::Tensor q, torch::Tensor k, torch::Tensor v, bool mask, bool normalize, bool exact_norm_grad, bool contiguous,
+                         double inv_t, double a0, double a1, double a2, double lim, int64_t p) {
+  return FastmaxNode::apply(q, k, v, mask, normalize, exact_norm_grad, contiguous, inv_t, a0, a1, a2, lim, p);
+}
+
+// one token per (batch, head) against the carried state: q, k, v (b, h, d) or (b, h, 1, d); returns o shaped like q
+torch::Tensor decode_step(torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor state, double inv_temp, double a0, double a1,
+                          double a2, int64_t p, c10::optional<torch::Tensor> out) {
+  CHECK_CUDA(q); CHECK_CUDA(k); CHECK_CUDA(v); CHECK_CUDA(state);
+  TORCH_CHECK(q.dim() == 3 || q.dim() == 4, "q, k, v must be (b, h, d) or (b, h, 1, d)");
+  TORCH_CHECK(k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(), "q, k, v dtypes differ");
+  const int64_t b = q.size(0), h = q.size(1), d = q.size(-1);
+  for (const torch::Tensor* t : {&q, &k, &v})
+    TORCH_CHECK(t->size(0) == b && t->size(1) == h && t->size(-1) == d && t->numel() == b * h * d && (d == 1 || t->stride(-1) == 1),
+                "q, k, v: one token per (batch, head), unit stride on the head dim");
+  const c10::cuda::CUDAGuard guard(q.device());
+  fastmax_problem pb{};
+  pb.batch = b; pb.heads = h; pb.nq = pb.nk = 1; pb.d = d; pb.order = (int)p; pb.causal = 1; pb.dtype = dtype_of(q);
+  pb.a0 = (float)a0; pb.a1 = (float)a1; pb.a2 = (float)a2; pb.inv_temperature = (float)inv_temp;
+  TORCH_CHECK(state.is_contiguous() && state.scalar_type() == torch::kFloat32 && (size_t)state.numel() * 4 == fastmax_state_bytes(&pb),
+              "state has the wrong size");
+  torch::Tensor o = out.has_value() && out->defined() ? *out : torch::empty(q.sizes(), q.options());
+  TORCH_CHECK(o.sizes() == q.sizes() && o.scalar_type() == q.scalar_type() && (d == 1 || o.stride(-1) == 1), "out must look like q");
+  auto view = [](const torch::Tensor& t) { return fastmax_tensor{t.data_ptr(), t.stride(0), t.stride(1), 0}; };
+  fastmax_decode_args a{};
+  a.q = view(q); a.k = view(k); a.v = view(v); a.o = view(o);
+  a.state = (float*)state.data_ptr();
+  check_status(fastmax_decode_step(&pb, &a, at::cuda::getCurrentCUDAStream().stream()), "fastmax decode_step");
+  return o;
+}
+
 int64_t launch_count() { return (int64_t)fastmax_launch_count(); }
 
 }  // namespace
@@ -415,6 +505,10 @@ PYBIND11_MODULE(fastmax_cuda, m) {
         py::arg("want_dstate") = false, py::arg("want_grads") = true, py::arg("flags") = 0,
         py::arg("grads_out") = py::none(), py::arg("key_moments") = py::none(), py::arg("grad_moments") = py::none(),
         py::arg("want_grad_moments") = false, release());
+  m.def("fastmax", &fastmax_op, "the operator as one autograd node: (b,h,n,d) tensors -> o", release());
+  m.def("decode_step", &decode_step, "one token per (batch, head) against the carried state: returns o", py::arg("q"), py::arg("k"),
+        py::arg("v"), py::arg("state"), py::arg("inv_temp"), py::arg("a0"), py::arg("a1"), py::arg("a2"), py::arg("p"),
+        py::arg("out") = py::none(), release());
   m.def("normalize_forward", &normalize_forward, "q/k normalisation: returns [y, stats]", release());
   m.def("normalize_backward", &normalize_backward, "gradient of the q/k normalisation", release());
   m.def("key_prologue", &key_prologue, "k <- k * inv_temp + rpe rows, in place", py::arg("k"), py::arg("inv_temp"),
