@@ -441,9 +441,36 @@ static int fwd_layout(const fastmax_problem* pb, const fastmax_forward_args* a, 
   return need_seg;
 }
 
+// the problem of a state-only call: as many (unused) queries as keys
+static fastmax_problem keys_only(const fastmax_problem* pb) {
+  fastmax_problem p = *pb;
+  p.nq = pb->nk;
+  return p;
+}
+// A prompt call (output and final state of a causal call that starts from nothing) as two independent ones where that is
+// cheaper: the output pair by pair, the state by the state-only form of the moment engines, which then need not apply it.
+static bool splits_prompt(const fastmax_problem* pb, const fastmax_forward_args* a, fastmax_forward_args& out, fastmax_forward_args& state) {
+  if (!a->o.ptr || !a->state_out || a->state_in || !pb->causal || pb->nq <= 0) return false;
+  out = *a;
+  out.state_out = nullptr;
+  out.key_moments_in = nullptr;
+  out.key_moments_out = nullptr;
+  if (!pair_takes_forward(pb, &out)) return false;
+  state = *a;
+  state.q = a->k;
+  state.o = fastmax_tensor{};
+  state.g = fastmax_tensor{};
+  return true;
+}
+
 size_t fastmax_forward_workspace(const fastmax_problem* pb, const fastmax_forward_args* args) {
   Plan pl;
   if (!args || make_plan(pb, pl) != FASTMAX_OK) return 0;
+  fastmax_forward_args out, state;
+  if (splits_prompt(pb, args, out, state)) {
+    const fastmax_problem keys = keys_only(pb);
+    return align_up(fastmax_forward_workspace(pb, &out), 256) + fastmax_forward_workspace(&keys, &state);
+  }
   if (pair_takes_forward(pb, args)) return pair_forward_workspace(pb) + 256;
   FwdLayout L;
   fwd_layout(pb, args, pl, L);
@@ -460,6 +487,11 @@ int32_t fastmax_forward_engine(const fastmax_problem* pb, const fastmax_forward_
 size_t fastmax_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_args* args) {
   Plan pl;
   if (!args || make_plan(pb, pl) != FASTMAX_OK || pb->nk == 0) return 0;
+  fastmax_forward_args out_call, state_call;
+  if (splits_prompt(pb, args, out_call, state_call)) {
+    const fastmax_problem keys = keys_only(pb);
+    return fastmax_key_moments_bytes(&keys, &state_call);
+  }
   if (pair_takes_forward(pb, args)) return 0;
   if (const size_t t = tc_key_moments_bytes(pb, args)) return t;   // a long sequence cut into segments for the tensor-memory kernels
   if (tc_takes_forward(pb, args)) return 0;   // the tensor-memory kernels take this call whole: no segment sums
@@ -491,6 +523,18 @@ int32_t fastmax_forward(const fastmax_problem* pb, const fastmax_forward_args* a
   if (ws_bytes < fastmax_forward_workspace(pb, a) || (ws_bytes && (!ws || ((uintptr_t)ws % 256))))
     return FASTMAX_ERR_WORKSPACE;
 
+  fastmax_forward_args out_call, state_call;
+  if (want_o && splits_prompt(pb, a, out_call, state_call)) {
+    // side by side, the state first: the other call's blocks fill the SMs its last round leaves idle
+    fastmax_problem keys = keys_only(pb);
+    keys.flags |= FASTMAX_FLAG_SINGLE_STREAM;
+    const size_t own = align_up(fastmax_forward_workspace(pb, &out_call), 256);
+    SideBranch branch(pb, st);
+    rc = fastmax_forward(&keys, &state_call, (char*)ws + own, ws_bytes - own, branch.side);
+    if (rc == FASTMAX_OK) rc = pair_forward(pb, &out_call, ws, st);
+    const cudaError_t e = branch.join();
+    return rc != FASTMAX_OK ? rc : e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
+  }
   if (want_o && pair_takes_forward(pb, a)) return pair_forward(pb, a, ws, st);
   int tcrc = tc_forward(pb, a, ws, ws_bytes, st);
   if (tcrc != FASTMAX_TC_NOT_HANDLED) return tcrc;

@@ -269,6 +269,7 @@ intra_fwd_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant_
 #include "tc_scan2.cuh"
 #include "tc_scan3.cuh"
 #include "tc_p1.cuh"
+#include "tc_moments.cuh"
 
 // Exclusive running sum over the segments of the states st[seg][head][n] (in place): forward order (prefix) or
 // reverse (suffix), starting from init[head][n] when given; total_out[head][n] (optional) = init + all segments.
@@ -434,6 +435,10 @@ static SideStreams* fork_streams(const fastmax_problem* pb, cudaStream_t st, int
   }
   return p;
 }
+struct SideBranch::Lease {
+  SideStreams* p = nullptr;
+  std::unique_lock<std::mutex> lock;
+};
 static cudaError_t join_streams(SideStreams* p, cudaStream_t st, int n) {
   if (!p) return cudaSuccess;
   for (int i = 1; i < n; ++i) {
@@ -443,6 +448,19 @@ static cudaError_t join_streams(SideStreams* p, cudaStream_t st, int n) {
   }
   return cudaSuccess;
 }
+
+SideBranch::SideBranch(const fastmax_problem* pb, cudaStream_t st) : main(st), side(st), lease(new Lease) {
+  cudaStream_t ss[2];
+  lease->p = fork_streams(pb, st, 2, ss, lease->lock);
+  side = ss[1];
+}
+cudaError_t SideBranch::join() {
+  if (!lease) return cudaSuccess;
+  const cudaError_t e = join_streams(lease->p, main, 2);
+  lease.reset();
+  return e;
+}
+SideBranch::~SideBranch() { join(); }
 
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per (device, kernel) instead of on every call: the attribute
 // sticks to the function on that device.  `slot` numbers the kernels of this file.
@@ -514,13 +532,12 @@ static ScanGeom scan_geom(const fastmax_problem* pb, bool backward = false) {
 }
 // Schedule of one scan.  Forward direction (forward pass, dq): query chunks apply, key chunks update.  Reverse
 // direction (dk, dv): key chunks apply, query chunks update, and scan index ci visits chunk nch - 1 - ci.
-static tc::Sched make_sched(const ScanGeom& g, bool reverse, bool has_init, bool want_apply, bool want_state) {
+static tc::Sched make_sched(const ScanGeom& g, bool reverse, bool has_init, bool want_state) {
   tc::Sched sc{};
   int a0, a1, u0, u1;
   if (!reverse) { a0 = g.qc0; a1 = g.qc1; u0 = g.kc0; u1 = g.kc1; }
   else { a0 = g.nch - 1 - g.kc1; a1 = g.nch - 1 - g.kc0; u0 = g.nch - 1 - g.qc1; u1 = g.nch - 1 - g.qc0; }
-  if (!want_apply) { a0 = 0; a1 = -1; }
-  else if (!has_init && a0 == 0) a0 = 1;           // the state is still zero in the first chunk
+  if (!has_init && a0 == 0) a0 = 1;           // the state is still zero in the first chunk
   if (!want_state && u1 > a1 - 1) u1 = a1 - 1;     // updates that nothing reads any more
   sc.a_first = a0; sc.a_last = a1; sc.u_first = u0; sc.u_last = u1;
   sc.c_first = u0 > a0 - 1 ? u0 : a0 - 1;
@@ -905,6 +922,61 @@ size_t tc_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_arg
   return tc_forward_segmentable(pb, a) ? seg_state_bytes(pb, tc_segments(pb)) : 0;
 }
 
+// moment states without an output (tc_moments.cuh): state = [init +] Phi(X)^T Y over n tokens per head.  tmxt: transposed copy
+// of X (column = token); y: Y (v, or dO' with 80 columns).
+static cudaError_t launch_moments(const fastmax_problem* pb, const CUtensorMap& tmxt, const fastmax_tensor& y, int n, bool dop,
+                                  const float* init, float* state, int kind, cudaStream_t st) {
+  const int bh = pb->batch * pb->heads;
+  CUtensorMap tmy;
+  if (!make_map(&tmy, y, pb->batch, pb->heads, n, 64, tc::CH, true, dop ? 80 : 64)) return cudaErrorInvalidValue;
+  tc::mo::Params P{};
+  P.out = state;
+  P.n = n;
+  P.heads = pb->heads;
+  P.nchunks = (n + tc::CH - 1) / tc::CH;
+  P.bh = bh;
+  P.tile_first = pb->order == 2 ? 0 : tc::NTILES - 1;
+  P.state_rows = pb->order == 2 ? 64 * 36 + 65 : 65;
+  P.dop = dop ? 1 : 0;
+  // Tiles per block and cuts of the token axis: the combination that ends first when the SMs take the blocks in order (full
+  // slices, then the shorter last ones), in clocks: 620 per tile and chunk, 12000 to start a block and write its rows, 20000 to
+  // add them, and 12000 for the memset that adding needs.  16 heads of 8192 tokens: 74 us with three tiles a block, 89 with
+  // four, 92 with four and two cuts; 128 heads of 4096: 220 us with four, 239 with three.
+  const int ntiles = pb->order == 2 ? tc::NTILES : 1, sms = device_sms();
+  long long best = -1;
+  for (int tps = 1; tps <= 4; ++tps)
+    for (int c = 1; c <= 16 && c <= P.nchunks; ++c) {
+      const bool add = c > 1 || init != nullptr;
+      const long long per = (P.nchunks + c - 1) / c, last = ntiles % tps, fixed = add ? 20000 : 12000;
+      const long long df = per * 620 * tps + fixed, dl = per * 620 * last + fixed;
+      const long long nf = (long long)(ntiles / tps) * bh * c, nl = last ? (long long)bh * c : 0;
+      const long long q = nf / sms, m = nf % sms;   // m SMs run q + 1 full blocks, the others q
+      long long cost = (q + (m > 0)) * df;
+      for (long long j = 1; nl > 0; ++j) {          // until j short blocks behind the q full ones are enough
+        const long long t = q * df + j * dl;
+        if ((sms - m) * j + (t >= (q + 1) * df ? m * ((t - (q + 1) * df) / dl) : 0) >= nl) {
+          if (t > cost) cost = t;
+          break;
+        }
+      }
+      if (add) cost += 12000;
+      if (best < 0 || cost < best) { best = cost; P.tps = tps; P.nsplit = c; }
+    }
+  P.nslices = (ntiles + P.tps - 1) / P.tps;
+  P.chunks_per_split = (P.nchunks + P.nsplit - 1) / P.nsplit;
+  P.nsplit = (P.nchunks + P.chunks_per_split - 1) / P.chunks_per_split;
+  const int ctas = P.nslices * bh;
+  P.add = P.nsplit > 1 || init != nullptr;
+  cudaError_t e = ensure_smem(tc::mo::moments_kernel, tc::mo::SMEM_BYTES, 7);
+  const size_t bytes = (size_t)bh * P.state_rows * 68 * sizeof(float);
+  if (e == cudaSuccess && init != nullptr && init != state) e = cudaMemcpyAsync(state, init, bytes, cudaMemcpyDeviceToDevice, st);
+  else if (e == cudaSuccess && P.add && init == nullptr) e = cudaMemsetAsync(state, 0, bytes, st);
+  if (e != cudaSuccess) return e;
+  LaunchScope ls(kind, st);
+  tc::mo::moments_kernel<<<dim3((unsigned)(ctas * P.nsplit)), tc::mo::THREADS, tc::mo::SMEM_BYTES, st>>>(tmxt, tmy, P);
+  return cudaGetLastError();
+}
+
 int tc_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, size_t ws_bytes, cudaStream_t st) {
   if (tc_forward_paddable(pb, a)) return tc_forward_padded(pb, a, ws, ws_bytes, st);
   if (tc_p1_supported(pb, a)) return tc_p1_forward(pb, a, st);
@@ -932,6 +1004,10 @@ int tc_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* w
   if (want_o) e = cudaMemsetAsync(oacc, 0, (size_t)bh * pb->nq * 68 * sizeof(float), st);
   if (e == cudaSuccess) e = launch_transpose(a->k, pb->batch, pb->heads, pb->nk, 0, kt, st);
   if (e != cudaSuccess) return report_cuda_error(e);
+  if (!want_o) {
+    e = launch_moments(pb, tmkt, a->v, pb->nk, false, a->state_in, a->state_out, KK_TC_FWD, st);
+    return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
+  }
   tc::FwdParams P{};
   P.oacc = oacc;
   P.heads = pb->heads;
@@ -947,7 +1023,7 @@ int tc_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* w
     e = ensure_smem(tc::intra_fwd_kernel, tc::I_SMEM_BYTES, 2);
   if (e != cudaSuccess) return report_cuda_error(e);
   // the scan and the intra-chunk kernel both ADD into the O' accumulator: independent, side by side
-  const bool intra = want_o && pb->causal;
+  const bool intra = pb->causal != 0;
   cudaStream_t ss[2];
   std::unique_lock<std::mutex> side_lock;
   SideStreams* side = intra ? fork_streams(pb, st, 2, ss, side_lock) : nullptr;
@@ -959,7 +1035,7 @@ int tc_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* w
     A.out = oacc; A.heads = pb->heads; A.nz = pb->nq; A.ny = pb->nk; A.z_shift = G.k0; A.y_shift = 0; A.nchunks = G.nch;
     A.c0 = P.c0; A.c1 = P.c1; A.c2 = P.c2;
     A.state_out = a->state_out; A.state_in = a->state_in;
-    A.sc = make_sched(G, false, a->state_in != nullptr, want_o, a->state_out != nullptr);
+    A.sc = make_sched(G, false, a->state_in != nullptr, a->state_out != nullptr);
     A.nslices = G.nslices; A.tps = G.tps; A.tile_first = G.tile_first; A.state_rows = G.state_rows;
     tc::s2::scan_apply_kernel<false><<<dim3(G.nslices * bh), tc::s2::THREADS, tc::s2::SMEM_BYTES, ss[0]>>>(tmq, tmkt, tmv, A);
   }
@@ -976,7 +1052,7 @@ int tc_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* w
     e = join_streams(side, st, 2);
   }
   if (e != cudaSuccess) return report_cuda_error(e);
-  return want_o ? launch_finalize_fwd(pb, a, oacc, st) : FASTMAX_OK;
+  return launch_finalize_fwd(pb, a, oacc, st);
 }
 
 static int device_sms() {
@@ -1213,24 +1289,20 @@ int tc_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void*
   const float c2 = pb->order == 2 ? pb->a2 * pb->inv_temperature * pb->inv_temperature : 0.f;
   e = ensure_smem(tc::s2::scan_apply_kernel<true>, tc::s2::SMEM_BYTES, 3);
   if (e != cudaSuccess) return report_cuda_error(e);
-  auto dv_params = [&](bool want_apply) {
+  auto dv_params = [&] {
     tc::s2::ApplyParams A{};
-    A.out = want_apply ? dva : nullptr; A.heads = pb->heads; A.nz = pb->nk; A.ny = pb->nk; A.z_shift = 0; A.y_shift = G.k0;
+    A.out = dva; A.heads = pb->heads; A.nz = pb->nk; A.ny = pb->nk; A.z_shift = 0; A.y_shift = G.k0;
     A.nchunks = G.nch; A.c0 = c0; A.c1 = c1; A.c2 = c2;
     A.state_out = a->dstate_out; A.state_in = a->dstate_in;
-    A.sc = make_sched(G, true, a->dstate_in != nullptr, want_apply, a->dstate_out != nullptr);
+    A.sc = make_sched(G, true, a->dstate_in != nullptr, a->dstate_out != nullptr);
     A.nslices = G.nslices; A.tps = G.tps; A.tile_first = G.tile_first; A.state_rows = G.state_rows;
     return A;
   };
   if (!want_grads) {
-    // only the gradient moments are wanted (what a sequence-parallel rank publishes): the dv scan, updates only
-    e = launch_transpose(a->q, pb->batch, pb->heads, pb->nq, G.k0, qt, st);
-    if (e != cudaSuccess) return report_cuda_error(e);
-    {
-      LaunchScope ls(KK_TC_BWD_DV, st);
-      tc::s2::scan_apply_kernel<true><<<dim3(G.nslices * bh), tc::s2::THREADS, tc::s2::SMEM_BYTES, st>>>(tmk, tmqt, tmdo, dv_params(false));
-    }
-    e = cudaGetLastError();
+    // only the gradient moments are wanted (what a sequence-parallel rank publishes); columns of the copy = queries
+    if (!make_map_t(&tmqt, qt, bh, pb->nq, tokens_padded(pb->nq))) return FASTMAX_TC_NOT_HANDLED;
+    e = launch_transpose(a->q, pb->batch, pb->heads, pb->nq, 0, qt, st);
+    if (e == cudaSuccess) e = launch_moments(pb, tmqt, dopt, pb->nq, true, a->dstate_in, a->dstate_out, KK_TC_BWD_DV, st);
     return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
   }
   // The chain-rule scans rebalance registers between their warp groups with setmaxnreg; that only terminates if
@@ -1295,7 +1367,7 @@ int tc_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void*
     C.heads = pb->heads; C.nz = dk ? pb->nk : pb->nq; C.nk = pb->nk; C.z_shift = dk ? 0 : G.k0; C.do_shift = G.k0;
     C.nchunks = G.nch; C.c1 = c1; C.c2 = c2;
     C.state_in = dk ? a->dstate_in : a->state_in;
-    C.sc = make_sched(G, dk, C.state_in != nullptr, true, false);
+    C.sc = make_sched(G, dk, C.state_in != nullptr, false);
     C.nslices = G.nslices; C.tps = G.tps; C.tile_first = G.tile_first; C.state_rows = G.state_rows;
     return C;
   };
@@ -1314,7 +1386,7 @@ int tc_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void*
   if (e != cudaSuccess) return report_cuda_error(e);
   {
     LaunchScope ls(KK_TC_BWD_DV, ss[0]);
-    tc::s2::scan_apply_kernel<true><<<dim3(G.nslices * bh), tc::s2::THREADS, tc::s2::SMEM_BYTES, ss[0]>>>(tmk, tmqt, tmdo, dv_params(true));
+    tc::s2::scan_apply_kernel<true><<<dim3(G.nslices * bh), tc::s2::THREADS, tc::s2::SMEM_BYTES, ss[0]>>>(tmk, tmqt, tmdo, dv_params());
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) return report_cuda_error(e);

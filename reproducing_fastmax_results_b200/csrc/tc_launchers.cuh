@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <memory>
+
 #include "../../include/fastmax_b200.h"
 
 namespace fm {
@@ -31,6 +33,20 @@ int tc_wait_selftest(long long cycles, int code, cudaStream_t st);
 // zero); false when the copy engine cannot describe the view
 bool tc_make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int heads, int n, int box_cols, int box_rows, bool swizzle128,
                  int cols);
+
+// A second stream for work that is independent of what the caller's stream gets meanwhile: forked from it here, joined back
+// by join() (or the destructor).  The caller's own stream when side streams are off.  Calls made on `side` must carry
+// FASTMAX_FLAG_SINGLE_STREAM: the device's side streams are leased until the join.
+struct SideBranch {
+  SideBranch(const fastmax_problem* pb, cudaStream_t st);
+  ~SideBranch();
+  cudaError_t join();
+  cudaStream_t main, side;
+
+ private:
+  struct Lease;
+  std::shared_ptr<Lease> lease;
+};
 
 // shared with the C-ABI translation unit
 int report_cuda_error(cudaError_t e);  // remembers e for fastmax_last_cuda_error(), returns FASTMAX_ERR_CUDA

@@ -55,7 +55,8 @@ class FastmaxDecoder:
         if q.dim() != 4 or q.shape[2] != k.shape[2]:
             raise ValueError("prefill takes (b, h, n, d) tensors with as many queries as keys")
         o, _, state = _lib.forward(q, k, v, True, self.inv_temperature, self.a0, self.a1, self.a2, self.p,
-                                   state_in=self.state if self.tokens_seen else None, want_state=True)
+                                   state_in=self.state if self.tokens_seen else None, want_state=True,
+                                   flags=_lib.FLAG_PAIRWISE)
         self.state = state
         self.tokens_seen += q.shape[2]
         return o

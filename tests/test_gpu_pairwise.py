@@ -93,5 +93,5 @@ def test_pairwise_form_is_left_to_the_moment_engines_where_it_does_not_apply():
     oe, ge, _ = L.forward(q, shared, v, True, 0.05, order=2, flags=L.FLAG_PAIRWISE)
     oc, gc, _ = L.forward(q, shared.contiguous(), v, True, 0.05, order=2, flags=L.FLAG_PAIRWISE)
     L.check_status()
-    for a, b, tol in ((o, o_ref, 2e-3), (state, state_ref, 1e-5), (oe, oc, 1e-2), (ge, gc, 1e-3)):
+    for a, b, tol in ((o, o_ref, 1e-2), (state, state_ref, 1e-4), (oe, oc, 1e-2), (ge, gc, 1e-3)):
         assert orc.max_norm_err(host(a), host(b)) < tol
