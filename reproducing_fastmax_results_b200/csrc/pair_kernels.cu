@@ -21,6 +21,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "common.cuh"
 #include "launchers.cuh"
@@ -179,6 +180,11 @@ struct Item {
   int t0;          // first streamed tile
   int n0, n1;      // streamed tiles of the held tile(s); n1: the second tile of a forward item
 };
+// The first rows of a causal sequence see few keys: their denominators are small, their gradients a hundred times the rest,
+// and what is rounded to bf16 there shows.  Their tile is therefore evaluated without the completed square (below), with the
+// roundings of the moment engines, and its denominators sum the rounded weights (the first row's output is then its value).
+__device__ __forceinline__ bool first_rows(const Params& P, int r0) { return P.causal && P.off < R && r0 + P.off < R; }
+
 // TILE: streamed rows per tile, HELD: rows of an item
 template <int KIND, int TILE, int HELD>
 __device__ __forceinline__ Item decode(int idx, const Params& P) {
@@ -337,10 +343,11 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
             if (KIND == DQ) { if (k >= 2) WAIT(B_READS + buf, (k >> 1) - 1u, 80); }   // the buffer's last scores have been read
             else if (k > 0) WAIT(B_READS + buf, k - 1u, 80);
             tc_fence_after_sync();
-            if (SQ) mma_ss_elect(tmem + C_S + buf * 128u, dHa, dHb, ID_S, 0u);
+            const bool add_h = SQ && !first_rows(P, it.r0 + m * R);
+            if (add_h) mma_ss_elect(tmem + C_S + buf * 128u, dHa, dHb, ID_S, 0u);
 #pragma unroll
             for (int ks = 0; ks < KS; ++ks)
-              mma_ss_elect(tmem + C_S + buf * 128u, dH + (uint64_t)(m * (X_BYTES >> 4) + 2 * ks), dX + (uint64_t)(2 * ks), ID_S, SQ || ks > 0);
+              mma_ss_elect(tmem + C_S + buf * 128u, dH + (uint64_t)(m * (X_BYTES >> 4) + 2 * ks), dX + (uint64_t)(2 * ks), ID_S, (add_h || ks > 0) ? 1u : 0u);
             if (KIND != FWD) {
               if (k > 0) WAIT(B_READD, k - 1u, 82);
               tc_fence_after_sync();
@@ -438,11 +445,13 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars[B_AFREE + grp]);
       const bool second = KIND == DKV && half == 0;   // dv
-      float wgt = second ? P.w1 : P.w0;
+      const bool first = first_rows(P, it.r0 + grp * R);
+      const float w1 = first ? 1.f : P.w1;
+      float wgt = second ? w1 : first ? 1.f : P.w0;
       if (KIND == FWD) {
         wgt = 1.f / total;   // the sum and the products carry the same factor
         if (row < P.nr)
-          reinterpret_cast<float*>(const_cast<void*>(P.out1.ptr))[(long long)it.b * P.out1.sb + (long long)it.h * P.out1.sh + (long long)row * P.out1.sn] = total * P.w1;
+          reinterpret_cast<float*>(const_cast<void*>(P.out1.ptr))[(long long)it.b * P.out1.sb + (long long)it.h * P.out1.sh + (long long)row * P.out1.sn] = total * w1;
       }
       if (second ? P.vec1 : P.vec0) {
         // rows -> the item's held set (its products are done), 128-byte swizzle -> the copy engine, which writes whole lines
@@ -486,6 +495,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
       const Item it = decode<KIND, T, HELD_ROWS>(idx, P);
       const int nt = (KIND == FWD && grp) ? it.n1 : it.n0;
       const int row = it.r0 + grp * R + quarter * 32 + lane;
+      const bool first = first_rows(P, it.r0 + grp * R);
       float total = 0.f;
       if (KIND == FWD) {
         float a, b;
@@ -514,6 +524,28 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
         const bool whole = __all_sync(0xffffffffu, lo <= 0 && hi >= W);
         const uint32_t sa = lane_addr + C_S + (uint32_t)(buf * 128 + W * half);
         if (KIND == FWD) {
+          if (first) {   // general form, the sum of the rounded weights
+            if (k > 0) WAIT(B_SFREE + grp, k - 1u, 83);
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+              uint32_t x32[32], pr[16];
+              tmem_ld32(sa + 32u * c, x32);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const uint64_t x = pack2u(x32[2 * j], x32[2 * j + 1]);
+                float p0, p1;
+                unpack2(fma2(fma2(C2, x, C1), x, C0), p0, p1);
+                pr[j] = bf16x2(32 * c + 2 * j < hi ? p0 : 0.f, 32 * c + 2 * j + 1 < hi ? p1 : 0.f);
+                sum[j & 3] = add2(sum[j & 3], pack2u(pr[j] << 16, pr[j] & 0xffff0000u));
+              }
+              tmem_st16(lane_addr + Cols<KIND>::P + 64u * grp + 16u * c, pr);
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars[B_READS + grp]);
+          } else {
           uint32_t s[4][32];
 #pragma unroll
           for (int c = 0; c < 4; ++c) tmem_ld32(sa + 32u * c, s[c]);
@@ -548,6 +580,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
             }
             tmem_st16(lane_addr + Cols<KIND>::P + 64u * grp + 16u * c, pr);
           }
+          }
         } else {
           uint32_t d[2][32], s[2][32], pr[2][16], dr[2][16];
           tmem_ld32(lane_addr + Cols<KIND>::DP + 64u * half, d[0]);
@@ -561,31 +594,30 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
             mbar_arrive(&bars[B_READS + buf]);
             mbar_arrive(&bars[B_READD]);
           }
+          auto weights = [&](auto square) {   // the element-wise part: f and f' (dP - delta), in bf16
+            constexpr bool Q = decltype(square)::value;
 #pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const ulonglong2* ndp = reinterpret_cast<const ulonglong2*>(sm + OFF_ND + (k & (STAGES - 1)) * T * 4 + half * 256 + c * 128);
+            for (int c = 0; c < 2; ++c) {
+              const ulonglong2* ndp = reinterpret_cast<const ulonglong2*>(sm + OFF_ND + (k & (STAGES - 1)) * T * 4 + half * 256 + c * 128);
 #pragma unroll
-            for (int j2 = 0; j2 < 8; ++j2) {
-              ulonglong2 n2;
-              n2.x = n2.y = ND;
-              if (KIND == DKV) n2 = ndp[j2];
+              for (int j2 = 0; j2 < 8; ++j2) {
+                ulonglong2 n2;
+                n2.x = n2.y = ND;
+                if (KIND == DKV) n2 = ndp[j2];
 #pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const int j = 2 * j2 + e;
-                const uint64_t x = pack2u(s[c][2 * j], s[c][2 * j + 1]);
-                const uint64_t dp = add2(pack2u(d[c][2 * j], d[c][2 * j + 1]), e ? n2.y : n2.x);
-                if (KIND == DQ || SQ) {
-                  const uint64_t u = SQ ? x : fma2(C22, x, C1);
+                for (int e = 0; e < 2; ++e) {
+                  const int j = 2 * j2 + e;
+                  const uint64_t x = pack2u(s[c][2 * j], s[c][2 * j + 1]);
+                  const uint64_t dp = add2(pack2u(d[c][2 * j], d[c][2 * j + 1]), e ? n2.y : n2.x);
+                  const uint64_t u = Q ? x : fma2(C22, x, C1);
                   dr[c][j] = bf16x2(mul2(u, dp));
-                  if (KIND == DKV) pr[c][j] = bf16x2(fma2(u, u, K));
-                } else {
-                  const uint64_t t = fma2(C2, x, C1);
-                  pr[c][j] = bf16x2(fma2(t, x, C0));
-                  dr[c][j] = bf16x2(mul2(fma2(C2, x, t), dp));
+                  if (KIND == DKV) pr[c][j] = bf16x2(Q ? fma2(u, u, K) : fma2(fma2(C2, x, C1), x, C0));
                 }
               }
             }
-          }
+          };
+          if (SQ && !first) weights(std::true_type{});
+          else weights(std::false_type{});
           if (!whole) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
@@ -646,7 +678,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
   if (w == W_ACC) tmem_dealloc(tmem, 512);
 }
 
-// dO' = dO / g in bf16 (dense [batch*heads][nq][D]) and -delta = -(dO . o) / g (zero from nq on).  D / 8 threads per row,
+// dO' = dO / g in bf16 (dense [batch*heads][nq][D]) and -delta = -(dO . o) / g, rounded to bf16 as everywhere (zero from nq on).  D / 8 threads per row,
 // 16-byte accesses (VEC) or element by element for views that do not allow them.
 template <int D, bool VEC>
 __global__ void __launch_bounds__(256) prologue_kernel(View dout, View o, View g, __nv_bfloat16* __restrict__ dop, float* __restrict__ ndelta,
@@ -681,7 +713,7 @@ __global__ void __launch_bounds__(256) prologue_kernel(View dout, View o, View g
     r.x = bf16x2(dv[0], dv[1]); r.y = bf16x2(dv[2], dv[3]); r.z = bf16x2(dv[4], dv[5]); r.w = bf16x2(dv[6], dv[7]);
     *reinterpret_cast<uint4*>(dop + ((long long)head * nq + row) * D + c) = r;
   }
-  if (c == 0 && row < nd_ld) ndelta[(long long)head * nd_ld + row] = row < nq ? -dot : 0.f;
+  if (c == 0 && row < nd_ld) ndelta[(long long)head * nd_ld + row] = row < nq ? __bfloat162float(__float2bfloat16(-dot)) : 0.f;
 }
 
 #include "pair_f32.cuh"

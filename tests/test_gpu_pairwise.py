@@ -54,7 +54,7 @@ def test_pairwise_kernels_match_oracle(case, poly, dtype):
         o_ref, g_ref = orc.fastmax_naive(a[0], a[1], a[2], causal, p)
         refs = (o_ref, g_ref) + tuple(orc.fastmax_naive_grads(a[0], a[1], a[2], a[3], causal, p))
         for name, x, r, tol in zip(("o", "g", "dq", "dk", "dv"), (o, gg, dq, dk, dv), refs,
-                                   (2e-2, 1e-5, 2e-2, 2e-2, 2e-2) if dtype == torch.bfloat16 else (5e-6,) * 5):
+                                   (2e-2, 2e-3, 2e-2, 2e-2, 2e-2) if dtype == torch.bfloat16 else (5e-6,) * 5):
             if np.abs(r).max() > 1e-9:   # dq and dk of a single visible key are analytically zero
                 assert orc.max_norm_err(host(x[b, h]), r) < tol, (name, b, h)
 
