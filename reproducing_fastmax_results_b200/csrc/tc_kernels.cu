@@ -22,6 +22,7 @@
 #include "launchers.cuh"
 #include "pair_launchers.cuh"
 #include "tc_launchers.cuh"
+#include "tc_phi.cuh"
 #include "tc_ptx.cuh"
 
 namespace fm {
@@ -81,10 +82,6 @@ struct FwdParams {
   float c0, c1, c2;
 };
 
-__device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
-  __nv_bfloat162 r = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
-  return *reinterpret_cast<uint32_t*>(&r);
-}
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&r);
@@ -328,13 +325,14 @@ static EncodeTiledFn encode_fn() {
 
 // bf16 (batch, head, token, cols) view -> 4-D tensor map with a [box_rows x box_cols] box.
 bool tc_make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int heads, int n, int box_cols, int box_rows,
-                     bool swizzle128, int cols) {
+                     bool swizzle128, int cols, bool f32) {
   EncodeTiledFn fn = encode_fn();
   if (!fn || n <= 0) return false;
   const cuuint64_t dims[4] = {(cuuint64_t)cols, (cuuint64_t)n, (cuuint64_t)heads, (cuuint64_t)batch};
   // a stride of a size-1 dimension is never used for addressing; any legal value will do.  A zero stride of a longer one
   // (a tensor expanded over tokens, heads or the batch) is left to the CUDA-core engine.
-  cuuint64_t sn = (cuuint64_t)t.stride_n * 2, sh = (cuuint64_t)t.stride_h * 2, sbb = (cuuint64_t)t.stride_b * 2;
+  const cuuint64_t es = f32 ? 4 : 2;
+  cuuint64_t sn = (cuuint64_t)t.stride_n * es, sh = (cuuint64_t)t.stride_h * es, sbb = (cuuint64_t)t.stride_b * es;
   if ((n > 1 && sn == 0) || (heads > 1 && sh == 0) || (batch > 1 && sbb == 0)) return false;
   if (n == 1) sn = 128;
   if (heads == 1) sh = sn * (cuuint64_t)n;
@@ -345,7 +343,7 @@ bool tc_make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int heads, 
   const cuuint32_t box[4] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   auto encode = [&] {
-    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, t.ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    return fn(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, t.ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
               swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   };
@@ -359,31 +357,32 @@ bool tc_make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int heads, 
 
 static bool make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int heads, int n, int box_cols, int box_rows,
                      bool swizzle128, int cols = 64) {
-  return tc_make_map(m, t, batch, heads, n, box_cols, box_rows, swizzle128, cols);
+  return tc_make_map(m, t, batch, heads, n, box_cols, box_rows, swizzle128, cols, false);
 }
 
 // Transposed bf16 copy xt [batch*heads][64][ntp] -> 3-D tensor map (tokens, 64 dims, batch*heads), box 72 x 64, no swizzle.
-static bool make_map_t(CUtensorMap* m, void* xt, int bh, int n, int ntp) {
+static bool make_map_t(CUtensorMap* m, void* xt, int bh, int n, int ntp, int d = 64) {
   EncodeTiledFn fn = encode_fn();
   if (!fn || n <= 0) return false;
-  const cuuint64_t dims[3] = {(cuuint64_t)n, 64, (cuuint64_t)bh};
-  const cuuint64_t strides[2] = {(cuuint64_t)ntp * 2, (cuuint64_t)ntp * 128};
-  const cuuint32_t box[3] = {72, 64, 1};  // 64 tokens + 8: shared-memory rows of 144 bytes spread over the banks
+  const cuuint64_t dims[3] = {(cuuint64_t)n, (cuuint64_t)d, (cuuint64_t)bh};
+  const cuuint64_t strides[2] = {(cuuint64_t)ntp * 2, (cuuint64_t)ntp * 2 * d};
+  const cuuint32_t box[3] = {72, (cuuint32_t)d, 1};  // 64 tokens + 8: shared-memory rows of 144 bytes spread over the banks
   const cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, xt, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 static inline int tokens_padded(int n) { return (n + 63) / 64 * 64; }
-static inline size_t transposed_bytes(int bh, int n) { return ((size_t)bh * 64 * tokens_padded(n) * 2 + 255) / 256 * 256; }
+static inline size_t transposed_bytes(int bh, int n, int d = 64) { return ((size_t)bh * d * tokens_padded(n) * 2 + 255) / 256 * 256; }
 
 // xt [batch*heads][64][tokens_padded(n + shift)]: column p = token p - shift of x
 static cudaError_t launch_transpose(const fastmax_tensor& x, int batch, int heads, int n, int shift, __nv_bfloat16* xt,
-                                    cudaStream_t st) {
+                                    cudaStream_t st, int d = 64) {
   LaunchScope ls(KK_TC_TRANSPOSE, st);
   const int ntp = tokens_padded(n + shift);
-  tc::s2::transpose_tokens_kernel<<<dim3(ntp / 64, batch * heads), 256, 0, st>>>(
-      View{x.ptr, x.stride_b, x.stride_h, x.stride_n}, xt, n, ntp, heads, shift);
+  const View v{x.ptr, x.stride_b, x.stride_h, x.stride_n};
+  if (d == 64) tc::s2::transpose_tokens_kernel<64><<<dim3(ntp / 64, batch * heads), 256, 0, st>>>(v, xt, n, ntp, heads, shift);
+  else tc::s2::transpose_tokens_kernel<32><<<dim3(ntp / 64, batch * heads), 256, 0, st>>>(v, xt, n, ntp, heads, shift);
   return cudaGetLastError();
 }
 
@@ -922,31 +921,40 @@ size_t tc_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_arg
   return tc_forward_segmentable(pb, a) ? seg_state_bytes(pb, tc_segments(pb)) : 0;
 }
 
-// moment states without an output (tc_moments.cuh): state = [init +] Phi(X)^T Y over n tokens per head.  tmxt: transposed copy
-// of X (column = token); y: Y (v, or dO' with 80 columns).
-static cudaError_t launch_moments(const fastmax_problem* pb, const CUtensorMap& tmxt, const fastmax_tensor& y, int n, bool dop,
-                                  const float* init, float* state, int kind, cudaStream_t st) {
-  const int bh = pb->batch * pb->heads;
-  CUtensorMap tmy;
-  if (!make_map(&tmy, y, pb->batch, pb->heads, n, 64, tc::CH, true, dop ? 80 : 64)) return cudaErrorInvalidValue;
+// Moment states without an output (tc_moments.cuh), head dim 32 or 64: state = [init +] Phi(X)^T [Y | tail] over n tokens per
+// head, or one state per segment of seg_tokens tokens.  x: keys (tail: ones) or queries (y = dO' with D + 16 columns, the tail
+// is column D).  xt: scratch of tc_moments_scratch() bytes.
+size_t tc_moments_scratch(const fastmax_problem* pb, int n) { return transposed_bytes(pb->batch * pb->heads, n, pb->d); }
+cudaError_t tc_moments(const fastmax_problem* pb, const fastmax_tensor& x, const fastmax_tensor& y, int n, bool dop, int seg_tokens,
+                       const float* init, float* state, void* xt, int kind, cudaStream_t st) {
+  const int bh = pb->batch * pb->heads, d = pb->d;
+  CUtensorMap tmxt, tmy, tmt;
+  if (!make_map_t(&tmxt, xt, bh, n, tokens_padded(n), d) || !make_map(&tmy, y, pb->batch, pb->heads, n, 64, tc::CH, true, d)) return cudaErrorInvalidValue;
+  tmt = tmy;
+  if (dop && !make_map(&tmt, y, pb->batch, pb->heads, n, 8, tc::CH, false, d + 16)) return cudaErrorInvalidValue;
+  cudaError_t e = launch_transpose(x, pb->batch, pb->heads, n, 0, (__nv_bfloat16*)xt, st, d);
+  if (e != cudaSuccess) return e;
+  const int npair = (d / 8) * (d / 8 + 1) / 2;
   tc::mo::Params P{};
   P.out = state;
   P.n = n;
+  P.bh = bh;
   P.heads = pb->heads;
   P.nchunks = (n + tc::CH - 1) / tc::CH;
-  P.bh = bh;
-  P.tile_first = pb->order == 2 ? 0 : tc::NTILES - 1;
-  P.state_rows = pb->order == 2 ? 64 * 36 + 65 : 65;
+  P.tile_first = pb->order == 2 ? 0 : npair / 2;
+  P.state_rows = (pb->order == 2 ? 64 * npair : 0) + d + 1;
   P.dop = dop ? 1 : 0;
+  P.per_split = seg_tokens > 0;
   // Tiles per block and cuts of the token axis: the combination that ends first when the SMs take the blocks in order (full
   // slices, then the shorter last ones), in clocks: 620 per tile and chunk, 12000 to start a block and write its rows, 20000 to
   // add them, and 12000 for the memset that adding needs.  16 heads of 8192 tokens: 74 us with three tiles a block, 89 with
   // four, 92 with four and two cuts; 128 heads of 4096: 220 us with four, 239 with three.
-  const int ntiles = pb->order == 2 ? tc::NTILES : 1, sms = device_sms();
+  const int ntiles = pb->order == 2 ? npair / 2 + 1 : 1, sms = device_sms();
+  const int segs = seg_tokens > 0 ? (n + seg_tokens - 1) / seg_tokens : 0;
   long long best = -1;
   for (int tps = 1; tps <= 4; ++tps)
-    for (int c = 1; c <= 16 && c <= P.nchunks; ++c) {
-      const bool add = c > 1 || init != nullptr;
+    for (int c = segs > 0 ? segs : 1; c <= (segs > 0 ? segs : 16) && c <= P.nchunks; ++c) {
+      const bool add = segs == 0 && (c > 1 || init != nullptr);
       const long long per = (P.nchunks + c - 1) / c, last = ntiles % tps, fixed = add ? 20000 : 12000;
       const long long df = per * 620 * tps + fixed, dl = per * 620 * last + fixed;
       const long long nf = (long long)(ntiles / tps) * bh * c, nl = last ? (long long)bh * c : 0;
@@ -963,17 +971,19 @@ static cudaError_t launch_moments(const fastmax_problem* pb, const CUtensorMap& 
       if (best < 0 || cost < best) { best = cost; P.tps = tps; P.nsplit = c; }
     }
   P.nslices = (ntiles + P.tps - 1) / P.tps;
-  P.chunks_per_split = (P.nchunks + P.nsplit - 1) / P.nsplit;
+  P.chunks_per_split = segs > 0 ? seg_tokens / tc::CH : (P.nchunks + P.nsplit - 1) / P.nsplit;
   P.nsplit = (P.nchunks + P.chunks_per_split - 1) / P.chunks_per_split;
-  const int ctas = P.nslices * bh;
-  P.add = P.nsplit > 1 || init != nullptr;
-  cudaError_t e = ensure_smem(tc::mo::moments_kernel, tc::mo::SMEM_BYTES, 7);
-  const size_t bytes = (size_t)bh * P.state_rows * 68 * sizeof(float);
-  if (e == cudaSuccess && init != nullptr && init != state) e = cudaMemcpyAsync(state, init, bytes, cudaMemcpyDeviceToDevice, st);
-  else if (e == cudaSuccess && P.add && init == nullptr) e = cudaMemsetAsync(state, 0, bytes, st);
+  const unsigned ctas = (unsigned)(P.nslices * bh * P.nsplit);
+  P.add = segs == 0 && (P.nsplit > 1 || init != nullptr);
+  const size_t bytes = (size_t)bh * P.state_rows * (d + 4) * sizeof(float);
+  if (P.add && init != nullptr && init != state) e = cudaMemcpyAsync(state, init, bytes, cudaMemcpyDeviceToDevice, st);
+  else if (P.add && init == nullptr) e = cudaMemsetAsync(state, 0, bytes, st);
+  if (e == cudaSuccess) e = d == 64 ? ensure_smem(tc::mo::moments_kernel<64>, tc::mo::Lay<64>::SMEM_BYTES, 7)
+                                    : ensure_smem(tc::mo::moments_kernel<32>, tc::mo::Lay<32>::SMEM_BYTES, 2);
   if (e != cudaSuccess) return e;
   LaunchScope ls(kind, st);
-  tc::mo::moments_kernel<<<dim3((unsigned)(ctas * P.nsplit)), tc::mo::THREADS, tc::mo::SMEM_BYTES, st>>>(tmxt, tmy, P);
+  if (d == 64) tc::mo::moments_kernel<64><<<dim3(ctas), tc::mo::THREADS, tc::mo::Lay<64>::SMEM_BYTES, st>>>(tmxt, tmy, tmt, P);
+  else tc::mo::moments_kernel<32><<<dim3(ctas), tc::mo::THREADS, tc::mo::Lay<32>::SMEM_BYTES, st>>>(tmxt, tmy, tmt, P);
   return cudaGetLastError();
 }
 
@@ -983,31 +993,25 @@ int tc_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* w
   if (tc_forward_segmentable(pb, a)) return tc_forward_segmented(pb, a, ws, ws_bytes, st);
   if (!tc_forward_supported(pb, a)) return FASTMAX_TC_NOT_HANDLED;
   if (ws_bytes < tc_forward_workspace(pb, a)) return FASTMAX_ERR_WORKSPACE;
-  const bool want_o = a->o.ptr && pb->nq > 0;
   CUtensorMap tmq, tmk, tmv;
   if (!make_map(&tmk, a->k, pb->batch, pb->heads, pb->nk, 64, tc::CH, true) ||
       !make_map(&tmv, a->v, pb->batch, pb->heads, pb->nk, 8, tc::CH, false))
     return FASTMAX_TC_NOT_HANDLED;  // layout the copy engine cannot describe: the CUDA-core engine takes it
-  if (want_o) {
-    if (!make_map(&tmq, a->q, pb->batch, pb->heads, pb->nq, 64, tc::CH, true)) return FASTMAX_TC_NOT_HANDLED;
-  } else {
-    tmq = tmk;   // a state-only call applies nothing: the tile is loaded and never read
+  if (!(a->o.ptr && pb->nq > 0)) {
+    const cudaError_t e = tc_moments(pb, a->k, a->v, pb->nk, false, 0, a->state_in, a->state_out, ws, KK_TC_FWD, st);
+    return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
   }
+  if (!make_map(&tmq, a->q, pb->batch, pb->heads, pb->nq, 64, tc::CH, true)) return FASTMAX_TC_NOT_HANDLED;
   const int bh = pb->batch * pb->heads;
   const ScanGeom G = scan_geom(pb);
   float* oacc = (float*)ws;
-  const size_t oacc_bytes = want_o ? ((size_t)bh * pb->nq * 68 * sizeof(float) + 255) / 256 * 256 : 0;
+  const size_t oacc_bytes = ((size_t)bh * pb->nq * 68 * sizeof(float) + 255) / 256 * 256;
   __nv_bfloat16* kt = (__nv_bfloat16*)((char*)ws + oacc_bytes);
   CUtensorMap tmkt;
   if (!make_map_t(&tmkt, kt, bh, pb->nk, tokens_padded(pb->nk))) return FASTMAX_TC_NOT_HANDLED;
-  cudaError_t e = cudaSuccess;
-  if (want_o) e = cudaMemsetAsync(oacc, 0, (size_t)bh * pb->nq * 68 * sizeof(float), st);
+  cudaError_t e = cudaMemsetAsync(oacc, 0, (size_t)bh * pb->nq * 68 * sizeof(float), st);
   if (e == cudaSuccess) e = launch_transpose(a->k, pb->batch, pb->heads, pb->nk, 0, kt, st);
   if (e != cudaSuccess) return report_cuda_error(e);
-  if (!want_o) {
-    e = launch_moments(pb, tmkt, a->v, pb->nk, false, a->state_in, a->state_out, KK_TC_FWD, st);
-    return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
-  }
   tc::FwdParams P{};
   P.oacc = oacc;
   P.heads = pb->heads;
@@ -1299,10 +1303,8 @@ int tc_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void*
     return A;
   };
   if (!want_grads) {
-    // only the gradient moments are wanted (what a sequence-parallel rank publishes); columns of the copy = queries
-    if (!make_map_t(&tmqt, qt, bh, pb->nq, tokens_padded(pb->nq))) return FASTMAX_TC_NOT_HANDLED;
-    e = launch_transpose(a->q, pb->batch, pb->heads, pb->nq, 0, qt, st);
-    if (e == cudaSuccess) e = launch_moments(pb, tmqt, dopt, pb->nq, true, a->dstate_in, a->dstate_out, KK_TC_BWD_DV, st);
+    // only the gradient moments are wanted (what a sequence-parallel rank publishes)
+    e = tc_moments(pb, a->q, dopt, pb->nq, true, 0, a->dstate_in, a->dstate_out, qt, KK_TC_BWD_DV, st);
     return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
   }
   // The chain-rule scans rebalance registers between their warp groups with setmaxnreg; that only terminates if

@@ -30,9 +30,13 @@ int tc_wait_histogram(int* out, int n);
 int tc_wait_selftest(long long cycles, int code, cudaStream_t st);
 
 // bf16 (batch, head, token, cols) view -> 4-D tensor map with a [box_rows x box_cols] box (columns past `cols` read as
-// zero); false when the copy engine cannot describe the view
+// zero); f32: the elements are float32; false when the copy engine cannot describe the view
 bool tc_make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int heads, int n, int box_cols, int box_rows, bool swizzle128,
-                 int cols);
+                 int cols, bool f32 = false);
+
+size_t tc_moments_scratch(const fastmax_problem* pb, int n);
+cudaError_t tc_moments(const fastmax_problem* pb, const fastmax_tensor& x, const fastmax_tensor& y, int n, bool dop, int seg_tokens,
+                       const float* init, float* state, void* xt, int kind, cudaStream_t st);
 
 // A second stream for work that is independent of what the caller's stream gets meanwhile: forked from it here, joined back
 // by join() (or the destructor).  The caller's own stream when side streams are off.  Calls made on `side` must carry

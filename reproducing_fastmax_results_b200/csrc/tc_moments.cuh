@@ -15,29 +15,44 @@ namespace mo {
 constexpr int THREADS = 576;
 constexpr int W_MMA = 16, W_TMA = 17;
 constexpr int STAGES = 4;
-constexpr int KT_BOX = 64 * s2::KT_ROW;            // 64 dims x 72 tokens
-// Y: two 64-column halves of 128 tokens, 128-byte swizzled rows (columns 0..63 and 64..127, of which 16 are used): whole rows
-// for the copy engine instead of 8-column boxes of 16 bytes a row
-constexpr int OFF_Y = 0, OFF_XT = 2 * REGION, STAGE = OFF_XT + 2 * KT_BOX;
-constexpr int OFF_BAR = STAGES * STAGE;
-constexpr int SMEM_BYTES = OFF_BAR + 512 + 1024;
-static_assert(KT_BOX % 128 == 0 && STAGE % 1024 == 0, "TMA destinations, swizzled tiles");
-static_assert(4 * CH * 68 * 4 <= STAGES * STAGE, "the output rows are staged over the tiles");
-static_assert(SMEM_BYTES <= 232448, "shared memory budget");
+// D: head dim.  Feature tiles: two 64-row pair units each, the last one holds the linear and constant rows.
+template <int D>
+struct Lay {
+  static constexpr int NB = D / 8;
+  static constexpr int PAIR_TILES = NB * (NB + 1) / 4;
+  static constexpr int TILES = PAIR_TILES + 1;
+  static constexpr int NC = D + 16;                       // accumulator columns of a tile: Y and its tail column
+  static constexpr int KT_BOX = D * s2::KT_ROW;           // D dims x 72 tokens
+  // Y: 128 tokens, 128-byte swizzled rows; tail (-delta of dO'): one 8-column block (8 columns used as 16: zeros follow)
+  static constexpr int OFF_T = REGION, OFF_XT = REGION + BLK, STAGE = (OFF_XT + 2 * KT_BOX + 1023) / 1024 * 1024;
+  static constexpr int OFF_ONES = STAGES * STAGE;         // the tail of [v | 1]: one constant block of ones, then a block of zeros
+  static constexpr int OFF_BAR = OFF_ONES + 2 * BLK;
+  static constexpr int SMEM_BYTES = OFF_BAR + 512 + 1024;
+  static constexpr int LD = D + 4;
+  static_assert((NB * (NB + 1) / 2) % 2 == 0, "whole tiles of two pair units");
+  static_assert(KT_BOX % 128 == 0, "TMA destinations");
+  static_assert(4 * CH * LD * 4 <= STAGES * STAGE, "the output rows are staged over the tiles");
+  static_assert(SMEM_BYTES <= 232448, "shared memory budget");
+};
 constexpr int B_FULL = 0, B_EMPTY = STAGES, B_SLOT = 2 * STAGES, B_FREE = B_SLOT + 3, B_DONE = B_FREE + 3, B_COUNT = B_DONE + 1;
-constexpr uint32_t COL_A = 320;
+constexpr uint32_t COL_A = 320;   // behind four accumulators of 80 columns
 
 struct Params {
-  float* out;          // [BH][state_rows][68]
+  float* out;          // [BH][state_rows][D + 4]; per_split: [BH][nsplit][state_rows][D + 4]
   int n;               // tokens
   int bh, heads, nchunks, chunks_per_split, nsplit;
   int nslices, tps, tile_first, state_rows;
-  int dop;             // Y has 80 columns in memory (dO'); else 64, and a ones column is put beside them
+  int dop;             // Y is dO' and its tail column comes from memory (column D); else the tail is ones
+  int per_split;       // every split has a state of its own
   int add;             // add to `out` instead of storing
 };
 
+template <int D>
 __global__ void __launch_bounds__(THREADS, 1)
-moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__ CUtensorMap tmy, const Params P) {
+moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__ CUtensorMap tmy, const __grid_constant__ CUtensorMap tmt,
+               const Params P) {
+  using L = Lay<D>;
+  constexpr int STAGE = L::STAGE, OFF_XT = L::OFF_XT, OFF_BAR = L::OFF_BAR, KT_BOX = L::KT_BOX, LIN = L::TILES - 1;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* sm = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
@@ -51,7 +66,7 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
   const int head = rest / P.nsplit, split = rest - head * P.nsplit;
   const int b_idx = head / P.heads, h_idx = head - b_idx * P.heads;
   const int tile0 = P.tile_first + slice * P.tps;
-  const int ntl = min(P.tps, NTILES - tile0);
+  const int ntl = min(P.tps, L::TILES - tile0);
   const int c0 = split * P.chunks_per_split, c1 = min(P.nchunks, c0 + P.chunks_per_split);
   const int nc = c1 - c0;
 
@@ -60,13 +75,9 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
     *abort_flag = 0;
     fence_mbar_init();
   }
-  if (!P.dop) {   // the ones column of Y: constant (features of tokens past the last one are zero)
-    for (int i = tid; i < STAGES * CH * 8; i += THREADS) {
-      const int r = (i >> 3) & (CH - 1), c = i & 7;   // 16-byte piece c of row r, swizzled
-      *reinterpret_cast<uint4*>(sm + (i >> 10) * STAGE + OFF_Y + REGION + r * 128 + ((c ^ (r & 7)) << 4)) = make_uint4(c ? 0u : 0x00003F80u, 0u, 0u, 0u);
-    }
-    fence_proxy_async_smem();
-  }
+  for (int i = tid; i < 2 * CH; i += THREADS)   // (features of tokens past the last one are zero)
+    *reinterpret_cast<uint4*>(sm + L::OFF_ONES + i * 16) = make_uint4(i < CH ? 0x00003F80u : 0u, 0u, 0u, 0u);
+  fence_proxy_async_smem();
   if (w == W_MMA) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
   __syncthreads();
@@ -85,29 +96,35 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
       if (lane == 0) {
         uint8_t* st = sm + s * STAGE;
         const int tok = (c0 + i) * CH;
-        mbar_arrive_expect_tx(&bars[B_FULL + s], 2 * KT_BOX + (P.dop ? 2 : 1) * REGION);
-        tma_load_4d(st + OFF_Y, &tmy, &bars[B_FULL + s], 0, tok, h_idx, b_idx);
-        if (P.dop) tma_load_4d(st + OFF_Y + REGION, &tmy, &bars[B_FULL + s], 64, tok, h_idx, b_idx);
+        mbar_arrive_expect_tx(&bars[B_FULL + s], 2 * KT_BOX + REGION + (P.dop ? BLK : 0));
+        tma_load_4d(st, &tmy, &bars[B_FULL + s], 0, tok, h_idx, b_idx);
+        if (P.dop) tma_load_4d(st + L::OFF_T, &tmt, &bars[B_FULL + s], D, tok, h_idx, b_idx);
         tma_load_3d(st + OFF_XT, &tmxt, &bars[B_FULL + s], tok, 0, head);
         tma_load_3d(st + OFF_XT + KT_BOX, &tmxt, &bars[B_FULL + s], tok + 64, 0, head);
       }
       loaded = i + 1;
     }
   } else if (w == W_MMA) {
-    constexpr uint32_t ID = make_idesc_bf16(128, 80, 0, 1);
-    const uint64_t dY = make_smem_desc(smem_u32(sm + OFF_Y), REGION, 1024, 2);
+    constexpr uint32_t ID = make_idesc_bf16(128, D, 0, 1), ID_T = make_idesc_bf16(128, 16, 0, 1);
+    const uint64_t dY = make_smem_desc(smem_u32(sm), REGION, 1024, 2);
+    const uint32_t zeros = smem_u32(sm + L::OFF_ONES + BLK);
     uint32_t k = 0;   // slabs so far
     for (int i = 0; i < nc; ++i) {
       const uint32_t s = (uint32_t)i % STAGES;
       WAIT(B_FULL + (int)s, (uint32_t)(i / STAGES), 111);
+      // tail operand: its block of eight columns, and the zeros a fixed distance behind it
+      const uint32_t tail = P.dop ? smem_u32(sm + s * STAGE + L::OFF_T) : smem_u32(sm + L::OFF_ONES);
+      const uint64_t dT = make_smem_desc(tail, 128, zeros - tail, 0);
       for (int t = 0; t < ntl; ++t, ++k) {
         const uint32_t slot = k % 3u;
         WAIT(B_SLOT + (int)slot, k / 3u, 112);
         tc_fence_after_sync();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          mma_ts_elect(tmem + 80u * t, tmem + COL_A + 64u * slot + 8u * kk, dY + (uint64_t)(s * (STAGE >> 4) + 128 * kk), ID,
-                       (i > 0 || kk > 0) ? 1u : 0u);
+        for (int kk = 0; kk < 8; ++kk) {
+          const uint32_t a = tmem + COL_A + 64u * slot + 8u * kk, acc = (i > 0 || kk > 0) ? 1u : 0u;
+          mma_ts_elect(tmem + L::NC * t, a, dY + (uint64_t)(s * (STAGE >> 4) + 128 * kk), ID, acc);
+          mma_ts_elect(tmem + L::NC * t + D, a, dT + (uint64_t)(16 * kk), ID_T, acc);
+        }
         mma_commit_elect(&bars[B_FREE + slot]);
       }
       mma_commit_elect(&bars[B_EMPTY + s]);
@@ -123,9 +140,9 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       int a = 0, b = 0;
-      if (t < ntl && tile0 + t < NTILES - 1) pair_decode(2 * (tile0 + t) + (row >> 6), 8, a, b);   // warp-uniform
+      if (t < ntl && tile0 + t < LIN) pair_decode(2 * (tile0 + t) + (row >> 6), L::NB, a, b);   // warp-uniform
       rows[t] = (uint32_t)((8 * a + (f >> 3)) * s2::KT_ROW) | (uint32_t)((8 * b + (f & 7)) * s2::KT_ROW) << 16;
-      if (tile0 + t == NTILES - 1) rows[t] = (uint32_t)(f * s2::KT_ROW) | (uint32_t)(f * s2::KT_ROW) << 16;
+      if (tile0 + t == LIN) rows[t] = (uint32_t)((f & (D - 1)) * s2::KT_ROW) | (uint32_t)((f & (D - 1)) * s2::KT_ROW) << 16;
     }
     uint32_t k = 0;
     for (int i = 0; i < nc; ++i) {
@@ -143,7 +160,7 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
       for (int t = 0; t < 4; ++t) {
         if (t < ntl) {
           uint32_t r[16];
-          if (tile0 + t < NTILES - 1) {
+          if (tile0 + t < LIN) {
             if (t == 0 || (rows[t] & 0xffffu) != (rows[t > 0 ? t - 1 : 0] & 0xffffu)) load(xa, rows[t] & 0xffffu);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -152,11 +169,11 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
               r[4 * c + 2] = hmul2_u32(xa[c].z, xb[c].z);
               r[4 * c + 3] = hmul2_u32(xa[c].w, xb[c].w);
             }
-          } else if (row < 64) {
+          } else if (row < D) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) { r[4 * c] = xb[c].x; r[4 * c + 1] = xb[c].y; r[4 * c + 2] = xb[c].z; r[4 * c + 3] = xb[c].w; }
-          } else {   // the constant feature (row 64), zero for tokens past the last one, and nothing
-            const int left = row == 64 ? P.n - ((c0 + i) * CH + 32 * g) : 0;
+          } else {   // the constant feature (row D), zero for tokens past the last one, and nothing
+            const int left = row == D ? P.n - ((c0 + i) * CH + 32 * g) : 0;
 #pragma unroll
             for (int c = 0; c < 16; ++c) r[c] = (2 * c < left ? 0x00003F80u : 0u) | (2 * c + 1 < left ? 0x3F800000u : 0u);
           }
@@ -179,31 +196,31 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
   __syncthreads();
   tc_fence_after_sync();
   if (*abort_flag == 0) {
-    // accumulators -> staging rows of 68 floats -> the state's rows, which lie one behind the other; producer group g: tile g
+    // accumulators -> staging rows of D + 4 floats -> the state's rows, which lie one behind the other; producer group g: tile g
     const int g = w >> 2;
     if (g < ntl) {
-      float* stage = reinterpret_cast<float*>(sm) + g * CH * 68;
+      float* stage = reinterpret_cast<float*>(sm) + g * CH * L::LD;
       const int row = (w & 3) * 32 + lane;
-      const uint32_t a = tmem + ((uint32_t)((w & 3) * 32) << 16) + 80u * g;
-      float4* dst = reinterpret_cast<float4*>(stage + row * 68);
+      const uint32_t a = tmem + ((uint32_t)((w & 3) * 32) << 16) + (uint32_t)(L::NC * g);
+      float4* dst = reinterpret_cast<float4*>(stage + row * L::LD);
       uint32_t r[32], r8[8];
-      tmem_ld8(a + 64u, r8);
+      tmem_ld8(a + (uint32_t)D, r8);
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
+      for (int half = 0; half < D / 32; ++half) {
         tmem_ld32(a + 32u * half, r);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 8; ++j)
           dst[8 * half + j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
       }
-      dst[16] = make_float4(__uint_as_float(r8[0]), 0.f, 0.f, 0.f);
+      dst[D / 4] = make_float4(__uint_as_float(r8[0]), 0.f, 0.f, 0.f);
       fence_proxy_async_smem();
       named_bar_sync(1 + g, 128);
       if ((w & 3) == 0 && lane == 0) {
         const int row0 = (tile0 + g - P.tile_first) * CH, rows = min(CH, P.state_rows - row0);
-        float* out = P.out + ((long long)head * P.state_rows + row0) * 68;
-        if (P.add) bulk_reduce_add_f32(out, stage, (uint32_t)rows * 272u);
-        else bulk_store(out, stage, (uint32_t)rows * 272u);
+        float* out = P.out + ((long long)(P.per_split ? head * P.nsplit + split : head) * P.state_rows + row0) * L::LD;
+        if (P.add) bulk_reduce_add_f32(out, stage, (uint32_t)(rows * L::LD * 4));
+        else bulk_store(out, stage, (uint32_t)(rows * L::LD * 4));
         bulk_commit_group();
         bulk_wait_read_all();
       }

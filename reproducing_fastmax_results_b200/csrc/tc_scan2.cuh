@@ -107,31 +107,6 @@ __device__ __forceinline__ void slab_kind(bool first_chunk, bool last_tile, int 
   else { is_q = !(j & 1); half = j >> 1; }
 }
 
-// Row `row` of a 128-byte-swizzled tile with 128-byte rows: 16-byte chunk cc.
-__device__ __forceinline__ uint4 sw_chunk(const uint8_t* tile, int row, int cc) {
-  return *reinterpret_cast<const uint4*>(tile + row * 128 + ((cc ^ (row & 7)) << 4));
-}
-
-// Apply slab: 64 features x[8a+mi] * x[8b+ri] of token row l of the raw [token][64] tile -> 32 packed registers
-// (register 4 mi + j holds ri = 2j, 2j + 1).  `dbl`: x[8a+mi] is doubled (exact) for an off-diagonal unit.
-__device__ __forceinline__ void apply_pair_slab(uint32_t (&r)[32], const uint8_t* raw, int l, int a, int b, bool dbl) {
-  uint4 xa4 = sw_chunk(raw, l, a);
-  const uint4 xb4 = sw_chunk(raw, l, b);
-  if (dbl) {
-    const uint32_t two = 0x40004000u;  // bf16x2 (2, 2)
-    xa4.x = hmul2_u32(xa4.x, two); xa4.y = hmul2_u32(xa4.y, two); xa4.z = hmul2_u32(xa4.z, two); xa4.w = hmul2_u32(xa4.w, two);
-  }
-  const uint32_t xa[4] = {xa4.x, xa4.y, xa4.z, xa4.w};
-#pragma unroll
-  for (int mi = 0; mi < 8; ++mi) {
-    const uint32_t pr = xa[mi >> 1];
-    const uint32_t bc = (mi & 1) ? __byte_perm(pr, pr, 0x3232) : __byte_perm(pr, pr, 0x1010);
-    r[4 * mi + 0] = hmul2_u32(bc, xb4.x);
-    r[4 * mi + 1] = hmul2_u32(bc, xb4.y);
-    r[4 * mi + 2] = hmul2_u32(bc, xb4.z);
-    r[4 * mi + 3] = hmul2_u32(bc, xb4.w);
-  }
-}
 // Update slab: products x[i][tok] * x[j][tok] for the 64 tokens of one box of the transposed tile ([64 dims] rows of
 // KT_ROW bytes, not swizzled: the pitch spreads consecutive rows over the banks) -> 32 packed registers
 // (register 4 cc + jj holds tokens 8cc + 2jj, +1).
@@ -630,14 +605,15 @@ scan_apply_kernel(const __grid_constant__ CUtensorMap tmz, const __grid_constant
 // (zero where there is none; ntp is a multiple of 64).  One block per (64-column group, batch*head).  The tile goes
 // through shared memory as 32-bit words (two dims each) with a row pitch of 33 words, so both the row-wise stores
 // and the column-wise loads spread over the banks.
+template <int D = 64>
 __global__ void __launch_bounds__(256) transpose_tokens_kernel(View x, __nv_bfloat16* __restrict__ xt, int n, int ntp, int heads,
                                                                int shift) {
   __shared__ uint32_t tile[64 * 33];
   const int head = blockIdx.y, t0 = blockIdx.x * 64;
   const int b = head / heads, h = head - b * heads;
   const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(x.ptr) + (long long)b * x.sb + (long long)h * x.sh;
-  for (int idx = threadIdx.x; idx < 512; idx += 256) {
-    const int r = idx >> 3, cv = idx & 7;
+  for (int idx = threadIdx.x; idx < 8 * D; idx += 256) {
+    const int r = idx / (D / 8), cv = idx % (D / 8);
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     const int tok = t0 + r - shift;
     if (tok >= 0 && tok < n) v = *reinterpret_cast<const uint4*>(src + (long long)tok * x.sn + cv * 8);
@@ -647,6 +623,7 @@ __global__ void __launch_bounds__(256) transpose_tokens_kernel(View x, __nv_bflo
   __syncthreads();
   // thread = (pair of dims dp, group of 8 tokens tg): eight words -> two output rows of eight tokens
   const int dp = threadIdx.x >> 3, tg = threadIdx.x & 7;
+  if (dp >= D / 2) return;
   uint32_t wv[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) wv[e] = tile[(tg * 8 + e) * 33 + dp];
@@ -655,7 +632,7 @@ __global__ void __launch_bounds__(256) transpose_tokens_kernel(View x, __nv_bflo
   lo.y = __byte_perm(wv[2], wv[3], 0x5410); hi.y = __byte_perm(wv[2], wv[3], 0x7632);
   lo.z = __byte_perm(wv[4], wv[5], 0x5410); hi.z = __byte_perm(wv[4], wv[5], 0x7632);
   lo.w = __byte_perm(wv[6], wv[7], 0x5410); hi.w = __byte_perm(wv[6], wv[7], 0x7632);
-  __nv_bfloat16* dst = xt + ((long long)head * 64 + 2 * dp) * ntp + t0 + tg * 8;
+  __nv_bfloat16* dst = xt + ((long long)head * D + 2 * dp) * ntp + t0 + tg * 8;
   *reinterpret_cast<uint4*>(dst) = lo;
   *reinterpret_cast<uint4*>(dst + ntp) = hi;
 }
