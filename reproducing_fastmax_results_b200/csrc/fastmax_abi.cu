@@ -450,7 +450,7 @@ static fastmax_problem keys_only(const fastmax_problem* pb) {
 // A prompt call (output and final state of a causal call that starts from nothing) as two independent ones where that is
 // cheaper: the output pair by pair, the state by the state-only form of the moment engines, which then need not apply it.
 static bool splits_prompt(const fastmax_problem* pb, const fastmax_forward_args* a, fastmax_forward_args& out, fastmax_forward_args& state) {
-  if (!a->o.ptr || !a->state_out || a->state_in || !pb->causal || pb->nq <= 0) return false;
+  if (!a->o.ptr || !a->state_out || a->state_in || !pb->causal || pb->nq <= 0 || pair_takes_forward(pb, a)) return false;
   out = *a;
   out.state_out = nullptr;
   out.key_moments_in = nullptr;
@@ -471,7 +471,7 @@ size_t fastmax_forward_workspace(const fastmax_problem* pb, const fastmax_forwar
     const fastmax_problem keys = keys_only(pb);
     return align_up(fastmax_forward_workspace(pb, &out), 256) + fastmax_forward_workspace(&keys, &state);
   }
-  if (pair_takes_forward(pb, args)) return pair_forward_workspace(pb) + 256;
+  if (pair_takes_forward(pb, args)) return pair_forward_workspace(pb, args) + 256;
   FwdLayout L;
   fwd_layout(pb, args, pl, L);
   size_t tc = tc_forward_workspace(pb, args);
@@ -492,7 +492,7 @@ size_t fastmax_key_moments_bytes(const fastmax_problem* pb, const fastmax_forwar
     const fastmax_problem keys = keys_only(pb);
     return fastmax_key_moments_bytes(&keys, &state_call);
   }
-  if (pair_takes_forward(pb, args)) return 0;
+  if (pair_takes_forward(pb, args)) return pair_key_moments_bytes(pb, args);
   if (const size_t t = tc_key_moments_bytes(pb, args)) return t;   // a long sequence cut into segments for the tensor-memory kernels
   if (tc_takes_forward(pb, args)) return 0;   // the tensor-memory kernels take this call whole: no segment sums
   FwdLayout L;
@@ -616,7 +616,7 @@ static void bwd_layout(const fastmax_problem* pb, const fastmax_backward_args* a
 size_t fastmax_backward_workspace(const fastmax_problem* pb, const fastmax_backward_args* args) {
   Plan pl;
   if (!args || make_plan(pb, pl, true) != FASTMAX_OK) return 0;
-  if (pair_takes_backward(pb, args)) return pair_backward_workspace(pb) + 256;
+  if (pair_takes_backward(pb, args)) return pair_backward_workspace(pb, args) + 256;
   BwdLayout L;
   bwd_layout(pb, args, pl, L);
   size_t tc = tc_backward_workspace(pb, args);

@@ -409,7 +409,7 @@ torch::Tensor readable(const torch::Tensor& t) {
 struct FastmaxNode : public torch::autograd::Function<FastmaxNode> {
   static torch::Tensor forward(torch::autograd::AutogradContext* ctx, torch::Tensor q, torch::Tensor k, torch::Tensor v, bool mask,
                                bool normalize, bool exact_norm_grad, bool contiguous, double inv_t, double a0, double a1, double a2,
-                               double lim, int64_t p) {
+                               double lim, int64_t p, bool train) {
     torch::Tensor stats_q, stats_k;
     if (contiguous) {   // the reference's wrapper takes tensors of any layout
       q = readable(q); k = readable(k); v = readable(v);
@@ -422,7 +422,9 @@ struct FastmaxNode : public torch::autograd::Function<FastmaxNode> {
     }
     c10::optional<torch::Tensor> out;
     if (contiguous) out = torch::empty(q.sizes(), q.options());
-    auto res = ::forward(q, k, v, mask, inv_t, a0, a1, a2, p, c10::nullopt, false, true, FASTMAX_FLAG_PAIRWISE, out, c10::nullopt, true);
+    // the states of the keys are kept for the backward only where there will be one
+    auto res = ::forward(q, k, v, mask, inv_t, a0, a1, a2, p, c10::nullopt, false, true, FASTMAX_FLAG_PAIRWISE, out, c10::nullopt, train);
+    if (!train) res.emplace_back();
     ctx->save_for_backward({q, k, v, res[0], res[1], stats_q, stats_k, res[3]});
     auto& d = ctx->saved_data;
     d["mask"] = mask; d["normalize"] = normalize && exact_norm_grad; d["contiguous"] = contiguous;
@@ -449,13 +451,14 @@ struct FastmaxNode : public torch::autograd::Function<FastmaxNode> {
       res[1] = normalize_backward(saved[1], res[1], saved[6], d["lim"].toDouble());
     }
     torch::Tensor none;
-    return {res[0], res[1], res[2], none, none, none, none, none, none, none, none, none, none};
+    return {res[0], res[1], res[2], none, none, none, none, none, none, none, none, none, none, none};
   }
 };
 
 torch::Tensor fastmax_op(torch::Tensor q, torch::Tensor k, torch::Tensor v, bool mask, bool normalize, bool exact_norm_grad, bool contiguous,
                          double inv_t, double a0, double a1, double a2, double lim, int64_t p) {
-  return FastmaxNode::apply(q, k, v, mask, normalize, exact_norm_grad, contiguous, inv_t, a0, a1, a2, lim, p);
+  const bool train = at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad());
+  return FastmaxNode::apply(q, k, v, mask, normalize, exact_norm_grad, contiguous, inv_t, a0, a1, a2, lim, p, train);
 }
 
 // one token per (batch, head) against the carried state: q, k, v (b, h, d) or (b, h, 1, d); returns o shaped like q

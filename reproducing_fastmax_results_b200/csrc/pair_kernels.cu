@@ -27,6 +27,7 @@
 #include "launchers.cuh"
 #include "pair_launchers.cuh"
 #include "tc_launchers.cuh"
+#include "tc_phi.cuh"
 #include "tc_ptx.cuh"
 
 namespace fm {
@@ -54,6 +55,8 @@ struct Params {
   int nd_ld;
   int heads, nr, nx;          // held rows, streamed rows per head
   int off, causal;            // query l sees the keys up to l + off
+  int window;                 // 0, or (causal, off = 0): only the keys of the query's own window of this many tokens
+  int part_lo, part_hi;       // rows whose results are partial: float32 into `part` (Maps::p0, p1), not divided
   int ntiles;                 // items per head
   uint32_t mul_t, mul_h;      // quotients by ntiles and heads without a division: (n * mul) >> shift
   int sh_t, sh_h;
@@ -203,10 +206,16 @@ __device__ __forceinline__ Item decode(int idx, const Params& P) {
     const int first = it.r0 - P.off;                 // first query that sees key r0
     if (P.causal && first > 0) it.t0 = first / TILE;
     it.n0 = all - it.t0;
+    if (P.window) it.n0 = min(it.n0, (it.r0 / P.window + 1) * P.window / TILE - it.t0);
   } else {
     it.r0 = (P.ntiles - 1 - ti) * HELD;
     it.n0 = P.causal ? min(all, (it.r0 + R - 1 + P.off) / TILE + 1) : all;
     if (HELD > R && it.r0 + R < P.nr) it.n1 = P.causal ? min(all, (it.r0 + 2 * R - 1 + P.off) / TILE + 1) : all;
+    if (P.window) {   // (a multiple of the item: both tiles are in the same window)
+      it.t0 = it.r0 / P.window * (P.window / TILE);
+      it.n0 -= it.t0;
+      if (it.n1 > 0) it.n1 -= it.t0;
+    }
   }
   return it;
 }
@@ -215,6 +224,7 @@ struct Maps {
   CUtensorMap x, y;     // streamed tiles
   CUtensorMap a, b;     // held tiles
   CUtensorMap o0, o1;   // outputs, 32-row boxes
+  CUtensorMap p0, p1;   // partial results in float32, 32-row boxes of 32 columns, dense over all heads
 };
 
 template <int D, int KIND, bool SQ>
@@ -448,12 +458,34 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
       const bool first = first_rows(P, it.r0 + grp * R);
       const float w1 = first ? 1.f : P.w1;
       float wgt = second ? w1 : first ? 1.f : P.w0;
+      const bool partial = row - lane >= P.part_lo && row - lane < P.part_hi;   // (bounds are multiples of a window)
+      if (KIND == FWD && partial) wgt = w1;
+      else if (KIND == FWD) wgt = 1.f / total;   // the sum and the products carry the same factor
       if (KIND == FWD) {
-        wgt = 1.f / total;   // the sum and the products carry the same factor
         if (row < P.nr)
           reinterpret_cast<float*>(const_cast<void*>(P.out1.ptr))[(long long)it.b * P.out1.sb + (long long)it.h * P.out1.sh + (long long)row * P.out1.sn] = total * w1;
       }
-      if (second ? P.vec1 : P.vec0) {
+      if (partial) {
+        uint8_t* stage = sm + OFF_HELD + (n & 1) * STAGE + (KIND == FWD ? grp : half) * X_BYTES + quarter * 4096;
+#pragma unroll
+        for (int c = 0; c < (D < 32 ? 1 : D / 32); ++c) {
+          if (c > 0) {   // one box of space per warp
+            if (lane == 0) bulk_wait_read_all();
+            __syncwarp();
+          }
+#pragma unroll
+          for (int q = 0; q < CH / 4; ++q)
+            *reinterpret_cast<float4*>(stage + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+                make_float4(__uint_as_float(r[c][4 * q]) * wgt, __uint_as_float(r[c][4 * q + 1]) * wgt, __uint_as_float(r[c][4 * q + 2]) * wgt,
+                            __uint_as_float(r[c][4 * q + 3]) * wgt);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && row < P.nr) {
+            tma_store_4d(second ? &M.p1 : &M.p0, stage, 32 * c, row, it.head, 0);
+            bulk_commit_group();
+          }
+        }
+      } else if (second ? P.vec1 : P.vec0) {
         // rows -> the item's held set (its products are done), 128-byte swizzle -> the copy engine, which writes whole lines
         // and clips what lies outside; stored by the threads, 32 lines per instruction, this took 1200 to 3000 clocks
         uint8_t* stage = sm + OFF_HELD + (n & 1) * STAGE + (KIND == FWD ? grp : half) * X_BYTES + quarter * 4096;
@@ -678,11 +710,11 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
   if (w == W_ACC) tmem_dealloc(tmem, 512);
 }
 
-// dO' = dO / g in bf16 (dense [batch*heads][nq][D]) and -delta = -(dO . o) / g, rounded to bf16 as everywhere (zero from nq on).  D / 8 threads per row,
+// dO' = dO / g in bf16 (dense [batch*heads][nq][ld], ld = D or D + 16) and -delta = -(dO . o) / g, rounded to bf16 as everywhere (zero from nq on).  D / 8 threads per row,
 // 16-byte accesses (VEC) or element by element for views that do not allow them.
 template <int D, bool VEC>
 __global__ void __launch_bounds__(256) prologue_kernel(View dout, View o, View g, __nv_bfloat16* __restrict__ dop, float* __restrict__ ndelta,
-                                                       int nq, int nd_ld, int heads) {
+                                                       int nq, int nd_ld, int heads, int ld) {
   constexpr int TPR = D / 8;
   const int head = blockIdx.y, b = head / heads, h = head - b * heads;
   const int row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, c = (threadIdx.x % TPR) * 8;
@@ -711,7 +743,12 @@ __global__ void __launch_bounds__(256) prologue_kernel(View dout, View o, View g
   if (row < nq) {
     uint4 r;
     r.x = bf16x2(dv[0], dv[1]); r.y = bf16x2(dv[2], dv[3]); r.z = bf16x2(dv[4], dv[5]); r.w = bf16x2(dv[6], dv[7]);
-    *reinterpret_cast<uint4*>(dop + ((long long)head * nq + row) * D + c) = r;
+    __nv_bfloat16* out = dop + ((long long)head * nq + row) * ld;
+    *reinterpret_cast<uint4*>(out + c) = r;
+    if (c == 0 && ld > D) {   // rows of D + 16 columns: -delta and zeros behind the values
+      *reinterpret_cast<uint4*>(out + D) = make_uint4(bf16x2(-dot, 0.f), 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(out + D + 8) = make_uint4(0u, 0u, 0u, 0u);
+    }
   }
   if (c == 0 && row < nd_ld) ndelta[(long long)head * nd_ld + row] = row < nq ? __bfloat162float(__float2bfloat16(-dot)) : 0.f;
 }
@@ -719,6 +756,8 @@ __global__ void __launch_bounds__(256) prologue_kernel(View dout, View o, View g
 #include "pair_f32.cuh"
 
 }  // namespace pair
+
+#include "long_kernels.cuh"
 
 // ------------------------------------------------------------------------------------------------------
 // host side
@@ -778,16 +817,30 @@ bool mappable(const fastmax_tensor& t, const fastmax_problem* pb, int n) {
   return t.ptr && ((uintptr_t)t.ptr & 15) == 0 && ok(t.stride_n, n) && ok(t.stride_h, pb->heads) && ok(t.stride_b, pb->batch);
 }
 
-// The pairwise kernels cost pairs x ~2.1e-7 us forward and ~7e-7 us backward (d = 64; narrower heads are bound by the
-// element-wise warps and cost the same), the moment scans tokens x ~1.2e-3 and ~4e-3 us at order 2: equal where a query sees
-// about 6000 keys.  At order 1 the scans run over one feature tile of nineteen: 5e-4 and 1.1e-3 us per token, equal at 2000
-// and 1300; without a mask and with at least 64 heads the order-1 forward is one pass over the tensors and always cheaper.
-// Measured crossings (causal, B x H x N, bf16): order 2 d = 64 32 heads 12000 tokens 1.30x / 1.08x for the pairs, 16 heads
-// 16384 tokens 0.85x / 0.88x; order 1 128 heads 2048 tokens 1.33x / 1.10x, 4096 tokens 0.96x / 0.67x.
-bool chosen(const fastmax_problem* pb, bool backward) {
-  if (!(pb->flags & FASTMAX_FLAG_PAIRWISE) || (pb->flags & FASTMAX_FLAG_NO_TENSOR_CORES)) return false;
-  if (pb->nq <= 0 || pb->nk <= 0) return false;
-  if ((long long)tiles(pb->nq > pb->nk ? pb->nq : pb->nk) * pb->batch * pb->heads >= (1ll << 31)) return false;
+// Which form takes a call.  USE_OUT: output alone; USE_TRAIN: forward and backward of a training call (the states of the forward
+// are handed on, so both take the same form); USE_PROMPT: output and final state.
+enum Use { USE_OUT, USE_TRAIN, USE_PROMPT };
+// The pairwise kernels cost about 1e-6 us per visible pair forward and backward (d = 64; narrower heads are bound by the
+// element-wise warps and cost the same), windows and states a time per token.  `per_token`, the keys a token sees on average,
+// at which both cost the same, from measurements at 64 to 128 heads (us, forward + backward, pairs / windows):
+//   order 2, mask:    d = 64 6144 tokens 1117 / 1240, 8192 1952 / 1790; d = 32 2048 358 / 433, 4096 1094 / 832
+//   order 2, no mask: d = 64 2048 302 / 473, 4096 1006 / 758;           d = 32 1024 108 / 118, 2048 272 / 163
+//   order 1, mask:    d = 64 1024 180 / 219, 2048 457 / 430;            d = 32 2048 371 / 323
+//   order 1, no mask: d = 64 512 89 / 107, 2048 568 / 192;              d = 32 1024 168 / 109
+// The forward alone crosses later (order 2, mask, d = 64: 8192 424 / 576, 16384 919 / 645), with a state to be returned earlier.
+double window_line(const fastmax_problem* pb, Use use) {
+  const bool wide = pb->d == 64;
+  if (pb->order == 2) {
+    if (pb->causal) return use == USE_TRAIN ? (wide ? 3600. : 1500.) : use == USE_PROMPT ? (wide ? 2500. : 1150.) : (wide ? 5500. : 2150.);
+    return use == USE_TRAIN ? (wide ? 3100. : 1100.) : (wide ? 4600. : 1600.);
+  }
+  if (pb->causal) return use == USE_TRAIN ? (wide ? 900. : 800.) : use == USE_PROMPT ? 600. : (wide ? 1450. : 1300.);
+  return use == USE_TRAIN ? (wide ? 550. : 600.) : (wide ? 800. : 1100.);
+}
+int chosen(const fastmax_problem* pb, bool backward, Use use) {   // 0: neither, 1: pair by pair, 2: windows and states
+  if (!(pb->flags & FASTMAX_FLAG_PAIRWISE) || (pb->flags & FASTMAX_FLAG_NO_TENSOR_CORES)) return 0;
+  if (pb->nq <= 0 || pb->nk <= 0) return 0;
+  if ((long long)tiles(pb->nq > pb->nk ? pb->nq : pb->nk) * pb->batch * pb->heads >= (1ll << 31)) return 0;
   const double nq = pb->nq, nk = pb->nk;
   const double pairs = pb->causal ? nq * (nk - 0.5 * (nq - 1.0)) : nq * nk;
   const double per_token = pairs / (0.5 * (nq + nk));
@@ -799,11 +852,15 @@ bool chosen(const fastmax_problem* pb, bool backward) {
     const double most = pb->order == 2 ? (pb->d == 64 ? 16000.0 : pb->d == 32 ? 5000.0 : 2000.0)
                         : pb->causal   ? (pb->d == 64 ? 2300.0 : pb->d == 32 ? 1050.0 : 900.0)
                                        : (pb->d == 64 ? 1300.0 : pb->d == 32 ? 800.0 : 600.0);
-    return per_token <= most && f32_registers_ok();
+    return per_token <= most && f32_registers_ok() ? 1 : 0;
   }
-  if (pb->order == 2) return per_token <= 6500.0;
-  if (!backward && !pb->causal && pb->d == 64 && (long long)pb->batch * pb->heads >= 64) return false;
-  return per_token <= (backward ? 1300.0 : 2000.0);
+  // order 1 without a mask: one pass over the tensors (p1_forward_kernel), always the cheapest where it fills the GPU
+  if (!backward && pb->order == 1 && !pb->causal && pb->d == 64 && (long long)pb->batch * pb->heads >= 64) return 0;
+  if (pb->d == 16) return per_token <= (pb->order == 2 ? 6500.0 : backward ? 1300.0 : 2000.0) ? 1 : 0;   // no states kernel
+  if (per_token <= window_line(pb, use)) return 1;
+  if (pb->causal && pb->nq != pb->nk) return per_token <= (pb->order == 2 ? 6500.0 : backward ? 1300.0 : 2000.0) ? 1 : 0;
+  if ((long long)(pb->nq > pb->nk ? pb->nq : pb->nk) >= (1ll << 30)) return 0;
+  return 2;
 }
 uint32_t bf16_bits(float x) {
   const __nv_bfloat16 v = __float2bfloat16(x);
@@ -840,22 +897,36 @@ bool fill(const fastmax_problem* pb, pair::Params& P) {
 
 }  // namespace
 
-bool pair_takes_forward(const fastmax_problem* pb, const fastmax_forward_args* a) {
-  return chosen(pb, false) && a->o.ptr && a->g.ptr && !a->state_in && !a->state_out && mappable(a->q, pb, pb->nq) &&
-         mappable(a->k, pb, pb->nk) && mappable(a->v, pb, pb->nk);
+static int forward_form(const fastmax_problem* pb, const fastmax_forward_args* a) {
+  if (!a->o.ptr || !a->g.ptr || a->state_in) return 0;
+  const Use use = a->state_out ? USE_PROMPT : a->key_moments_out || a->key_moments_in ? USE_TRAIN : USE_OUT;
+  const int form = chosen(pb, false, use);
+  if (form == 0 || !mappable(a->q, pb, pb->nq) || !mappable(a->k, pb, pb->nk) || !mappable(a->v, pb, pb->nk)) return 0;
+  if (form == 2) return rows16(a->o) && mappable(a->o, pb, pb->nq) && (!a->state_out || pb->causal) ? 2 : 0;
+  return a->state_out ? 0 : 1;
 }
-bool pair_takes_backward(const fastmax_problem* pb, const fastmax_backward_args* a) {
-  return chosen(pb, true) && a->dq.ptr && a->dk.ptr && a->dv.ptr && !a->state_in && !a->dstate_in && !a->dstate_out &&
-         mappable(a->q, pb, pb->nq) && mappable(a->k, pb, pb->nk) && mappable(a->v, pb, pb->nk);
+static int backward_form(const fastmax_problem* pb, const fastmax_backward_args* a) {
+  if (!a->dq.ptr || !a->dk.ptr || !a->dv.ptr || a->state_in || a->dstate_in || a->dstate_out) return 0;
+  const int form = chosen(pb, true, USE_TRAIN);
+  if (form == 0 || !mappable(a->q, pb, pb->nq) || !mappable(a->k, pb, pb->nk) || !mappable(a->v, pb, pb->nk)) return 0;
+  if (form == 2)
+    return rows16(a->dq) && rows16(a->dk) && rows16(a->dv) && mappable(a->dq, pb, pb->nq) && mappable(a->dk, pb, pb->nk) && mappable(a->dv, pb, pb->nk) ? 2 : 0;
+  return 1;
 }
+bool pair_takes_forward(const fastmax_problem* pb, const fastmax_forward_args* a) { return forward_form(pb, a) != 0; }
+bool pair_takes_backward(const fastmax_problem* pb, const fastmax_backward_args* a) { return backward_form(pb, a) != 0; }
 
 // ---- float32 ------------------------------------------------------------------------------------------------------------
 // bf16 pieces [3][batch*heads][n][d] as a tensor map: piece = batch index, head = batch*heads
 static size_t pieces_bytes(const fastmax_problem* pb, int n) { return up256((size_t)3 * pb->batch * pb->heads * n * pb->d * 2); }
-size_t pair_forward_workspace(const fastmax_problem* pb) {
-  return pb->dtype == FASTMAX_F32 ? pieces_bytes(pb, pb->nq) + 2 * pieces_bytes(pb, pb->nk) : 0;
+static size_t long_forward_workspace(const fastmax_problem* pb);
+static size_t long_backward_workspace(const fastmax_problem* pb);
+size_t pair_forward_workspace(const fastmax_problem* pb, const fastmax_forward_args* a) {
+  if (pb->dtype == FASTMAX_F32) return pieces_bytes(pb, pb->nq) + 2 * pieces_bytes(pb, pb->nk);
+  return forward_form(pb, a) == 2 ? long_forward_workspace(pb) : 0;
 }
-size_t pair_backward_workspace(const fastmax_problem* pb) {
+size_t pair_backward_workspace(const fastmax_problem* pb, const fastmax_backward_args* a) {
+  if (pb->dtype != FASTMAX_F32 && backward_form(pb, a) == 2) return long_backward_workspace(pb);
   if (pb->dtype == FASTMAX_F32)
     return 2 * pieces_bytes(pb, pb->nq) + 2 * pieces_bytes(pb, pb->nk) + up256((size_t)pb->batch * pb->heads * nd_ld(pb->nq) * sizeof(float));
   const size_t bh = (size_t)pb->batch * pb->heads;
@@ -1009,8 +1080,272 @@ static int out_map(CUtensorMap* m, const fastmax_tensor& t, const fastmax_proble
   return rows16(t) && tc_make_map(m, t, pb->batch, pb->heads, n, 64, 32, true, pb->d) ? 1 : 0;
 }
 
+template <int D>
+static void launch_prologue(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
+  const int ld = nd_ld(pb->nq), rows = 256 / (D / 8);
+  const dim3 grid((unsigned)((ld + rows - 1) / rows), (unsigned)(pb->batch * pb->heads));
+  if (rows16(a->o) && rows16(a->d_out))
+    pair::prologue_kernel<D, true><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+  else
+    pair::prologue_kernel<D, false><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+}
+static void launch_prologue_any(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
+  LaunchScope ls(KK_PROLOGUE, st, pb->d < 64 ? KK_TC_PAD : -1);
+  switch (pb->d) {
+    case 16: launch_prologue<16>(pb, a, dop, nd, dld, st); break;
+    case 32: launch_prologue<32>(pb, a, dop, nd, dld, st); break;
+    default: launch_prologue<64>(pb, a, dop, nd, dld, st); break;
+  }
+}
+
+// ---- long bf16 sequences (long_kernels.cuh) -----------------------------------------------------------------------------
+namespace {
+
+// Window of the pairwise part: its cost grows with the window, what a state costs (written, packed, read: 1 us per head at
+// d = 64, order 2) does not.
+int long_window(const fastmax_problem* pb) {
+  return pb->order == 1 ? 512 : pb->d == 64 ? 1536 : 768;
+}
+struct LongGeo {
+  int L, ns;         // window, states per head (segments before the last, or after the first)
+  int rows;          // state rows
+  size_t raw, packed, cst;
+};
+LongGeo long_geo(const fastmax_problem* pb) {
+  LongGeo g;
+  const size_t bh = (size_t)pb->batch * pb->heads;
+  const int nb = pb->d / 8, npair = nb * (nb + 1) / 2;
+  g.L = pb->causal ? long_window(pb) : 0;
+  g.ns = pb->causal ? (pb->nk + g.L - 1) / g.L - 1 : 1;
+  g.rows = (pb->order == 2 ? 64 * npair : 0) + pb->d + 1;
+  g.raw = up256(bh * (g.ns + 1) * g.rows * (pb->d + 4) * sizeof(float));   // (+ 1: a prompt's last segment)
+  g.packed = up256(bh * g.ns * (npair + 1) * (size_t)(pb->d / 8 + 2) * 1024);
+  g.cst = up256(bh * g.ns * (pb->d + 8) * sizeof(float));
+  return g;
+}
+fastmax_tensor after(const fastmax_tensor& t, int tokens, int es) {
+  fastmax_tensor r = t;
+  r.ptr = (char*)t.ptr + (int64_t)tokens * t.stride_n * es;
+  return r;
+}
+bool f32_map(CUtensorMap* m, float* p, const fastmax_problem* pb, int n, int rows) {
+  const int64_t bh = (int64_t)pb->batch * pb->heads;
+  return tc_make_map(m, fastmax_tensor{p, bh * n * pb->d, (int64_t)n * pb->d, pb->d}, 1, (int)bh, n, 32, rows, true, pb->d, true);
+}
+void launch_pack(const fastmax_problem* pb, const LongGeo& g, const float* raw, uint8_t* S, float* cst, bool reverse, float* total, cudaStream_t st) {
+  const float c0 = pb->a0, c1 = pb->a1 * pb->inv_temperature, c2 = pb->order == 2 ? pb->a2 * pb->inv_temperature * pb->inv_temperature : 0.f;
+  const int nb = pb->d / 8, units = (pb->order == 2 ? nb * (nb + 1) / 2 : 0) + 1;
+  const dim3 grid((unsigned)units, (unsigned)(pb->batch * pb->heads));
+  LaunchScope ls(KK_STATE_SCAN, st);
+  if (pb->d == 64) lng::pack_kernel<64><<<grid, 640, 0, st>>>(raw, S, cst, g.ns, reverse, pb->order, c0, c1, c2, total);
+  else lng::pack_kernel<32><<<grid, 384, 0, st>>>(raw, S, cst, g.ns, reverse, pb->order, c0, c1, c2, total);
+}
+int sm_total() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    cached[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+template <typename K>
+cudaError_t launch_items(K kernel, std::atomic<bool>* done, int bytes, int threads, const lng::Maps& M, const lng::Params& P, int kind, cudaStream_t st) {
+  if (P.nitems <= 0) return cudaSuccess;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64 || !done[dev].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+  }
+  const int sms = sm_total();
+  LaunchScope ls(kind, st);
+  kernel<<<dim3((unsigned)(P.nitems < sms ? P.nitems : sms)), threads, bytes, st>>>(M, P);
+  return cudaGetLastError();
+}
+template <int D, bool FWD>
+cudaError_t launch_apply(const lng::Maps& M, const lng::Params& P, int kind, cudaStream_t st) {
+  static std::atomic<bool> done[64];
+  return launch_items(lng::ap::apply_kernel<D, FWD>, done, lng::ap::Lay<D>::BYTES, lng::ap::THREADS, M, P, kind, st);
+}
+template <int D, bool DK>
+cudaError_t launch_chain(const lng::Maps& M, const lng::Params& P, int kind, cudaStream_t st) {
+  static std::atomic<bool> done[64];
+  return launch_items(lng::ch::chain_kernel<D, DK>, done, lng::ch::Lay<D>::BYTES, lng::ch::THREADS, M, P, kind, st);
+}
+// tokens [row0, end) of n, state of token r: (r - row0) / L
+lng::Params long_params(const fastmax_problem* pb, const LongGeo& g, const uint8_t* S, int n, int row0, int end) {
+  lng::Params P{};
+  const int nb = pb->d / 8;
+  P.S = S;
+  P.cst = (const float*)(S + g.packed);
+  P.heads = pb->heads;
+  P.n = end;
+  P.row0 = row0;
+  P.seg = g.L > 0 ? g.L : (n + lng::ROWS) / lng::ROWS * lng::ROWS;
+  P.ns = g.ns;
+  P.items_per_head = (end - row0 + lng::ROWS - 1) / lng::ROWS;
+  P.nitems = P.items_per_head * pb->batch * pb->heads;
+  P.u0 = pb->order == 2 ? 0 : nb * (nb + 1) / 2;
+  P.part = pb->causal ? 1 : 0;
+  P.w1 = 1.f;
+  return P;
+}
+
+}  // namespace
+
+static size_t long_forward_workspace(const fastmax_problem* pb) {
+  const LongGeo g = long_geo(pb);
+  return g.raw + g.packed + g.cst + up256(tc_moments_scratch(pb, pb->nk)) +
+         (pb->causal ? up256((size_t)pb->batch * pb->heads * pb->nq * pb->d * sizeof(float)) : 0);
+}
+static size_t long_backward_workspace(const fastmax_problem* pb) {
+  const LongGeo g = long_geo(pb);
+  const size_t bh = (size_t)pb->batch * pb->heads;
+  const int n = pb->nq > pb->nk ? pb->nq : pb->nk;
+  return g.raw + 2 * (g.packed + g.cst) + up256(tc_moments_scratch(pb, n)) + up256(bh * pb->nq * (pb->d + 16) * 2) +
+         up256(bh * nd_ld(pb->nq) * sizeof(float)) + (pb->causal ? 3 * up256(bh * pb->nq * pb->d * sizeof(float)) : 0);
+}
+size_t pair_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_args* a) {
+  fastmax_forward_args train = *a;   // who asks is about to hand them on
+  train.key_moments_out = (float*)a->q.ptr;
+  return pb->dtype != FASTMAX_F32 && forward_form(pb, &train) == 2 ? long_geo(pb).packed + long_geo(pb).cst : 0;
+}
+
+// Packed states of the keys before every segment but the first (no mask: of all keys): S, then the constant rows behind it
+static cudaError_t long_key_states(const fastmax_problem* pb, const LongGeo& g, const fastmax_tensor& k, const fastmax_tensor& v, float* raw, void* xt,
+                                   uint8_t* S, float* total, cudaStream_t st) {
+  const cudaError_t e = tc_moments(pb, k, v, pb->causal && !total ? g.ns * g.L : pb->nk, false, g.L, nullptr, raw, xt, KK_TC_MOMENTS, st);
+  if (e != cudaSuccess) return e;
+  launch_pack(pb, g, raw, S, (float*)(S + g.packed), false, total, st);
+  return cudaGetLastError();
+}
+
+static int long_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st) {
+  const LongGeo g = long_geo(pb);
+  const int bh = pb->batch * pb->heads;
+  char* base = (char*)ws;
+  float* raw = (float*)base; base += g.raw;
+  uint8_t* S = a->key_moments_in ? (uint8_t*)const_cast<float*>(a->key_moments_in) : a->key_moments_out ? (uint8_t*)a->key_moments_out : (uint8_t*)base;
+  base += g.packed + g.cst;
+  void* xt = base; base += up256(tc_moments_scratch(pb, pb->nk));
+  float* part = (float*)base;
+  pair::Maps M;
+  lng::Maps A;
+  if (!tc_make_map(&M.a, a->q, pb->batch, pb->heads, pb->nq, 64, pair::R, true, pb->d) ||
+      !tc_make_map(&M.x, a->k, pb->batch, pb->heads, pb->nk, 64, pair::T, true, pb->d) ||
+      !tc_make_map(&M.y, a->v, pb->batch, pb->heads, pb->nk, 64, pair::T, true, pb->d) || !out_map(&M.o0, a->o, pb, pb->nq))
+    return FASTMAX_ERR_UNSUPPORTED;
+  M.b = M.o1 = M.p0 = M.p1 = M.a;
+  A.x = A.y = A.part = M.a;
+  A.out = M.o0;
+  cudaError_t e = cudaSuccess;
+  if (pb->causal) {
+    if (!f32_map(&M.p0, part, pb, pb->nq, 32) || !f32_map(&A.part, part, pb, pb->nq, 128)) return FASTMAX_ERR_UNSUPPORTED;
+    pair::Params P{};
+    const bool sq = fill(pb, P);
+    P.window = g.L;
+    P.part_lo = g.L;
+    P.part_hi = 1 << 30;
+    P.out0 = view_of(a->o);
+    P.out1 = view_of(a->g);
+    P.nr = P.nx = pb->nq;
+    P.ntiles = tiles(pb->nq, 2 * pair::R);
+    P.vec0 = 1;
+    if (sq) P.w1 = P.c2;
+    LaunchScope ls(KK_TC_INTRA_FWD, st);
+    e = sq ? launch_d<pair::FWD, true>(pb->d, M, P, bh, st) : launch_d<pair::FWD, false>(pb->d, M, P, bh, st);
+  }
+  if (e == cudaSuccess && (!a->key_moments_in || a->state_out)) e = long_key_states(pb, g, a->k, a->v, raw, xt, S, a->state_out, st);
+  lng::Params P = long_params(pb, g, S, pb->nq, g.L, pb->nq);
+  P.g = view_of(a->g);
+  if (e == cudaSuccess) e = pb->d == 64 ? launch_apply<64, true>(A, P, KK_TC_FWD, st) : launch_apply<32, true>(A, P, KK_TC_FWD, st);
+  return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
+}
+
+static int long_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
+  const LongGeo g = long_geo(pb);
+  const int bh = pb->batch * pb->heads, d = pb->d, ld = d + 16;
+  char* base = (char*)ws;
+  float* raw = (float*)base; base += g.raw;
+  uint8_t* S = a->key_moments_in ? (uint8_t*)const_cast<float*>(a->key_moments_in) : (uint8_t*)base; base += g.packed + g.cst;
+  uint8_t* dS = (uint8_t*)base; base += g.packed + g.cst;
+  void* xt = base; base += up256(tc_moments_scratch(pb, pb->nq > pb->nk ? pb->nq : pb->nk));
+  __nv_bfloat16* dop = (__nv_bfloat16*)base; base += up256((size_t)bh * pb->nq * ld * 2);
+  float* nd = (float*)base; base += up256((size_t)bh * nd_ld(pb->nq) * sizeof(float));
+  const size_t pbytes = up256((size_t)bh * pb->nq * d * sizeof(float));
+  float *pq = (float*)base, *pk = (float*)(base + pbytes), *pv = (float*)(base + 2 * pbytes);
+  const fastmax_tensor dflat{dop, (int64_t)bh * pb->nq * ld, (int64_t)pb->nq * ld, ld};                   // one batch of bh heads
+  const fastmax_tensor dhead{dop, (int64_t)pb->heads * pb->nq * ld, (int64_t)pb->nq * ld, ld};
+  pair::Maps M, N;   // M: dq, N: dk and dv
+  if (!tc_make_map(&M.x, a->k, pb->batch, pb->heads, pb->nk, 64, pair::T, true, d) ||
+      !tc_make_map(&M.y, a->v, pb->batch, pb->heads, pb->nk, 64, pair::T, true, d) ||
+      !tc_make_map(&M.a, a->q, pb->batch, pb->heads, pb->nq, 64, pair::R, true, d) ||
+      !tc_make_map(&M.b, dflat, 1, bh, pb->nq, 64, pair::R, true, d) || !out_map(&M.o0, a->dq, pb, pb->nq) || !out_map(&N.o0, a->dk, pb, pb->nk) ||
+      !out_map(&N.o1, a->dv, pb, pb->nk))
+    return FASTMAX_ERR_UNSUPPORTED;
+  N.x = M.a; N.y = M.b; N.a = M.x; N.b = M.y;
+  M.o1 = M.o0;
+  M.p0 = M.p1 = N.p0 = N.p1 = M.a;
+  lng::Maps Q, K, V;   // dq, dk, dv
+  Q.x = M.a; Q.y = M.b; Q.out = M.o0; Q.part = M.a;
+  K.x = M.x; K.y = M.y; K.out = N.o0; K.part = M.a;
+  V.x = M.x; V.y = M.x; V.out = N.o1; V.part = M.a;
+  if (pb->causal && (!f32_map(&M.p0, pq, pb, pb->nq, 32) || !f32_map(&N.p0, pk, pb, pb->nk, 32) || !f32_map(&N.p1, pv, pb, pb->nk, 32) ||
+                     !f32_map(&Q.part, pq, pb, pb->nq, 128) || !f32_map(&K.part, pk, pb, pb->nk, 128) || !f32_map(&V.part, pv, pb, pb->nk, 128)))
+    return FASTMAX_ERR_UNSUPPORTED;
+  launch_prologue_any(pb, a, dop, nd, ld, st);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return report_cuda_error(e);
+  if (pb->causal) {
+    pair::Params P{};
+    const bool sq = fill(pb, P);
+    P.window = g.L;
+    P.ndelta = nd;
+    P.nd_ld = nd_ld(pb->nq);
+    P.nr = P.nx = pb->nq;
+    P.ntiles = tiles(pb->nq);
+    P.vec0 = P.vec1 = 1;
+    pair::Params B = P;
+    B.part_lo = 0;
+    B.part_hi = g.ns * g.L;   // the last window's keys have no later queries
+    B.out0 = view_of(a->dk);
+    B.out1 = view_of(a->dv);
+    if (sq) { B.w0 = 2.f * B.c2; B.w1 = B.c2; P.w0 = 2.f * P.c2; }
+    {
+      LaunchScope ls(KK_TC_INTRA_BWD, st);
+      e = sq ? launch_d<pair::DKV, true>(d, N, B, bh, st) : launch_d<pair::DKV, false>(d, N, B, bh, st);
+    }
+    P.part_lo = g.L;
+    P.part_hi = 1 << 30;
+    P.out0 = P.out1 = view_of(a->dq);
+    LaunchScope ls(KK_TC_INTRA_BWD, st);
+    if (e == cudaSuccess) e = sq ? launch_d<pair::DQ, true>(d, M, P, bh, st) : launch_d<pair::DQ, false>(d, M, P, bh, st);
+  }
+  if (e == cudaSuccess && !a->key_moments_in) e = long_key_states(pb, g, a->k, a->v, raw, xt, S, nullptr, st);
+  if (e != cudaSuccess) return report_cuda_error(e);
+  // gradient moments of every segment but the first (no mask: of all queries); raw may be reused: the stream orders it
+  e = tc_moments(pb, after(a->q, g.L, 2), after(dhead, g.L, 2), pb->nq - g.L, true, g.L, nullptr, raw, xt, KK_TC_MOMENTS, st);
+  if (e != cudaSuccess) return report_cuda_error(e);
+  launch_pack(pb, g, raw, dS, (float*)(dS + g.packed), true, nullptr, st);
+  e = cudaGetLastError();
+  lng::Params P = long_params(pb, g, S, pb->nq, g.L, pb->nq);
+  P.ndelta = nd;
+  P.nd_ld = nd_ld(pb->nq);
+  if (e == cudaSuccess) e = d == 64 ? launch_chain<64, false>(Q, P, KK_TC_BWD_Q, st) : launch_chain<32, false>(Q, P, KK_TC_BWD_Q, st);
+  P = long_params(pb, g, dS, pb->nk, 0, pb->causal ? g.ns * g.L : pb->nk);
+  if (e == cudaSuccess) e = d == 64 ? launch_chain<64, true>(K, P, KK_TC_BWD_KV, st) : launch_chain<32, true>(K, P, KK_TC_BWD_KV, st);
+  if (e == cudaSuccess) e = d == 64 ? launch_apply<64, false>(V, P, KK_TC_BWD_DV, st) : launch_apply<32, false>(V, P, KK_TC_BWD_DV, st);
+  return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
+}
+
 int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st) {
   if (pb->dtype == FASTMAX_F32) return pair_f32_forward(pb, a, ws, st);
+  if (forward_form(pb, a) == 2) return long_forward(pb, a, ws, st);
   pair::Maps M;
   if (!tc_make_map(&M.a, a->q, pb->batch, pb->heads, pb->nq, 64, pair::R, true, pb->d) ||
       !tc_make_map(&M.x, a->k, pb->batch, pb->heads, pb->nk, 64, pair::T, true, pb->d) ||
@@ -1032,18 +1367,9 @@ int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void*
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
 
-template <int D>
-static void launch_prologue(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, cudaStream_t st) {
-  const int ld = nd_ld(pb->nq), rows = 256 / (D / 8);
-  const dim3 grid((unsigned)((ld + rows - 1) / rows), (unsigned)(pb->batch * pb->heads));
-  if (rows16(a->o) && rows16(a->d_out))
-    pair::prologue_kernel<D, true><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads);
-  else
-    pair::prologue_kernel<D, false><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads);
-}
-
 int pair_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
   if (pb->dtype == FASTMAX_F32) return pair_f32_backward(pb, a, ws, st);
+  if (backward_form(pb, a) == 2) return long_backward(pb, a, ws, st);
   const int bh = pb->batch * pb->heads;
   __nv_bfloat16* dop = (__nv_bfloat16*)ws;
   float* nd = (float*)((char*)ws + up256((size_t)bh * pb->nq * pb->d * 2));
@@ -1057,14 +1383,7 @@ int pair_backward(const fastmax_problem* pb, const fastmax_backward_args* a, voi
   M.o0 = M.o1 = M.a;
   pair::Maps N;   // dk, dv: the other way round (held and streamed tiles have the same 128-row box)
   N.x = M.a; N.y = M.b; N.a = M.x; N.b = M.y; N.o0 = N.o1 = M.a;
-  {
-    LaunchScope ls(KK_PROLOGUE, st, pb->d < 64 ? KK_TC_PAD : -1);
-    switch (pb->d) {
-      case 16: launch_prologue<16>(pb, a, dop, nd, st); break;
-      case 32: launch_prologue<32>(pb, a, dop, nd, st); break;
-      default: launch_prologue<64>(pb, a, dop, nd, st); break;
-    }
-  }
+  launch_prologue_any(pb, a, dop, nd, pb->d, st);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return report_cuda_error(e);
   pair::Params P{};

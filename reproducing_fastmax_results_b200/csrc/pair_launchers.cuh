@@ -9,8 +9,10 @@ namespace fm {
 // Whether the pairwise kernels take the call: allowed by the caller, the cheaper form, and in a layout the copy engine reads.
 bool pair_takes_forward(const fastmax_problem* pb, const fastmax_forward_args* a);
 bool pair_takes_backward(const fastmax_problem* pb, const fastmax_backward_args* a);
-size_t pair_forward_workspace(const fastmax_problem* pb);
-size_t pair_backward_workspace(const fastmax_problem* pb);
+// Bytes of the moment arrays a call on long sequences hands from forward to backward (0: none)
+size_t pair_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_args* a);
+size_t pair_forward_workspace(const fastmax_problem* pb, const fastmax_forward_args* a);
+size_t pair_backward_workspace(const fastmax_problem* pb, const fastmax_backward_args* a);
 int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st);
 int pair_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st);
 // Device-side error word and per-wait-site give-up counters (see tc_device_status / tc_wait_histogram, which include them).

@@ -1,0 +1,84 @@
+"""Long bf16 sequences as windows of pairs plus moment states (FASTMAX_FLAG_PAIRWISE beyond the lengths the pairwise form is
+cheaper for), against the CPU oracle's sampled rows and columns: ragged last windows, a last window of one token, no mask,
+order 1, head-split views, the states handed from forward to backward or built again, the final state of a prompt."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import fastmax_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def host(t):
+    return t.detach().double().cpu().numpy()
+
+
+CASES = [  # B, H, nq, nk, D, causal, order
+    (1, 2, 7681, 7681, 64, True, 2),   # five windows of 1536 and one token
+    (2, 2, 8000, 8000, 64, True, 2),
+    (1, 3, 3840, 3840, 32, True, 2),   # five whole windows
+    (2, 1, 4001, 4001, 32, True, 2),
+    (1, 2, 5000, 4700, 64, False, 2),
+    (1, 2, 1400, 9000, 32, False, 2),
+    (1, 2, 2305, 2305, 64, True, 1),
+    (1, 2, 1700, 900, 32, False, 1),
+]
+
+
+@pytest.mark.parametrize("hand_over", [True, False])
+@pytest.mark.parametrize("case", CASES)
+def test_windows_match_oracle(case, hand_over):
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    B, H, nq, nk, D, causal, order = case
+    g = torch.Generator(device="cuda").manual_seed(nq + nk + D)
+    mk = lambda n: torch.randn(B, n, H, D, device="cuda", generator=g).bfloat16().transpose(1, 2)
+    q, do, k, v = mk(nq), mk(nq), mk(nk), mk(nk)
+    p = orc.Poly(0.9, 1.1, 0.45, 1.0 / (8.0 * math.sqrt(D)), order)
+    args = (causal, p.inv_temp, p.a0, p.a1, p.a2, order)
+    km = L.KeyMoments()
+    L.profile_collect()
+    L.profile(True)
+    o, gg, _ = L.forward(q, k, v, *args, flags=L.FLAG_PAIRWISE, key_moments=km)
+    assert km.buf is not None
+    dq, dk, dv, _ = L.backward(q, k, v, o, gg, do, *args, flags=L.FLAG_PAIRWISE, key_moments=km if hand_over else None)
+    L.check_status()
+    L.profile(False)
+    assert L.profile_collect()["tc_moments"][1] == (2 if hand_over else 3)
+    assert L.wait_histogram() == {}
+    rng = np.random.default_rng(nq)
+    for b, h in {(0, 0), (B - 1, H - 1)}:
+        a = [host(t[b, h]) for t in (q, k, v, do)]
+        oh, gh = host(o[b, h]), host(gg[b, h])
+        win = [w for w in (127, 511, 512, 767, 768, 1535, 1536, 3071, 3072) if w < min(nq, nk)]
+        rq = np.unique(np.concatenate([win, [nq - 1], rng.integers(64, nq, 24)]))
+        rk = np.unique(np.concatenate([win, [nk - 1], rng.integers(64, nk, 24)]))
+        o_ref, g_ref = orc.sampled_forward_rows(a[0], a[1], a[2], rq, causal, p)
+        assert orc.max_norm_err(oh[rq], o_ref) < 2e-2 and orc.max_norm_err(gh[rq], g_ref) < 1e-3
+        dq_ref = orc.sampled_dq_rows(a[0], a[1], a[2], oh, gh, a[3], rq, causal, p)
+        dk_ref, dv_ref = orc.sampled_dkv_cols(a[0], a[1], a[2], oh, gh, a[3], rk, causal, p)
+        for name, x, ref, rows in (("dq", dq, dq_ref, rq), ("dk", dk, dk_ref, rk), ("dv", dv, dv_ref, rk)):
+            err = np.linalg.norm(host(x[b, h])[rows] - ref) / np.linalg.norm(ref)
+            assert err < 2e-2, (name, b, h, err)
+
+
+@pytest.mark.parametrize("D,N", [(64, 5200), (32, 2500)])
+def test_prompt_of_windows_returns_its_state(D, N):
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    g = torch.Generator(device="cuda").manual_seed(N)
+    q, k, v = (torch.randn(1, 20, N, D, device="cuda", generator=g).bfloat16() for _ in range(3))
+    L.profile_collect()
+    L.profile(True)
+    o, gg, state = L.forward(q, k, v, True, 0.02, order=2, want_state=True, flags=L.FLAG_PAIRWISE)
+    L.check_status()
+    L.profile(False)
+    assert L.profile_collect()["tc_moments"][1] == 1
+    o2, g2, state2 = L.forward(q, k, v, True, 0.02, order=2, want_state=True, flags=L.FLAG_NO_TENSOR_CORES)
+    torch.cuda.synchronize()
+    for a, b, tol in ((o, o2, 2e-2), (gg, g2, 1e-3), (state, state2, 5e-3)):
+        assert orc.max_norm_err(host(a), host(b)) < tol
+    assert float(state[..., D + 1:].abs().max()) == 0.0
