@@ -670,4 +670,6 @@ __global__ void __launch_bounds__(64 * (D / 8 + 2)) pack_kernel(const float* __r
   }
 }
 
+#include "long_f32.cuh"
+
 }  // namespace lng

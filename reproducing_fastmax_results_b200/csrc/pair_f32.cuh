@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
             named_bar_sync(1 + quarter, 64);
             const float g = sums[quarter * 32 + lane] + sums[R + quarter * 32 + lane];
             named_bar_sync(1 + quarter, 64);
-            wgt = 1.f / g;
+            wgt = it.r0 >= P.part_lo && it.r0 < P.part_hi ? 1.f : 1.f / g;   // partial rows: not divided yet
             if (half == 0 && row < P.nr)
               reinterpret_cast<float*>(const_cast<void*>(P.out1.ptr))[(long long)it.b * P.out1.sb + (long long)it.h * P.out1.sh + (long long)row * P.out1.sn] = g;
           }
@@ -452,11 +452,12 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
   if (w == W_ACC) tmem_dealloc(tmem, 512);
 }
 
-// Splits float32 views into bf16 pieces: out[piece][batch*heads][n][D].  A thread takes eight columns; blockIdx.z picks the tensor.
+// Splits float32 views into bf16 pieces: out[piece][batch*heads][n][ld], ld = D, or D + 16: [values, 1, 0 ...].  A thread takes
+// eight columns; blockIdx.z picks the tensor.
 struct SplitArgs {
   View x[3];
   __nv_bfloat16* out[3];
-  int n[3];
+  int n[3], ld[3];
 };
 __device__ __forceinline__ void store_pieces(__nv_bfloat16* out, long long plane, long long at, const float (&v)[8]) {
   uint32_t r[3][4];
@@ -464,6 +465,17 @@ __device__ __forceinline__ void store_pieces(__nv_bfloat16* out, long long plane
   for (int i = 0; i < 4; ++i) split3(pack2(v[2 * i], v[2 * i + 1]), r[0][i], r[1][i], r[2][i]);
 #pragma unroll
   for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(out + p * plane + at) = make_uint4(r[p][0], r[p][1], r[p][2], r[p][3]);
+}
+// the sixteen columns behind the values: x, then zeros
+__device__ __forceinline__ void store_tail(__nv_bfloat16* out, long long plane, long long at, float x) {
+  uint32_t r[3];
+  split3(pack2(x, 0.f), r[0], r[1], r[2]);
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    uint4* t = reinterpret_cast<uint4*>(out + p * plane + at);
+    t[0] = make_uint4(r[p], 0u, 0u, 0u);
+    t[1] = make_uint4(0u, 0u, 0u, 0u);
+  }
 }
 template <int D>
 __global__ void __launch_bounds__(256) split_kernel(const SplitArgs A, int heads) {
@@ -475,13 +487,16 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitArgs A, int heads
                                                     (long long)row * A.x[t].sn + c);
   const float4 u = p[0], w = p[1];
   const float v[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
-  store_pieces(A.out[t], (long long)gridDim.y * A.n[t] * D, ((long long)head * A.n[t] + row) * D + c, v);
+  const int ld = A.ld[t];
+  const long long plane = (long long)gridDim.y * A.n[t] * ld, at = ((long long)head * A.n[t] + row) * ld;
+  store_pieces(A.out[t], plane, at + c, v);
+  if (c == 0 && ld > D) store_tail(A.out[t], plane, at + D, 1.f);
 }
 
-// dO' = dO / g in pieces and -delta = -(dO . o) / g
+// dO' = dO / g in pieces (ld = D + 16: with -delta behind the values) and -delta = -(dO . o) / g
 template <int D, bool VEC>
 __global__ void __launch_bounds__(256) prologue_f32_kernel(View dout, View o, View g, __nv_bfloat16* __restrict__ dop, float* __restrict__ ndelta,
-                                                           int nq, int nd_ld, int heads) {
+                                                           int nq, int nd_ld, int heads, int ld) {
   constexpr int TPR = D / 8;
   const int head = blockIdx.y, b = head / heads, h = head - b * heads;
   const int row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, c = (threadIdx.x % TPR) * 8;
@@ -508,7 +523,11 @@ __global__ void __launch_bounds__(256) prologue_f32_kernel(View dout, View o, Vi
   }
 #pragma unroll
   for (int m = TPR / 2; m > 0; m >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, m);
-  if (row < nq) store_pieces(dop, (long long)gridDim.y * nq * D, ((long long)head * nq + row) * D + c, v);
+  if (row < nq) {
+    const long long plane = (long long)gridDim.y * nq * ld, at = ((long long)head * nq + row) * ld;
+    store_pieces(dop, plane, at + c, v);
+    if (c == 0 && ld > D) store_tail(dop, plane, at + D, -dot);
+  }
   if (c == 0 && row < nd_ld) ndelta[(long long)head * nd_ld + row] = row < nq ? -dot : 0.f;
 }
 

@@ -817,6 +817,12 @@ bool mappable(const fastmax_tensor& t, const fastmax_problem* pb, int n) {
   return t.ptr && ((uintptr_t)t.ptr & 15) == 0 && ok(t.stride_n, n) && ok(t.stride_h, pb->heads) && ok(t.stride_b, pb->batch);
 }
 
+// rows of a float32 view as the copy engine reads and writes them
+bool rows_f32(const fastmax_tensor& t, const fastmax_problem* pb, int n) {
+  const int64_t big = (int64_t)1 << 38;
+  auto ok = [&](int64_t s, int extent) { return extent == 1 || (s > 0 && s < big && (s & 3) == 0); };
+  return t.ptr && ((uintptr_t)t.ptr & 15) == 0 && ok(t.stride_n, n) && ok(t.stride_h, pb->heads) && ok(t.stride_b, pb->batch);
+}
 // Which form takes a call.  USE_OUT: output alone; USE_TRAIN: forward and backward of a training call (the states of the forward
 // are handed on, so both take the same form); USE_PROMPT: output and final state.
 enum Use { USE_OUT, USE_TRAIN, USE_PROMPT };
@@ -852,6 +858,9 @@ int chosen(const fastmax_problem* pb, bool backward, Use use) {   // 0: neither,
     const double most = pb->order == 2 ? (pb->d == 64 ? 16000.0 : pb->d == 32 ? 5000.0 : 2000.0)
                         : pb->causal   ? (pb->d == 64 ? 2300.0 : pb->d == 32 ? 1050.0 : 900.0)
                                        : (pb->d == 64 ? 1300.0 : pb->d == 32 ? 800.0 : 600.0);
+    // d = 32 with a mask: windows and states (us, forward + backward, pairs / windows: order 2 64 heads 2048 tokens 724 / 589,
+    // 128 heads 1024 tokens 434 / 512; order 1 128 heads 1024 tokens 436 / 377)
+    if (pb->d == 32 && pb->causal && pb->nq == pb->nk && pb->nq < (1 << 30) && f32_registers_ok() && per_token > (pb->order == 2 ? 900. : 450.)) return 2;
     return per_token <= most && f32_registers_ok() ? 1 : 0;
   }
   // order 1 without a mask: one pass over the tensors (p1_forward_kernel), always the cheapest where it fills the GPU
@@ -902,6 +911,8 @@ static int forward_form(const fastmax_problem* pb, const fastmax_forward_args* a
   const Use use = a->state_out ? USE_PROMPT : a->key_moments_out || a->key_moments_in ? USE_TRAIN : USE_OUT;
   const int form = chosen(pb, false, use);
   if (form == 0 || !mappable(a->q, pb, pb->nq) || !mappable(a->k, pb, pb->nk) || !mappable(a->v, pb, pb->nk)) return 0;
+  if (form == 2 && pb->dtype == FASTMAX_F32)
+    return !a->state_out && rows_f32(a->q, pb, pb->nq) && rows_f32(a->k, pb, pb->nk) && rows_f32(a->o, pb, pb->nq) ? 2 : 0;
   if (form == 2) return rows16(a->o) && mappable(a->o, pb, pb->nq) && (!a->state_out || pb->causal) ? 2 : 0;
   return a->state_out ? 0 : 1;
 }
@@ -909,6 +920,8 @@ static int backward_form(const fastmax_problem* pb, const fastmax_backward_args*
   if (!a->dq.ptr || !a->dk.ptr || !a->dv.ptr || a->state_in || a->dstate_in || a->dstate_out) return 0;
   const int form = chosen(pb, true, USE_TRAIN);
   if (form == 0 || !mappable(a->q, pb, pb->nq) || !mappable(a->k, pb, pb->nk) || !mappable(a->v, pb, pb->nk)) return 0;
+  if (form == 2 && pb->dtype == FASTMAX_F32)
+    return rows_f32(a->q, pb, pb->nq) && rows_f32(a->k, pb, pb->nk) && rows_f32(a->dq, pb, pb->nq) && rows_f32(a->dk, pb, pb->nk) && rows_f32(a->dv, pb, pb->nk) ? 2 : 0;
   if (form == 2)
     return rows16(a->dq) && rows16(a->dk) && rows16(a->dv) && mappable(a->dq, pb, pb->nq) && mappable(a->dk, pb, pb->nk) && mappable(a->dv, pb, pb->nk) ? 2 : 0;
   return 1;
@@ -918,24 +931,29 @@ bool pair_takes_backward(const fastmax_problem* pb, const fastmax_backward_args*
 
 // ---- float32 ------------------------------------------------------------------------------------------------------------
 // bf16 pieces [3][batch*heads][n][d] as a tensor map: piece = batch index, head = batch*heads
-static size_t pieces_bytes(const fastmax_problem* pb, int n) { return up256((size_t)3 * pb->batch * pb->heads * n * pb->d * 2); }
+static size_t pieces_bytes(const fastmax_problem* pb, int n, int ld = 0) { return up256((size_t)3 * pb->batch * pb->heads * n * (ld > 0 ? ld : pb->d) * 2); }
 static size_t long_forward_workspace(const fastmax_problem* pb);
+static size_t long_f32_forward_workspace(const fastmax_problem* pb);
+static size_t long_f32_backward_workspace(const fastmax_problem* pb);
 static size_t long_backward_workspace(const fastmax_problem* pb);
 size_t pair_forward_workspace(const fastmax_problem* pb, const fastmax_forward_args* a) {
-  if (pb->dtype == FASTMAX_F32) return pieces_bytes(pb, pb->nq) + 2 * pieces_bytes(pb, pb->nk);
+  if (pb->dtype == FASTMAX_F32) return forward_form(pb, a) == 2 ? long_f32_forward_workspace(pb) : pieces_bytes(pb, pb->nq) + 2 * pieces_bytes(pb, pb->nk);
   return forward_form(pb, a) == 2 ? long_forward_workspace(pb) : 0;
 }
 size_t pair_backward_workspace(const fastmax_problem* pb, const fastmax_backward_args* a) {
-  if (pb->dtype != FASTMAX_F32 && backward_form(pb, a) == 2) return long_backward_workspace(pb);
+  if (backward_form(pb, a) == 2) return pb->dtype == FASTMAX_F32 ? long_f32_backward_workspace(pb) : long_backward_workspace(pb);
   if (pb->dtype == FASTMAX_F32)
     return 2 * pieces_bytes(pb, pb->nq) + 2 * pieces_bytes(pb, pb->nk) + up256((size_t)pb->batch * pb->heads * nd_ld(pb->nq) * sizeof(float));
   const size_t bh = (size_t)pb->batch * pb->heads;
   return up256(bh * pb->nq * pb->d * 2) + up256(bh * nd_ld(pb->nq) * sizeof(float));
 }
 
-static bool pieces_map(CUtensorMap* m, void* p, const fastmax_problem* pb, int n, int rows) {
+// rows [first, n) of every piece and head; columns past `cols` read as zero
+static bool pieces_map(CUtensorMap* m, void* p, const fastmax_problem* pb, int n, int rows, int ld = 0, int cols = 0, int first = 0) {
   const int64_t bh = (int64_t)pb->batch * pb->heads;
-  return tc_make_map(m, fastmax_tensor{p, bh * n * pb->d, (int64_t)n * pb->d, pb->d}, 3, (int)bh, n, 64, rows, true, pb->d);
+  if (ld == 0) ld = pb->d;
+  const fastmax_tensor t{(__nv_bfloat16*)p + (int64_t)first * ld, bh * n * ld, (int64_t)n * ld, ld};
+  return tc_make_map(m, t, 3, (int)bh, n - first, 64, rows, true, cols > 0 ? cols : pb->d);
 }
 static void launch_split(const fastmax_problem* pb, const pair::f32::SplitArgs& A, int count, cudaStream_t st) {
   int n = A.n[0];
@@ -995,7 +1013,7 @@ static int pair_f32_forward(const fastmax_problem* pb, const fastmax_forward_arg
     return FASTMAX_ERR_UNSUPPORTED;
   M.b = M.o0 = M.o1 = M.a;
   launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
-                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {pb->nq, pb->nk, pb->nk}}, 3, st);
+                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {pb->nq, pb->nk, pb->nk}, {pb->d, pb->d, pb->d}}, 3, st);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return report_cuda_error(e);
   pair::Params P{};
@@ -1011,16 +1029,16 @@ static int pair_f32_forward(const fastmax_problem* pb, const fastmax_forward_arg
 }
 
 template <int D>
-static void launch_prologue_f32(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, cudaStream_t st) {
+static void launch_prologue_f32(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
   const int ld = nd_ld(pb->nq), rows = 256 / (D / 8);
   const dim3 grid((unsigned)((ld + rows - 1) / rows), (unsigned)(pb->batch * pb->heads));
   auto vec = [](const fastmax_tensor& t) {
     return ((uintptr_t)t.ptr & 15) == 0 && (t.stride_b & 3) == 0 && (t.stride_h & 3) == 0 && (t.stride_n & 3) == 0;
   };
   if (vec(a->o) && vec(a->d_out))
-    pair::f32::prologue_f32_kernel<D, true><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads);
+    pair::f32::prologue_f32_kernel<D, true><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
   else
-    pair::f32::prologue_f32_kernel<D, false><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads);
+    pair::f32::prologue_f32_kernel<D, false><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
 }
 
 static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
@@ -1037,13 +1055,13 @@ static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
     return FASTMAX_ERR_UNSUPPORTED;
   M.o0 = M.o1 = N.o0 = N.o1 = M.a;
   launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
-                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {pb->nq, pb->nk, pb->nk}}, 3, st);
+                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {pb->nq, pb->nk, pb->nk}, {pb->d, pb->d, pb->d}}, 3, st);
   {
     LaunchScope ls(KK_PROLOGUE, st);
     switch (pb->d) {
-      case 16: launch_prologue_f32<16>(pb, a, (__nv_bfloat16*)dp, nd, st); break;
-      case 32: launch_prologue_f32<32>(pb, a, (__nv_bfloat16*)dp, nd, st); break;
-      default: launch_prologue_f32<64>(pb, a, (__nv_bfloat16*)dp, nd, st); break;
+      case 16: launch_prologue_f32<16>(pb, a, (__nv_bfloat16*)dp, nd, pb->d, st); break;
+      case 32: launch_prologue_f32<32>(pb, a, (__nv_bfloat16*)dp, nd, pb->d, st); break;
+      default: launch_prologue_f32<64>(pb, a, (__nv_bfloat16*)dp, nd, pb->d, st); break;
     }
   }
   cudaError_t e = cudaGetLastError();
@@ -1151,8 +1169,8 @@ int sm_total() {
   }
   return n;
 }
-template <typename K>
-cudaError_t launch_items(K kernel, std::atomic<bool>* done, int bytes, int threads, const lng::Maps& M, const lng::Params& P, int kind, cudaStream_t st) {
+template <typename K, typename MAPS, typename PARAMS>
+cudaError_t launch_items(K kernel, std::atomic<bool>* done, int bytes, int threads, const MAPS& M, const PARAMS& P, int kind, cudaStream_t st) {
   if (P.nitems <= 0) return cudaSuccess;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -1210,12 +1228,6 @@ static size_t long_backward_workspace(const fastmax_problem* pb) {
   return g.raw + 2 * (g.packed + g.cst) + up256(tc_moments_scratch(pb, n)) + up256(bh * pb->nq * (pb->d + 16) * 2) +
          up256(bh * nd_ld(pb->nq) * sizeof(float)) + (pb->causal ? 3 * up256(bh * pb->nq * pb->d * sizeof(float)) : 0);
 }
-size_t pair_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_args* a) {
-  fastmax_forward_args train = *a;   // who asks is about to hand them on
-  train.key_moments_out = (float*)a->q.ptr;
-  return pb->dtype != FASTMAX_F32 && forward_form(pb, &train) == 2 ? long_geo(pb).packed + long_geo(pb).cst : 0;
-}
-
 // Packed states of the keys before every segment but the first (no mask: of all keys): S, then the constant rows behind it
 static cudaError_t long_key_states(const fastmax_problem* pb, const LongGeo& g, const fastmax_tensor& k, const fastmax_tensor& v, float* raw, void* xt,
                                    uint8_t* S, float* total, cudaStream_t st) {
@@ -1343,8 +1355,187 @@ static int long_backward(const fastmax_problem* pb, const fastmax_backward_args*
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
 
+// ---- long float32 sequences (long_f32.cuh) --------------------------------------------------------------------------------
+namespace {
+
+LongGeo long_geo_f32(const fastmax_problem* pb) {
+  LongGeo g;
+  const size_t bh = (size_t)pb->batch * pb->heads;
+  // window: 8 heads of 131072 tokens forward + backward 4.26 / 4.49 / 4.85 / 5.27 ms for 256 / 512 / 768 / 1024; the states, which a
+  // training call keeps, take half the memory at 512 (414 MB there)
+  g.L = 512;
+  g.ns = (pb->nk + g.L - 1) / g.L - 1;
+  g.rows = (pb->order == 2 ? 64 * lng::f32::NPAIR : 0) + pb->d + 1;
+  g.raw = up256(bh * g.ns * g.rows * lng::f32::LD * sizeof(float));
+  g.packed = up256(bh * g.ns * lng::f32::UNITS * (size_t)lng::f32::UNIT);
+  g.cst = up256(bh * g.ns * lng::f32::CST * sizeof(float));
+  return g;
+}
+bool view_map_f32(CUtensorMap* m, const fastmax_tensor& t, const fastmax_problem* pb, int n, int rows, bool swizzle) {
+  return tc_make_map(m, t, pb->batch, pb->heads, n, 32, rows, swizzle, pb->d, true);
+}
+// the three pieces of [dO' | -delta] or [v | 1] as 128-row boxes of 48 columns
+bool g_map_f32(CUtensorMap* m, void* p, const fastmax_problem* pb, int n) {
+  const int64_t bh = (int64_t)pb->batch * pb->heads, ld = lng::f32::NC;
+  return tc_make_map(m, fastmax_tensor{p, bh * n * ld, n * ld, ld}, 3, (int)bh, n, (int)ld, 128, false, (int)ld);
+}
+// packed states of x (keys or queries) and y (pieces with 48 columns), rows [first, n): S, then the constant rows behind it
+cudaError_t long_states_f32(const fastmax_problem* pb, const LongGeo& g, const fastmax_tensor& x, void* y, int n_all, int first, int n, bool reverse, float* raw,
+                            uint8_t* S, cudaStream_t st) {
+  using namespace lng::f32;
+  mo::Maps M;
+  if (!view_map_f32(&M.x, after(x, first, 4), pb, n - first, CHUNK, false) || !pieces_map(&M.y, y, pb, n_all, CHUNK, NC, NC, first)) return cudaErrorInvalidValue;
+  mo::Params P{};
+  P.out = raw;
+  P.n = n - first;
+  P.heads = pb->heads;
+  P.seg = g.L;
+  P.nsplit = g.ns;
+  P.tile_first = pb->order == 2 ? 0 : mo::LIN;
+  P.nslices = pb->order == 2 ? 3 : 1;
+  P.nitems = P.nslices * g.ns * pb->batch * pb->heads;
+  P.state_rows = g.rows;
+  static std::atomic<bool> done[64];
+  cudaError_t e = launch_items(mo::moments_kernel, done, mo::BYTES, mo::THREADS, M, P, KK_TC_MOMENTS, st);
+  if (e != cudaSuccess) return e;
+  const float c0 = pb->a0, c1 = pb->a1 * pb->inv_temperature, c2 = pb->order == 2 ? pb->a2 * pb->inv_temperature * pb->inv_temperature : 0.f;
+  const dim3 grid((unsigned)((pb->order == 2 ? UNITS : 1) + 1), NC / 8, (unsigned)(pb->batch * pb->heads));
+  LaunchScope ls(KK_STATE_SCAN, st);
+  pack_kernel<<<grid, 64, 0, st>>>(raw, S, (float*)(S + g.packed), g.ns, g.ns, reverse, pb->order, c0, c1, c2);
+  return cudaGetLastError();
+}
+template <bool FWD>
+cudaError_t launch_apply_f32(const lng::Maps& M, const lng::Params& P, int kind, cudaStream_t st) {
+  static std::atomic<bool> done[64];
+  return launch_items(lng::f32::ap::apply_kernel<FWD>, done, lng::f32::ap::BYTES, lng::f32::ap::THREADS, M, P, kind, st);
+}
+cudaError_t launch_chain_f32(const lng::Maps& M, const lng::Params& P, int kind, cudaStream_t st) {
+  static std::atomic<bool> done[64];
+  return launch_items(lng::f32::ch::chain_kernel, done, lng::f32::ch::BYTES, lng::f32::ch::THREADS, M, P, kind, st);
+}
+
+}  // namespace
+
+static size_t long_f32_forward_workspace(const fastmax_problem* pb) {
+  const LongGeo g = long_geo_f32(pb);
+  return g.raw + g.packed + g.cst + pieces_bytes(pb, pb->nq) + pieces_bytes(pb, pb->nk) + pieces_bytes(pb, pb->nk, lng::f32::NC);
+}
+static size_t long_f32_backward_workspace(const fastmax_problem* pb) {
+  const LongGeo g = long_geo_f32(pb);
+  return g.raw + 2 * (g.packed + g.cst) + 2 * pieces_bytes(pb, pb->nq) + 2 * pieces_bytes(pb, pb->nk, lng::f32::NC) +
+         up256((size_t)pb->batch * pb->heads * nd_ld(pb->nq) * sizeof(float));
+}
+
+static int long_f32_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st) {
+  const LongGeo g = long_geo_f32(pb);
+  const int bh = pb->batch * pb->heads, n = pb->nq;
+  char* base = (char*)ws;
+  float* raw = (float*)base; base += g.raw;
+  uint8_t* S = a->key_moments_in ? (uint8_t*)const_cast<float*>(a->key_moments_in) : a->key_moments_out ? (uint8_t*)a->key_moments_out : (uint8_t*)base;
+  base += g.packed + g.cst;
+  void *qp = base, *kp = base + pieces_bytes(pb, n), *vp = base + 2 * pieces_bytes(pb, n);
+  pair::Maps M;
+  lng::Maps A;
+  if (!pieces_map(&M.a, qp, pb, n, pair::R) || !pieces_map(&M.x, kp, pb, n, pair::f32::TF) || !pieces_map(&M.y, vp, pb, n, pair::f32::TF, lng::f32::NC) ||
+      !view_map_f32(&A.x, a->q, pb, n, 128, true) || !view_map_f32(&A.part, a->o, pb, n, 128, true) || !view_map_f32(&A.out, a->o, pb, n, 32, true))
+    return FASTMAX_ERR_UNSUPPORTED;
+  M.b = M.o0 = M.o1 = M.p0 = M.p1 = M.a;
+  A.y = A.x;
+  launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
+                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {n, n, n}, {pb->d, pb->d, lng::f32::NC}}, 3, st);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return report_cuda_error(e);
+  {
+    pair::Params P{};
+    fill(pb, P);
+    P.window = P.part_lo = g.L;
+    P.part_hi = 1 << 30;
+    P.out0 = view_of(a->o);
+    P.out1 = view_of(a->g);
+    P.nr = P.nx = n;
+    P.ntiles = tiles(n);
+    LaunchScope ls(KK_TC_INTRA_FWD, st);
+    e = launch_f32_d<pair::FWD>(pb->d, M, P, bh, st);
+  }
+  if (e == cudaSuccess && !a->key_moments_in) e = long_states_f32(pb, g, a->k, vp, n, 0, g.ns * g.L, false, raw, S, st);
+  lng::Params P = long_params(pb, g, S, n, g.L, n);
+  P.g = view_of(a->g);
+  if (e == cudaSuccess) e = launch_apply_f32<true>(A, P, KK_TC_FWD, st);
+  return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
+}
+
+static int long_f32_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
+  using lng::f32::NC;
+  const LongGeo g = long_geo_f32(pb);
+  const int bh = pb->batch * pb->heads, n = pb->nq;
+  const size_t narrow = pieces_bytes(pb, n), wide = pieces_bytes(pb, n, NC);
+  char* base = (char*)ws;
+  float* raw = (float*)base; base += g.raw;
+  uint8_t* S = a->key_moments_in ? (uint8_t*)const_cast<float*>(a->key_moments_in) : (uint8_t*)base; base += g.packed + g.cst;
+  uint8_t* dS = (uint8_t*)base; base += g.packed + g.cst;
+  void *qp = base, *kp = base + narrow, *vp = base + 2 * narrow, *dp = base + 2 * narrow + wide;
+  float* nd = (float*)(base + 2 * narrow + 2 * wide);
+  pair::Maps M, N;   // M: dq, N: dk and dv
+  lng::Maps Q, K, V;
+  if (!pieces_map(&M.a, qp, pb, n, pair::R) || !pieces_map(&M.b, dp, pb, n, pair::R, NC) || !pieces_map(&M.x, kp, pb, n, pair::f32::TF) ||
+      !pieces_map(&M.y, vp, pb, n, pair::f32::TF, NC) || !pieces_map(&N.a, kp, pb, n, pair::R) || !pieces_map(&N.b, vp, pb, n, pair::R, NC) ||
+      !pieces_map(&N.x, qp, pb, n, pair::f32::TF) || !pieces_map(&N.y, dp, pb, n, pair::f32::TF, NC) ||
+      !view_map_f32(&Q.x, a->q, pb, n, 128, true) || !view_map_f32(&K.x, a->k, pb, n, 128, true) ||
+      !view_map_f32(&Q.part, a->dq, pb, n, 128, true) || !view_map_f32(&Q.out, a->dq, pb, n, 32, true) ||
+      !view_map_f32(&K.part, a->dk, pb, n, 128, true) || !view_map_f32(&K.out, a->dk, pb, n, 32, true) ||
+      !view_map_f32(&V.part, a->dv, pb, n, 128, true) || !view_map_f32(&V.out, a->dv, pb, n, 32, true) ||
+      !g_map_f32(&Q.y, dp, pb, n) || !g_map_f32(&K.y, vp, pb, n))
+    return FASTMAX_ERR_UNSUPPORTED;
+  M.o0 = M.o1 = M.p0 = M.p1 = N.o0 = N.o1 = N.p0 = N.p1 = M.a;
+  V.x = K.x;
+  V.y = K.y;
+  launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
+                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {n, n, n}, {pb->d, pb->d, NC}}, 3, st);
+  {
+    LaunchScope ls(KK_PROLOGUE, st);
+    launch_prologue_f32<32>(pb, a, (__nv_bfloat16*)dp, nd, NC, st);
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return report_cuda_error(e);
+  pair::Params P{};
+  fill(pb, P);
+  P.window = g.L;
+  P.ndelta = nd;
+  P.nd_ld = nd_ld(n);
+  P.nr = P.nx = n;
+  P.ntiles = tiles(n);
+  pair::Params B = P;
+  B.out0 = view_of(a->dk);
+  B.out1 = view_of(a->dv);
+  {
+    LaunchScope ls(KK_TC_INTRA_BWD, st);
+    e = launch_f32_d<pair::DKV>(pb->d, N, B, bh, st);
+  }
+  P.out0 = P.out1 = view_of(a->dq);
+  if (e == cudaSuccess) {
+    LaunchScope ls(KK_TC_INTRA_BWD, st);
+    e = launch_f32_d<pair::DQ>(pb->d, M, P, bh, st);
+  }
+  if (e == cudaSuccess && !a->key_moments_in) e = long_states_f32(pb, g, a->k, vp, n, 0, g.ns * g.L, false, raw, S, st);
+  // gradient moments of every segment but the first; raw may be reused: the stream orders it
+  if (e == cudaSuccess) e = long_states_f32(pb, g, a->q, dp, n, g.L, n, true, raw, dS, st);
+  if (e == cudaSuccess) e = launch_chain_f32(Q, long_params(pb, g, S, n, g.L, n), KK_TC_BWD_Q, st);
+  const lng::Params R = long_params(pb, g, dS, n, 0, g.ns * g.L);
+  if (e == cudaSuccess) e = launch_chain_f32(K, R, KK_TC_BWD_KV, st);
+  if (e == cudaSuccess) e = launch_apply_f32<false>(V, R, KK_TC_BWD_DV, st);
+  return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
+}
+
+size_t pair_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_args* a) {
+  fastmax_forward_args train = *a;   // who asks is about to hand them on
+  train.key_moments_out = (float*)a->q.ptr;
+  if (forward_form(pb, &train) != 2) return 0;
+  const LongGeo g = pb->dtype == FASTMAX_F32 ? long_geo_f32(pb) : long_geo(pb);
+  return g.packed + g.cst;
+}
+
 int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st) {
-  if (pb->dtype == FASTMAX_F32) return pair_f32_forward(pb, a, ws, st);
+  if (pb->dtype == FASTMAX_F32) return forward_form(pb, a) == 2 ? long_f32_forward(pb, a, ws, st) : pair_f32_forward(pb, a, ws, st);
   if (forward_form(pb, a) == 2) return long_forward(pb, a, ws, st);
   pair::Maps M;
   if (!tc_make_map(&M.a, a->q, pb->batch, pb->heads, pb->nq, 64, pair::R, true, pb->d) ||
@@ -1368,7 +1559,7 @@ int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void*
 }
 
 int pair_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
-  if (pb->dtype == FASTMAX_F32) return pair_f32_backward(pb, a, ws, st);
+  if (pb->dtype == FASTMAX_F32) return backward_form(pb, a) == 2 ? long_f32_backward(pb, a, ws, st) : pair_f32_backward(pb, a, ws, st);
   if (backward_form(pb, a) == 2) return long_backward(pb, a, ws, st);
   const int bh = pb->batch * pb->heads;
   __nv_bfloat16* dop = (__nv_bfloat16*)ws;

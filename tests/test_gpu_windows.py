@@ -82,3 +82,47 @@ def test_prompt_of_windows_returns_its_state(D, N):
     for a, b, tol in ((o, o2, 2e-2), (gg, g2, 1e-3), (state, state2, 5e-3)):
         assert orc.max_norm_err(host(a), host(b)) < tol
     assert float(state[..., D + 1:].abs().max()) == 0.0
+
+
+F32_CASES = [  # B, H, n, order, head-split views
+    (1, 2, 4097, 2, False),   # eight windows of 512 and one token
+    (2, 2, 4500, 2, True),
+    (1, 3, 4608, 2, True),    # nine whole windows
+    (1, 2, 1300, 1, False),
+]
+
+
+@pytest.mark.parametrize("hand_over", [True, False])
+@pytest.mark.parametrize("case", F32_CASES)
+def test_float32_windows_match_oracle(case, hand_over):
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    B, H, n, order, split = case
+    D = 32
+    g = torch.Generator(device="cuda").manual_seed(n)
+    mk = lambda: (torch.randn(B, n, H, D, device="cuda", generator=g).transpose(1, 2) if split else torch.randn(B, H, n, D, device="cuda", generator=g))
+    q, k, v, do = (mk() for _ in range(4))
+    p = orc.Poly(0.9, 1.1, 0.45, 1.0 / (8.0 * math.sqrt(D)), order)
+    args = (True, p.inv_temp, p.a0, p.a1, p.a2, order)
+    km = L.KeyMoments()
+    L.profile_collect()
+    L.profile(True)
+    o, gg, _ = L.forward(q, k, v, *args, flags=L.FLAG_PAIRWISE, key_moments=km)
+    assert km.buf is not None
+    dq, dk, dv, _ = L.backward(q, k, v, o, gg, do, *args, flags=L.FLAG_PAIRWISE, key_moments=km if hand_over else None)
+    L.check_status()
+    L.profile(False)
+    assert L.profile_collect()["tc_moments"][1] == (2 if hand_over else 3)
+    assert L.wait_histogram() == {}
+    rng = np.random.default_rng(n)
+    for b, h in {(0, 0), (B - 1, H - 1)}:
+        a = [host(t[b, h]) for t in (q, k, v, do)]
+        oh, gh = host(o[b, h]), host(gg[b, h])
+        rows = np.unique(np.concatenate([[0, 127, 511, 512, 639, 1023, 1024, n - 1], rng.integers(0, n, 24)]))
+        o_ref, g_ref = orc.sampled_forward_rows(a[0], a[1], a[2], rows, True, p)
+        assert orc.max_norm_err(oh[rows], o_ref) < 2e-6 and orc.max_norm_err(gh[rows], g_ref) < 2e-6
+        dq_ref = orc.sampled_dq_rows(a[0], a[1], a[2], oh, gh, a[3], rows, True, p)
+        dk_ref, dv_ref = orc.sampled_dkv_cols(a[0], a[1], a[2], oh, gh, a[3], rows, True, p)
+        for name, x, ref in (("dq", dq, dq_ref), ("dk", dk, dk_ref), ("dv", dv, dv_ref)):
+            err = np.linalg.norm(host(x[b, h])[rows] - ref) / np.linalg.norm(ref)
+            assert err < 3e-6, (name, b, h, err)
