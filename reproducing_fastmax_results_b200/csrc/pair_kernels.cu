@@ -58,8 +58,9 @@ struct Params {
   int window;                 // 0, or (causal, off = 0): only the keys of the query's own window of this many tokens
   int part_lo, part_hi;       // rows whose results are partial: float32 into `part` (Maps::p0, p1), not divided
   int ntiles;                 // items per head
-  uint32_t mul_t, mul_h;      // quotients by ntiles and heads without a division: (n * mul) >> shift
-  int sh_t, sh_h;
+  int group, last, ngroups;   // heads per group of the item order, and in its last group
+  uint32_t mul_g, mul_t, mul_l, mul_h;   // quotients by group * ntiles, group, last and heads without a division: (n * mul) >> shift
+  int sh_g, sh_t, sh_l, sh_h;
   int vec0, vec1;             // rows of out0 / out1 start on 16-byte boundaries: written by the copy engine
   float c0, c1, c2;
   float k, w0, w1;            // completed square (see SQ): c0 / c2 - h^2; factors of out0 and out1
@@ -191,11 +192,15 @@ __device__ __forceinline__ bool first_rows(const Params& P, int r0) { return P.c
 // TILE: streamed rows per tile, HELD: rows of an item
 template <int KIND, int TILE, int HELD>
 __device__ __forceinline__ Item decode(int idx, const Params& P) {
-  // Head-major, the longest item of a head first: the blocks at work share a few heads' streamed tiles in L2, and the
-  // last items are short.
+  // Groups of heads one after the other; within a group the longest items of all its heads first.  Blocks at work share a few
+  // heads' streamed tiles in L2 (see order_items), and the last items are short: in the order of the heads, the last head's long
+  // items started when everything else was done (64 heads of 4096 tokens: the SMs were idle for 20 % of the forward).
   Item it;
-  it.head = (int)(((uint64_t)(uint32_t)idx * P.mul_t) >> P.sh_t);
-  const int ti = idx - it.head * P.ntiles;
+  const int gr = (int)(((uint64_t)(uint32_t)idx * P.mul_g) >> P.sh_g);
+  const uint32_t rest = (uint32_t)(idx - gr * P.group * P.ntiles);
+  const bool end = gr == P.ngroups - 1;
+  const int ti = end ? (int)(((uint64_t)rest * P.mul_l) >> P.sh_l) : (int)(((uint64_t)rest * P.mul_t) >> P.sh_t);
+  it.head = gr * P.group + (int)rest - ti * (end ? P.last : P.group);
   it.b = (int)(((uint64_t)(uint32_t)it.head * P.mul_h) >> P.sh_h);
   it.h = it.head - it.b * P.heads;
   it.t0 = 0;
@@ -787,10 +792,28 @@ cudaError_t launch(const pair::Maps& M, const pair::Params& P, int bh, cudaStrea
   kernel<<<dim3((unsigned)(P.ntiles * bh)), pair::THREADS, pair::SMEM_BYTES, st>>>(M, P);
   return cudaGetLastError();
 }
+// Heads per group of the item order (decode).  With a mask, items differ in length: as many heads as have their streamed tiles in
+// a quarter of L2 (us forward / backward, one head at a time, 32, 128: 128 heads of 4096 x 64 252/862, 241/838, 262/939; 128 heads
+// of 2048 x 32 78/237, 70/218, 66/214; of 1024 x 64 44/105, 42/98, 42/92).  Without one (and within windows) the items are alike, and the order of the heads is best for L2.
+void order_items(int d, int es, pair::Params& P, int bh) {
+  long long group = 1;
+  if (P.causal && !P.window) {
+    group = (32ll << 20) / ((long long)P.nx * d * 2 * es);
+    group = group < 1 ? 1 : group > bh ? bh : group;
+    const long long n = (bh + group - 1) / group;
+    group = (bh + n - 1) / n;
+  }
+  P.group = (int)group;
+  P.ngroups = (bh + P.group - 1) / P.group;
+  P.last = bh - (P.ngroups - 1) * P.group;
+  quotient(P.group * P.ntiles, P.mul_g, P.sh_g);
+  quotient(P.group, P.mul_t, P.sh_t);
+  quotient(P.last, P.mul_l, P.sh_l);
+  quotient(P.heads, P.mul_h, P.sh_h);
+}
 template <int KIND, bool SQ>
 cudaError_t launch_d(int d, const pair::Maps& M, pair::Params& P, int bh, cudaStream_t st) {
-  quotient(P.ntiles, P.mul_t, P.sh_t);
-  quotient(P.heads, P.mul_h, P.sh_h);
+  order_items(d, 2, P, bh);
   switch (d) {
     case 16: return launch<16, KIND, SQ>(M, P, bh, st);
     case 32: return launch<32, KIND, SQ>(M, P, bh, st);
@@ -985,8 +1008,7 @@ static cudaError_t launch_f32(const pair::Maps& M, const pair::Params& P, int bh
 }
 template <int KIND>
 static cudaError_t launch_f32_d(int d, const pair::Maps& M, pair::Params& P, int bh, cudaStream_t st) {
-  quotient(P.ntiles, P.mul_t, P.sh_t);
-  quotient(P.heads, P.mul_h, P.sh_h);
+  order_items(d, 6, P, bh);
   switch (d) {
     case 16: return launch_f32<16, KIND>(M, P, bh, st);
     case 32: return launch_f32<32, KIND>(M, P, bh, st);

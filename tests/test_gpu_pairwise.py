@@ -95,3 +95,28 @@ def test_pairwise_form_is_left_to_the_moment_engines_where_it_does_not_apply():
     L.check_status()
     for a, b, tol in ((o, o_ref, 1e-2), (state, state_ref, 1e-4), (oe, oc, 1e-2), (ge, gc, 1e-3)):
         assert orc.max_norm_err(host(a), host(b)) < tol
+
+
+@pytest.mark.parametrize("dtype,n", [(torch.bfloat16, 5500), (torch.float32, 2000)])
+def test_more_heads_than_one_group_of_the_item_order(dtype, n):
+    """25 heads whose streamed tiles exceed the share of L2: two groups, the last one smaller; every head, forward and backward."""
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v, do = (torch.randn(1, 25, n, 64, device="cuda", generator=g).to(dtype) for _ in range(4))
+    p = orc.Poly(1.0, 1.0, 0.5, 1.0 / 64.0, 2)
+    args = (True, p.inv_temp, p.a0, p.a1, p.a2, 2)
+    o, gg, _ = L.forward(q, k, v, *args, flags=L.FLAG_PAIRWISE)
+    dq, dk, dv, _ = L.backward(q, k, v, o, gg, do, *args, flags=L.FLAG_PAIRWISE)
+    L.check_status()
+    rows = np.array([300, 1023, n - 1])
+    tol = 2e-2 if dtype == torch.bfloat16 else 5e-6
+    for h in range(25):
+        a = [host(t[0, h]) for t in (q, k, v, do)]
+        oh, gh = host(o[0, h]), host(gg[0, h])
+        o_ref, _ = orc.sampled_forward_rows(a[0], a[1], a[2], rows, True, p)
+        dq_ref = orc.sampled_dq_rows(a[0], a[1], a[2], oh, gh, a[3], rows, True, p)
+        dk_ref, dv_ref = orc.sampled_dkv_cols(a[0], a[1], a[2], oh, gh, a[3], rows, True, p)
+        for name, x, r in (("o", o, o_ref), ("dq", dq, dq_ref), ("dk", dk, dk_ref), ("dv", dv, dv_ref)):
+            err = np.linalg.norm(host(x[0, h])[rows] - r) / np.linalg.norm(r)
+            assert err < tol, (name, h, err)
