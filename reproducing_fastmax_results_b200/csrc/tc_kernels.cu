@@ -381,8 +381,8 @@ static cudaError_t launch_transpose(const fastmax_tensor& x, int batch, int head
   LaunchScope ls(KK_TC_TRANSPOSE, st);
   const int ntp = tokens_padded(n + shift);
   const View v{x.ptr, x.stride_b, x.stride_h, x.stride_n};
-  if (d == 64) tc::s2::transpose_tokens_kernel<64><<<dim3(ntp / 64, batch * heads), 256, 0, st>>>(v, xt, n, ntp, heads, shift);
-  else tc::s2::transpose_tokens_kernel<32><<<dim3(ntp / 64, batch * heads), 256, 0, st>>>(v, xt, n, ntp, heads, shift);
+  if (d == 64) tc::s2::transpose_tokens_kernel<64><<<dim3((ntp + 127) / 128, batch * heads), 256, 0, st>>>(v, xt, n, ntp, heads, shift);
+  else tc::s2::transpose_tokens_kernel<32><<<dim3((ntp + 127) / 128, batch * heads), 256, 0, st>>>(v, xt, n, ntp, heads, shift);
   return cudaGetLastError();
 }
 
