@@ -815,7 +815,7 @@ static int tc_p1_forward(const fastmax_problem* pb, const fastmax_forward_args* 
   CUtensorMap tmq, tmk, tmv, tmo;
   if (!make_map(&tmq, a->q, pb->batch, pb->heads, pb->nq, 64, tc::CH, true) ||
       !make_map(&tmk, a->k, pb->batch, pb->heads, pb->nk, 64, tc::CH, true) ||
-      !make_map(&tmv, a->v, pb->batch, pb->heads, pb->nk, 8, tc::CH, false) ||
+      !make_map(&tmv, a->v, pb->batch, pb->heads, pb->nk, 64, tc::CH, true) ||
       !make_map(&tmo, a->o, pb->batch, pb->heads, pb->nq, 64, 32, true))   // output: 32-row boxes, one per epilogue warp
     return FASTMAX_TC_NOT_HANDLED;
   cudaError_t e = ensure_smem(tc::p1::p1_forward_kernel, tc::p1::SMEM_BYTES, 0);

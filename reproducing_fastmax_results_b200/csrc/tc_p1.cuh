@@ -5,11 +5,13 @@
 //     O'_c = Q_c (c1 S)  + a0 s0     per 128-query chunk;  o = O'[:, :64] / O'[:, 64],  g = O'[:, 64]
 //
 // 33 flop per byte: the call is bound by HBM (read q, k, v once, write o and g once).  One CTA per (batch, head)
-// streams the head's K and V chunks through a two-deep TMA ring into the moment MMAs, rounds c1 S to bf16 into a
-// K-major operand tile, then streams the Q chunks through the same ring; every epilogue warp stages its 32 output
+// streams the head's K and V tiles through a four-deep TMA ring into the moment MMAs (the ones column is a constant tile, the
+// second half of the A operand's rows), rounds c1 S to bf16 into a
+// K-major operand tile, then streams the Q tiles through the same ring; every epilogue warp stages its 32 output
 // rows in shared memory and hands them to the copy engine (tiled bulk store: whole 128-byte lines, rows past the
 // last query clipped by the tensor map).  Two CTAs fit on an SM, so one head's phase change hides behind the other's
-// streaming.
+// streaming.  Measured: 768 heads of 1024 tokens (405 MB) 72.8 us, 85 % of the copy bandwidth; 78.7 us with V in 8-column boxes
+// (16-byte rows: half of every sector unused) and a ring of two chunks.
 // Warp roles (160 threads): 0-3 epilogue (TMEM lane = moment row, then = token), 4 TMA loads + MMA issue.
 // TMEM columns (256 allocated): 0..63 S^T, 64..79 s0, 96..175 and 176..255 the two output accumulators.
 #pragma once
@@ -17,21 +19,20 @@
 namespace p1 {
 
 constexpr int THREADS = 160;
-constexpr int OFF_X = 0;                      // two 128 x 64 swizzled tiles: K chunks, later Q chunks
-constexpr int OFF_V = 2 * REGION;             // two [V | 1] chunks of 10 column blocks; the moment MMA reads 16 blocks
-constexpr int OFF_SB = OFF_V + 2 * 10 * BLK;  // 73728: c1 S as a K-major B operand, 80 rows x 128 B, 128-byte swizzle
-constexpr int OFF_ONES = OFF_SB + 80 * 128;   // 83968: 1 KB of bf16 ones (B operand of the s0 MMA)
+constexpr int RING = 4;
+constexpr int OFF_X = 0;                      // 128 x 64 swizzled tiles: K, V, K, V, ... later Q
+constexpr int OFF_V1 = RING * REGION;         // rows 64..127 of the moment MMA's A operand: a column of ones, then zeros
+constexpr int OFF_SB = OFF_V1 + REGION;       // c1 S as a K-major B operand, 80 rows x 128 B, 128-byte swizzle
+constexpr int OFF_ONES = OFF_SB + 80 * 128;   // 1 KB of bf16 ones (B operand of the s0 MMA)
 constexpr int OFF_T0 = OFF_ONES + 1024;       // 80 floats: a0 s0
 constexpr int OFF_BAR = OFF_T0 + 512;
-constexpr int OFF_OST = OFF_BAR + 512;        // 86016: output staging, one 32-row x 128-byte swizzled box per epilogue warp
+constexpr int OFF_OST = OFF_BAR + 512;        // output staging, one 32-row x 128-byte swizzled box per epilogue warp
 constexpr int OFF_END = OFF_OST + 4 * 4096;
-// rows 80..127 of the moment MMA's A operand read the 12 KB that follow a [V | 1] buffer (the other buffer, the
-// S tile, the ones): finite or not, they only reach TMEM lanes 80..127, which nobody reads
-static_assert(OFF_V + 10 * BLK + 16 * BLK <= OFF_END + 1024, "the moment MMA's A operand stays inside the allocation");
-constexpr int SMEM_BYTES = OFF_END + 1024 + 1024;
-static_assert(OFF_SB % 1024 == 0 && OFF_V % 1024 == 0 && OFF_OST % 1024 == 0, "swizzled tiles need 1024-byte alignment");
+constexpr int SMEM_BYTES = OFF_END + 1024;
+static_assert(OFF_SB % 1024 == 0 && OFF_OST % 1024 == 0, "swizzled tiles need 1024-byte alignment");
+static_assert(2 * (SMEM_BYTES + 1024) <= 233472, "two blocks on an SM");
 constexpr uint32_t COL_S = 0u, COL_S0 = 64u, COL_O = 96u;
-constexpr int B_X_READY = 0, B_X_FREE = 2, B_S_DONE = 4, B_SB_READY = 5, B_O_DONE = 6, B_O_FREE = 8, B_COUNT = 10;
+constexpr int B_X_READY = 0, B_X_FREE = RING, B_S_DONE = 2 * RING, B_SB_READY = B_S_DONE + 1, B_O_DONE = B_SB_READY + 1, B_O_FREE = B_O_DONE + 2;
 
 struct P1Params {
   View g;
@@ -46,7 +47,6 @@ p1_forward_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* sm = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
   uint8_t* xbuf = sm + OFF_X;
-  uint8_t* vbuf = sm + OFF_V;
   uint8_t* sb = sm + OFF_SB;
   float* t0 = reinterpret_cast<float*>(sm + OFF_T0);
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + OFF_BAR);
@@ -59,9 +59,8 @@ p1_forward_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant
   const int nkc = (P.nk + CH - 1) / CH, nqc = (P.nq + CH - 1) / CH;
 
   if (tid == 0) {
+    for (int i = 0; i < 2 * RING; ++i) mbar_init(&bars[B_X_READY + i], 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bars[B_X_READY + i], 1);
-      mbar_init(&bars[B_X_FREE + i], 1);
       mbar_init(&bars[B_O_DONE + i], 1);
       mbar_init(&bars[B_O_FREE + i], 4);
     }
@@ -71,12 +70,10 @@ p1_forward_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant
     fence_mbar_init();
   }
   if (w == 0) tmem_alloc(tmem_slot, 256);
-  // ones for the s0 MMA; zero pad blocks (column block 9 of both [V | 1] buffers; block 8 is rewritten per chunk)
+  // ones for the s0 MMA; the constant tile
   for (int i = tid; i < 1024 / 16; i += THREADS) reinterpret_cast<uint4*>(sm + OFF_ONES)[i] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
-  for (int i = tid; i < 2 * (2 * BLK / 16); i += THREADS) {
-    const int b = i / (2 * BLK / 16), r = i - b * (2 * BLK / 16);
-    reinterpret_cast<uint4*>(vbuf + b * 10 * BLK + 8 * BLK)[r] = make_uint4(0u, 0u, 0u, 0u);
-  }
+  for (int i = tid; i < REGION / 16; i += THREADS)   // 16-byte piece c of row r lies at c ^ (r & 7)
+    reinterpret_cast<uint4*>(sm + OFF_V1)[i] = make_uint4((i & 7) == ((i >> 3) & 7) ? 0x00003F80u : 0u, 0u, 0u, 0u);
   fence_proxy_async_smem();
   tc_fence_before_sync();
   __syncthreads();
@@ -90,75 +87,67 @@ p1_forward_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant
     atomicExch(&g_tc_status, code);
   };
 
+  int loads = 0;   // tiles asked for
   if (w == 4) {
     // ================= TMA loads and MMA issue =================
-    // The ring of two (X, [V | 1]) buffers carries the K / V chunks of the moment phase, then the Q chunks of the
-    // apply phase (X only).  Load number n uses buffer n & 1; its `free` barrier counts the MMAs that read the buffer.
+    // Tiles in order: K and V of every key chunk, then Q.  Tile i uses buffer i & 3; its `free` barrier counts the MMAs that
+    // read it.
     bool ok = true;
-    uint32_t loads = 0;   // loads issued so far (both phases)
-    auto load = [&](int chunk, bool moment) -> bool {
-      const uint32_t buf = loads & 1u;
-      if (loads >= 2 && !WAIT(B_X_FREE + buf, (loads >> 1) - 1u)) { FAIL(400); return false; }
-      const int pos0 = chunk * CH;
-      uint8_t* vb = vbuf + buf * 10 * BLK;
-      if (moment) {
-        for (int r = lane; r < CH; r += 32)  // the ones column of [V | 1] (zero for rows past the last key)
-          *reinterpret_cast<uint4*>(vb + 8 * BLK + r * 16) = make_uint4((pos0 + r < P.nk) ? 0x00003F80u : 0u, 0u, 0u, 0u);
-        fence_proxy_async_smem();
-      }
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&bars[B_X_READY + buf], moment ? REGION + 8 * BLK : REGION);
-        tma_load_4d(xbuf + buf * REGION, moment ? &tmk : &tmq, &bars[B_X_READY + buf], 0, pos0, h_idx, b_idx);
-        if (moment) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) tma_load_4d(vb + j * BLK, &tmv, &bars[B_X_READY + buf], 8 * j, pos0, h_idx, b_idx);
+    const int total = 2 * nkc + nqc;
+    int used = 0;   // tiles consumed so far
+    auto load_ahead = [&]() -> bool {   // as many tiles as the ring holds
+      for (; loads < total && loads < used + RING; ++loads) {
+        const int buf = loads & (RING - 1);
+        if (loads >= RING && !WAIT(B_X_FREE + buf, (uint32_t)(loads / RING) - 1u)) { FAIL(400); return false; }
+        if (lane == 0) {
+          const bool key = loads < 2 * nkc;
+          mbar_arrive_expect_tx(&bars[B_X_READY + buf], REGION);
+          tma_load_4d(xbuf + buf * REGION, !key ? &tmq : (loads & 1) ? &tmv : &tmk, &bars[B_X_READY + buf], 0, (key ? loads >> 1 : loads - 2 * nkc) * CH, h_idx, b_idx);
         }
+        __syncwarp();
       }
-      __syncwarp();
-      ++loads;
       return true;
     };
-    uint32_t used = 0;    // loads consumed so far
+    auto ready = [&](int i) -> bool { return WAIT(B_X_READY + (i & (RING - 1)), (uint32_t)(i / RING)); };
     constexpr uint32_t IDESC_M = make_idesc_bf16(128, 64, 1, 1);    // A MN-major ([V | 1]), B MN-major (K tile)
     constexpr uint32_t IDESC_S0 = make_idesc_bf16(128, 16, 1, 0);   // A MN-major, B K-major (ones)
     constexpr uint32_t IDESC_A = make_idesc_bf16(128, 80, 0, 0);    // A K-major (Q tile), B K-major (c1 S)
     const uint64_t d_ones = make_smem_desc(smem_u32(sm + OFF_ONES), 128, 256, 0);
     // ---- moments ----
-    if (nkc > 0) ok = load(0, true);
-    for (int c = 0; c < nkc && ok; ++c) {
-      if (c + 1 < nkc) ok = load(c + 1, true);
+    for (int c = 0; c < nkc && ok; ++c, used += 2) {
+      ok = load_ahead();
       if (!ok) break;
-      const uint32_t buf = used & 1u;
-      if (!WAIT(B_X_READY + buf, used >> 1)) { FAIL(401); ok = false; break; }
+      if (!ready(used) || !ready(used + 1)) { FAIL(401); ok = false; break; }
       __syncwarp();
       tc_fence_after_sync();
       if (elect_one()) {
-        const uint64_t dV = make_smem_desc(smem_u32(vbuf + buf * 10 * BLK), 128, 2048, 0);
-        const uint64_t dK = make_smem_desc(smem_u32(xbuf + buf * REGION), REGION, 1024, 2);
+        const int bk = used & (RING - 1), bv = bk + 1;
+        const uint64_t dV = make_smem_desc(smem_u32(xbuf + bv * REGION), OFF_V1 - bv * REGION, 1024, 2);
+        const uint64_t dK = make_smem_desc(smem_u32(xbuf + bk * REGION), REGION, 1024, 2);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-          mma_ss(tmem_base + COL_S, dV + (uint64_t)(16 * ks), dK + (uint64_t)(128 * ks), IDESC_M, (c > 0 || ks > 0) ? 1u : 0u);
-          mma_ss(tmem_base + COL_S0, dV + (uint64_t)(16 * ks), d_ones, IDESC_S0, (c > 0 || ks > 0) ? 1u : 0u);
+          mma_ss(tmem_base + COL_S, dV + (uint64_t)(128 * ks), dK + (uint64_t)(128 * ks), IDESC_M, (c > 0 || ks > 0) ? 1u : 0u);
+          mma_ss(tmem_base + COL_S0, dV + (uint64_t)(128 * ks), d_ones, IDESC_S0, (c > 0 || ks > 0) ? 1u : 0u);
         }
-        mma_commit(&bars[B_X_FREE + buf]);
+        mma_commit(&bars[B_X_FREE + bk]);
+        mma_commit(&bars[B_X_FREE + bv]);
         if (c == nkc - 1) mma_commit(&bars[B_S_DONE]);
       }
       __syncwarp();
-      ++used;
     }
     // ---- apply ----
-    if (ok && nqc > 0) ok = load(0, false);
+    if (ok) ok = load_ahead();
     if (ok && nkc > 0 && !WAIT(B_SB_READY, 0)) { FAIL(402); ok = false; }
-    for (int c = 0; c < nqc && ok; ++c) {
-      if (c + 1 < nqc) ok = load(c + 1, false);
+    for (int c = 0; c < nqc && ok; ++c, ++used) {
+      ok = load_ahead();
       if (!ok) break;
-      const uint32_t buf = used & 1u, ob = (uint32_t)c & 1u;
-      if (!WAIT(B_X_READY + buf, used >> 1)) { FAIL(403); ok = false; break; }
+      const uint32_t ob = (uint32_t)c & 1u;
+      if (!ready(used)) { FAIL(403); ok = false; break; }
       if (c >= 2 && !WAIT(B_O_FREE + ob, (uint32_t)(c >> 1) - 1u)) { FAIL(404); ok = false; break; }
       __syncwarp();
       tc_fence_after_sync();
       if (elect_one()) {
+        const int buf = used & (RING - 1);
         const uint64_t dQ = make_smem_desc(smem_u32(xbuf + buf * REGION), 16, 1024, 2);
         const uint64_t dS = make_smem_desc(smem_u32(sb), 16, 1024, 2);
 #pragma unroll
@@ -168,10 +157,9 @@ p1_forward_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant
         mma_commit(&bars[B_O_DONE + ob]);
       }
       __syncwarp();
-      ++used;
     }
     // every MMA has completed before the CTA gives its tensor memory back
-    if (ok && used > 0 && !WAIT(B_X_FREE + ((used - 1u) & 1u), (used - 1u) >> 1)) FAIL(405);
+    if (ok && used > 0 && !WAIT(B_X_FREE + ((used - 1) & (RING - 1)), (uint32_t)((used - 1) / RING))) FAIL(405);
     tc_fence_after_sync();
   } else {
     // ================= epilogues: moment rows -> bf16 operand tile; output rows -> global memory =================
@@ -199,7 +187,7 @@ p1_forward_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant
                            pack_bf16(__uint_as_float(r[4]) * P.c1, __uint_as_float(r[5]) * P.c1),
                            pack_bf16(__uint_as_float(r[6]) * P.c1, __uint_as_float(r[7]) * P.c1));
           }
-          t0[l] = P.c0 * __uint_as_float(r8[0]);
+          t0[l] = P.c0 * (l == 64 ? (float)P.nk : __uint_as_float(r8[0]));   // (the constant tile counts rows past the last key)
         }
         fence_proxy_async_smem();
         tc_fence_before_sync();
@@ -257,6 +245,12 @@ p1_forward_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant
 
   tc_fence_before_sync();
   __syncthreads();
+  if (*abort_flag != 0) {   // a wait ran out: copies in flight still land in this block's shared memory
+    if (w == 4)
+      for (int i = loads > RING ? loads - RING : 0; i < loads; ++i)
+        mbar_wait_bounded(&bars[B_X_READY + (i & (RING - 1))], (uint32_t)(i / RING) & 1u, WAIT_CYCLES);
+    __syncthreads();
+  }
   if (w == 0) tmem_dealloc(tmem_base, 256);
 }
 
