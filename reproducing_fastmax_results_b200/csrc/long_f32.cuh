@@ -325,6 +325,12 @@ __global__ void __launch_bounds__(64) pack_kernel(const float* __restrict__ raw,
         uint32_t o[3][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) split3(pack2(s[2 * j] * wgt, s[2 * j + 1] * wgt), o[0][j], o[1][j], o[2][j]);
+        if (cb == D / 8) {   // piece 0: the column that counts, and the pieces as the chain kernel pairs them with G's
+          const uint32_t hi = o[0][0] & 0xffffu, mid = o[1][0] & 0xffffu, lo = o[2][0] & 0xffffu;
+          o[0][0] = hi | hi << 16;
+          o[0][1] = mid | hi << 16;
+          o[0][2] = mid | lo << 16;
+        }
 #pragma unroll
         for (int p = 0; p < 3; ++p)
           *reinterpret_cast<uint4*>(dst + (long long)k * UNITS * UNIT + p * PIECE) = make_uint4(o[p][0], o[p][1], o[p][2], o[p][3]);
@@ -583,6 +589,9 @@ __global__ void __launch_bounds__(THREADS, 1) apply_kernel(const __grid_constant
 }  // namespace ap
 
 // ---- chain: out += sum_u chain rule through Phi of dphi_u, dphi_u = G S_u^T (see long_kernels.cuh) ---------------------------
+// The six piece products of the denominator column share one K = 16 step: [hi mid hi lo mid hi] of G against [hi hi mid hi mid lo]
+// of S: 13 MMAs per unit instead of 18, and G of two items fits into TMEM, so the next item's is there before this one's
+// products end.
 namespace ch {
 constexpr int THREADS = 384, W_LOAD = 2, W_CHAIN = 4;
 constexpr int S_STAGES = 3;
@@ -591,7 +600,8 @@ constexpr int OFF_X = 0, OFF_P = 4 * LT, OFF_G = OFF_P + 2 * LT, OFF_S = OFF_G +
 static_assert(BYTES <= 232448, "shared memory budget");
 constexpr int B_XFULL = 0, B_XFREE = 2, B_GFULL = 4, B_GFREE = 5, B_GT = 6, B_SFULL = 8, B_SEMPTY = B_SFULL + S_STAGES,
               B_D = B_SEMPTY + S_STAGES, B_DFREE = B_D + 4, B_PFULL = B_DFREE + 4, B_PFREE = B_PFULL + 1, B_DRAIN = B_PFREE + 1, B_COUNT = B_DRAIN + 2;
-constexpr uint32_t COL_D = 256;   // dphi: tile m, buffer b at COL_D + 128 m + 64 b; piece p of G of tile m at 72 m + 24 p
+constexpr uint32_t COL_D = 224;   // dphi: tile m, buffer b at COL_D + 128 m + 64 b
+constexpr uint32_t G_TILE = 56;    // G of item n, tile m at 112 (n & 1) + 56 m: three pieces of 16 columns, the tail of 8
 
 __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant__ lng::Maps M, const lng::Params P) {
   extern __shared__ uint8_t smem_raw[];
@@ -623,12 +633,12 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
 
   int xs = 0, gs = 0, parts = 0, ss = 0;
   if (w == W_LOAD) {
-    int n = 0;
-    for (int idx = blockIdx.x; idx < P.nitems && *abort_flag == 0; idx += gridDim.x, ++n) {
+    // x and G of item n (of this block), as soon as the last users have let go
+    auto load_item = [&](int idx, int n) {
       const Work k = work(idx, P);
       if (n >= 2) WAIT(B_XFREE + (n & 1), (uint32_t)(n >> 1) - 1u, 160);
       if (n >= 1) WAIT(B_GFREE, (uint32_t)n - 1u, 161);
-      if (*abort_flag != 0) break;
+      if (*abort_flag != 0) return;
       if (lane == 0) {
         mbar_arrive_expect_tx(&bars[B_GFULL], 6 * GT);
         for (int i = 0; i < 6; ++i) tma_load_4d(sm + OFF_G + i * GT, &M.y, &bars[B_GFULL], 0, k.tok + (i / 3) * 128, k.head, i % 3);
@@ -637,6 +647,12 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
         for (int m = 0; m < 2; ++m) tma_load_4d(sm + ((n & 1) * 2 + m) * LT, &M.x, bar, 0, k.tok + m * 128, k.h, k.b);
       }
       xs = gs = n + 1;
+    };
+    int n = 0;
+    if ((int)blockIdx.x < P.nitems) load_item(blockIdx.x, 0);
+    const int ahead = min(3, units - 1);   // unit after which the next item's tiles are asked for: the chain warps take G later
+    for (int idx = blockIdx.x; idx < P.nitems && *abort_flag == 0; idx += gridDim.x, ++n) {
+      const Work k = work(idx, P);
       const uint8_t* src = P.S + ((long long)k.st * UNITS + u0) * UNIT;
       for (int j = 0; j < units; ++j, ++ss) {
         const int s = ss % S_STAGES;
@@ -646,6 +662,7 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
           mbar_arrive_expect_tx(&bars[B_SFULL + s], UNIT);
           bulk_load(sm + OFF_S + s * UNIT, src + (long long)j * UNIT, UNIT, &bars[B_SFULL + s]);
         }
+        if (j == ahead && idx + (int)gridDim.x < P.nitems) load_item(idx + gridDim.x, n + 1);
       }
       if (P.part) {
         if (n >= 1) WAIT(B_PFREE, (uint32_t)n - 1u, 163);
@@ -669,7 +686,9 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
         if (sg >= 2) WAIT(B_DFREE + 2 * w + (int)buf, (sg >> 1) - 1u, 166);
         tc_fence_after_sync();
         const uint64_t dS = make_smem_desc(smem_u32(sm + OFF_S) + s * UNIT, 1024, 128, 0);
-        product<3>(tmem + COL_D + 128u * w + 64u * buf, tmem + 72u * w, 24u, dS, PIECE >> 4, 128u, ID, 3);
+        const uint32_t acc = tmem + COL_D + 128u * w + 64u * buf, ga = tmem + G_TILE * (2u * (n & 1) + w);
+        product<2>(acc, ga, 16u, dS, PIECE >> 4, 128u, ID, 2);
+        mma_ts_elect(acc, ga + 48u, dS + (uint64_t)256, ID, 1u);
         mma_commit_elect(&bars[B_D + 2 * w + buf]);
         mma_commit_elect(&bars[B_SEMPTY + s]);
       }
@@ -681,25 +700,24 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
   } else if (w >= W_CHAIN) {
     const int m = (w - W_CHAIN) >> 2, quarter = w & 3, l = quarter * 32 + lane, sw = lane & 7;
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-    uint32_t sg = 0;
-    int n = 0;
-    for (int idx = blockIdx.x; idx < P.nitems && *abort_flag == 0; idx += gridDim.x, ++n) {
-      const Work k = work(idx, P);
-      const int row = k.tok + m * 128 + l;
+    auto take_g = [&](int n) {   // G of item n: shared memory -> TMEM
       WAIT(B_GFULL, (uint32_t)n, 167);
+      const uint32_t dst = lane_addr + G_TILE * (2u * (n & 1) + m);
+      uint32_t tail[3];
 #pragma unroll
       for (int p = 0; p < 3; ++p) {
         const uint4* src = reinterpret_cast<const uint4*>(sm + OFF_G + (3 * m + p) * GT + l * (NC * 2));
-        uint32_t r[16], r8[8];
+        uint32_t r[16];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) {
+        for (int c = 0; c < 4; ++c) {
           const uint4 v = src[c];
-          uint32_t* d = c < 4 ? r + 4 * c : r8 + 4 * (c - 4);
-          d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+          r[4 * c] = v.x; r[4 * c + 1] = v.y; r[4 * c + 2] = v.z; r[4 * c + 3] = v.w;
         }
-        tmem_st16(lane_addr + 72u * m + 24u * p, r);
-        tmem_st8(lane_addr + 72u * m + 24u * p + 16u, r8);
+        tail[p] = src[4].x & 0xffffu;
+        tmem_st16(dst + 16u * p, r);
       }
+      const uint32_t r8[8] = {tail[0] | tail[1] << 16, tail[0] | tail[2] << 16, tail[1] | tail[0] << 16, 0u, 0u, 0u, 0u, 0u};
+      tmem_st8(dst + 48u, r8);
       tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
@@ -707,6 +725,13 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
         mbar_arrive(&bars[B_GT + m]);
         mbar_arrive(&bars[B_GFREE]);
       }
+    };
+    if ((int)blockIdx.x < P.nitems) take_g(0);
+    uint32_t sg = 0;
+    int n = 0;
+    for (int idx = blockIdx.x; idx < P.nitems && *abort_flag == 0; idx += gridDim.x, ++n) {
+      const Work k = work(idx, P);
+      const int row = k.tok + m * 128 + l;
       WAIT(B_XFULL + (n & 1), (uint32_t)(n >> 1), 168);
       const uint8_t* x = sm + ((n & 1) * 2 + m) * LT + l * 128;
       uint64_t acc[16];
@@ -731,6 +756,7 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
       if (u0 == 0) {
 #pragma unroll
         for (int a = 0; a < NB; ++a) {
+          if (a == 1 && idx + (int)gridDim.x < P.nitems) take_g(n + 1);
           uint64_t xa[4], t[8];
           block(a, xa);
 #pragma unroll
@@ -771,6 +797,7 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
           }
         }
       }
+      if (u0 > 0 && idx + (int)gridDim.x < P.nitems) take_g(n + 1);
       {   // the linear unit
         const uint32_t addr = next_unit();
         uint32_t d[32];
