@@ -221,6 +221,17 @@ int32_t fastmax_normalize_backward(int32_t batch, int32_t heads, int32_t n, int3
                                    const fastmax_tensor* dx, const uint64_t* stats, float* scratch_bh,
                                    void* cuda_stream);
 
+/* The same for the queries and the keys of a call, in one launch where both are large enough. */
+int32_t fastmax_normalize_forward_qk(int32_t batch, int32_t heads, int32_t nq, int32_t nk, int32_t d, int32_t dtype,
+                                     float lim, const fastmax_tensor* q, const fastmax_tensor* yq,
+                                     const fastmax_tensor* k, const fastmax_tensor* yk,
+                                     uint64_t* stats_q, uint64_t* stats_k, void* cuda_stream);
+int32_t fastmax_normalize_backward_qk(int32_t batch, int32_t heads, int32_t nq, int32_t nk, int32_t d, int32_t dtype,
+                                      float lim, const fastmax_tensor* yq, const fastmax_tensor* dyq, const fastmax_tensor* dxq,
+                                      const fastmax_tensor* yk, const fastmax_tensor* dyk, const fastmax_tensor* dxk,
+                                      const uint64_t* stats_q, const uint64_t* stats_k, float* scratch_bh,
+                                      void* cuda_stream);
+
 /* ---- diagnostics ---------------------------------------------------------------------------------- */
 const char* fastmax_status_string(int32_t status);
 int32_t fastmax_last_cuda_error(void);           /* cudaError_t of the calling thread's last failing runtime call */

@@ -424,7 +424,8 @@ __global__ void norm_bwd_apply_vec_kernel(View y, View dy, View dx, int n, int h
 }
 
 // ---- one-launch variants: a thread-block cluster per (batch, head) ---------------------------------------------
-// gridDim = (CL, batch*heads) with CL blocks of 256 threads per cluster.  Pass 1: every block walks its share of the
+// gridDim = (CL, batch*heads, tensors) with CL blocks of 256 threads per cluster; q and k of a call go in one launch (two of
+// 1024 blocks each were 31 us for 128 heads of 1024 tokens, most of it the start and the end of a launch).  Pass 1: every block walks its share of the
 // head's tokens and reduces (max squared norm / sum dy.y); the CL partial results meet through distributed shared
 // memory (each block reads its peers' partial after a cluster barrier, in rank order, so the sum does not depend on
 // timing).  Pass 2 walks the same tokens in the opposite order and writes the result; what it reads again comes from
@@ -432,8 +433,21 @@ __global__ void norm_bwd_apply_vec_kernel(View y, View dy, View dx, int n, int h
 // (Measured against this form on B8 H16 N4096 D64 bf16, forward + backward, 0.113 ms: blocks of 1024 threads, one
 // per SM, that keep their loads in registers between the passes took 0.156 ms, since with one block per SM nothing
 // overlaps the barrier between the passes; fewer resident blocks of this form, for more L2 hits, took 0.119 ms.)
+struct NormArgs {
+  View x[2], y[2];
+  int n[2];
+  unsigned long long* stats[2];
+};
+struct NormBwdArgs {
+  View y[2], dy[2], dx[2];
+  int n[2];
+  const unsigned long long* stats[2];
+};
 template <typename T, int LPR>
-__global__ void __launch_bounds__(256) norm_fused_vec_kernel(View x, View y, int n, int heads, unsigned long long* stats, float lim) {
+__global__ void __launch_bounds__(256) norm_fused_vec_kernel(const NormArgs A, int heads, float lim) {
+  const View x = A.x[blockIdx.z], y = A.y[blockIdx.z];
+  const int n = A.n[blockIdx.z];
+  unsigned long long* stats = A.stats[blockIdx.z];
   constexpr int D = 8 * LPR, RPI = 256 / LPR;
   namespace cgx = cooperative_groups;
   cgx::cluster_group cluster = cgx::this_cluster();
@@ -513,8 +527,10 @@ __global__ void __launch_bounds__(256) norm_fused_vec_kernel(View x, View y, int
 }
 
 template <typename T, int LPR>
-__global__ void __launch_bounds__(256) norm_bwd_fused_vec_kernel(View y, View dy, View dx, int n, int heads,
-                                                                  const unsigned long long* stats, float lim) {
+__global__ void __launch_bounds__(256) norm_bwd_fused_vec_kernel(const NormBwdArgs A, int heads, float lim) {
+  const View y = A.y[blockIdx.z], dy = A.dy[blockIdx.z], dx = A.dx[blockIdx.z];
+  const int n = A.n[blockIdx.z];
+  const unsigned long long* stats = A.stats[blockIdx.z];
   constexpr int D = 8 * LPR, RPI = 256 / LPR;
   namespace cgx = cooperative_groups;
   cgx::cluster_group cluster = cgx::this_cluster();

@@ -530,8 +530,8 @@ int32_t fastmax_forward(const fastmax_problem* pb, const fastmax_forward_args* a
     keys.flags |= FASTMAX_FLAG_SINGLE_STREAM;
     const size_t own = align_up(fastmax_forward_workspace(pb, &out_call), 256);
     SideBranch branch(pb, st);
-    rc = fastmax_forward(&keys, &state_call, (char*)ws + own, ws_bytes - own, branch.side);
-    if (rc == FASTMAX_OK) rc = pair_forward(pb, &out_call, ws, st);
+    rc = pair_forward(pb, &out_call, ws, st);
+    if (rc == FASTMAX_OK) rc = fastmax_forward(&keys, &state_call, (char*)ws + own, ws_bytes - own, branch.side);
     const cudaError_t e = branch.join();
     return rc != FASTMAX_OK ? rc : e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
   }
@@ -870,10 +870,10 @@ static int norm_cluster_size(int batch, int heads, int n, int d) {
   if (bh * cl < 2LL * sm_count()) return 0;
   return cl;
 }
-#define FM_NORM_FUSED(KERNEL, CL, ...)                                                                  \
+#define FM_NORM_FUSED(KERNEL, CL, COUNT, ...)                                                                  \
   do {                                                                                                  \
     cudaLaunchConfig_t cfg = {};                                                                        \
-    cfg.gridDim = dim3((unsigned)(CL), (unsigned)(batch * heads));                                      \
+    cfg.gridDim = dim3((unsigned)(CL), (unsigned)(batch * heads), (unsigned)(COUNT));                                      \
     cfg.blockDim = dim3(256);                                                                           \
     cfg.stream = st;                                                                                    \
     cudaLaunchAttribute attr[1];                                                                        \
@@ -903,15 +903,17 @@ int32_t fastmax_normalize_forward(int32_t batch, int32_t heads, int32_t n, int32
   if (dtype != FASTMAX_F32 && dtype != FASTMAX_BF16) return FASTMAX_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   long long nrows = (long long)batch * heads * n;
-  FM_CUDA(cudaMemsetAsync(stats, 0, (size_t)batch * heads * sizeof(uint64_t), st));
+  const int cl = nrows > 0 && norm_vec_ok(d, dtype, {x, y}) && (long long)batch * heads <= 65535 ? norm_cluster_size(batch, heads, n, d) : 0;
+  if (cl == 0) FM_CUDA(cudaMemsetAsync(stats, 0, (size_t)batch * heads * sizeof(uint64_t), st));   // (the cluster kernel writes all of it)
   if (nrows == 0) return FASTMAX_OK;
   int threads = 256;
   unsigned blocks = (unsigned)((nrows * 32 + threads - 1) / threads);
   unsigned long long* sp = reinterpret_cast<unsigned long long*>(stats);
   if (norm_vec_ok(d, dtype, {x, y}) && (long long)batch * heads <= 65535) {
-    if (const int cl = norm_cluster_size(batch, heads, n, d)) {
+    if (cl > 0) {
+      const NormArgs A{{to_view(*x)}, {to_view(*y)}, {(int)n}, {sp}};
       LaunchScope ls(KK_NORMALIZE, st);
-      FM_NORM_FUSED(norm_fused_vec_kernel, cl, to_view(*x), to_view(*y), (int)n, (int)heads, sp, lim);
+      FM_NORM_FUSED(norm_fused_vec_kernel, cl, 1, A, (int)heads, lim);
       return FASTMAX_OK;
     }
     {
@@ -952,15 +954,17 @@ int32_t fastmax_normalize_backward(int32_t batch, int32_t heads, int32_t n, int3
   if (dtype != FASTMAX_F32 && dtype != FASTMAX_BF16) return FASTMAX_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   long long nrows = (long long)batch * heads * n;
-  FM_CUDA(cudaMemsetAsync(scratch, 0, (size_t)batch * heads * sizeof(float), st));
+  const int cl = nrows > 0 && norm_vec_ok(d, dtype, {y, dy, dx}) && (long long)batch * heads <= 65535 ? norm_cluster_size(batch, heads, n, d) : 0;
+  if (cl == 0) FM_CUDA(cudaMemsetAsync(scratch, 0, (size_t)batch * heads * sizeof(float), st));
   if (nrows == 0) return FASTMAX_OK;
   int threads = 256;
   unsigned blocks = (unsigned)((nrows * 32 + threads - 1) / threads);
   const unsigned long long* sp = reinterpret_cast<const unsigned long long*>(stats);
   if (norm_vec_ok(d, dtype, {y, dy, dx}) && (long long)batch * heads <= 65535) {
-    if (const int cl = norm_cluster_size(batch, heads, n, d)) {
+    if (cl > 0) {
+      const NormBwdArgs A{{to_view(*y)}, {to_view(*dy)}, {to_view(*dx)}, {(int)n}, {sp}};
       LaunchScope ls(KK_NORMALIZE, st);
-      FM_NORM_FUSED(norm_bwd_fused_vec_kernel, cl, to_view(*y), to_view(*dy), to_view(*dx), (int)n, (int)heads, sp, lim);
+      FM_NORM_FUSED(norm_bwd_fused_vec_kernel, cl, 1, A, (int)heads, lim);
       return FASTMAX_OK;
     }
     {
@@ -990,6 +994,46 @@ int32_t fastmax_normalize_backward(int32_t batch, int32_t heads, int32_t n, int3
   }
   FM_CUDA(cudaGetLastError());
   return FASTMAX_OK;
+}
+
+// Queries and keys of a call: one launch where both take the cluster kernel, else one after the other.
+int32_t fastmax_normalize_forward_qk(int32_t batch, int32_t heads, int32_t nq, int32_t nk, int32_t d, int32_t dtype, float lim,
+                                     const fastmax_tensor* q, const fastmax_tensor* yq, const fastmax_tensor* k, const fastmax_tensor* yk,
+                                     uint64_t* stats_q, uint64_t* stats_k, void* stream) {
+  const int most = nq > nk ? nq : nk;
+  if (q && yq && k && yk && q->ptr && yq->ptr && k->ptr && yk->ptr && stats_q && stats_k && batch > 0 && heads > 0 && nq > 0 && nk > 0 && lim > 0.f &&
+      (dtype == FASTMAX_F32 || dtype == FASTMAX_BF16) && norm_vec_ok(d, dtype, {q, yq, k, yk}) && (long long)batch * heads <= 65535) {
+    if (const int cl = norm_cluster_size(batch, heads, most, d)) {
+      cudaStream_t st = (cudaStream_t)stream;
+      const NormArgs A{{to_view(*q), to_view(*k)}, {to_view(*yq), to_view(*yk)}, {(int)nq, (int)nk},
+                       {reinterpret_cast<unsigned long long*>(stats_q), reinterpret_cast<unsigned long long*>(stats_k)}};
+      LaunchScope ls(KK_NORMALIZE, st);
+      FM_NORM_FUSED(norm_fused_vec_kernel, cl, 2, A, (int)heads, lim);
+      return FASTMAX_OK;
+    }
+  }
+  const int32_t rc = fastmax_normalize_forward(batch, heads, nq, d, dtype, lim, q, yq, stats_q, stream);
+  return rc != FASTMAX_OK ? rc : fastmax_normalize_forward(batch, heads, nk, d, dtype, lim, k, yk, stats_k, stream);
+}
+int32_t fastmax_normalize_backward_qk(int32_t batch, int32_t heads, int32_t nq, int32_t nk, int32_t d, int32_t dtype, float lim,
+                                      const fastmax_tensor* yq, const fastmax_tensor* dyq, const fastmax_tensor* dxq, const fastmax_tensor* yk,
+                                      const fastmax_tensor* dyk, const fastmax_tensor* dxk, const uint64_t* stats_q, const uint64_t* stats_k,
+                                      float* scratch, void* stream) {
+  const int most = nq > nk ? nq : nk;
+  if (yq && dyq && dxq && yk && dyk && dxk && yq->ptr && dyq->ptr && dxq->ptr && yk->ptr && dyk->ptr && dxk->ptr && stats_q && stats_k && batch > 0 &&
+      heads > 0 && nq > 0 && nk > 0 && lim > 0.f && (dtype == FASTMAX_F32 || dtype == FASTMAX_BF16) &&
+      norm_vec_ok(d, dtype, {yq, dyq, dxq, yk, dyk, dxk}) && (long long)batch * heads <= 65535) {
+    if (const int cl = norm_cluster_size(batch, heads, most, d)) {
+      cudaStream_t st = (cudaStream_t)stream;
+      const NormBwdArgs A{{to_view(*yq), to_view(*yk)}, {to_view(*dyq), to_view(*dyk)}, {to_view(*dxq), to_view(*dxk)}, {(int)nq, (int)nk},
+                          {reinterpret_cast<const unsigned long long*>(stats_q), reinterpret_cast<const unsigned long long*>(stats_k)}};
+      LaunchScope ls(KK_NORMALIZE, st);
+      FM_NORM_FUSED(norm_bwd_fused_vec_kernel, cl, 2, A, (int)heads, lim);
+      return FASTMAX_OK;
+    }
+  }
+  const int32_t rc = fastmax_normalize_backward(batch, heads, nq, d, dtype, lim, yq, dyq, dxq, stats_q, scratch, stream);
+  return rc != FASTMAX_OK ? rc : fastmax_normalize_backward(batch, heads, nk, d, dtype, lim, yk, dyk, dxk, stats_k, scratch, stream);
 }
 
 }  // extern "C"

@@ -84,12 +84,15 @@ torch::Tensor forwardpass(torch::Tensor q, torch::Tensor k, torch::Tensor v, tor
   // the reference scales k by 1/temperature in place (fwd.cu:282-292) and normalises q, k in place
   // (fwd.cu:424-433); callers keep the mutated tensors for backward (model.py:29-37).
   if (normalize) {
-    auto stats = torch::empty({bh}, q.options().dtype(torch::kInt64));
+    auto stats = torch::empty({2 * bh}, q.options().dtype(torch::kInt64));
+    uint64_t* sp = (uint64_t*)stats.data_ptr();
     fastmax_tensor qv = view_nbd(q), kv = view_nbd(k);
-    check_status(fastmax_normalize_forward(1, bh, nq, d, FASTMAX_F32, lim, &qv, &qv, (uint64_t*)stats.data_ptr(), stream),
-                 "fastmax normalize(q)");
-    check_status(fastmax_normalize_forward(1, bh, nk, d, FASTMAX_F32, lim, &kv, &kv, (uint64_t*)stats.data_ptr(), stream),
-                 "fastmax normalize(k)");
+    if (qv.ptr == kv.ptr) {   // one tensor for both: one after the other
+      check_status(fastmax_normalize_forward(1, bh, nq, d, FASTMAX_F32, lim, &qv, &qv, sp, stream), "fastmax normalize(q)");
+      check_status(fastmax_normalize_forward(1, bh, nk, d, FASTMAX_F32, lim, &kv, &kv, sp, stream), "fastmax normalize(k)");
+    } else {
+      check_status(fastmax_normalize_forward_qk(1, bh, nq, nk, d, FASTMAX_F32, lim, &qv, &qv, &kv, &kv, sp, sp + bh, stream), "fastmax normalize");
+    }
   }
   if (temperature != 1.0f) {   // k <- k / temperature in place, as apply_rpe_and_temp does (fwd.cu:282-292)
     fastmax_tensor kv = view_nbd(k);
@@ -352,6 +355,39 @@ torch::Tensor normalize_backward(torch::Tensor y, torch::Tensor dy, torch::Tenso
   return dx;
 }
 
+// q and k of a call: (yq, stats_q, yk, stats_k), one launch where both are large enough
+static std::vector<torch::Tensor> normalize_forward_qk(const torch::Tensor& q, const torch::Tensor& k, double lim) {
+  if (q.scalar_type() != k.scalar_type() || q.size(0) != k.size(0) || q.size(1) != k.size(1) || q.size(3) != k.size(3)) {
+    auto a = normalize_forward(q, lim), b = normalize_forward(k, lim);
+    return {a[0], a[1], b[0], b[1]};
+  }
+  CHECK_CUDA(q); CHECK_CUDA(k);
+  const c10::cuda::CUDAGuard guard(q.device());
+  auto stream = at::cuda::getCurrentCUDAStream().stream();
+  auto yq = torch::empty_like(q), yk = torch::empty_like(k);
+  auto stats = torch::empty({2, q.size(0), q.size(1)}, q.options().dtype(torch::kInt64));
+  auto sq = stats.select(0, 0), sk = stats.select(0, 1);
+  fastmax_tensor qv = view_bhnd(q), yqv = view_bhnd(yq), kv = view_bhnd(k), ykv = view_bhnd(yk);
+  check_status(fastmax_normalize_forward_qk(q.size(0), q.size(1), q.size(2), k.size(2), q.size(3), dtype_of(q), (float)lim, &qv, &yqv, &kv, &ykv,
+                                            (uint64_t*)sq.data_ptr(), (uint64_t*)sk.data_ptr(), stream),
+               "fastmax normalize_forward");
+  return {yq, sq, yk, sk};
+}
+static void normalize_backward_qk(const torch::Tensor& yq, torch::Tensor& dq, const torch::Tensor& sq, const torch::Tensor& yk, torch::Tensor& dk,
+                                  const torch::Tensor& sk, double lim) {
+  const c10::cuda::CUDAGuard guard(yq.device());
+  auto stream = at::cuda::getCurrentCUDAStream().stream();
+  auto dxq = torch::empty_like(yq), dxk = torch::empty_like(yk);
+  auto scratch = torch::empty({yq.size(0) * yq.size(1)}, yq.options().dtype(torch::kFloat32));
+  fastmax_tensor yqv = view_bhnd(yq), dqv = view_bhnd(dq), dxqv = view_bhnd(dxq), ykv = view_bhnd(yk), dkv = view_bhnd(dk), dxkv = view_bhnd(dxk);
+  check_status(fastmax_normalize_backward_qk(yq.size(0), yq.size(1), yq.size(2), yk.size(2), yq.size(3), dtype_of(yq), (float)lim, &yqv, &dqv, &dxqv,
+                                             &ykv, &dkv, &dxkv, (const uint64_t*)sq.data_ptr(), (const uint64_t*)sk.data_ptr(),
+                                             (float*)scratch.data_ptr(), stream),
+               "fastmax normalize_backward");
+  dq = dxq;
+  dk = dxk;
+}
+
 // k <- k * inv_temp (+ rpe rows) in place; returns k
 torch::Tensor key_prologue(torch::Tensor k, double inv_temp, c10::optional<torch::Tensor> rpe) {
   CHECK_CUDA(k);
@@ -415,10 +451,9 @@ struct FastmaxNode : public torch::autograd::Function<FastmaxNode> {
       q = readable(q); k = readable(k); v = readable(v);
     }
     if (normalize) {
-      auto nq = normalize_forward(q, lim);
-      auto nk = normalize_forward(k, lim);
-      q = nq[0]; stats_q = nq[1];
-      k = nk[0]; stats_k = nk[1];
+      auto n = normalize_forward_qk(q, k, lim);
+      q = n[0]; stats_q = n[1];
+      k = n[2]; stats_k = n[3];
     }
     c10::optional<torch::Tensor> out;
     if (contiguous) out = torch::empty(q.sizes(), q.options());
@@ -446,10 +481,7 @@ struct FastmaxNode : public torch::autograd::Function<FastmaxNode> {
     auto res = ::backward(saved[0], saved[1], saved[2], saved[3], saved[4], go, d["mask"].toBool(), d["inv_t"].toDouble(), d["a0"].toDouble(),
                           d["a1"].toDouble(), d["a2"].toDouble(), d["p"].toInt(), c10::nullopt, c10::nullopt, false, true,
                           FASTMAX_FLAG_PAIRWISE, outs, km, c10::nullopt, false);
-    if (d["normalize"].toBool()) {
-      res[0] = normalize_backward(saved[0], res[0], saved[5], d["lim"].toDouble());
-      res[1] = normalize_backward(saved[1], res[1], saved[6], d["lim"].toDouble());
-    }
+    if (d["normalize"].toBool()) normalize_backward_qk(saved[0], res[0], saved[5], saved[1], res[1], saved[6], d["lim"].toDouble());
     torch::Tensor none;
     return {res[0], res[1], res[2], none, none, none, none, none, none, none, none, none, none, none};
   }

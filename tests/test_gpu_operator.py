@@ -353,3 +353,31 @@ def test_medium_matmul_precision_with_every_option_of_the_operator_switched_on()
     assert {"tc_pad", "tc_scan_fwd", "tc_scan_bwd_q"} <= kinds_fast and "scan_fwd" not in kinds_fast, kinds_fast
     for a, b, name in zip(fast, exact, ("out", "dq", "dk", "dv")):
         assert orc.max_norm_err(host(a), host(b)) < 2e-2, name
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_normalisation_of_q_and_k_in_one_launch(dtype):
+    """Enough heads for the one-launch form, more queries than keys: same values as tensor by tensor, and one launch each way."""
+    from reproducing_fastmax_results_b200 import _lib as L
+    from reproducing_fastmax_results_b200.attention import fastmax_custom
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, do = (torch.randn(4, 40, 300, 32, device="cuda", generator=g).to(dtype) for _ in range(2))
+    k, v = (torch.randn(4, 40, 131, 32, device="cuda", generator=g).to(dtype) for _ in range(2))
+    yq, sq = L.normalize_forward(q, 1.0)
+    yk, sk = L.normalize_forward(k, 1.0)
+    plain = [t.clone().requires_grad_(True) for t in (yq, yk, v)]
+    options = (1.0, 1.0, 1.0, 0.5, 1.0, 2)
+    ref = fastmax_custom(*plain, None, None, False, 0.0, False, *options)
+    dyq, dyk, _ = torch.autograd.grad(ref, plain, do)
+    dq_ref, dk_ref = L.normalize_backward(yq, dyq, sq, 1.0), L.normalize_backward(yk, dyk, sk, 1.0)
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    L.profile_collect()
+    L.profile(True)
+    o = fastmax_custom(*leaves, None, None, False, 0.0, True, *options)
+    dq, dk, _ = torch.autograd.grad(o, leaves, do)
+    torch.cuda.synchronize()
+    L.profile(False)
+    assert L.profile_collect()["normalize"][1] == 2
+    assert torch.equal(o, ref) and torch.equal(dq, dq_ref)
+    assert (dk - dk_ref).float().norm() < (1e-6 if dtype == torch.float32 else 1e-2) * dk_ref.float().norm()   # sums in another order
