@@ -888,7 +888,10 @@ int chosen(const fastmax_problem* pb, bool backward, Use use) {   // 0: neither,
   }
   // order 1 without a mask: one pass over the tensors (p1_forward_kernel), always the cheapest where it fills the GPU
   if (!backward && pb->order == 1 && !pb->causal && pb->d == 64 && (long long)pb->batch * pb->heads >= 64) return 0;
-  if (pb->d == 16) return per_token <= (pb->order == 2 ? 6500.0 : backward ? 1300.0 : 2000.0) ? 1 : 0;   // no states kernel
+  // d = 16 has no states kernel.  Causal calls beyond 3000 tokens stay with the CUDA-core engine: the first tokens' gradients are
+  // a hundred times the others there, and the float32 weights of that engine round their bf16 results to the last bit.
+  if (pb->d == 16)
+    return per_token <= (pb->order == 2 ? (pb->causal ? 1500.0 : 6500.0) : backward || pb->causal ? 1300.0 : 2000.0) ? 1 : 0;
   if (per_token <= window_line(pb, use)) return 1;
   if (pb->causal && pb->nq != pb->nk) return per_token <= (pb->order == 2 ? 6500.0 : backward ? 1300.0 : 2000.0) ? 1 : 0;
   if ((long long)(pb->nq > pb->nk ? pb->nq : pb->nk) >= (1ll << 30)) return 0;
