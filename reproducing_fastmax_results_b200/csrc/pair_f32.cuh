@@ -10,6 +10,8 @@
 // for every streamed tile (64 rows: four additions of hi hi behind the twenty small ones, which go first) and the
 // element-wise warps add the tile's result to float32 totals in registers, rounding to nearest.
 //
+// Measured: 128 heads of 1024 x 64, causal, forward + backward with splitting 13400 us in the CUDA-core engine (FFMA), 600 here.
+//
 // Roles and hand-offs are those of the bf16 kernels; the streamed pair's two tiles have barriers of their own, because with
 // three pieces each only two or three stages fit and each tile can be let go at a different time.
 #pragma once
