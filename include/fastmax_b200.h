@@ -98,7 +98,9 @@ size_t fastmax_state_bytes(const fastmax_problem* pb); /* all batch*heads states
  *       (not on state_in), so a caller that comes back with the same k and v -- the forward after a state-only call
  *       of a sequence-parallel rank, the backward after the forward -- can hand them back and save that pass.
  *       key_moments_out receives them (fastmax_key_moments_bytes() bytes, float32); key_moments_in must hold what an
- *       earlier call with the same problem, k and v wrote.  No counterpart in the reference, which has no segments. */
+ *       earlier call with the same problem, k and v wrote, and that call must have been given the same number of bytes:
+ *       the array has a form per engine (segment sums, or the packed window states of FASTMAX_FLAG_PAIRWISE), and no two
+ *       forms have the same size.  No counterpart in the reference, which has no segments. */
 typedef struct {
   fastmax_tensor q, k, v;
   fastmax_tensor o;
@@ -115,7 +117,7 @@ size_t fastmax_forward_workspace(const fastmax_problem* pb, const fastmax_forwar
  * this for the bfloat16 form of its problem before it converts anything. */
 int32_t fastmax_forward_engine(const fastmax_problem* pb, const fastmax_forward_args* args);
 /* Size of the key_moments arrays for this problem and these arguments, or 0 when this call would neither write nor
- * read them (one segment per head, no keys, or a call the tensor-memory kernels take). */
+ * read them (one segment per head, no keys, pairs without windows, or a call the tensor-memory kernels take whole). */
 size_t fastmax_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_args* args);
 int32_t fastmax_forward(const fastmax_problem* pb, const fastmax_forward_args* args,
                         void* workspace, size_t workspace_bytes, void* cuda_stream);
@@ -145,7 +147,10 @@ int32_t fastmax_forward_static_scratch(const fastmax_problem* pb, const fastmax_
  *   dstate_in    : gradient moments sum Phi(q)^T dO' of LATER queries (sequence-parallel), or NULL.
  *   dstate_out   : dstate_in + this call's gradient moments, or NULL.
  *   If dq.ptr, dk.ptr and dv.ptr are all NULL only dstate_out is produced.
- *   key_moments_in (optional): what the forward call of the same problem, k and v wrote to key_moments_out.
+ *   key_moments_in (optional): what the forward call of the same problem, k and v wrote to key_moments_out.  Read where
+ *       fastmax_backward_key_moments_bytes() is the number of bytes that call was given: which form a backward call reads
+ *       depends on its own arguments (carried states, rows of the gradients).  An array of the other form is not read: the
+ *       call then passes over k and v itself.
  *   grad_moments_out / grad_moments_in (optional): the same for the per-segment sums Phi(Q)^T dO' of this call's
  *       q, o, g and d_out: the state-only call of a sequence-parallel rank writes them, its gradient call reads them
  *       (fastmax_grad_moments_bytes() bytes, float32). */
@@ -161,6 +166,8 @@ typedef struct {
 } fastmax_backward_args;
 
 size_t fastmax_backward_workspace(const fastmax_problem* pb, const fastmax_backward_args* args);
+/* Size of the key_moments array this backward call reads, or 0 when it reads none. */
+size_t fastmax_backward_key_moments_bytes(const fastmax_problem* pb, const fastmax_backward_args* args);
 /* Size of the grad_moments arrays, or 0 when this call would neither write nor read them. */
 size_t fastmax_grad_moments_bytes(const fastmax_problem* pb, const fastmax_backward_args* args);
 int32_t fastmax_backward(const fastmax_problem* pb, const fastmax_backward_args* args,

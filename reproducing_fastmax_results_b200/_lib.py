@@ -21,7 +21,7 @@ EXPORTED_SYMBOLS = [
     "fastmax_state_rows", "fastmax_state_ld", "fastmax_state_bytes",
     "fastmax_forward_workspace", "fastmax_forward", "fastmax_key_moments_bytes", "fastmax_forward_engine",
     "fastmax_static_scratch_bytes", "fastmax_forward_static_scratch",
-    "fastmax_backward_workspace", "fastmax_backward", "fastmax_grad_moments_bytes",
+    "fastmax_backward_workspace", "fastmax_backward", "fastmax_backward_key_moments_bytes", "fastmax_grad_moments_bytes",
     "fastmax_decode_step",
     "fastmax_normalize_forward", "fastmax_normalize_backward",
     "fastmax_key_prologue", "fastmax_output_noise",
@@ -112,6 +112,8 @@ def load():
     lib.fastmax_forward_static_scratch.argtypes = [C.POINTER(Problem), C.POINTER(ForwardArgs), C.c_void_p]
     lib.fastmax_backward_workspace.restype = C.c_size_t
     lib.fastmax_backward_workspace.argtypes = [C.POINTER(Problem), C.POINTER(BackwardArgs)]
+    lib.fastmax_backward_key_moments_bytes.restype = C.c_size_t
+    lib.fastmax_backward_key_moments_bytes.argtypes = [C.POINTER(Problem), C.POINTER(BackwardArgs)]
     lib.fastmax_grad_moments_bytes.restype = C.c_size_t
     lib.fastmax_grad_moments_bytes.argtypes = [C.POINTER(Problem), C.POINTER(BackwardArgs)]
     lib.fastmax_backward.restype = C.c_int32
@@ -202,19 +204,19 @@ def _workspace(nbytes, device):
     return ws, C.c_void_p(ptr)
 
 
-def _attach_key_moments(lib, pb, fargs, key_moments, device, sink, allow_fill):
-    """Points sink.key_moments_in at the holder's buffer when it fits this call, or (allow_fill) gives the call a new
-    buffer to fill.  `fargs`: the ForwardArgs that describe the call to fastmax_key_moments_bytes."""
+def _attach_key_moments(lib, pb, args, key_moments, device):
+    """Points args.key_moments_in at the holder's buffer when it has the size, and with it the form, of this forward call,
+    else gives the call a new buffer to fill."""
     import torch
 
-    nbytes = lib.fastmax_key_moments_bytes(C.byref(pb), C.byref(fargs))
+    nbytes = lib.fastmax_key_moments_bytes(C.byref(pb), C.byref(args))
     if nbytes == 0:
         return
     if key_moments.buf is not None and key_moments.buf.numel() * 4 == nbytes:
-        sink.key_moments_in = key_moments.buf.data_ptr()
-    elif allow_fill:
+        args.key_moments_in = key_moments.buf.data_ptr()
+    else:
         key_moments.buf = torch.empty(nbytes // 4, dtype=torch.float32, device=device)
-        sink.key_moments_out = key_moments.buf.data_ptr()
+        args.key_moments_out = key_moments.buf.data_ptr()
 
 
 def forward(q, k, v, causal, inv_temp, a0=1.0, a1=1.0, a2=0.5, order=2, state_in=None, want_state=False,
@@ -242,7 +244,7 @@ def forward(q, k, v, causal, inv_temp, a0=1.0, a1=1.0, a2=0.5, order=2, state_in
                            dtype=torch.float32, device=q.device)
         args.state_out = sout.data_ptr()
     if key_moments is not None:
-        _attach_key_moments(lib, pb, args, key_moments, q.device, args, True)
+        _attach_key_moments(lib, pb, args, key_moments, q.device)
     need = lib.fastmax_forward_workspace(C.byref(pb), C.byref(args))
     ws, wptr = _workspace(need, q.device)
     check(lib.fastmax_forward(C.byref(pb), C.byref(args), wptr, need, _stream()), "fastmax_forward")
@@ -291,9 +293,8 @@ def backward(q, k, v, o, g, d_out, causal, inv_temp, a0=1.0, a1=1.0, a2=0.5, ord
                             dtype=torch.float32, device=q.device)
         args.dstate_out = dsout.data_ptr()
     if key_moments is not None and key_moments.buf is not None and want_grads:
-        fargs = ForwardArgs()
-        fargs.q, fargs.k, fargs.v, fargs.o, fargs.g = args.q, args.k, args.v, args.o, args.g
-        _attach_key_moments(lib, pb, fargs, key_moments, q.device, args, False)
+        if key_moments.buf.numel() * 4 == lib.fastmax_backward_key_moments_bytes(C.byref(pb), C.byref(args)):
+            args.key_moments_in = key_moments.buf.data_ptr()
     if key_moments is not None:
         nbytes = lib.fastmax_grad_moments_bytes(C.byref(pb), C.byref(args))
         if nbytes:

@@ -453,20 +453,34 @@ static bool splits_prompt(const fastmax_problem* pb, const fastmax_forward_args*
   if (!a->o.ptr || !a->state_out || a->state_in || !pb->causal || pb->nq <= 0 || pair_takes_forward(pb, a)) return false;
   out = *a;
   out.state_out = nullptr;
-  out.key_moments_in = nullptr;
-  out.key_moments_out = nullptr;
-  if (!pair_takes_forward(pb, &out)) return false;
   state = *a;
   state.q = a->k;
   state.o = fastmax_tensor{};
   state.g = fastmax_tensor{};
-  return true;
+  fastmax_forward_args& other = pair_packs_key_moments(pb, a) ? state : out;   // the one that does not handle the key moments
+  other.key_moments_in = nullptr;
+  other.key_moments_out = nullptr;
+  return pair_takes_forward(pb, &out);
+}
+// Key moments that no other call of this problem could read (the call is one that writes segment sums, while the calls of
+// the problem with an output and without a state write packed states) are neither written nor read.
+static bool drops_key_moments(const fastmax_problem* pb, const fastmax_forward_args* a) {
+  fastmax_forward_args out, state;
+  return (a->key_moments_in || a->key_moments_out) && pair_packs_key_moments(pb, a) && !pair_takes_forward(pb, a) && !splits_prompt(pb, a, out, state);
+}
+static const fastmax_forward_args* without_unusable_moments(const fastmax_problem* pb, const fastmax_forward_args* a, fastmax_forward_args& copy) {
+  if (!drops_key_moments(pb, a)) return a;
+  copy = *a;
+  copy.key_moments_in = nullptr;
+  copy.key_moments_out = nullptr;
+  return &copy;
 }
 
 size_t fastmax_forward_workspace(const fastmax_problem* pb, const fastmax_forward_args* args) {
   Plan pl;
   if (!args || make_plan(pb, pl) != FASTMAX_OK) return 0;
-  fastmax_forward_args out, state;
+  fastmax_forward_args copy, out, state;
+  args = without_unusable_moments(pb, args, copy);
   if (splits_prompt(pb, args, out, state)) {
     const fastmax_problem keys = keys_only(pb);
     return align_up(fastmax_forward_workspace(pb, &out), 256) + fastmax_forward_workspace(&keys, &state);
@@ -487,12 +501,17 @@ int32_t fastmax_forward_engine(const fastmax_problem* pb, const fastmax_forward_
 size_t fastmax_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_args* args) {
   Plan pl;
   if (!args || make_plan(pb, pl) != FASTMAX_OK || pb->nk == 0) return 0;
+  fastmax_forward_args asked = *args;   // the call as it will be: who asks is about to hand an array over
+  if (!asked.key_moments_in && !asked.key_moments_out) asked.key_moments_out = (float*)args->k.ptr;
+  args = &asked;
+  if (drops_key_moments(pb, args)) return 0;
   fastmax_forward_args out_call, state_call;
   if (splits_prompt(pb, args, out_call, state_call)) {
+    if (pair_packs_key_moments(pb, args)) return pair_key_moments_bytes(pb);
     const fastmax_problem keys = keys_only(pb);
     return fastmax_key_moments_bytes(&keys, &state_call);
   }
-  if (pair_takes_forward(pb, args)) return pair_key_moments_bytes(pb, args);
+  if (pair_takes_forward(pb, args)) return pair_packs_key_moments(pb, args) ? pair_key_moments_bytes(pb) : 0;
   if (const size_t t = tc_key_moments_bytes(pb, args)) return t;   // a long sequence cut into segments for the tensor-memory kernels
   if (tc_takes_forward(pb, args)) return 0;   // the tensor-memory kernels take this call whole: no segment sums
   FwdLayout L;
@@ -523,6 +542,8 @@ int32_t fastmax_forward(const fastmax_problem* pb, const fastmax_forward_args* a
   if (ws_bytes < fastmax_forward_workspace(pb, a) || (ws_bytes && (!ws || ((uintptr_t)ws % 256))))
     return FASTMAX_ERR_WORKSPACE;
 
+  fastmax_forward_args copy;
+  a = without_unusable_moments(pb, a, copy);
   fastmax_forward_args out_call, state_call;
   if (want_o && splits_prompt(pb, a, out_call, state_call)) {
     // side by side, the state first: the other call's blocks fill the SMs its last round leaves idle
@@ -637,6 +658,27 @@ size_t fastmax_grad_moments_bytes(const fastmax_problem* pb, const fastmax_backw
   return (size_t)pl.bh * nsegD * pl.n_state * sizeof(float);
 }
 
+size_t fastmax_backward_key_moments_bytes(const fastmax_problem* pb, const fastmax_backward_args* args) {
+  Plan pl;
+  if (!args || make_plan(pb, pl, true) != FASTMAX_OK || pb->nk == 0 || !args->dq.ptr) return 0;
+  if (pair_takes_backward(pb, args)) return pair_reads_key_moments(pb, args) ? pair_key_moments_bytes(pb) : 0;
+  if (const size_t t = tc_grad_moments_bytes(pb, args)) return t;   // (one state per segment and head, as the gradient moments)
+  if (tc_takes_backward(pb, args)) return 0;
+  BwdLayout L;
+  bwd_layout(pb, args, pl, L);
+  return L.need_segS ? (size_t)pl.bh * pl.k_nseg * pl.n_state * sizeof(float) : 0;
+}
+
+// The key moments handed to a backward call come from the forward call of the same problem: they are packed window states if
+// that call wrote those, else segment sums.  A backward call that reads the other form builds its own.
+static bool foreign_key_moments(const fastmax_problem* pb, const fastmax_backward_args* a) {
+  if (!a->key_moments_in) return false;
+  fastmax_forward_args f{};
+  f.q = a->q; f.k = a->k; f.v = a->v; f.o = a->o; f.g = a->g;
+  f.state_in = a->state_in;
+  return pair_packs_key_moments(pb, &f) != pair_reads_key_moments(pb, a);
+}
+
 int32_t fastmax_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, size_t ws_bytes,
                          void* stream) {
   Plan pl;
@@ -679,6 +721,12 @@ int32_t fastmax_backward(const fastmax_problem* pb, const fastmax_backward_args*
     return FASTMAX_OK;
   }
 
+  fastmax_backward_args own_moments;
+  if (foreign_key_moments(pb, a)) {
+    own_moments = *a;
+    own_moments.key_moments_in = nullptr;
+    a = &own_moments;
+  }
   if (pair_takes_backward(pb, a)) return pair_backward(pb, a, ws, st);
   int tcrc = tc_backward(pb, a, ws, ws_bytes, st);
   if (tcrc != FASTMAX_TC_NOT_HANDLED) return tcrc;

@@ -297,10 +297,8 @@ std::vector<torch::Tensor> backward(torch::Tensor q, torch::Tensor k, torch::Ten
     a.dstate_out = (float*)dsout.data_ptr();
   }
   if (want_grads && key_moments.has_value() && key_moments->defined()) {
-    // what the forward call of the same q, k, v wrote: valid when it has the size this problem's segments give
-    fastmax_forward_args fa{};
-    fa.q = a.q; fa.k = a.k; fa.v = a.v; fa.o = a.o; fa.g = a.g;
-    const size_t nbytes = fastmax_key_moments_bytes(&pb, &fa);
+    // what the forward call of the same q, k, v wrote: read when it has the size, and with it the form, this call takes
+    const size_t nbytes = fastmax_backward_key_moments_bytes(&pb, &a);
     if (nbytes != 0 && key_moments->is_contiguous() && key_moments->scalar_type() == torch::kFloat32 &&
         (size_t)key_moments->numel() * 4 == nbytes)
       a.key_moments_in = (const float*)key_moments->data_ptr();

@@ -938,7 +938,8 @@ bool fill(const fastmax_problem* pb, pair::Params& P) {
 
 static int forward_form(const fastmax_problem* pb, const fastmax_forward_args* a) {
   if (!a->o.ptr || !a->g.ptr || a->state_in) return 0;
-  const Use use = a->state_out ? USE_PROMPT : a->key_moments_out || a->key_moments_in ? USE_TRAIN : USE_OUT;
+  // (key moments before the state: whether they are packed does not depend on it)
+  const Use use = a->key_moments_out || a->key_moments_in ? USE_TRAIN : a->state_out ? USE_PROMPT : USE_OUT;
   const int form = chosen(pb, false, use);
   if (form == 0 || !mappable(a->q, pb, pb->nq) || !mappable(a->k, pb, pb->nk) || !mappable(a->v, pb, pb->nk)) return 0;
   if (form == 2 && pb->dtype == FASTMAX_F32)
@@ -1555,13 +1556,19 @@ static int long_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
 
-size_t pair_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_args* a) {
-  fastmax_forward_args train = *a;   // who asks is about to hand them on
+bool pair_packs_key_moments(const fastmax_problem* pb, const fastmax_forward_args* a) {
+  fastmax_forward_args train = *a;
+  train.state_out = nullptr;
+  train.key_moments_in = nullptr;
   train.key_moments_out = (float*)a->q.ptr;
-  if (forward_form(pb, &train) != 2) return 0;
-  const LongGeo g = pb->dtype == FASTMAX_F32 ? long_geo_f32(pb) : long_geo(pb);
-  return g.packed + g.cst;
+  return forward_form(pb, &train) == 2;
 }
+// one float more than the states take: every array of segment sums is a multiple of 16 bytes, so a size tells the form
+size_t pair_key_moments_bytes(const fastmax_problem* pb) {
+  const LongGeo g = pb->dtype == FASTMAX_F32 ? long_geo_f32(pb) : long_geo(pb);
+  return g.packed + g.cst + sizeof(float);
+}
+bool pair_reads_key_moments(const fastmax_problem* pb, const fastmax_backward_args* a) { return backward_form(pb, a) == 2; }
 
 int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st) {
   if (pb->dtype == FASTMAX_F32) return forward_form(pb, a) == 2 ? long_f32_forward(pb, a, ws, st) : pair_f32_forward(pb, a, ws, st);

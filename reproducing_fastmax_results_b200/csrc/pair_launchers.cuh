@@ -9,8 +9,12 @@ namespace fm {
 // Whether the pairwise kernels take the call: allowed by the caller, the cheaper form, and in a layout the copy engine reads.
 bool pair_takes_forward(const fastmax_problem* pb, const fastmax_forward_args* a);
 bool pair_takes_backward(const fastmax_problem* pb, const fastmax_backward_args* a);
-// Bytes of the moment arrays a call on long sequences hands from forward to backward (0: none)
-size_t pair_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_args* a);
+// Moment arrays that a call on long sequences hands from forward to backward: packed window states, a form of their own.  Whether
+// the forward call of these arguments writes them when it is asked for key moments, a requested final state aside; their
+// bytes, which are those of no array of segment sums; and whether a backward call reads them.
+bool pair_packs_key_moments(const fastmax_problem* pb, const fastmax_forward_args* a);
+size_t pair_key_moments_bytes(const fastmax_problem* pb);
+bool pair_reads_key_moments(const fastmax_problem* pb, const fastmax_backward_args* a);
 size_t pair_forward_workspace(const fastmax_problem* pb, const fastmax_forward_args* a);
 size_t pair_backward_workspace(const fastmax_problem* pb, const fastmax_backward_args* a);
 int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st);

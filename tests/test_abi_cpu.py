@@ -86,6 +86,48 @@ def test_backward_rejects_bad_arguments():
     assert lib.fastmax_launch_count() == 0
 
 
+def test_size_of_key_moments_tells_their_form():
+    """Packed window states (FASTMAX_FLAG_PAIRWISE, long sequences) and segment sums never have the same size, and what a
+    backward call reads is asked for with its own arguments: carried states and unaligned gradient rows change the form."""
+    lib = _lib.load()
+    B, H, N, D = 1, 8, 8192, 64
+    pb = _lib.Problem(B, H, N, N, D, 2, 1, 1, 1, 1, 0.5, 1.0, _lib.FLAG_PAIRWISE, 0)
+    plain = _lib.Problem(B, H, N, N, D, 2, 1, 1, 1, 1, 0.5, 1.0, 0, 0)
+
+    def args(cls, fields):
+        a = cls()
+        for f in fields:
+            t = getattr(a, f)
+            t.ptr, t.stride_b, t.stride_h, t.stride_n = 4096, H * N * D, N * D, D
+        a.g.stride_b, a.g.stride_h, a.g.stride_n = H * N, N, 1
+        return a
+
+    fwd = args(_lib.ForwardArgs, ("q", "k", "v", "o", "g"))
+    packed = lib.fastmax_key_moments_bytes(C.byref(pb), C.byref(fwd))
+    sums = lib.fastmax_key_moments_bytes(C.byref(plain), C.byref(fwd))
+    assert packed % 16 == 4 and sums > 0 and sums % 16 == 0
+    bwd = lambda: args(_lib.BackwardArgs, ("q", "k", "v", "o", "g", "d_out", "dq", "dk", "dv"))
+    size = lambda problem, a: lib.fastmax_backward_key_moments_bytes(C.byref(problem), C.byref(a))
+    a = bwd()
+    assert size(pb, a) == packed and size(plain, a) == sums
+    for field in ("state_in", "dstate_in", "dstate_out"):
+        a = bwd()
+        setattr(a, field, 4096)
+        assert size(pb, a) == sums, field
+    a = bwd()
+    a.dq.stride_n = D + 1
+    assert size(pb, a) == sums
+    a = bwd()
+    a.dq.ptr = a.dk.ptr = a.dv.ptr = None   # gradient moments alone: the keys are not passed over
+    a.dstate_out = 4096
+    assert size(pb, a) == 0
+    state = args(_lib.ForwardArgs, ("q", "k", "v", "o", "g"))   # a prompt's call writes what the backward of the problem reads
+    state.state_out = 4096
+    assert lib.fastmax_key_moments_bytes(C.byref(pb), C.byref(state)) == packed
+    state.o.ptr = None                                          # a state-only call sums segments
+    assert lib.fastmax_key_moments_bytes(C.byref(pb), C.byref(state)) == sums
+
+
 def test_python_extension_module_is_importable_under_reference_name():
     import reproducing_fastmax_results_b200 as pkg
 

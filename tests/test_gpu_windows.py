@@ -126,3 +126,46 @@ def test_float32_windows_match_oracle(case, hand_over):
         for name, x, ref in (("dq", dq, dq_ref), ("dk", dk, dk_ref), ("dv", dv, dv_ref)):
             err = np.linalg.norm(host(x[b, h])[rows] - ref) / np.linalg.norm(ref)
             assert err < 3e-6, (name, b, h, err)
+
+
+@pytest.mark.parametrize("binding", ["ctypes", "extension"])
+@pytest.mark.parametrize("variant", ["dstate_in", "dstate_out", "gradient rows", "prompt"])
+@pytest.mark.parametrize("dtype,D,N", [(torch.bfloat16, 64, 8192), (torch.float32, 32, 4096)])
+def test_key_moments_of_another_form_are_not_read(dtype, D, N, variant, binding):
+    """A forward of the window form leaves packed states; a backward of the same problem that also takes or returns gradient
+    moments, or writes into rows the copy engine cannot, runs on the moment engines and must not read them (nor may the
+    window form read what a prompt's state left).  Same gradients with and without the hand-over."""
+    import reproducing_fastmax_results_b200 as pkg
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    ext = pkg.load_extension()
+    B, H = 1, 8
+    g = torch.Generator(device="cuda").manual_seed(N + D)
+    q, k, v, do = (torch.randn(B, H, N, D, device="cuda", generator=g).to(dtype) for _ in range(4))
+    it = 1.0 / (8.0 * math.sqrt(D))
+    poly = (1.0, 1.0, 0.5, 2)
+    dstate = torch.randn(L.new_state(B, H, D).shape, device="cuda", generator=g) * 1e-2 if variant == "dstate_in" else None
+    want_state, want_dstate = variant == "prompt", variant == "dstate_out"
+
+    def rows():
+        if variant != "gradient rows":
+            return None
+        return [torch.zeros(B, H, N, D + 1, device="cuda", dtype=dtype)[..., :D] for _ in range(3)]
+
+    def run(hand_over):
+        if binding == "ctypes":
+            km = L.KeyMoments()
+            o, gg, _ = L.forward(q, k, v, True, it, *poly, want_state=want_state, flags=L.FLAG_PAIRWISE, key_moments=km)
+            res = L.backward(q, k, v, o, gg, do, True, it, *poly, dstate_in=dstate, want_dstate=want_dstate, grads_out=rows(),
+                             flags=L.FLAG_PAIRWISE, key_moments=km if hand_over else None)
+            buf = km.buf
+        else:
+            o, gg, _, buf = ext.forward(q, k, v, True, it, *poly, None, want_state, True, ext.PAIRWISE, None, None, True)
+            res = ext.backward(q, k, v, o, gg, do, True, it, *poly, None, dstate, want_dstate, True, ext.PAIRWISE, rows(),
+                               buf if hand_over else None)[:4]
+        L.check_status()
+        assert buf.numel() % 4 == 1   # packed states, whatever else the forward returned
+        return [t for t in res if t is not None and t.numel()]
+
+    for a, b in zip(run(True), run(False)):
+        assert orc.max_norm_err(host(a), host(b)) < (1e-2 if dtype == torch.bfloat16 else 2e-6)
