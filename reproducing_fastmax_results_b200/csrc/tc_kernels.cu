@@ -763,9 +763,15 @@ static bool tc_forward_supported(const fastmax_problem* pb, const fastmax_forwar
   return true;
 }
 
+// A tensor expanded over tokens or heads (zero stride) has no tensor map: such a call goes to the CUDA-core engine whole, it
+// must not be taken apart first.
+static bool seg_mappable(const fastmax_tensor& t, const fastmax_problem* pb, int n) {
+  return (n == 1 || t.stride_n != 0) && (pb->heads == 1 || t.stride_h != 0);
+}
 static bool tc_forward_segmentable(const fastmax_problem* pb, const fastmax_forward_args* a) {
   if (tc_segments(pb) <= 0 || !a->k.ptr || !a->v.ptr) return false;
-  if (a->o.ptr) return a->q.ptr && a->g.ptr;
+  if (!seg_mappable(a->k, pb, pb->nk) || !seg_mappable(a->v, pb, pb->nk)) return false;
+  if (a->o.ptr) return a->q.ptr && a->g.ptr && seg_mappable(a->q, pb, pb->nq);
   return a->state_out != nullptr;   // a state-only call: the segment moments and their sum
 }
 
@@ -1106,7 +1112,7 @@ static bool tc_backward_segmentable(const fastmax_problem* pb, const fastmax_bac
   if (!(a->dq.ptr && a->dk.ptr && a->dv.ptr) && !(a->dstate_out && !a->dq.ptr)) return false;   // gradients, or a state-only call
   for (const fastmax_tensor* t : {&a->o, &a->d_out})
     if (((uintptr_t)t->ptr & 3) || (t->stride_b & 1) || (t->stride_h & 1) || (t->stride_n & 1)) return false;
-  return true;
+  return seg_mappable(a->q, pb, pb->nq) && seg_mappable(a->k, pb, pb->nk) && seg_mappable(a->v, pb, pb->nk);
 }
 
 size_t tc_backward_workspace(const fastmax_problem* pb, const fastmax_backward_args* a) {

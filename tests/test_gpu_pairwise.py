@@ -97,6 +97,29 @@ def test_pairwise_form_is_left_to_the_moment_engines_where_it_does_not_apply():
         assert orc.max_norm_err(host(a), host(b)) < tol
 
 
+@pytest.mark.parametrize("flags", [0, 4])
+@pytest.mark.parametrize("D", [64, 32])
+def test_expanded_keys_of_a_long_sequence_with_few_heads(D, flags):
+    """One key and value head for all eight query heads (zero stride) at a length that the tensor-memory engine cuts into
+    segments: accepted, forward, state-only call and backward, with the results of contiguous copies."""
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    B, H, N = 1, 8, 8192
+    g = torch.Generator(device="cuda").manual_seed(6)
+    q, do = (torch.randn(B, H, N, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    k1, v1 = (torch.randn(B, 1, N, D, device="cuda", generator=g).bfloat16().expand(B, H, N, D) for _ in range(2))
+
+    def run(k, v):
+        o, gg, _ = L.forward(q, k, v, True, 0.05, order=2, flags=flags)
+        state = L.forward(k, k, v, True, 0.05, order=2, want_state=True, want_output=False, flags=flags)[2]
+        grads = L.backward(q, k, v, o, gg, do, True, 0.05, order=2, flags=flags)[:3]
+        L.check_status()
+        return (o, gg, state) + tuple(grads)
+
+    for a, b in zip(run(k1, v1), run(k1.contiguous(), v1.contiguous())):
+        assert orc.max_norm_err(host(a), host(b)) < 2e-2
+
+
 @pytest.mark.parametrize("dtype,n", [(torch.bfloat16, 5500), (torch.float32, 2000)])
 def test_more_heads_than_one_group_of_the_item_order(dtype, n):
     """25 heads whose streamed tiles exceed the share of L2: two groups, the last one smaller; every head, forward and backward."""
