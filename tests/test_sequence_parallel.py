@@ -145,6 +145,37 @@ def test_cuda_engine_pieces_match_whole_sequence(D, dtype, pieces):
             assert orc.max_norm_err(got, ref) < tol, ("dq", "dk", "dv")[j]
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,dtype,kind", [(32, torch.float32, "moments_kv"), (64, torch.float32, "moments_kv"),
+                                          (64, torch.bfloat16, "tc_scan_fwd")])
+def test_cuda_engine_sums_the_key_moments_of_a_piece_once(D, dtype, kind):
+    """A long piece with few heads and a carried state: the per-segment key moments of the state call reach the forward and
+    the backward, which launch no pass over k and v of their own.  `kind`: the launches that sum them."""
+    from reproducing_fastmax_results_b200 import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v, do = (torch.randn(1, 4, 8192, D, device="cuda", generator=g).to(dtype) for _ in range(4))
+    eng = sp.CudaEngine(1.0 / (2.0 * math.sqrt(D)))
+    km = sp.KeyMoments()
+
+    def launches(fn):
+        _lib.profile_collect()
+        _lib.profile(True)
+        out = fn()
+        _lib.check_status()
+        _lib.profile(False)
+        return out, _lib.profile_collect().get(kind, (0.0, 0))[1]
+
+    total, first = launches(lambda: eng.key_state(k, v, moments=km))
+    (o, gg), forward = launches(lambda: eng.forward(q, k, v, total, moments=km))
+    gtot, _ = launches(lambda: eng.grad_state(q, k, v, o, gg, do, total, moments=km))
+    grads, backward = launches(lambda: eng.backward(q, k, v, o, gg, do, total, gtot, moments=km))
+    # (the tensor-memory forward is itself one launch of this kind)
+    assert (first, forward, backward) == ((1, 1, 0) if kind == "tc_scan_fwd" else (1, 0, 0))
+    for a, b in zip(grads, eng.backward(q, k, v, o, gg, do, total, gtot)):
+        assert orc.max_norm_err(a.double().cpu().numpy(), b.double().cpu().numpy()) < (1e-2 if dtype == torch.bfloat16 else 2e-6)
+
+
 def _failing_peer_worker(rank, world, port, out_dir):
     """Rank 1 raises before the exchange; rank 0 must come back from the collective with an error, not hang."""
     import datetime
