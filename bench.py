@@ -1248,22 +1248,22 @@ def main():
     #   executed:    contraction passes the kernel really runs, over the block-symmetric feature rows (x 0.569):
     #                every scan recomputes its state (apply/dphi + update = 2 passes).
     units_alg = {"scan_fwd": 2.0, "tc_scan_fwd": 2.0, "scan_bwd_q": 1.0, "tc_scan_bwd_q": 1.0, "scan_bwd_kv": 3.0,
-                 "tc_scan_bwd_kv": 2.0, "tc_scan_bwd_dv": 1.0, "moments_kv": 1.0, "moments_qg": 1.0, "tc_moments": 1.0}
+                 "tc_scan_bwd_kv": 2.0, "tc_scan_bwd_dv": 1.0, "moments_kv": 1.0, "moments_qg": 1.0, "tc_moments": 1.0,
+                 "pair_fwd": 2.0, "pair_bwd_q": 1.0, "pair_bwd_kv": 3.0, "pair_f32_fwd": 2.0, "pair_f32_bwd_q": 1.0,
+                 "pair_f32_bwd_kv": 3.0}
     units_exec = {"tc_scan_fwd": 2.0, "tc_scan_bwd_q": 2.0, "tc_scan_bwd_kv": 2.0, "tc_scan_bwd_dv": 2.0}
     m_full = 1 + D + (D * D if order == 2 else 0)
     ratio_exec = executed_units(D, order) / m_full
 
-    # The pairwise kernels report under the same kinds; their products per visible pair: forward 4 d, dq 6 d, dk and dv 8 d
-    # from one launch (listed under both kinds).  The scans are told apart by the transposed copies they read.
-    pairwise = bool(flags & _lib.FLAG_PAIRWISE) and dtype_name == "bf16" and "tc_transpose" not in kernels
+    # the pairwise kernels' products per visible pair: forward 4 d, dq 6 d, dk and dv 8 d from one launch
     visible = B * H * (N * (N + 1) / 2 if causal else N * N)
-    pair_flops = {"tc_scan_fwd": 4.0, "tc_scan_bwd_q": 6.0, "tc_scan_bwd_kv": 4.0, "tc_scan_bwd_dv": 4.0}
+    pair_flops = {"fwd": 4.0, "bwd_q": 6.0, "bwd_kv": 8.0}
 
     def counted_flops(name):
         """min(algorithmic, executed) flops of one launch: never credits more than the hardware did."""
         alg = units_alg.get(name, 0.0) * U
-        if pairwise:
-            return min(alg, pair_flops.get(name, 0.0) * D * visible), alg
+        if name.startswith("pair_"):
+            return min(alg, pair_flops.get(name.removeprefix("pair_").removeprefix("f32_"), 0.0) * D * visible), alg
         ex = units_exec.get(name, units_alg.get(name, 0.0)) * U * (ratio_exec if name.startswith("tc_") else 1.0)
         return min(alg, ex), alg
 
@@ -1275,6 +1275,7 @@ def main():
         dur_s = kernels[dominant]["ms_per_launch"] * 1e-3
         peak = pk["bf16_tflops_sustained"]
         achieved = counted * per_launch / dur_s / 1e12
+        pairwise = dominant.startswith("pair_")
         roofline = {
             "kernel": dominant, "bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak, "peak_source": pk["_source"] + " (sustained cuBLAS bf16: kernel timed inside a long step)",

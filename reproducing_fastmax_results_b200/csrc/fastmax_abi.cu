@@ -20,7 +20,7 @@ static thread_local int g_last_cuda_error = 0;
 
 // ---- optional per-kernel timing -----------------------------------------------------------------
 struct ProfRec {
-  int kind, also;
+  int kind;
   cudaEvent_t a, b;
 };
 static std::atomic<int> g_prof_on{0};
@@ -38,14 +38,14 @@ void launch_begin(int kind, cudaStream_t st) {
   cudaEventRecord(a, st);
   g_prof_open = a;
 }
-void launch_end(int kind, cudaStream_t st, int also) {
+void launch_end(int kind, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (g_prof_open == nullptr) return;
   cudaEvent_t b = nullptr;
   if (cudaEventCreate(&b) == cudaSuccess) {
     cudaEventRecord(b, st);
     std::lock_guard<std::mutex> lk(g_prof_mu);
-    g_prof_recs.push_back(ProfRec{kind, also, g_prof_open, b});
+    g_prof_recs.push_back(ProfRec{kind, g_prof_open, b});
   } else {
     cudaEventDestroy(g_prof_open);
   }
@@ -53,7 +53,9 @@ void launch_end(int kind, cudaStream_t st, int also) {
 }
 static const char* kKindNames[KK_COUNT] = {
     "moments_kv", "moments_qg", "state_scan", "scan_fwd", "scan_bwd_q", "scan_bwd_kv", "finalize_fwd",
-    "bwd_prologue", "cast_out", "normalize", "tc_scan_fwd", "tc_scan_bwd_q", "tc_scan_bwd_kv", "tc_moments", "p1_fwd", "tc_intra_fwd", "tc_intra_bwd", "tc_transpose", "tc_scan_bwd_dv", "decode_step", "key_prologue", "output_noise", "tc_pad"};
+    "bwd_prologue", "cast_out", "normalize", "tc_scan_fwd", "tc_scan_bwd_q", "tc_scan_bwd_kv", "tc_moments", "p1_fwd", "tc_intra_fwd", "tc_intra_bwd", "tc_transpose", "tc_scan_bwd_dv", "decode_step", "key_prologue", "output_noise", "tc_pad",
+    "pair_fwd", "pair_bwd_q", "pair_bwd_kv", "pair_f32_fwd", "pair_f32_bwd_q", "pair_f32_bwd_kv", "pair_split",
+    "window_pack", "window_fwd", "window_bwd_q", "window_bwd_k", "window_bwd_v"};
 
 static int sm_count() {
   static int cached[64] = {0};
@@ -410,13 +412,8 @@ int32_t fastmax_profile_collect(double* ms, uint64_t* count, int32_t nkinds) {
       g_last_cuda_error = (int)e;
       rc = FASTMAX_ERR_CUDA;
     } else if (r.kind >= 0 && r.kind < nkinds) {
-      const bool both = r.also >= 0 && r.also < nkinds;
-      ms[r.kind] += both ? 0.5 * t : t;
+      ms[r.kind] += t;
       count[r.kind] += 1;
-      if (both) {
-        ms[r.also] += 0.5 * t;
-        count[r.also] += 1;
-      }
     }
     cudaEventDestroy(r.a);
     cudaEventDestroy(r.b);

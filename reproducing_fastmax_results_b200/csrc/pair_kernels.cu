@@ -991,7 +991,7 @@ static void launch_split(const fastmax_problem* pb, const pair::f32::SplitArgs& 
   for (int i = 1; i < count; ++i) n = A.n[i] > n ? A.n[i] : n;
   const int rows = 256 / (pb->d / 8);
   const dim3 grid((unsigned)((n + rows - 1) / rows), (unsigned)(pb->batch * pb->heads), (unsigned)count);
-  LaunchScope ls(KK_CAST, st);
+  LaunchScope ls(KK_PAIR_SPLIT, st);
   switch (pb->d) {
     case 16: pair::f32::split_kernel<16><<<grid, 256, 0, st>>>(A, pb->heads); break;
     case 32: pair::f32::split_kernel<32><<<grid, 256, 0, st>>>(A, pb->heads); break;
@@ -1053,7 +1053,7 @@ static int pair_f32_forward(const fastmax_problem* pb, const fastmax_forward_arg
   P.nr = pb->nq;
   P.nx = pb->nk;
   P.ntiles = tiles(pb->nq);
-  LaunchScope ls(KK_SCAN_FWD, st);
+  LaunchScope ls(KK_PAIR_F32_FWD, st);
   e = launch_f32_d<pair::FWD>(pb->d, M, P, pb->batch * pb->heads, st);
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
@@ -1107,7 +1107,7 @@ static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   K.nx = pb->nq;
   K.ntiles = tiles(pb->nk);
   {
-    LaunchScope ls(KK_SCAN_BWD_KV, st);
+    LaunchScope ls(KK_PAIR_F32_BWD_KV, st);
     e = launch_f32_d<pair::DKV>(pb->d, N, K, bh, st);
   }
   if (e != cudaSuccess) return report_cuda_error(e);
@@ -1116,7 +1116,7 @@ static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   P.nx = pb->nk;
   P.ntiles = tiles(pb->nq);
   {
-    LaunchScope ls(KK_SCAN_BWD_Q, st);
+    LaunchScope ls(KK_PAIR_F32_BWD_Q, st);
     e = launch_f32_d<pair::DQ>(pb->d, M, P, bh, st);
   }
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
@@ -1138,7 +1138,7 @@ static void launch_prologue(const fastmax_problem* pb, const fastmax_backward_ar
     pair::prologue_kernel<D, false><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
 }
 static void launch_prologue_any(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
-  LaunchScope ls(KK_PROLOGUE, st, pb->d < 64 ? KK_TC_PAD : -1);
+  LaunchScope ls(KK_PROLOGUE, st);
   switch (pb->d) {
     case 16: launch_prologue<16>(pb, a, dop, nd, dld, st); break;
     case 32: launch_prologue<32>(pb, a, dop, nd, dld, st); break;
@@ -1184,7 +1184,7 @@ void launch_pack(const fastmax_problem* pb, const LongGeo& g, const float* raw, 
   const float c0 = pb->a0, c1 = pb->a1 * pb->inv_temperature, c2 = pb->order == 2 ? pb->a2 * pb->inv_temperature * pb->inv_temperature : 0.f;
   const int nb = pb->d / 8, units = (pb->order == 2 ? nb * (nb + 1) / 2 : 0) + 1;
   const dim3 grid((unsigned)units, (unsigned)(pb->batch * pb->heads));
-  LaunchScope ls(KK_STATE_SCAN, st);
+  LaunchScope ls(KK_WINDOW_PACK, st);
   if (pb->d == 64) lng::pack_kernel<64><<<grid, 640, 0, st>>>(raw, S, cst, g.ns, reverse, pb->order, c0, c1, c2, total);
   else lng::pack_kernel<32><<<grid, 384, 0, st>>>(raw, S, cst, g.ns, reverse, pb->order, c0, c1, c2, total);
 }
@@ -1261,7 +1261,7 @@ static size_t long_backward_workspace(const fastmax_problem* pb) {
 // Packed states of the keys before every segment but the first (no mask: of all keys): S, then the constant rows behind it
 static cudaError_t long_key_states(const fastmax_problem* pb, const LongGeo& g, const fastmax_tensor& k, const fastmax_tensor& v, float* raw, void* xt,
                                    uint8_t* S, float* total, cudaStream_t st) {
-  const cudaError_t e = tc_moments(pb, k, v, pb->causal && !total ? g.ns * g.L : pb->nk, false, g.L, nullptr, raw, xt, KK_TC_MOMENTS, st);
+  const cudaError_t e = tc_moments(pb, k, v, pb->causal && !total ? g.ns * g.L : pb->nk, false, g.L, nullptr, raw, xt, st);
   if (e != cudaSuccess) return e;
   launch_pack(pb, g, raw, S, (float*)(S + g.packed), false, total, st);
   return cudaGetLastError();
@@ -1299,13 +1299,13 @@ static int long_forward(const fastmax_problem* pb, const fastmax_forward_args* a
     P.ntiles = tiles(pb->nq, 2 * pair::R);
     P.vec0 = 1;
     if (sq) P.w1 = P.c2;
-    LaunchScope ls(KK_TC_INTRA_FWD, st);
+    LaunchScope ls(KK_PAIR_FWD, st);
     e = sq ? launch_d<pair::FWD, true>(pb->d, M, P, bh, st) : launch_d<pair::FWD, false>(pb->d, M, P, bh, st);
   }
   if (e == cudaSuccess && (!a->key_moments_in || a->state_out)) e = long_key_states(pb, g, a->k, a->v, raw, xt, S, a->state_out, st);
   lng::Params P = long_params(pb, g, S, pb->nq, g.L, pb->nq);
   P.g = view_of(a->g);
-  if (e == cudaSuccess) e = pb->d == 64 ? launch_apply<64, true>(A, P, KK_TC_FWD, st) : launch_apply<32, true>(A, P, KK_TC_FWD, st);
+  if (e == cudaSuccess) e = pb->d == 64 ? launch_apply<64, true>(A, P, KK_WINDOW_FWD, st) : launch_apply<32, true>(A, P, KK_WINDOW_FWD, st);
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
 
@@ -1359,29 +1359,29 @@ static int long_backward(const fastmax_problem* pb, const fastmax_backward_args*
     B.out1 = view_of(a->dv);
     if (sq) { B.w0 = 2.f * B.c2; B.w1 = B.c2; P.w0 = 2.f * P.c2; }
     {
-      LaunchScope ls(KK_TC_INTRA_BWD, st);
+      LaunchScope ls(KK_PAIR_BWD_KV, st);
       e = sq ? launch_d<pair::DKV, true>(d, N, B, bh, st) : launch_d<pair::DKV, false>(d, N, B, bh, st);
     }
     P.part_lo = g.L;
     P.part_hi = 1 << 30;
     P.out0 = P.out1 = view_of(a->dq);
-    LaunchScope ls(KK_TC_INTRA_BWD, st);
+    LaunchScope ls(KK_PAIR_BWD_Q, st);
     if (e == cudaSuccess) e = sq ? launch_d<pair::DQ, true>(d, M, P, bh, st) : launch_d<pair::DQ, false>(d, M, P, bh, st);
   }
   if (e == cudaSuccess && !a->key_moments_in) e = long_key_states(pb, g, a->k, a->v, raw, xt, S, nullptr, st);
   if (e != cudaSuccess) return report_cuda_error(e);
   // gradient moments of every segment but the first (no mask: of all queries); raw may be reused: the stream orders it
-  e = tc_moments(pb, after(a->q, g.L, 2), after(dhead, g.L, 2), pb->nq - g.L, true, g.L, nullptr, raw, xt, KK_TC_MOMENTS, st);
+  e = tc_moments(pb, after(a->q, g.L, 2), after(dhead, g.L, 2), pb->nq - g.L, true, g.L, nullptr, raw, xt, st);
   if (e != cudaSuccess) return report_cuda_error(e);
   launch_pack(pb, g, raw, dS, (float*)(dS + g.packed), true, nullptr, st);
   e = cudaGetLastError();
   lng::Params P = long_params(pb, g, S, pb->nq, g.L, pb->nq);
   P.ndelta = nd;
   P.nd_ld = nd_ld(pb->nq);
-  if (e == cudaSuccess) e = d == 64 ? launch_chain<64, false>(Q, P, KK_TC_BWD_Q, st) : launch_chain<32, false>(Q, P, KK_TC_BWD_Q, st);
+  if (e == cudaSuccess) e = d == 64 ? launch_chain<64, false>(Q, P, KK_WINDOW_BWD_Q, st) : launch_chain<32, false>(Q, P, KK_WINDOW_BWD_Q, st);
   P = long_params(pb, g, dS, pb->nk, 0, pb->causal ? g.ns * g.L : pb->nk);
-  if (e == cudaSuccess) e = d == 64 ? launch_chain<64, true>(K, P, KK_TC_BWD_KV, st) : launch_chain<32, true>(K, P, KK_TC_BWD_KV, st);
-  if (e == cudaSuccess) e = d == 64 ? launch_apply<64, false>(V, P, KK_TC_BWD_DV, st) : launch_apply<32, false>(V, P, KK_TC_BWD_DV, st);
+  if (e == cudaSuccess) e = d == 64 ? launch_chain<64, true>(K, P, KK_WINDOW_BWD_K, st) : launch_chain<32, true>(K, P, KK_WINDOW_BWD_K, st);
+  if (e == cudaSuccess) e = d == 64 ? launch_apply<64, false>(V, P, KK_WINDOW_BWD_V, st) : launch_apply<32, false>(V, P, KK_WINDOW_BWD_V, st);
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
 
@@ -1430,7 +1430,7 @@ cudaError_t long_states_f32(const fastmax_problem* pb, const LongGeo& g, const f
   if (e != cudaSuccess) return e;
   const float c0 = pb->a0, c1 = pb->a1 * pb->inv_temperature, c2 = pb->order == 2 ? pb->a2 * pb->inv_temperature * pb->inv_temperature : 0.f;
   const dim3 grid((unsigned)((pb->order == 2 ? UNITS : 1) + 1), NC / 8, (unsigned)(pb->batch * pb->heads));
-  LaunchScope ls(KK_STATE_SCAN, st);
+  LaunchScope ls(KK_WINDOW_PACK, st);
   pack_kernel<<<grid, 64, 0, st>>>(raw, S, (float*)(S + g.packed), g.ns, g.ns, reverse, pb->order, c0, c1, c2);
   return cudaGetLastError();
 }
@@ -1484,13 +1484,13 @@ static int long_f32_forward(const fastmax_problem* pb, const fastmax_forward_arg
     P.out1 = view_of(a->g);
     P.nr = P.nx = n;
     P.ntiles = tiles(n);
-    LaunchScope ls(KK_TC_INTRA_FWD, st);
+    LaunchScope ls(KK_PAIR_F32_FWD, st);
     e = launch_f32_d<pair::FWD>(pb->d, M, P, bh, st);
   }
   if (e == cudaSuccess && !a->key_moments_in) e = long_states_f32(pb, g, a->k, vp, n, 0, g.ns * g.L, false, raw, S, st);
   lng::Params P = long_params(pb, g, S, n, g.L, n);
   P.g = view_of(a->g);
-  if (e == cudaSuccess) e = launch_apply_f32<true>(A, P, KK_TC_FWD, st);
+  if (e == cudaSuccess) e = launch_apply_f32<true>(A, P, KK_WINDOW_FWD, st);
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
 
@@ -1538,21 +1538,21 @@ static int long_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   B.out0 = view_of(a->dk);
   B.out1 = view_of(a->dv);
   {
-    LaunchScope ls(KK_TC_INTRA_BWD, st);
+    LaunchScope ls(KK_PAIR_F32_BWD_KV, st);
     e = launch_f32_d<pair::DKV>(pb->d, N, B, bh, st);
   }
   P.out0 = P.out1 = view_of(a->dq);
   if (e == cudaSuccess) {
-    LaunchScope ls(KK_TC_INTRA_BWD, st);
+    LaunchScope ls(KK_PAIR_F32_BWD_Q, st);
     e = launch_f32_d<pair::DQ>(pb->d, M, P, bh, st);
   }
   if (e == cudaSuccess && !a->key_moments_in) e = long_states_f32(pb, g, a->k, vp, n, 0, g.ns * g.L, false, raw, S, st);
   // gradient moments of every segment but the first; raw may be reused: the stream orders it
   if (e == cudaSuccess) e = long_states_f32(pb, g, a->q, dp, n, g.L, n, true, raw, dS, st);
-  if (e == cudaSuccess) e = launch_chain_f32(Q, long_params(pb, g, S, n, g.L, n), KK_TC_BWD_Q, st);
+  if (e == cudaSuccess) e = launch_chain_f32(Q, long_params(pb, g, S, n, g.L, n), KK_WINDOW_BWD_Q, st);
   const lng::Params R = long_params(pb, g, dS, n, 0, g.ns * g.L);
-  if (e == cudaSuccess) e = launch_chain_f32(K, R, KK_TC_BWD_KV, st);
-  if (e == cudaSuccess) e = launch_apply_f32<false>(V, R, KK_TC_BWD_DV, st);
+  if (e == cudaSuccess) e = launch_chain_f32(K, R, KK_WINDOW_BWD_K, st);
+  if (e == cudaSuccess) e = launch_apply_f32<false>(V, R, KK_WINDOW_BWD_V, st);
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
 
@@ -1589,7 +1589,7 @@ int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void*
   P.vec0 = out_map(&M.o0, a->o, pb, pb->nq);
   if (sq) P.w1 = P.c2;
   const int bh = pb->batch * pb->heads;
-  LaunchScope ls(KK_TC_FWD, st);
+  LaunchScope ls(KK_PAIR_FWD, st);
   const cudaError_t e = sq ? launch_d<pair::FWD, true>(pb->d, M, P, bh, st) : launch_d<pair::FWD, false>(pb->d, M, P, bh, st);
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
@@ -1627,7 +1627,7 @@ int pair_backward(const fastmax_problem* pb, const fastmax_backward_args* a, voi
   K.vec1 = out_map(&N.o1, a->dv, pb, pb->nk);
   if (sq) { K.w0 = 2.f * K.c2; K.w1 = K.c2; }
   {
-    LaunchScope ls(KK_TC_BWD_KV, st, KK_TC_BWD_DV);
+    LaunchScope ls(KK_PAIR_BWD_KV, st);
     e = sq ? launch_d<pair::DKV, true>(pb->d, N, K, bh, st) : launch_d<pair::DKV, false>(pb->d, N, K, bh, st);
   }
   if (e != cudaSuccess) return report_cuda_error(e);
@@ -1638,7 +1638,7 @@ int pair_backward(const fastmax_problem* pb, const fastmax_backward_args* a, voi
   P.vec0 = out_map(&M.o0, a->dq, pb, pb->nq);
   if (sq) P.w0 = 2.f * P.c2;
   {
-    LaunchScope ls(KK_TC_BWD_Q, st);
+    LaunchScope ls(KK_PAIR_BWD_Q, st);
     e = sq ? launch_d<pair::DQ, true>(pb->d, M, P, bh, st) : launch_d<pair::DQ, false>(pb->d, M, P, bh, st);
   }
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);

@@ -932,7 +932,7 @@ size_t tc_key_moments_bytes(const fastmax_problem* pb, const fastmax_forward_arg
 // is column D).  xt: scratch of tc_moments_scratch() bytes.
 size_t tc_moments_scratch(const fastmax_problem* pb, int n) { return transposed_bytes(pb->batch * pb->heads, n, pb->d); }
 cudaError_t tc_moments(const fastmax_problem* pb, const fastmax_tensor& x, const fastmax_tensor& y, int n, bool dop, int seg_tokens,
-                       const float* init, float* state, void* xt, int kind, cudaStream_t st) {
+                       const float* init, float* state, void* xt, cudaStream_t st) {
   const int bh = pb->batch * pb->heads, d = pb->d;
   CUtensorMap tmxt, tmy, tmt;
   if (!make_map_t(&tmxt, xt, bh, n, tokens_padded(n), d) || !make_map(&tmy, y, pb->batch, pb->heads, n, 64, tc::CH, true, d)) return cudaErrorInvalidValue;
@@ -987,7 +987,7 @@ cudaError_t tc_moments(const fastmax_problem* pb, const fastmax_tensor& x, const
   if (e == cudaSuccess) e = d == 64 ? ensure_smem(tc::mo::moments_kernel<64>, tc::mo::Lay<64>::SMEM_BYTES, 7)
                                     : ensure_smem(tc::mo::moments_kernel<32>, tc::mo::Lay<32>::SMEM_BYTES, 2);
   if (e != cudaSuccess) return e;
-  LaunchScope ls(kind, st);
+  LaunchScope ls(KK_TC_MOMENTS, st);
   if (d == 64) tc::mo::moments_kernel<64><<<dim3(ctas), tc::mo::THREADS, tc::mo::Lay<64>::SMEM_BYTES, st>>>(tmxt, tmy, tmt, P);
   else tc::mo::moments_kernel<32><<<dim3(ctas), tc::mo::THREADS, tc::mo::Lay<32>::SMEM_BYTES, st>>>(tmxt, tmy, tmt, P);
   return cudaGetLastError();
@@ -1004,7 +1004,7 @@ int tc_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* w
       !make_map(&tmv, a->v, pb->batch, pb->heads, pb->nk, 8, tc::CH, false))
     return FASTMAX_TC_NOT_HANDLED;  // layout the copy engine cannot describe: the CUDA-core engine takes it
   if (!(a->o.ptr && pb->nq > 0)) {
-    const cudaError_t e = tc_moments(pb, a->k, a->v, pb->nk, false, 0, a->state_in, a->state_out, ws, KK_TC_FWD, st);
+    const cudaError_t e = tc_moments(pb, a->k, a->v, pb->nk, false, 0, a->state_in, a->state_out, ws, st);
     return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
   }
   if (!make_map(&tmq, a->q, pb->batch, pb->heads, pb->nq, 64, tc::CH, true)) return FASTMAX_TC_NOT_HANDLED;
@@ -1310,7 +1310,7 @@ int tc_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void*
   };
   if (!want_grads) {
     // only the gradient moments are wanted (what a sequence-parallel rank publishes)
-    e = tc_moments(pb, a->q, dopt, pb->nq, true, 0, a->dstate_in, a->dstate_out, qt, KK_TC_BWD_DV, st);
+    e = tc_moments(pb, a->q, dopt, pb->nq, true, 0, a->dstate_in, a->dstate_out, qt, st);
     return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
   }
   // The chain-rule scans rebalance registers between their warp groups with setmaxnreg; that only terminates if

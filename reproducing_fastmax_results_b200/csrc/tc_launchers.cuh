@@ -36,7 +36,7 @@ bool tc_make_map(CUtensorMap* m, const fastmax_tensor& t, int batch, int heads, 
 
 size_t tc_moments_scratch(const fastmax_problem* pb, int n);
 cudaError_t tc_moments(const fastmax_problem* pb, const fastmax_tensor& x, const fastmax_tensor& y, int n, bool dop, int seg_tokens,
-                       const float* init, float* state, void* xt, int kind, cudaStream_t st);
+                       const float* init, float* state, void* xt, cudaStream_t st);
 
 // A second stream for work that is independent of what the caller's stream gets meanwhile: forked from it here, joined back
 // by join() (or the destructor).  The caller's own stream when side streams are off.  Calls made on `side` must carry

@@ -88,7 +88,7 @@ def test_config4_bf16_noncausal_p1_full_size():
 def test_config2_shape_with_32_wide_bf16_heads_full_size():
     """B=8, H=16, N=4096, D=32, bf16, causal, order 2: the zero-padded form of the tensor-memory kernels at full size,
     forward + backward against exact sampled rows / columns; and the long float32 sequence of config 3 under the
-    "medium" float32 matmul precision (bfloat16 copies, padded, cut into segments) at the bfloat16 tolerance."""
+    "medium" float32 matmul precision (bfloat16 copies, windows of pairs plus states) at the bfloat16 tolerance."""
     from reproducing_fastmax_results_b200 import _lib as L
     from reproducing_fastmax_results_b200.attention import FastMax
 
@@ -122,7 +122,9 @@ def test_config2_shape_with_32_wide_bf16_heads_full_size():
     finally:
         torch.set_float32_matmul_precision(before)
     kinds = set(L.profile_collect())
-    assert {"tc_pad", "tc_scan_fwd", "state_scan"} <= kinds and "scan_fwd" not in kinds, kinds
+    assert {"pair_fwd", "pair_bwd_q", "pair_bwd_kv", "tc_moments", "window_pack", "window_fwd", "window_bwd_q", "window_bwd_k",
+            "window_bwd_v"} <= kinds, kinds
+    assert not ({"scan_fwd", "pair_f32_fwd", "tc_pad"} & kinds), kinds
     assert out.dtype == torch.float32 and qg.grad.dtype == torch.float32
     # the denominators of the bfloat16 run, for the sampled-row check of the gradients
     qb, kb, vb = (t.bfloat16() for t in (q, k, v))

@@ -299,21 +299,22 @@ def test_float32_callers_reach_the_tensor_memory_kernels_under_medium_matmul_pre
     try:
         torch.set_float32_matmul_precision("highest")
         exact, kinds_exact = run()
-        assert "tc_scan_fwd" not in kinds_exact and "scan_fwd" in kinds_exact, kinds_exact
+        assert {"pair_f32_fwd", "pair_f32_bwd_q", "pair_f32_bwd_kv"} <= kinds_exact and "pair_fwd" not in kinds_exact, kinds_exact
         torch.set_float32_matmul_precision("medium")
         fast, kinds_fast = run()
-        assert {"tc_scan_fwd", "tc_scan_bwd_q", "tc_scan_bwd_kv", "tc_scan_bwd_dv"} <= kinds_fast, kinds_fast
-        assert not ({"scan_fwd", "scan_bwd_q", "scan_bwd_kv"} & kinds_fast), kinds_fast
+        assert {"pair_fwd", "pair_bwd_q", "pair_bwd_kv"} <= kinds_fast, kinds_fast
+        assert not ({"scan_fwd", "scan_bwd_q", "scan_bwd_kv", "pair_f32_fwd", "pair_f32_bwd_q", "pair_f32_bwd_kv"} & kinds_fast), kinds_fast
         for a, b in zip(fast, exact):
             assert orc.max_norm_err(host(a), host(b)) < 2e-2
-        # a shape the tensor-memory kernels do not take (head dim 16) stays on the exact engine, in float32
+        # a shape the tensor-memory engine does not take (head dim 16) stays in float32
         q, k, v = (torch.randn(2, 16, 128, 16, device="cuda", generator=g) for _ in range(3))
         _lib.profile_collect()
         _lib.profile(True)
         FastMax.apply(q, k, v, None, None, True, 0.0, False, 8.0, 1.0, 1.0, 0.5, 1.0, 2)
         torch.cuda.synchronize()
         _lib.profile(False)
-        assert "scan_fwd" in set(_lib.profile_collect())
+        kinds = set(_lib.profile_collect())
+        assert "pair_f32_fwd" in kinds and "pair_fwd" not in kinds, kinds
     finally:
         torch.set_float32_matmul_precision(before)
 
@@ -324,7 +325,7 @@ def test_medium_matmul_precision_with_every_option_of_the_operator_switched_on()
     import reproducing_fastmax_results_b200 as pkg
     from reproducing_fastmax_results_b200 import _lib
 
-    B, H, N, D, rate = 2, 16, 256, 32, 0.1   # 32-wide heads: zero-padded on top
+    B, H, N, D, rate = 2, 16, 256, 32, 0.1
     g = torch.Generator(device="cuda").manual_seed(8)
     q0, k0, v0, do, noise = (torch.randn(B, H, N, D, device="cuda", generator=g) * 0.7 for _ in range(5))
     rpe = 0.05 * torch.randn(2 * N - 1, D, device="cuda", generator=g)
@@ -349,8 +350,8 @@ def test_medium_matmul_precision_with_every_option_of_the_operator_switched_on()
         fast, kinds_fast = run()
     finally:
         torch.set_float32_matmul_precision(before)
-    assert "scan_fwd" in kinds_exact and "tc_scan_fwd" not in kinds_exact
-    assert {"tc_pad", "tc_scan_fwd", "tc_scan_bwd_q"} <= kinds_fast and "scan_fwd" not in kinds_fast, kinds_fast
+    assert "pair_f32_fwd" in kinds_exact and "pair_fwd" not in kinds_exact, kinds_exact
+    assert {"pair_fwd", "pair_bwd_q", "pair_bwd_kv"} <= kinds_fast and not ({"scan_fwd", "pair_f32_fwd"} & kinds_fast), kinds_fast
     for a, b, name in zip(fast, exact, ("out", "dq", "dk", "dv")):
         assert orc.max_norm_err(host(a), host(b)) < 2e-2, name
 

@@ -147,7 +147,7 @@ def test_cuda_engine_pieces_match_whole_sequence(D, dtype, pieces):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("D,dtype,kind", [(32, torch.float32, "moments_kv"), (64, torch.float32, "moments_kv"),
-                                          (64, torch.bfloat16, "tc_scan_fwd")])
+                                          (64, torch.bfloat16, "tc_moments")])
 def test_cuda_engine_sums_the_key_moments_of_a_piece_once(D, dtype, kind):
     """A long piece with few heads and a carried state: the per-segment key moments of the state call reach the forward and
     the backward, which launch no pass over k and v of their own.  `kind`: the launches that sum them."""
@@ -170,8 +170,7 @@ def test_cuda_engine_sums_the_key_moments_of_a_piece_once(D, dtype, kind):
     (o, gg), forward = launches(lambda: eng.forward(q, k, v, total, moments=km))
     gtot, _ = launches(lambda: eng.grad_state(q, k, v, o, gg, do, total, moments=km))
     grads, backward = launches(lambda: eng.backward(q, k, v, o, gg, do, total, gtot, moments=km))
-    # (the tensor-memory forward is itself one launch of this kind)
-    assert (first, forward, backward) == ((1, 1, 0) if kind == "tc_scan_fwd" else (1, 0, 0))
+    assert (first, forward, backward) == (1, 0, 0)
     for a, b in zip(grads, eng.backward(q, k, v, o, gg, do, total, gtot)):
         assert orc.max_norm_err(a.double().cpu().numpy(), b.double().cpu().numpy()) < (1e-2 if dtype == torch.bfloat16 else 2e-6)
 
