@@ -52,8 +52,10 @@ def _float32_in_bfloat16(q):
 
 class FASTMultiHeadAttention_Function(torch.autograd.Function):
     """Behavioural twin of transformer/model.py:14-74.  float32 CUDA tensors go through the extension's native autograd node,
-    which reads them where they are (no (n, b*h, d) copies; same values, same gradients, contiguous results); what that node
-    does not cover goes through forwardpass / backwardpass on top of the `fastmax_cuda` extension, as in the reference."""
+    which reads them where they are (no (n, b*h, d) copies; same values, same gradients, contiguous results, and like the
+    reference it keeps copies of its own for the backward: what the caller writes into q, k, v or the result afterwards does
+    not matter); what that node does not cover goes through forwardpass / backwardpass on top of the `fastmax_cuda`
+    extension, as in the reference."""
 
     @classmethod
     def apply(cls, q, k, v, drop_noise, rpe_matrix=None, mask=False, dropout=0.0, normalize=False,

@@ -382,3 +382,30 @@ def test_normalisation_of_q_and_k_in_one_launch(dtype):
     assert L.profile_collect()["normalize"][1] == 2
     assert torch.equal(o, ref) and torch.equal(dq, dq_ref)
     assert (dk - dk_ref).float().norm() < (1e-6 if dtype == torch.float32 else 1e-2) * dk_ref.float().norm()   # sums in another order
+
+
+@pytest.mark.parametrize("normalize", [False, True])
+@pytest.mark.parametrize("three_d", [False, True])
+def test_writing_into_the_boundary_operators_tensors_after_the_call(normalize, three_d):
+    """FASTMultiHeadAttention_Function keeps copies of its own (model.py:29-37): overwriting q, k, v and the output between the
+    forward and the backward changes no gradient."""
+    from reproducing_fastmax_results_b200.attention import FASTMultiHeadAttention_Function
+
+    g = torch.Generator(device="cuda").manual_seed(12)
+    shape = (6, 150, 32) if three_d else (2, 3, 150, 32)
+    q0, k0, v0, do, noise = (torch.randn(*shape, device="cuda", generator=g) for _ in range(5))
+    rpe = torch.zeros(2 * 150 - 1, 32, device="cuda")
+
+    def run(overwrite):
+        leaves = [t.clone().requires_grad_(True) for t in (q0, k0, v0)]
+        q, k, v = (t * 1.0 for t in leaves)   # what a projection leaves: no leaf, may be written to
+        o = FASTMultiHeadAttention_Function.apply(q, k, v, noise, rpe, True, 0.0, normalize, 4.0, 1.0, 1.0, 0.5, 1.0, 2)
+        out = o.detach().clone()
+        if overwrite:
+            with torch.no_grad():
+                for t in (q, k, v, o):
+                    t.zero_()
+        return [out] + list(torch.autograd.grad(o, leaves, do))
+
+    for a, b in zip(run(False), run(True)):
+        assert torch.equal(a, b)
