@@ -144,7 +144,8 @@ class FastMax(torch.autograd.Function):
             return super().apply(q, k, v, drop_noise, rpe_matrix, mask, dropout, normalize, temperature, a0, a1, a2, lim, p,
                                  apply_rpe, noise_dropout)
         _alert_not_deterministic("FastMax (fastmax_custom)")
-        return _ext().fastmax(q, k, v, mask, normalize, True, False, 1.0 / temperature, a0, a1, a2, lim, p)
+        return _ext().fastmax(q, k, v, bool(mask), bool(normalize), True, False, 1.0 / float(temperature), float(a0), float(a1),
+                              float(a2), float(lim), int(p))
 
     @staticmethod
     def forward(ctx, q, k, v, drop_noise=None, rpe_matrix=None, mask=False, dropout=0.0, normalize=False,

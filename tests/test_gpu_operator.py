@@ -409,3 +409,14 @@ def test_writing_into_the_boundary_operators_tensors_after_the_call(normalize, t
 
     for a, b in zip(run(False), run(True)):
         assert torch.equal(a, b)
+
+
+def test_operator_arguments_that_convert():
+    """Numbers that are not of the declared Python type: p as a float, coefficients and the temperature as one-element tensors."""
+    from reproducing_fastmax_results_b200.attention import FastMax
+
+    g = torch.Generator(device="cuda").manual_seed(2)
+    q, k, v = (torch.randn(1, 2, 40, 16, device="cuda", generator=g) for _ in range(3))
+    ref = FastMax.apply(q, k, v, None, None, True, 0.0, False, 4.0, 1.0, 1.0, 0.5, 1.0, 2)
+    got = FastMax.apply(q, k, v, None, None, 1, 0.0, 0, torch.tensor(4.0), np.float32(1.0), torch.tensor([1.0]), 0.5, 1, 2.0)
+    assert torch.equal(ref, got)
