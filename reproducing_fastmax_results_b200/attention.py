@@ -60,8 +60,11 @@ class FASTMultiHeadAttention_Function(torch.autograd.Function):
     @classmethod
     def apply(cls, q, k, v, drop_noise, rpe_matrix=None, mask=False, dropout=0.0, normalize=False,
               temperature=1.0, a0=1.0, a1=1.0, a2=0.5, lim=1.0, p=2):
-        if (rpe_matrix is None or q.dim() not in (3, 4) or not q.is_cuda or q.dtype != torch.float32 or k.dtype != torch.float32
-                or v.dtype != torch.float32 or _float32_in_bfloat16(q)):
+        lead = q.dim() - 2   # (b, h) or (b*h): the native node reads the three tensors head by head
+        if (not isinstance(rpe_matrix, torch.Tensor) or not isinstance(drop_noise, torch.Tensor) or drop_noise.dim() != q.dim()
+                or lead not in (1, 2) or k.dim() != q.dim() or k.shape[:lead] != q.shape[:lead] or v.shape != k.shape
+                or not q.is_cuda or q.dtype != torch.float32 or k.dtype != torch.float32 or v.dtype != torch.float32
+                or _float32_in_bfloat16(q)):
             return super().apply(q, k, v, drop_noise, rpe_matrix, mask, dropout, normalize, temperature, a0, a1, a2, lim, p)
         _alert_not_deterministic("FASTMultiHeadAttention_Function")
         three_d = q.dim() == 3

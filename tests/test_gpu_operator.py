@@ -420,3 +420,23 @@ def test_operator_arguments_that_convert():
     ref = FastMax.apply(q, k, v, None, None, True, 0.0, False, 4.0, 1.0, 1.0, 0.5, 1.0, 2)
     got = FastMax.apply(q, k, v, None, None, 1, 0.0, 0, torch.tensor(4.0), np.float32(1.0), torch.tensor([1.0]), 0.5, 1, 2.0)
     assert torch.equal(ref, got)
+
+
+def test_boundary_operator_with_heads_folded_in_another_way():
+    """q as (2, 3, n, d), k and v as (3, 2, n, d): six heads each, which is what the reference's reshape to (b*h, n, d) reads.
+    A noise tensor of another rank is refused, as that reshape refuses it."""
+    from reproducing_fastmax_results_b200.attention import FASTMultiHeadAttention_Function
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q0, k0, v0 = (torch.randn(6, 50, 32, device="cuda", generator=g) for _ in range(3))
+    rpe = torch.zeros(99, 32, device="cuda")
+    options = (True, 0.0, False, 4.0, 1.0, 1.0, 0.5, 1.0, 2)
+
+    def run(shape_k):
+        q, k, v = (t.view(*shape, 50, 32) for t, shape in ((q0, (2, 3)), (k0, shape_k), (v0, shape_k)))
+        return FASTMultiHeadAttention_Function.apply(q, k, v, torch.zeros_like(q), rpe, *options)
+
+    assert orc.max_norm_err(host(run((3, 2))), host(run((2, 3)))) < 5e-6
+    q = q0.view(2, 3, 50, 32)
+    with pytest.raises(Exception):
+        FASTMultiHeadAttention_Function.apply(q, q, q, q0, rpe, *options)
