@@ -515,7 +515,9 @@ torch::Tensor decode_step(torch::Tensor q, torch::Tensor k, torch::Tensor v, tor
   TORCH_CHECK(state.is_contiguous() && state.scalar_type() == torch::kFloat32 && (size_t)state.numel() * 4 == fastmax_state_bytes(&pb),
               "state has the wrong size");
   torch::Tensor o = out.has_value() && out->defined() ? *out : torch::empty(q.sizes(), q.options());
-  TORCH_CHECK(o.sizes() == q.sizes() && o.scalar_type() == q.scalar_type() && (d == 1 || o.stride(-1) == 1), "out must look like q");
+  TORCH_CHECK((o.dim() == 3 || o.dim() == 4) && o.size(0) == b && o.size(1) == h && o.size(-1) == d && o.numel() == b * h * d &&
+                  o.scalar_type() == q.scalar_type() && (d == 1 || o.stride(-1) == 1),
+              "out must be (b, h, d) or (b, h, 1, d) of q's type, unit stride on the head dim");
   auto view = [](const torch::Tensor& t) { return fastmax_tensor{t.data_ptr(), t.stride(0), t.stride(1), 0}; };
   fastmax_decode_args a{};
   a.q = view(q); a.k = view(k); a.v = view(v); a.o = view(o);

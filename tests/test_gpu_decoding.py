@@ -204,3 +204,18 @@ def test_decoding_is_bit_for_bit_repeatable():
         runs.append((outs, state))
     assert all(torch.equal(a, b) for a, b in zip(runs[0][0], runs[1][0]))
     assert torch.equal(runs[0][1], runs[1][1])
+
+
+def test_step_into_an_output_of_either_rank():
+    """A (b, h, 1, d) token may be written into a (b, h, d) tensor and the other way round."""
+    from reproducing_fastmax_results_b200.decoding import FastmaxDecoder
+
+    g = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v = (torch.randn(2, 4, 1, 32, device="cuda", generator=g) for _ in range(3))
+    outs = []
+    for token, shape in (((q, k, v), (2, 4, 1, 32)), ((q, k, v), (2, 4, 32)), (tuple(t[:, :, 0] for t in (q, k, v)), (2, 4, 1, 32))):
+        dec = FastmaxDecoder(2, 4, 32, p=2, temperature=8.0)
+        out = torch.zeros(shape, device="cuda")
+        assert dec.step(*token, out=out) is out
+        outs.append(out.reshape(2, 4, 32))
+    assert float(outs[0].abs().max()) > 0 and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
