@@ -440,3 +440,22 @@ def test_boundary_operator_with_heads_folded_in_another_way():
     q = q0.view(2, 3, 50, 32)
     with pytest.raises(Exception):
         FASTMultiHeadAttention_Function.apply(q, q, q, q0, rpe, *options)
+
+
+@pytest.mark.parametrize("shift", [0, 1, 37])
+def test_forwardpass_normalises_overlapping_tensors_one_after_the_other(shift):
+    """q and k as windows of one buffer, `shift` tokens apart: forwardpass normalises in place, q first, then k on what q left."""
+    import reproducing_fastmax_results_b200 as pkg
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    ext = pkg.load_extension()
+    n, bh, d = 400, 160, 32   # enough heads for the one-launch form
+    g = torch.Generator(device="cuda").manual_seed(shift)
+    buf = torch.randn(n + shift, bh, d, device="cuda", generator=g)
+    v, noise, rpe = torch.randn(n, bh, d, device="cuda", generator=g), torch.zeros(n, bh, d, device="cuda"), torch.zeros(2 * n - 1, d, device="cuda")
+    ref = buf.clone()
+    for window in (slice(0, n), slice(shift, n + shift)):
+        x = ref[window].permute(1, 0, 2).unsqueeze(0)
+        ref[window] = L.normalize_forward(x, 1.0)[0][0].permute(1, 0, 2)
+    ext.forwardpass(buf[:n], buf[shift:], v, noise, rpe, True, 0.0, True, 1.0, 1.0, 1.0, 0.5, 1.0, 2)
+    assert torch.allclose(buf, ref, rtol=1e-5, atol=1e-6)
