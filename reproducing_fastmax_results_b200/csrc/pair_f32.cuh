@@ -1,4 +1,4 @@
-// Pairwise kernels for float32 tensors.  Included by pair_kernels.cu inside fm::pair.
+// Pairwise kernels with float32 weights: float32 tensors, and bf16 heads of 16 dims.  Included by pair_kernels.cu inside fm::pair.
 //
 // Every float32 operand is the exact sum of three bf16 numbers (8 + 8 + 8 bits), so a product is the sum of the six piece
 // products that reach 2^-24 of the largest: hi hi, hi mid, mid hi, mid mid, hi lo, lo hi.  q, k, v and dO' are split once, by
@@ -10,7 +10,8 @@
 // for every streamed tile (64 rows: four additions of hi hi behind the twenty small ones, which go first) and the
 // element-wise warps add the tile's result to float32 totals in registers, rounding to nearest.
 //
-// Measured: 128 heads of 1024 x 64, causal, forward + backward with splitting 13400 us in the CUDA-core engine (FFMA), 600 here.
+// Measured: 128 heads of 1024 x 64, causal, forward + backward with splitting 13400 us in the CUDA-core engine (FFMA), 600 here;
+// bf16, 128 heads of 1024 x 16 (q, k, v are one piece each: 1 or 3 products instead of 6, no pass that splits) 771 and 233.
 //
 // Roles and hand-offs are those of the bf16 kernels; the streamed pair's two tiles have barriers of their own, because with
 // three pieces each only two or three stages fit and each tile can be let go at a different time.
@@ -46,6 +47,9 @@ constexpr int THREADS_F = KIND == DKV ? (W_SUM + 4) * 32 : THREADS;
 constexpr int REG_LAUNCH = 128, REG_REST = 48, REG_EW = 136, REG_SUM = 192;
 static_assert(REG_REST * W_EW + REG_EW * EW + REG_SUM * 4 <= REG_LAUNCH * (W_SUM + 4), "setmaxnreg.inc waits for registers the block does not have");
 
+// the piece products that count, the smallest first
+__device__ constexpr int PIECE_A[6] = {0, 2, 1, 0, 1, 0}, PIECE_B[6] = {2, 0, 1, 1, 0, 0};
+
 // two float32 numbers -> their three bf16 pieces
 __device__ __forceinline__ void split3(uint64_t x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   const uint64_t minus = 0xBF800000BF800000ull;
@@ -70,10 +74,13 @@ __device__ __forceinline__ void wait_inline(uint64_t* bar, uint32_t parity, int 
   }
 }
 
-template <int D, int KIND>
+// IN: pieces of q, k and v: 3, from a pass over float32 tensors, or 1: bf16 tensors, read as they are (their results are bf16)
+template <int D, int KIND, int IN>
 __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __grid_constant__ Maps M, const Params P) {
   using L = Lay<KIND>;
   constexpr int KS = D / 16, STAGES = L::STAGES;
+  constexpr int PY = KIND == DKV ? 3 : IN, PB = KIND == DQ ? 3 : IN;   // dO', wherever it is an operand, has three pieces
+  using Out = typename std::conditional<IN == 1, __nv_bfloat16, float>::type;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* sm = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
@@ -127,9 +134,14 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
         uint64_t* bar = &bars[(y ? B_FY : B_FX) + s];
         const int row = (it.t0 + i) * TF;
         const bool nd = KIND == DKV && y;
-        mbar_arrive_expect_tx(bar, 3 * XF + (nd ? TF * 4 : 0));
+        const int pieces = y ? PY : IN;
+        mbar_arrive_expect_tx(bar, pieces * XF + (nd ? TF * 4 : 0));
+        if (pieces == 1) {
+          tma_load_4d(x, y ? &M.y : &M.x, bar, 0, row, it.h, it.b);
+        } else {
 #pragma unroll
-        for (int p = 0; p < 3; ++p) tma_load_4d(x + p * XF, y ? &M.y : &M.x, bar, 0, row, it.head, p);
+          for (int p = 0; p < 3; ++p) tma_load_4d(x + p * XF, y ? &M.y : &M.x, bar, 0, row, it.head, p);
+        }
         if (nd) bulk_load(sm + L::OFF_ND + s * TF * 4, P.ndelta + (long long)it.head * P.nd_ld + row, TF * 4, bar);
       }
       ++issued;
@@ -148,12 +160,15 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
       if (n >= 1) WAIT(B_HEMPTY, (uint32_t)n - 1u, 78);
       if (*abort_flag != 0) break;
       if (lane == 0) {
-        mbar_arrive_expect_tx(&bars[B_HFULL], L::HELD);
+        mbar_arrive_expect_tx(&bars[B_HFULL], (IN + (KIND == FWD ? 0 : PB)) * AF);
+        auto load_held = [&](uint8_t* dst, const CUtensorMap* m, int pieces) {
+          if (pieces == 1) tma_load_4d(dst, m, &bars[B_HFULL], 0, it.r0, it.h, it.b);
+          else
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
-          tma_load_4d(sm + p * AF, &M.a, &bars[B_HFULL], 0, it.r0, it.head, p);
-          if (KIND != FWD) tma_load_4d(sm + (3 + p) * AF, &M.b, &bars[B_HFULL], 0, it.r0, it.head, p);
-        }
+            for (int p = 0; p < 3; ++p) tma_load_4d(dst + p * AF, m, &bars[B_HFULL], 0, it.r0, it.head, p);
+        };
+        load_held(sm, &M.a, IN);
+        if (KIND != FWD) load_held(sm + 3 * AF, &M.b, PB);
       }
       helds = n + 1;
       for (int i = 0; i < it.n0 && *abort_flag == 0; ++i) {   // in the order in which the tiles are used
@@ -168,14 +183,17 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
     constexpr uint32_t ID_S = make_idesc_bf16(R, TF, 0, 0);
     const uint64_t dH = make_smem_desc(smem_u32(sm), 16, 1024, 2);
     const uint64_t dX0 = make_smem_desc(smem_u32(sm + L::OFF_X), 16, 1024, 2);
-    // sum over the piece products, the smallest first
-    auto product = [&](uint32_t acc, uint64_t a, uint64_t b) {
+    // sum over the piece products of a held tile with `na` pieces and a streamed one with `nb`, the smallest first
+    auto product = [&](uint32_t acc, uint64_t a, int na, uint64_t b, int nb) {
+      bool more = false;
 #pragma unroll
       for (int t = 0; t < 6; ++t) {
-        constexpr int PA[6] = {0, 2, 1, 0, 1, 0}, PB[6] = {2, 0, 1, 1, 0, 0};
+        if (PIECE_A[t] >= na || PIECE_B[t] >= nb) continue;
 #pragma unroll
-        for (int ks = 0; ks < KS; ++ks)
-          mma_ss_elect(acc, a + (uint64_t)(PA[t] * (AF >> 4) + 2 * ks), b + (uint64_t)(PB[t] * (XF >> 4) + 2 * ks), ID_S, t > 0 || ks > 0);
+        for (int ks = 0; ks < KS; ++ks) {
+          mma_ss_elect(acc, a + (uint64_t)(PIECE_A[t] * (AF >> 4) + 2 * ks), b + (uint64_t)(PIECE_B[t] * (XF >> 4) + 2 * ks), ID_S, more);
+          more = true;
+        }
       }
     };
     uint32_t k = 0;
@@ -190,17 +208,17 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
         if (KIND == DQ) {   // v is needed here only: it can go before k, which the second product reads too
           WAIT(B_FY + (int)s, k / STAGES, 74);
           tc_fence_after_sync();
-          product(tmem + C_DP, dH + (uint64_t)(3 * AF >> 4), dY);
+          product(tmem + C_DP, dH + (uint64_t)(3 * AF >> 4), PB, dY, PY);
           mma_commit_elect(&bars[B_EY + s]);
         }
         WAIT(B_FX + (int)s, k / STAGES, 73);
         tc_fence_after_sync();
-        product(tmem + C_S, dH, dX);
+        product(tmem + C_S, dH, IN, dX, IN);
         if (KIND == FWD) mma_commit_elect(&bars[B_EX + s]);
         if (KIND == DKV) {
           WAIT(B_FY + (int)s, k / STAGES, 74);
           tc_fence_after_sync();
-          product(tmem + C_DP, dH + (uint64_t)(3 * AF >> 4), dY);
+          product(tmem + C_DP, dH + (uint64_t)(3 * AF >> 4), PB, dY, PY);
         }
         mma_commit_elect(&bars[B_S]);
         ++k;
@@ -217,13 +235,16 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
     // ================= issuer of the second products =================
     constexpr uint32_t ID_ACC = make_idesc_bf16(R, D, 0, 1);
     const uint64_t dX0 = make_smem_desc(smem_u32(sm + L::OFF_X), XF, 1024, 2);
-    auto product = [&](uint32_t acc, uint32_t a, uint64_t b) {
+    auto product = [&](uint32_t acc, uint32_t a, uint64_t b, int nb) {   // P or dS (three pieces) with a streamed tile
+      bool more = false;
 #pragma unroll
       for (int t = 0; t < 6; ++t) {
-        constexpr int PA[6] = {0, 2, 1, 0, 1, 0}, PB[6] = {2, 0, 1, 1, 0, 0};
+        if (PIECE_B[t] >= nb) continue;
 #pragma unroll
-        for (int kk = 0; kk < TF / 16; ++kk)
-          mma_ts_elect(acc, a + 32u * PA[t] + 8u * kk, b + (uint64_t)(PB[t] * (XF >> 4) + 128 * kk), ID_ACC, t > 0 || kk > 0);
+        for (int kk = 0; kk < TF / 16; ++kk) {
+          mma_ts_elect(acc, a + 32u * PIECE_A[t] + 8u * kk, b + (uint64_t)(PIECE_B[t] * (XF >> 4) + 128 * kk), ID_ACC, more);
+          more = true;
+        }
       }
     };
     uint32_t k = 0;
@@ -238,11 +259,11 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
         if (k > 0) WAIT(B_AFREE, k - 1u, 82);   // the last tile's results are in the totals
         tc_fence_after_sync();
         if (KIND != FWD) {
-          product(tmem + (KIND == DKV ? C_ACC1 : C_ACC), tmem + C_DS, dX);
+          product(tmem + (KIND == DKV ? C_ACC1 : C_ACC), tmem + C_DS, dX, IN);
           mma_commit_elect(&bars[B_EX + s]);
         }
         if (KIND != DQ) {
-          product(tmem + C_ACC, tmem + C_P, dY);
+          product(tmem + C_ACC, tmem + C_P, dY, PY);
           mma_commit_elect(&bars[B_EY + s]);
         }
         mma_commit_elect(&bars[B_ACC]);
@@ -289,8 +310,8 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
 #pragma unroll
       for (int c = 0; c < NA / CH; ++c) {
         const View& out = KIND == DKV && c * CH < D ? P.out1 : P.out0;
-        float* base = reinterpret_cast<float*>(const_cast<void*>(out.ptr)) + (long long)it.b * out.sb + (long long)it.h * out.sh +
-                      (KIND == DKV ? c * CH % D : half * NA + CH * c);
+        Out* base = reinterpret_cast<Out*>(const_cast<void*>(out.ptr)) + (long long)it.b * out.sb + (long long)it.h * out.sh +
+                    (KIND == DKV ? c * CH % D : half * NA + CH * c);
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < CH / 2; ++j) {
@@ -306,7 +327,7 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
         for (int r = 0; r < 32; r += RP) {
           const int g = it.r0 + quarter * 32 + r + rr;
           const float v = stage[(r + rr) * 32 + (cc ^ (r + rr))];
-          if (g < P.nr) base[(long long)g * out.sn + cc] = v;
+          if (g < P.nr) base[(long long)g * out.sn + cc] = static_cast<Out>(v);
         }
       }
     };
@@ -495,8 +516,8 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitArgs A, int heads
   if (c == 0 && ld > D) store_tail(A.out[t], plane, at + D, 1.f);
 }
 
-// dO' = dO / g in pieces (ld = D + 16: with -delta behind the values) and -delta = -(dO . o) / g
-template <int D, bool VEC>
+// dO' = dO / g in pieces (ld = D + 16: with -delta behind the values) and -delta = -(dO . o) / g; T: the type of dO and o
+template <typename T, int D, bool VEC>
 __global__ void __launch_bounds__(256) prologue_f32_kernel(View dout, View o, View g, __nv_bfloat16* __restrict__ dop, float* __restrict__ ndelta,
                                                            int nq, int nd_ld, int heads, int ld) {
   constexpr int TPR = D / 8;
@@ -504,21 +525,25 @@ __global__ void __launch_bounds__(256) prologue_f32_kernel(View dout, View o, Vi
   const int row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, c = (threadIdx.x % TPR) * 8;
   float v[8], dot = 0.f;
   if (row < nq) {
-    const float* pd = reinterpret_cast<const float*>(dout.ptr) + (long long)b * dout.sb + (long long)h * dout.sh + (long long)row * dout.sn + c;
-    const float* po = reinterpret_cast<const float*>(o.ptr) + (long long)b * o.sb + (long long)h * o.sh + (long long)row * o.sn + c;
+    const T* pd = reinterpret_cast<const T*>(dout.ptr) + (long long)b * dout.sb + (long long)h * dout.sh + (long long)row * dout.sn + c;
+    const T* po = reinterpret_cast<const T*>(o.ptr) + (long long)b * o.sb + (long long)h * o.sh + (long long)row * o.sn + c;
     const float inv = 1.f / reinterpret_cast<const float*>(g.ptr)[(long long)b * g.sb + (long long)h * g.sh + (long long)row * g.sn];
     float x[8];
+    alignas(16) T td[8], to[8];
     if (VEC) {
-      *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(pd);
-      *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(pd + 4);
-      *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(po);
-      *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(po + 4);
+#pragma unroll
+      for (int i = 0; i < (int)sizeof(T) / 2; ++i) {
+        reinterpret_cast<uint4*>(td)[i] = reinterpret_cast<const uint4*>(pd)[i];
+        reinterpret_cast<uint4*>(to)[i] = reinterpret_cast<const uint4*>(po)[i];
+      }
     } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) { v[i] = pd[i]; x[i] = po[i]; }
+      for (int i = 0; i < 8; ++i) { td[i] = pd[i]; to[i] = po[i]; }
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
+      v[i] = static_cast<float>(td[i]);
+      x[i] = static_cast<float>(to[i]);
       v[i] *= inv;
       dot += v[i] * x[i];
     }

@@ -18,7 +18,8 @@
 //
 // Bound by neither pipe alone: the tensor pipe is busy 55 to 65 % of the time at d = 64 (21 to 29 % at d = 32), the element-wise
 // warps issue in 40 to 47 % of their slots.  Measured (us; the scans of the moment engine before): 128 heads of 4096 x 64, causal,
-// forward + backward 2930 -> 1080; 128 heads of 1024 x 64 570 -> 135; 128 heads of 2048 x 32 1533 -> 285.
+// forward + backward 2930 -> 1080; 128 heads of 1024 x 64 570 -> 135; 128 heads of 2048 x 32 1533 -> 285.  Heads of 16 dims have
+// the kernels of pair_f32.cuh.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -455,7 +456,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
       ++done;
       if (!writes) return;
       tc_fence_after_sync();
-      constexpr int CH = D < 32 ? D : 32;
+      constexpr int CH = 32;
       uint32_t r[D / CH][CH];
 #pragma unroll
       for (int c = 0; c < D / CH; ++c) tmem_ld<CH>(lane_addr + (KIND == FWD ? 64u * grp : 64u * half) + (uint32_t)(CH * c), r[c]);
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
       if (partial) {
         uint8_t* stage = sm + OFF_HELD + (n & 1) * STAGE + (KIND == FWD ? grp : half) * X_BYTES + quarter * 4096;
 #pragma unroll
-        for (int c = 0; c < (D < 32 ? 1 : D / 32); ++c) {
+        for (int c = 0; c < D / 32; ++c) {
           if (c > 0) {   // one box of space per warp
             if (lane == 0) bulk_wait_read_all();
             __syncwarp();
@@ -819,7 +820,6 @@ template <int KIND, bool SQ>
 cudaError_t launch_d(int d, const pair::Maps& M, pair::Params& P, int bh, cudaStream_t st) {
   order_items(d, 2, P, bh);
   switch (d) {
-    case 16: return launch<16, KIND, SQ>(M, P, bh, st);
     case 32: return launch<32, KIND, SQ>(M, P, bh, st);
     default: return launch<64, KIND, SQ>(M, P, bh, st);
   }
@@ -836,6 +836,10 @@ size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 }  // namespace
 bool f32_registers_ok();
 namespace {
+// bf16 heads of 16 dims have no tensor-memory engine beside the pairs: their weights stay float32 there (split into pieces, results
+// rounded once) as in the CUDA-core engine.  Relative error of dq, 16 heads of 1024 tokens: 1.7e-3 that way, which is the
+// rounding of the result, 3.2e-3 with bf16 weights.
+bool float32_weights(const fastmax_problem* pb) { return pb->dtype == FASTMAX_F32 || pb->d == 16; }
 // a view the copy engine can read (a stride of a size-1 dimension is never used)
 bool mappable(const fastmax_tensor& t, const fastmax_problem* pb, int n) {
   if (pb->dtype == FASTMAX_F32) return t.ptr != nullptr;   // split by ordinary loads
@@ -892,10 +896,13 @@ int chosen(const fastmax_problem* pb, bool backward, Use use) {   // 0: neither,
   }
   // order 1 without a mask: one pass over the tensors (p1_forward_kernel), always the cheapest where it fills the GPU
   if (!backward && pb->order == 1 && !pb->causal && pb->d == 64 && (long long)pb->batch * pb->heads >= 64) return 0;
-  // d = 16 has no states kernel.  Causal calls beyond 3000 tokens stay with the CUDA-core engine: the first tokens' gradients are
-  // a hundred times the others there, and the float32 weights of that engine round their bf16 results to the last bit.
+  // d = 16: float32 weights (float32_weights) against the CUDA-core engine; there is no states kernel.  us, forward / backward,
+  // pairs against engine: order 2, mask, 64 heads 4096 tokens 359 / 1041 against 574 / 1565, 32 heads 8192 687 / 1996 against
+  // 543 / 1495; no mask, 64 heads 2048 182 / 521 against 202 / 602, 4096 680 / 1987 against 384 / 1175; order 1, mask, 64 heads
+  // 2048 103 / 295 against 122 / 350, 4096 359 / 1041 against 229 / 705; no mask, 64 heads 256 31 / 49 against 45 / 74, 128
+  // heads 1024 97 / 278 against 67 / 188.
   if (pb->d == 16)
-    return per_token <= (pb->order == 2 ? (pb->causal ? 1500.0 : 6500.0) : backward || pb->causal ? 1300.0 : 2000.0) ? 1 : 0;
+    return per_token <= (pb->order == 2 ? (pb->causal ? 3000.0 : 2300.0) : pb->causal ? 1200.0 : 700.0) && f32_registers_ok() ? 1 : 0;
   if (per_token <= window_line(pb, use)) return 1;
   if (pb->causal && pb->nq != pb->nk) return per_token <= (pb->order == 2 ? 6500.0 : backward ? 1300.0 : 2000.0) ? 1 : 0;
   if ((long long)(pb->nq > pb->nk ? pb->nq : pb->nk) >= (1ll << 30)) return 0;
@@ -963,20 +970,20 @@ bool pair_takes_backward(const fastmax_problem* pb, const fastmax_backward_args*
 // ---- float32 ------------------------------------------------------------------------------------------------------------
 // bf16 pieces [3][batch*heads][n][d] as a tensor map: piece = batch index, head = batch*heads
 static size_t pieces_bytes(const fastmax_problem* pb, int n, int ld = 0) { return up256((size_t)3 * pb->batch * pb->heads * n * (ld > 0 ? ld : pb->d) * 2); }
+static size_t input_bytes(const fastmax_problem* pb, int n) { return pb->dtype == FASTMAX_F32 ? pieces_bytes(pb, n) : 0; }   // pieces of q, k or v
 static size_t long_forward_workspace(const fastmax_problem* pb);
 static size_t long_f32_forward_workspace(const fastmax_problem* pb);
 static size_t long_f32_backward_workspace(const fastmax_problem* pb);
 static size_t long_backward_workspace(const fastmax_problem* pb);
 size_t pair_forward_workspace(const fastmax_problem* pb, const fastmax_forward_args* a) {
-  if (pb->dtype == FASTMAX_F32) return forward_form(pb, a) == 2 ? long_f32_forward_workspace(pb) : pieces_bytes(pb, pb->nq) + 2 * pieces_bytes(pb, pb->nk);
-  return forward_form(pb, a) == 2 ? long_forward_workspace(pb) : 0;
+  if (forward_form(pb, a) == 2) return pb->dtype == FASTMAX_F32 ? long_f32_forward_workspace(pb) : long_forward_workspace(pb);
+  return input_bytes(pb, pb->nq) + 2 * input_bytes(pb, pb->nk);
 }
 size_t pair_backward_workspace(const fastmax_problem* pb, const fastmax_backward_args* a) {
   if (backward_form(pb, a) == 2) return pb->dtype == FASTMAX_F32 ? long_f32_backward_workspace(pb) : long_backward_workspace(pb);
-  if (pb->dtype == FASTMAX_F32)
-    return 2 * pieces_bytes(pb, pb->nq) + 2 * pieces_bytes(pb, pb->nk) + up256((size_t)pb->batch * pb->heads * nd_ld(pb->nq) * sizeof(float));
-  const size_t bh = (size_t)pb->batch * pb->heads;
-  return up256(bh * pb->nq * pb->d * 2) + up256(bh * nd_ld(pb->nq) * sizeof(float));
+  const size_t bh = (size_t)pb->batch * pb->heads, delta = up256(bh * nd_ld(pb->nq) * sizeof(float));
+  if (float32_weights(pb)) return pieces_bytes(pb, pb->nq) + input_bytes(pb, pb->nq) + 2 * input_bytes(pb, pb->nk) + delta;
+  return up256(bh * pb->nq * pb->d * 2) + delta;
 }
 
 // rows [first, n) of every piece and head; columns past `cols` read as zero
@@ -998,9 +1005,9 @@ static void launch_split(const fastmax_problem* pb, const pair::f32::SplitArgs& 
     default: pair::f32::split_kernel<64><<<grid, 256, 0, st>>>(A, pb->heads); break;
   }
 }
-template <int D, int KIND>
+template <int D, int KIND, int IN>
 static cudaError_t launch_f32(const pair::Maps& M, const pair::Params& P, int bh, cudaStream_t st) {
-  auto kernel = pair::f32::pair_f32_kernel<D, KIND>;
+  auto kernel = pair::f32::pair_f32_kernel<D, KIND, IN>;
   constexpr int bytes = pair::f32::Lay<KIND>::BYTES;
   static std::atomic<bool> done[64];
   int dev = 0;
@@ -1015,36 +1022,50 @@ static cudaError_t launch_f32(const pair::Maps& M, const pair::Params& P, int bh
   return cudaGetLastError();
 }
 template <int KIND>
-static cudaError_t launch_f32_d(int d, const pair::Maps& M, pair::Params& P, int bh, cudaStream_t st) {
-  order_items(d, 6, P, bh);
-  switch (d) {
-    case 16: return launch_f32<16, KIND>(M, P, bh, st);
-    case 32: return launch_f32<32, KIND>(M, P, bh, st);
-    default: return launch_f32<64, KIND>(M, P, bh, st);
+static cudaError_t launch_f32_d(const fastmax_problem* pb, const pair::Maps& M, pair::Params& P, cudaStream_t st) {
+  const int bh = pb->batch * pb->heads;
+  order_items(pb->d, pb->dtype == FASTMAX_F32 ? 6 : 2, P, bh);
+  if (pb->dtype == FASTMAX_BF16) return launch_f32<16, KIND, 1>(M, P, bh, st);
+  switch (pb->d) {
+    case 16: return launch_f32<16, KIND, 3>(M, P, bh, st);
+    case 32: return launch_f32<32, KIND, 3>(M, P, bh, st);
+    default: return launch_f32<64, KIND, 3>(M, P, bh, st);
   }
 }
 // dk / dv move registers between their warps (setmaxnreg), which only ends if the blocks are launched with what the budget
 // in pair_f32.cuh assumes
 bool f32_registers_ok() {
   static const bool ok = [] {
-    cudaFuncAttributes a{}, b{}, c{};
-    return cudaFuncGetAttributes(&a, pair::f32::pair_f32_kernel<16, pair::DKV>) == cudaSuccess && a.numRegs == pair::f32::REG_LAUNCH &&
-           cudaFuncGetAttributes(&b, pair::f32::pair_f32_kernel<32, pair::DKV>) == cudaSuccess && b.numRegs == pair::f32::REG_LAUNCH &&
-           cudaFuncGetAttributes(&c, pair::f32::pair_f32_kernel<64, pair::DKV>) == cudaSuccess && c.numRegs == pair::f32::REG_LAUNCH;
+    auto right = [](auto kernel) {
+      cudaFuncAttributes a{};
+      return cudaFuncGetAttributes(&a, kernel) == cudaSuccess && a.numRegs == pair::f32::REG_LAUNCH;
+    };
+    return right(pair::f32::pair_f32_kernel<16, pair::DKV, 3>) && right(pair::f32::pair_f32_kernel<32, pair::DKV, 3>) &&
+           right(pair::f32::pair_f32_kernel<64, pair::DKV, 3>) && right(pair::f32::pair_f32_kernel<16, pair::DKV, 1>);
   }();
   return ok;
 }
 
+// Tensor map of q, k or v: their pieces, or (bf16) the tensor itself
+static bool input_map(CUtensorMap* m, const fastmax_tensor& t, void* pieces, const fastmax_problem* pb, int n, int rows) {
+  return pb->dtype == FASTMAX_F32 ? pieces_map(m, pieces, pb, n, rows) : tc_make_map(m, t, pb->batch, pb->heads, n, 64, rows, true, pb->d);
+}
+static cudaError_t split_inputs(const fastmax_problem* pb, const fastmax_tensor& q, const fastmax_tensor& k, const fastmax_tensor& v, void* qp, void* kp, void* vp,
+                                cudaStream_t st) {
+  if (pb->dtype != FASTMAX_F32) return cudaSuccess;
+  launch_split(pb, pair::f32::SplitArgs{{view_of(q), view_of(k), view_of(v)}, {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp},
+                                        {pb->nq, pb->nk, pb->nk}, {pb->d, pb->d, pb->d}}, 3, st);
+  return cudaGetLastError();
+}
 static int pair_f32_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st) {
   char* base = (char*)ws;
-  void *qp = base, *kp = base + pieces_bytes(pb, pb->nq), *vp = base + pieces_bytes(pb, pb->nq) + pieces_bytes(pb, pb->nk);
+  void *qp = base, *kp = base + input_bytes(pb, pb->nq), *vp = base + input_bytes(pb, pb->nq) + input_bytes(pb, pb->nk);
   pair::Maps M;
-  if (!pieces_map(&M.a, qp, pb, pb->nq, pair::R) || !pieces_map(&M.x, kp, pb, pb->nk, pair::f32::TF) || !pieces_map(&M.y, vp, pb, pb->nk, pair::f32::TF))
+  if (!input_map(&M.a, a->q, qp, pb, pb->nq, pair::R) || !input_map(&M.x, a->k, kp, pb, pb->nk, pair::f32::TF) ||
+      !input_map(&M.y, a->v, vp, pb, pb->nk, pair::f32::TF))
     return FASTMAX_ERR_UNSUPPORTED;
   M.b = M.o0 = M.o1 = M.a;
-  launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
-                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {pb->nq, pb->nk, pb->nk}, {pb->d, pb->d, pb->d}}, 3, st);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = split_inputs(pb, a->q, a->k, a->v, qp, kp, vp, st);
   if (e != cudaSuccess) return report_cuda_error(e);
   pair::Params P{};
   fill(pb, P);
@@ -1054,47 +1075,47 @@ static int pair_f32_forward(const fastmax_problem* pb, const fastmax_forward_arg
   P.nx = pb->nk;
   P.ntiles = tiles(pb->nq);
   LaunchScope ls(KK_PAIR_F32_FWD, st);
-  e = launch_f32_d<pair::FWD>(pb->d, M, P, pb->batch * pb->heads, st);
+  e = launch_f32_d<pair::FWD>(pb, M, P, st);
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
 
-template <int D>
+template <typename T, int D>
 static void launch_prologue_f32(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
   const int ld = nd_ld(pb->nq), rows = 256 / (D / 8);
   const dim3 grid((unsigned)((ld + rows - 1) / rows), (unsigned)(pb->batch * pb->heads));
   auto vec = [](const fastmax_tensor& t) {
-    return ((uintptr_t)t.ptr & 15) == 0 && (t.stride_b & 3) == 0 && (t.stride_h & 3) == 0 && (t.stride_n & 3) == 0;
+    constexpr int64_t odd = 16 / sizeof(T) - 1;
+    return ((uintptr_t)t.ptr & 15) == 0 && (t.stride_b & odd) == 0 && (t.stride_h & odd) == 0 && (t.stride_n & odd) == 0;
   };
   if (vec(a->o) && vec(a->d_out))
-    pair::f32::prologue_f32_kernel<D, true><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+    pair::f32::prologue_f32_kernel<T, D, true><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
   else
-    pair::f32::prologue_f32_kernel<D, false><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+    pair::f32::prologue_f32_kernel<T, D, false><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
 }
 
 static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
-  const int bh = pb->batch * pb->heads;
-  const size_t nqb = pieces_bytes(pb, pb->nq), nkb = pieces_bytes(pb, pb->nk);
+  const size_t nqb = input_bytes(pb, pb->nq), nkb = input_bytes(pb, pb->nk), dob = pieces_bytes(pb, pb->nq);
   char* base = (char*)ws;
-  void *qp = base, *dp = base + nqb, *kp = base + 2 * nqb, *vp = base + 2 * nqb + nkb;
-  float* nd = (float*)(base + 2 * nqb + 2 * nkb);
+  void *dp = base, *qp = base + dob, *kp = base + dob + nqb, *vp = base + dob + nqb + nkb;
+  float* nd = (float*)(base + dob + nqb + 2 * nkb);
   pair::Maps M, N;   // M: dq, N: dk and dv
-  if (!pieces_map(&M.a, qp, pb, pb->nq, pair::R) || !pieces_map(&M.b, dp, pb, pb->nq, pair::R) ||
-      !pieces_map(&M.x, kp, pb, pb->nk, pair::f32::TF) || !pieces_map(&M.y, vp, pb, pb->nk, pair::f32::TF) ||
-      !pieces_map(&N.a, kp, pb, pb->nk, pair::R) || !pieces_map(&N.b, vp, pb, pb->nk, pair::R) ||
-      !pieces_map(&N.x, qp, pb, pb->nq, pair::f32::TF) || !pieces_map(&N.y, dp, pb, pb->nq, pair::f32::TF))
+  if (!input_map(&M.a, a->q, qp, pb, pb->nq, pair::R) || !pieces_map(&M.b, dp, pb, pb->nq, pair::R) ||
+      !input_map(&M.x, a->k, kp, pb, pb->nk, pair::f32::TF) || !input_map(&M.y, a->v, vp, pb, pb->nk, pair::f32::TF) ||
+      !input_map(&N.a, a->k, kp, pb, pb->nk, pair::R) || !input_map(&N.b, a->v, vp, pb, pb->nk, pair::R) ||
+      !input_map(&N.x, a->q, qp, pb, pb->nq, pair::f32::TF) || !pieces_map(&N.y, dp, pb, pb->nq, pair::f32::TF))
     return FASTMAX_ERR_UNSUPPORTED;
   M.o0 = M.o1 = N.o0 = N.o1 = M.a;
-  launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
-                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {pb->nq, pb->nk, pb->nk}, {pb->d, pb->d, pb->d}}, 3, st);
+  cudaError_t e = split_inputs(pb, a->q, a->k, a->v, qp, kp, vp, st);
+  if (e != cudaSuccess) return report_cuda_error(e);
   {
     LaunchScope ls(KK_PROLOGUE, st);
-    switch (pb->d) {
-      case 16: launch_prologue_f32<16>(pb, a, (__nv_bfloat16*)dp, nd, pb->d, st); break;
-      case 32: launch_prologue_f32<32>(pb, a, (__nv_bfloat16*)dp, nd, pb->d, st); break;
-      default: launch_prologue_f32<64>(pb, a, (__nv_bfloat16*)dp, nd, pb->d, st); break;
-    }
+    __nv_bfloat16* dop = (__nv_bfloat16*)dp;
+    if (pb->dtype == FASTMAX_BF16) launch_prologue_f32<__nv_bfloat16, 16>(pb, a, dop, nd, pb->d, st);
+    else if (pb->d == 16) launch_prologue_f32<float, 16>(pb, a, dop, nd, pb->d, st);
+    else if (pb->d == 32) launch_prologue_f32<float, 32>(pb, a, dop, nd, pb->d, st);
+    else launch_prologue_f32<float, 64>(pb, a, dop, nd, pb->d, st);
   }
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) return report_cuda_error(e);
   pair::Params P{};
   fill(pb, P);
@@ -1108,7 +1129,7 @@ static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   K.ntiles = tiles(pb->nk);
   {
     LaunchScope ls(KK_PAIR_F32_BWD_KV, st);
-    e = launch_f32_d<pair::DKV>(pb->d, N, K, bh, st);
+    e = launch_f32_d<pair::DKV>(pb, N, K, st);
   }
   if (e != cudaSuccess) return report_cuda_error(e);
   P.out0 = P.out1 = view_of(a->dq);
@@ -1117,7 +1138,7 @@ static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   P.ntiles = tiles(pb->nq);
   {
     LaunchScope ls(KK_PAIR_F32_BWD_Q, st);
-    e = launch_f32_d<pair::DQ>(pb->d, M, P, bh, st);
+    e = launch_f32_d<pair::DQ>(pb, M, P, st);
   }
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
@@ -1139,11 +1160,8 @@ static void launch_prologue(const fastmax_problem* pb, const fastmax_backward_ar
 }
 static void launch_prologue_any(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
   LaunchScope ls(KK_PROLOGUE, st);
-  switch (pb->d) {
-    case 16: launch_prologue<16>(pb, a, dop, nd, dld, st); break;
-    case 32: launch_prologue<32>(pb, a, dop, nd, dld, st); break;
-    default: launch_prologue<64>(pb, a, dop, nd, dld, st); break;
-  }
+  if (pb->d == 32) launch_prologue<32>(pb, a, dop, nd, dld, st);
+  else launch_prologue<64>(pb, a, dop, nd, dld, st);
 }
 
 // ---- long bf16 sequences (long_kernels.cuh) -----------------------------------------------------------------------------
@@ -1485,7 +1503,7 @@ static int long_f32_forward(const fastmax_problem* pb, const fastmax_forward_arg
     P.nr = P.nx = n;
     P.ntiles = tiles(n);
     LaunchScope ls(KK_PAIR_F32_FWD, st);
-    e = launch_f32_d<pair::FWD>(pb->d, M, P, bh, st);
+    e = launch_f32_d<pair::FWD>(pb, M, P, st);
   }
   if (e == cudaSuccess && !a->key_moments_in) e = long_states_f32(pb, g, a->k, vp, n, 0, g.ns * g.L, false, raw, S, st);
   lng::Params P = long_params(pb, g, S, n, g.L, n);
@@ -1523,7 +1541,7 @@ static int long_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
                                         {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {n, n, n}, {pb->d, pb->d, NC}}, 3, st);
   {
     LaunchScope ls(KK_PROLOGUE, st);
-    launch_prologue_f32<32>(pb, a, (__nv_bfloat16*)dp, nd, NC, st);
+    launch_prologue_f32<float, 32>(pb, a, (__nv_bfloat16*)dp, nd, NC, st);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return report_cuda_error(e);
@@ -1539,12 +1557,12 @@ static int long_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   B.out1 = view_of(a->dv);
   {
     LaunchScope ls(KK_PAIR_F32_BWD_KV, st);
-    e = launch_f32_d<pair::DKV>(pb->d, N, B, bh, st);
+    e = launch_f32_d<pair::DKV>(pb, N, B, st);
   }
   P.out0 = P.out1 = view_of(a->dq);
   if (e == cudaSuccess) {
     LaunchScope ls(KK_PAIR_F32_BWD_Q, st);
-    e = launch_f32_d<pair::DQ>(pb->d, M, P, bh, st);
+    e = launch_f32_d<pair::DQ>(pb, M, P, st);
   }
   if (e == cudaSuccess && !a->key_moments_in) e = long_states_f32(pb, g, a->k, vp, n, 0, g.ns * g.L, false, raw, S, st);
   // gradient moments of every segment but the first; raw may be reused: the stream orders it
@@ -1571,8 +1589,8 @@ size_t pair_key_moments_bytes(const fastmax_problem* pb) {
 bool pair_reads_key_moments(const fastmax_problem* pb, const fastmax_backward_args* a) { return backward_form(pb, a) == 2; }
 
 int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st) {
-  if (pb->dtype == FASTMAX_F32) return forward_form(pb, a) == 2 ? long_f32_forward(pb, a, ws, st) : pair_f32_forward(pb, a, ws, st);
-  if (forward_form(pb, a) == 2) return long_forward(pb, a, ws, st);
+  if (forward_form(pb, a) == 2) return pb->dtype == FASTMAX_F32 ? long_f32_forward(pb, a, ws, st) : long_forward(pb, a, ws, st);
+  if (float32_weights(pb)) return pair_f32_forward(pb, a, ws, st);
   pair::Maps M;
   if (!tc_make_map(&M.a, a->q, pb->batch, pb->heads, pb->nq, 64, pair::R, true, pb->d) ||
       !tc_make_map(&M.x, a->k, pb->batch, pb->heads, pb->nk, 64, pair::T, true, pb->d) ||
@@ -1595,8 +1613,8 @@ int pair_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void*
 }
 
 int pair_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
-  if (pb->dtype == FASTMAX_F32) return backward_form(pb, a) == 2 ? long_f32_backward(pb, a, ws, st) : pair_f32_backward(pb, a, ws, st);
-  if (backward_form(pb, a) == 2) return long_backward(pb, a, ws, st);
+  if (backward_form(pb, a) == 2) return pb->dtype == FASTMAX_F32 ? long_f32_backward(pb, a, ws, st) : long_backward(pb, a, ws, st);
+  if (float32_weights(pb)) return pair_f32_backward(pb, a, ws, st);
   const int bh = pb->batch * pb->heads;
   __nv_bfloat16* dop = (__nv_bfloat16*)ws;
   float* nd = (float*)((char*)ws + up256((size_t)bh * pb->nq * pb->d * 2));
