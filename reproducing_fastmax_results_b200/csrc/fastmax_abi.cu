@@ -543,7 +543,7 @@ int32_t fastmax_forward(const fastmax_problem* pb, const fastmax_forward_args* a
   a = without_unusable_moments(pb, a, copy);
   fastmax_forward_args out_call, state_call;
   if (want_o && splits_prompt(pb, a, out_call, state_call)) {
-    // side by side, the state first: the other call's blocks fill the SMs its last round leaves idle
+    // side by side: the state's blocks fill the SMs that the output's last round leaves idle
     fastmax_problem keys = keys_only(pb);
     keys.flags |= FASTMAX_FLAG_SINGLE_STREAM;
     const size_t own = align_up(fastmax_forward_workspace(pb, &out_call), 256);

@@ -266,30 +266,29 @@ __global__ void __launch_bounds__(THREADS, 1) moments_kernel(const __grid_consta
 }
 }  // namespace mo
 
-// ---- raw states -> weighted pieces of the state before (reverse: after) each segment, or of all of them --------------------
+// ---- raw states -> weighted pieces of the state before (reverse: after) each segment ----------------------------------------
 // Running sum over the segments, times the polynomial weights, split.  A thread owns (unit, block of eight columns, row) of a
 // head; four segments' loads are in flight (one at a time, the sum over 255 segments was a chain of memory latencies).
-__global__ void __launch_bounds__(64) pack_kernel(const float* __restrict__ raw, uint8_t* __restrict__ S, float* __restrict__ cst, int nraw, int ns, int reverse,
+__global__ void __launch_bounds__(64) pack_kernel(const float* __restrict__ raw, uint8_t* __restrict__ S, float* __restrict__ cst, int ns, int reverse,
                                                   int order, float c0, float c1, float c2) {
   const int u0 = order == 2 ? 0 : NPAIR, u = u0 + blockIdx.x, cb = blockIdx.y, head = blockIdx.z, r = threadIdx.x;
   const int rows = (order == 2 ? 64 * NPAIR : 0) + D + 1;
   const long long step = (long long)rows * LD;
-  const float* src = raw + (long long)head * nraw * step;
+  const float* src = raw + (long long)head * ns * step;
   constexpr int AHEAD = 4;
   if (u == UNITS) {   // the constant row
     if (cb > 0 || r >= CST) return;
     float s = 0.f;
     src += (long long)(rows - 1) * LD + r;
-    for (int i0 = 0; i0 < nraw; i0 += AHEAD) {
+    for (int i0 = 0; i0 < ns; i0 += AHEAD) {
       float v[AHEAD];
 #pragma unroll
-      for (int e = 0; e < AHEAD; ++e) v[e] = r <= D && i0 + e < nraw ? src[(reverse ? nraw - 1 - i0 - e : i0 + e) * step] : 0.f;
+      for (int e = 0; e < AHEAD; ++e) v[e] = r <= D && i0 + e < ns ? src[(reverse ? ns - 1 - i0 - e : i0 + e) * step] : 0.f;
 #pragma unroll
       for (int e = 0; e < AHEAD; ++e) {
         const int i = i0 + e;
         s += v[e];
-        const int k = ns == nraw ? (reverse ? ns - 1 - i : i) : 0;
-        if (i < nraw && (ns == nraw || i == nraw - 1)) cst[((long long)head * ns + k) * CST + r] = s * c0;
+        if (i < ns) cst[((long long)head * ns + (reverse ? ns - 1 - i : i)) * CST + r] = s * c0;
       }
     }
     return;
@@ -304,13 +303,13 @@ __global__ void __launch_bounds__(64) pack_kernel(const float* __restrict__ raw,
   src += (long long)(64 * (u - u0) + r) * LD + 8 * cb;
   uint8_t* dst = S + ((long long)head * ns * UNITS + u) * UNIT + cb * 1024 + r * 16;
   float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int i0 = 0; i0 < nraw; i0 += AHEAD) {
+  for (int i0 = 0; i0 < ns; i0 += AHEAD) {
     float4 v[AHEAD][2];
 #pragma unroll
     for (int e = 0; e < AHEAD; ++e) {
       v[e][0] = v[e][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (live && i0 + e < nraw) {
-        const float4* p = reinterpret_cast<const float4*>(src + (reverse ? nraw - 1 - i0 - e : i0 + e) * step);
+      if (live && i0 + e < ns) {
+        const float4* p = reinterpret_cast<const float4*>(src + (reverse ? ns - 1 - i0 - e : i0 + e) * step);
         v[e][0] = p[0];
         if (cb < D / 8) v[e][1] = p[1];
       }
@@ -320,8 +319,8 @@ __global__ void __launch_bounds__(64) pack_kernel(const float* __restrict__ raw,
       const int i = i0 + e;
       s[0] += v[e][0].x; s[1] += v[e][0].y; s[2] += v[e][0].z; s[3] += v[e][0].w;
       s[4] += v[e][1].x; s[5] += v[e][1].y; s[6] += v[e][1].z; s[7] += v[e][1].w;
-      const int k = ns == nraw ? (reverse ? ns - 1 - i : i) : 0;
-      if (i < nraw && (ns == nraw || i == nraw - 1)) {
+      const int k = reverse ? ns - 1 - i : i;
+      if (i < ns) {
         uint32_t o[3][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) split3(pack2(s[2 * j] * wgt, s[2 * j + 1] * wgt), o[0][j], o[1][j], o[2][j]);
@@ -399,15 +398,13 @@ __global__ void __launch_bounds__(THREADS, 1) apply_kernel(const __grid_constant
           bulk_load(sm + OFF_S + s * UNIT, src + (long long)j * UNIT, UNIT, &bars[B_SFULL + s]);
         }
       }
-      if (P.part) {
-        if (n >= 1) WAIT(B_PFREE, (uint32_t)n - 1u, 152);
-        if (*abort_flag != 0) break;
-        if (lane == 0) {
-          mbar_arrive_expect_tx(&bars[B_PFULL], 2 * LT);
-          for (int m = 0; m < 2; ++m) tma_load_4d(sm + OFF_P + m * LT, &M.part, &bars[B_PFULL], 0, k.tok + m * 128, k.h, k.b);
-        }
-        parts = n + 1;
+      if (n >= 1) WAIT(B_PFREE, (uint32_t)n - 1u, 152);
+      if (*abort_flag != 0) break;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&bars[B_PFULL], 2 * LT);
+        for (int m = 0; m < 2; ++m) tma_load_4d(sm + OFF_P + m * LT, &M.part, &bars[B_PFULL], 0, k.tok + m * 128, k.h, k.b);
       }
+      parts = n + 1;
     }
   } else if (w == W_MMA) {
     constexpr uint32_t ID = make_idesc_bf16(128, NC, 0, 1);
@@ -518,12 +515,7 @@ __global__ void __launch_bounds__(THREADS, 1) apply_kernel(const __grid_constant
           drain(tot[m], lane_addr + NC * ab, &bars[B_AFREE + ab], lane);
         }
       }
-      if (P.part) {
-        WAIT(B_PFULL, (uint32_t)n, 159);
-      } else if (n > 0) {   // the rows staged for the last item have been read
-        if (lane == 0) bulk_wait_read_all();
-        __syncwarp();
-      }
+      WAIT(B_PFULL, (uint32_t)n, 159);
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
         const int row = k.tok + m * 128 + quarter * 32 + lane;
@@ -534,7 +526,7 @@ __global__ void __launch_bounds__(THREADS, 1) apply_kernel(const __grid_constant
           unpack2(tot[m][16], gs, unused);
           if (row < P.n) {
             float* g = reinterpret_cast<float*>(const_cast<void*>(P.g.ptr)) + (long long)k.b * P.g.sb + (long long)k.h * P.g.sh + (long long)row * P.g.sn;
-            if (P.part) gs += *g;
+            gs += *g;
             *g = gs;
           }
           wgt = 1.f / gs;
@@ -543,14 +535,10 @@ __global__ void __launch_bounds__(THREADS, 1) apply_kernel(const __grid_constant
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           ulonglong2* at = reinterpret_cast<ulonglong2*>(own + ((q ^ sw) << 4));
+          const ulonglong2 p = *at;
           ulonglong2 o;
-          o.x = tot[m][2 * q];
-          o.y = tot[m][2 * q + 1];
-          if (P.part) {
-            const ulonglong2 p = *at;
-            o.x = add2(o.x, p.x);
-            o.y = add2(o.y, p.y);
-          }
+          o.x = add2(tot[m][2 * q], p.x);
+          o.y = add2(tot[m][2 * q + 1], p.y);
           if (FWD) {
             o.x = mul2(o.x, ww);
             o.y = mul2(o.y, ww);
@@ -564,13 +552,11 @@ __global__ void __launch_bounds__(THREADS, 1) apply_kernel(const __grid_constant
           bulk_commit_group();
         }
       }
-      if (P.part) {
-        if (lane == 0) {
-          bulk_wait_read_all();
-          mbar_arrive(&bars[B_PFREE]);
-        }
-        __syncwarp();
+      if (lane == 0) {
+        bulk_wait_read_all();
+        mbar_arrive(&bars[B_PFREE]);
       }
+      __syncwarp();
     }
     if (lane == 0) bulk_wait_read_all();
   }
@@ -664,15 +650,13 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
         }
         if (j == ahead && idx + (int)gridDim.x < P.nitems) load_item(idx + gridDim.x, n + 1);
       }
-      if (P.part) {
-        if (n >= 1) WAIT(B_PFREE, (uint32_t)n - 1u, 163);
-        if (*abort_flag != 0) break;
-        if (lane == 0) {
-          mbar_arrive_expect_tx(&bars[B_PFULL], 2 * LT);
-          for (int m = 0; m < 2; ++m) tma_load_4d(sm + OFF_P + m * LT, &M.part, &bars[B_PFULL], 0, k.tok + m * 128, k.h, k.b);
-        }
-        parts = n + 1;
+      if (n >= 1) WAIT(B_PFREE, (uint32_t)n - 1u, 163);
+      if (*abort_flag != 0) break;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&bars[B_PFULL], 2 * LT);
+        for (int m = 0; m < 2; ++m) tma_load_4d(sm + OFF_P + m * LT, &M.part, &bars[B_PFULL], 0, k.tok + m * 128, k.h, k.b);
       }
+      parts = n + 1;
     }
   } else if (w < 2) {
     constexpr uint32_t ID = make_idesc_bf16(128, 64, 0, 0);
@@ -809,23 +793,14 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
       }
       if (lane == 0) mbar_arrive(&bars[B_XFREE + (n & 1)]);
       uint8_t* own = sm + OFF_P + m * LT + l * 128;
-      if (P.part) {
-        WAIT(B_PFULL, (uint32_t)n, 170);
-      } else if (n > 0) {
-        if (lane == 0) bulk_wait_read_all();
-        __syncwarp();
-      }
+      WAIT(B_PFULL, (uint32_t)n, 170);
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         ulonglong2* at = reinterpret_cast<ulonglong2*>(own + ((q ^ sw) << 4));
+        const ulonglong2 p = *at;
         ulonglong2 o;
-        o.x = acc[2 * q];
-        o.y = acc[2 * q + 1];
-        if (P.part) {
-          const ulonglong2 p = *at;
-          o.x = add2(o.x, p.x);
-          o.y = add2(o.y, p.y);
-        }
+        o.x = add2(acc[2 * q], p.x);
+        o.y = add2(acc[2 * q + 1], p.y);
         *at = o;
       }
       fence_proxy_async_smem();
@@ -834,13 +809,11 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
         tma_store_4d(&M.out, own, 0, row, k.h, k.b);
         bulk_commit_group();
       }
-      if (P.part) {
-        if (lane == 0) {
-          bulk_wait_read_all();
-          mbar_arrive(&bars[B_PFREE]);
-        }
-        __syncwarp();
+      if (lane == 0) {
+        bulk_wait_read_all();
+        mbar_arrive(&bars[B_PFREE]);
       }
+      __syncwarp();
     }
     if (lane == 0) bulk_wait_read_all();
   }

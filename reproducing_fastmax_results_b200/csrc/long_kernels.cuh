@@ -32,7 +32,7 @@ struct Geo {
   static constexpr int NB = D / 8;
   static constexpr int NPAIR = NB * (NB + 1) / 2;
   static constexpr int UNITS = NPAIR + 1;              // pair units and the linear unit; the constant row is added by the epilogue
-  static constexpr int CB = D / 8 + 2;                 // 8-column blocks: values, [denominator, denominator, 0 ...], 0
+  static constexpr int CB = D / 8 + 2;                 // 8-column blocks: values, [denominator, 0 ...], 0
   static constexpr int UNIT_BYTES = CB * 1024;         // [block][64 rows][8 columns] bf16
   static constexpr int CST = D + 8;                    // constant row, float32
   static constexpr int STATE_LD = D + 4;
@@ -458,13 +458,8 @@ __global__ void __launch_bounds__(THREADS, 1) chain_kernel(const __grid_constant
           r[4 * c] = v.x; r[4 * c + 1] = v.y; r[4 * c + 2] = v.z; r[4 * c + 3] = v.w;
         }
         pair::tmem_st<D / 2>(lane_addr + 64u * m, r);
-        if (DK) {
-          r8[0] = 0x00003F80u;
-        } else {   // -delta as the sum of two bf16 numbers: both columns meet the denominator moment
-          const float nd = row < P.n ? __ldg(P.ndelta + (long long)k.head * P.nd_ld + row) : 0.f;
-          const float hi = __bfloat162float(__float2bfloat16(nd));
-          r8[0] = bf16x2(hi, nd - hi);
-        }
+        // one, or -delta (a bf16 number, see prologue_kernel)
+        r8[0] = DK ? 0x00003F80u : bf16x2(row < P.n ? __ldg(P.ndelta + (long long)k.head * P.nd_ld + row) : 0.f, 0.f);
         tmem_st8(lane_addr + 64u * m + D / 2, r8);
         tmem_st_wait();
         tc_fence_before_sync();
@@ -644,7 +639,7 @@ __global__ void __launch_bounds__(64 * (D / 8 + 2)) pack_kernel(const float* __r
       o.x = bf16x2(s[0] * wgt, s[1] * wgt); o.y = bf16x2(s[2] * wgt, s[3] * wgt);
       o.z = bf16x2(s[4] * wgt, s[5] * wgt); o.w = bf16x2(s[6] * wgt, s[7] * wgt);
     } else {
-      o = make_uint4(bf16x2(s[0] * wgt, s[0] * wgt), 0u, 0u, 0u);   // the denominator moment twice (see chain_kernel)
+      o = make_uint4(bf16x2(s[0] * wgt, 0.f), 0u, 0u, 0u);
     }
     if (k < ns) *reinterpret_cast<uint4*>(dst + k * dst_step) = o;
     if (is_const && cb <= D / 8) {

@@ -1449,7 +1449,7 @@ cudaError_t long_states_f32(const fastmax_problem* pb, const LongGeo& g, const f
   const float c0 = pb->a0, c1 = pb->a1 * pb->inv_temperature, c2 = pb->order == 2 ? pb->a2 * pb->inv_temperature * pb->inv_temperature : 0.f;
   const dim3 grid((unsigned)((pb->order == 2 ? UNITS : 1) + 1), NC / 8, (unsigned)(pb->batch * pb->heads));
   LaunchScope ls(KK_WINDOW_PACK, st);
-  pack_kernel<<<grid, 64, 0, st>>>(raw, S, (float*)(S + g.packed), g.ns, g.ns, reverse, pb->order, c0, c1, c2);
+  pack_kernel<<<grid, 64, 0, st>>>(raw, S, (float*)(S + g.packed), g.ns, reverse, pb->order, c0, c1, c2);
   return cudaGetLastError();
 }
 template <bool FWD>
