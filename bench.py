@@ -35,18 +35,18 @@ WORKLOADS = {
     "cfg2_bf16_causal_p2_B8_H16_N4096_D64": (8, 16, 4096, 64, 2, True, "bf16", 1.0),
     # profiling case: same per-CTA work as config 2, a few GB on the device, inputs (134 MB) larger than L2
     "prof_bf16_causal_p2_B4_H16_N4096_D64": (4, 16, 4096, 64, 2, True, "bf16", 1.0),
-    # the config-2 shape without a mask: the moment build over all keys, then the apply over all queries (and the
-    # matching backward), on the same tensor-memory scans
+    # the config-2 shape without a mask: one moment state per head over all keys, then the apply over all queries (and the
+    # matching backward)
     "nc_bf16_noncausal_p2_B8_H16_N4096_D64": (8, 16, 4096, 64, 2, False, "bf16", 1.0),
     "ncprof_bf16_noncausal_p2_B4_H16_N4096_D64": (4, 16, 4096, 64, 2, False, "bf16", 1.0),
     # one long causal sequence with few heads in bf16 / D=64 (config 3's shape at the tensor-memory engine's dtype and
-    # head dim): the library cuts it into segments so that the scans still cover the GPU
+    # head dim): windows of pairs plus the moment states before them
     "long_bf16_causal_p2_B1_H8_N131072_D64": (1, 8, 131072, 64, 2, True, "bf16", 1.0),
     # one long causal sequence, cut into contiguous pieces across the ranks (strong scaling)
     "cfg3_f32_causal_p2_B1_H8_N131072_D32": (1, 8, 131072, 32, 2, True, "f32", 1.0),
     # order 1, non-causal, wide batch, forward (run with --mode fwd): HBM-bound
     "cfg4_bf16_noncausal_p1_B64_H12_N1024_D64": (64, 12, 1024, 64, 1, False, "bf16", 0.5),
-    # config 2's shape with narrower heads (bf16): zero-padded to 64 on the tensor-memory kernels
+    # config 2's shape with narrower heads (bf16)
     "d32_bf16_causal_p2_B8_H16_N4096_D32": (8, 16, 4096, 32, 2, True, "bf16", 1.0),
     # incremental decoding: one new token per (batch, head) per step against the carried state (N = prefix length is
     # irrelevant to the cost; 512 head states = 330 MB, larger than L2)
@@ -313,8 +313,8 @@ def config1_record(torch, dev):
     inv_temp = 1.0 / (8.0 * math.sqrt(D))
 
     def gpu_step():
-        o, g, _ = _lib.forward(qd, kd, vd, False, inv_temp, order=2)
-        return (o,) + tuple(_lib.backward(qd, kd, vd, o, g, dod, False, inv_temp, order=2)[:3])
+        o, g, _ = _lib.forward(qd, kd, vd, False, inv_temp, order=2, flags=_lib.FLAG_PAIRWISE)
+        return (o,) + tuple(_lib.backward(qd, kd, vd, o, g, dod, False, inv_temp, order=2, flags=_lib.FLAG_PAIRWISE)[:3])
 
     for _ in range(5):
         got = gpu_step()
@@ -637,7 +637,7 @@ def measure_sequence_sharded(workload, steps, warmup, torch, dist, dev, rank, wo
     medium = None
     if check and dtype == torch.float32:
         # the same float32 step after torch.set_float32_matmul_precision("medium"): the pieces run on bfloat16 copies on the
-        # tensor-memory kernels (32-wide heads zero-padded to 64), the exchanged states stay float32; bfloat16 tolerance
+        # tensor-memory kernels, the exchanged states stay float32; bfloat16 tolerance
         saved_precision = torch.get_float32_matmul_precision()
         torch.set_float32_matmul_precision("medium")
         try:
@@ -688,12 +688,13 @@ def run_sequence_sharded(args, torch, dist, dev, rank, world):
                        "parallelism": f"sequence pieces over {world} rank(s); all_gather of {r['state_bytes_per_rank']} state bytes per rank, "
                                       "once forward (exclusive prefix) and once backward (exclusive suffix)",
                        "l2": "inputs exceed the 126 MB L2 at 1-2 ranks; no explicit flush"},
-            "roofline": {"kernel": "whole step (fp32 CUDA-core engine)", "bound": "tensor",
+            "roofline": {"kernel": "whole step (%s)" % ("windows of pairs and moment states" if world == 1 else "fp32 CUDA-core engine"), "bound": "tensor",
                          "achieved": executed / (ms_step * 1e-3) / 1e12, "peak": pk["bf16_tflops_sustained"] / 2.0,
                          "unit": "TFLOP/s", "frac": executed / (ms_step * 1e-3) / 1e12 / (pk["bf16_tflops_sustained"] / 2.0),
                          "peak_source": pk["_source"] + " bf16 sustained / 2 (TF32 runs at half the bf16 rate; no TF32 peak was measured)",
-                         "note": "executed flops of one rank over the step time; the fp32 engine runs on the FFMA pipe because "
-                                 "TF32 operands miss the 1e-4 tolerance", "traffic": None},
+                         "note": "flops of the moment formulation of one rank over the step time; one rank runs windows of pairs "
+                                 "and moment states on bf16 pieces of the float32 operands, pieces with a carried state the "
+                                 "FFMA pipe", "traffic": None},
             "exchange_ms_per_step": r["exchange_ms_per_step"], "parity": r["parity"],
             "kernels": kernels, "cpu_baseline": None, "e2e": None, "gpu_launches": r["gpu_launches"], "clocks": r["clocks"],
         }
@@ -1016,9 +1017,9 @@ def measure_cfg2_strong(torch, dist, dev, rank, world, steps=10, warmup=3):
     q, k, v, do = ((torch.randn(b, H, N, D, device=dev, generator=gen) * scale).bfloat16() for _ in range(4))
     inv_temp = 1.0 / (8.0 * math.sqrt(D))
 
-    def step():
-        o, g, _ = _lib.forward(q, k, v, causal, inv_temp, order=order)
-        return _lib.backward(q, k, v, o, g, do, causal, inv_temp, order=order)
+    def step():   # as the Python operators call it
+        o, g, _ = _lib.forward(q, k, v, causal, inv_temp, order=order, flags=_lib.FLAG_PAIRWISE)
+        return _lib.backward(q, k, v, o, g, do, causal, inv_temp, order=order, flags=_lib.FLAG_PAIRWISE)
 
     for _ in range(warmup):
         step()
@@ -1048,9 +1049,9 @@ def measure_cfg2_strong(torch, dist, dev, rank, world, steps=10, warmup=3):
 
 def measure_reference_boundary(torch, dist, dev, rank, world, steps=3, warmup=1):
     """Config 2's shape through the reference's own boundary, per rank (weak): float32 (b, h, n, d) tensors into
-    `FASTMultiHeadAttention_Function` (the twin of transformer/model.py:14-74: reshape, permute to (n, b*h, d) with
-    copies, `fastmax_cuda.forwardpass` / `backwardpass`, permute back), forward + backward.  float32 puts the call on
-    the CUDA-core engine; the figure says what a caller gets who changes nothing but the import."""
+    `FASTMultiHeadAttention_Function` (the twin of transformer/model.py:14-74), forward + backward.  float32 tensors run
+    pair by pair on tensor memory, every operand as three bf16 pieces (float32 results); the figure says what a caller
+    gets who changes nothing but the import."""
     from reproducing_fastmax_results_b200.attention import FASTMultiHeadAttention_Function
 
     B, H, N, D, order, causal, _, scale = WORKLOADS[DEFAULT]
@@ -1103,8 +1104,8 @@ def measure_reference_boundary(torch, dist, dev, rank, world, steps=3, warmup=1)
     finally:
         torch.set_float32_matmul_precision(saved_precision)
     return {"ms_per_step": ms, "value": world * B * N / (ms * 1e-3) / 1e6, "unit": "Mtokens/s", "scaling": "weak", "dtype": "f32",
-            "api": "FASTMultiHeadAttention_Function.apply + backward: the reference wrapper's permutes and copies around "
-                   "fastmax_cuda.forwardpass / backwardpass (float32 contract, CUDA-core engine)",
+            "api": "FASTMultiHeadAttention_Function.apply + backward: float32 contract, float32 results; a native autograd node "
+                   "that reads the (b, h, n, d) tensors where they are (pairwise kernels on bf16 pieces)",
             "medium_matmul_precision": {"ms_per_step": ms_medium, "value": world * B * N / (ms_medium * 1e-3) / 1e6,
                                         "note": "same float32 tensors and calls after torch.set_float32_matmul_precision('medium'): "
                                                 "the extension converts q, k, v and the upstream gradient to bfloat16 and runs the "
