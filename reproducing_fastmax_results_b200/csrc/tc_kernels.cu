@@ -954,12 +954,13 @@ cudaError_t tc_moments(const fastmax_problem* pb, const fastmax_tensor& x, const
   // Tiles per block and cuts of the token axis: the combination that ends first when the SMs take the blocks in order (full
   // slices, then the shorter last ones), in clocks: 620 per tile and chunk, 12000 to start a block and write its rows, 20000 to
   // add them, and 12000 for the memset that adding needs.  16 heads of 8192 tokens: 74 us with three tiles a block, 89 with
-  // four, 92 with four and two cuts; 128 heads of 4096: 220 us with four, 239 with three.
+  // four, 92 with four and two cuts; 128 heads of 4096: 220 us with four, 239 with three.  No more cuts than give the same bits
+  // whatever order they end in: two that add to zeros, one that adds to a carried state.
   const int ntiles = pb->order == 2 ? npair / 2 + 1 : 1, sms = device_sms();
-  const int segs = seg_tokens > 0 ? (n + seg_tokens - 1) / seg_tokens : 0;
+  const int segs = seg_tokens > 0 ? (n + seg_tokens - 1) / seg_tokens : 0, most = segs > 0 ? segs : init != nullptr ? 1 : 2;
   long long best = -1;
   for (int tps = 1; tps <= 4; ++tps)
-    for (int c = segs > 0 ? segs : 1; c <= (segs > 0 ? segs : 16) && c <= P.nchunks; ++c) {
+    for (int c = segs > 0 ? segs : 1; c <= most && c <= P.nchunks; ++c) {
       const bool add = segs == 0 && (c > 1 || init != nullptr);
       const long long per = (P.nchunks + c - 1) / c, last = ntiles % tps, fixed = add ? 20000 : 12000;
       const long long df = per * 620 * tps + fixed, dl = per * 620 * last + fixed;
