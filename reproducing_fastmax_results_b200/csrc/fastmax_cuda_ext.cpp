@@ -446,15 +446,9 @@ struct FastmaxNode : public torch::autograd::Function<FastmaxNode> {
                                bool normalize, bool exact_norm_grad, bool contiguous, double inv_t, double a0, double a1, double a2,
                                double lim, int64_t p, bool train) {
     torch::Tensor stats_q, stats_k;
-    const bool own = contiguous && train;   // the reference's wrapper keeps copies of its own: callers may write into theirs after the call
-    if (contiguous) {                       // ... and takes tensors of any layout
-      const torch::Tensor given[3] = {q, k, v};
+    const torch::Tensor given[3] = {q, k, v};
+    if (contiguous) {   // the reference's wrapper takes tensors of any layout
       q = readable(q); k = readable(k); v = readable(v);
-      if (own && !normalize) {
-        if (q.is_same(given[0])) q = q.clone(at::MemoryFormat::Contiguous);
-        if (k.is_same(given[1])) k = k.clone(at::MemoryFormat::Contiguous);
-      }
-      if (own && v.is_same(given[2])) v = v.clone(at::MemoryFormat::Contiguous);
     }
     if (normalize) {
       auto n = normalize_forward_qk(q, k, lim);
@@ -466,7 +460,21 @@ struct FastmaxNode : public torch::autograd::Function<FastmaxNode> {
     // the states of the keys are kept for the backward only where there will be one
     auto res = ::forward(q, k, v, mask, inv_t, a0, a1, a2, p, c10::nullopt, false, true, FASTMAX_FLAG_PAIRWISE, out, c10::nullopt, train);
     if (!train) res.emplace_back();
-    ctx->save_for_backward({q, k, v, own ? res[0].clone() : res[0], res[1], stats_q, stats_k, res[3]});
+    torch::Tensor o = res[0];
+    if (contiguous && train) {   // ... and keeps copies of its own: callers may write into theirs, and into the result, after the call
+      std::vector<torch::Tensor*> shared{&o};
+      if (q.is_same(given[0])) shared.push_back(&q);
+      if (k.is_same(given[1])) shared.push_back(&k);
+      if (v.is_same(given[2])) shared.push_back(&v);
+      std::vector<torch::Tensor> from, copy;
+      for (torch::Tensor* t : shared) {
+        from.push_back(*t);
+        copy.push_back(torch::empty(t->sizes(), t->options()));
+      }
+      at::_foreach_copy_(copy, from);   // one launch
+      for (size_t i = 0; i < shared.size(); ++i) *shared[i] = copy[i];
+    }
+    ctx->save_for_backward({q, k, v, o, res[1], stats_q, stats_k, res[3]});
     auto& d = ctx->saved_data;
     d["mask"] = mask; d["normalize"] = normalize && exact_norm_grad; d["contiguous"] = contiguous;
     d["inv_t"] = inv_t; d["a0"] = a0; d["a1"] = a1; d["a2"] = a2; d["lim"] = lim; d["p"] = p;
