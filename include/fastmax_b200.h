@@ -112,7 +112,8 @@ typedef struct {
 } fastmax_forward_args;
 
 size_t fastmax_forward_workspace(const fastmax_problem* pb, const fastmax_forward_args* args);
-/* Which engine takes this forward call: 1 = the tensor-memory (tcgen05) kernels, 0 = the CUDA-core engine.  A host
+/* Which of the two moment engines covers this forward call, FASTMAX_FLAG_PAIRWISE aside: 1 = the tensor-memory (tcgen05)
+ * kernels, 0 = the CUDA-core engine.  A host
  * that holds float32 tensors and is allowed to compute in bfloat16 (PyTorch's float32 matmul precision "medium") asks
  * this for the bfloat16 form of its problem before it converts anything. */
 int32_t fastmax_forward_engine(const fastmax_problem* pb, const fastmax_forward_args* args);

@@ -4,8 +4,9 @@
 // Products are sums of six bf16 piece products (see pair_f32.cuh).  The features are formed and split into their three pieces in
 // registers, in float32 from the tensors themselves; states are split once, when they are packed.  The tensor pipe adds with
 // truncation, so an accumulator lives for one unit (64 features, or 64 tokens of a moment) and the drain warps add it to
-// float32 totals in registers.  All three kernels are bound by the tensor pipe: 24 MMAs of 33 clocks (18 in the chain) per 64
-// features and tile.  Measured, 8 heads x 131072 tokens, order 2: moments 419 us, packing 128, apply 370, chain 293; forward and
+// float32 totals in registers.  What bounds all three kernels is starting products: 24 MMAs (13 in the chain) of N = 48 per 64
+// features and tile, one every 33 clocks, each 24 clocks of the tensor pipe, which is active in 48 % (apply) and 62 % (chain) of
+// the clocks (ncu, 8 heads of 32768).  Measured, 8 heads x 131072 tokens, order 2: moments 419 us, packing 128, apply 370, chain 293; forward and
 // backward with the pairwise windows 4.5 ms, where the CUDA-core engine (multiply-adds bound by its shared-memory reads, a scan
 // over segments) took 22.5.
 #pragma once

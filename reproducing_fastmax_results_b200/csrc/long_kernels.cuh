@@ -6,7 +6,8 @@
 // written once.  Without a mask there are no pairs and one state per head.  Included by pair_kernels.cu inside fm.
 //
 // Measured, 8 heads of 131072 x 64, forward + backward: 7.9 ms by segmented scans (their serial chains and float32 partial sums in
-// memory), 4.1 here: moments 2 x 495 us, pairs 230 + 740, apply 2 x 295, chain rule 380 + 370, packing 2 x 156.
+// memory), 4.0 to 4.5 here from box to box; of 4.1: moments 2 x 495 us, pairs 230 + 740, apply 2 x 295, chain rule 380 + 370,
+// packing 2 x 156.
 #pragma once
 
 namespace lng {

@@ -16,8 +16,8 @@
 // control: it takes over a block that has not started), so the items' lengths may differ by any factor; the loads and
 // first products of the next item run under the last tiles and the stores of the current one.
 //
-// Bound by neither pipe alone: the tensor pipe is busy 55 to 65 % of the time at d = 64 (21 to 29 % at d = 32), the element-wise
-// warps issue in 40 to 47 % of their slots.  Measured (us; the scans of the moment engine before): 128 heads of 4096 x 64, causal,
+// Bound by neither pipe alone: the tensor pipe is active in 64 to 72 % of the clocks at d = 64 (31 to 38 % at d = 32), the
+// schedulers issue in 40 to 47 % (ncu, 64 heads of 4096 x 64 and 128 heads of 2048 x 32).  Measured (us; the scans of the moment engine before): 128 heads of 4096 x 64, causal,
 // forward + backward 2930 -> 1080; 128 heads of 1024 x 64 570 -> 135; 128 heads of 2048 x 32 1533 -> 285.  Heads of 16 dims have
 // the kernels of pair_f32.cuh.
 #include <cuda.h>

@@ -8,6 +8,9 @@
 // factor is kept in registers across the tiles that share it: 1.25 rows read per feature instead of two (a 128-bit load of a
 // warp takes four wavefronts whatever its lanes share).
 // TMEM: four 80-column accumulators, three 64-column slots.
+//
+// 620 clocks per tile and chunk.  No unit is full: 64 heads of 4096 x 64 (130 us) keep the shared-memory pipe busy for 58 % of the
+// time, the tensor pipe for 43 % (two products per K step, N = D and N = 16), the schedulers for 48 %.
 #pragma once
 
 namespace mo {
