@@ -128,13 +128,14 @@ def test_float32_windows_match_oracle(case, hand_over):
             assert err < 3e-6, (name, b, h, err)
 
 
-@pytest.mark.parametrize("binding", ["ctypes", "extension"])
+@pytest.mark.parametrize("binding", ["ctypes", "extension", "entry point"])
 @pytest.mark.parametrize("variant", ["dstate_in", "dstate_out", "gradient rows", "prompt"])
 @pytest.mark.parametrize("dtype,D,N", [(torch.bfloat16, 64, 8192), (torch.float32, 32, 4096)])
-def test_key_moments_of_another_form_are_not_read(dtype, D, N, variant, binding):
+def test_key_moments_of_another_form_are_not_read(dtype, D, N, variant, binding, monkeypatch):
     """A forward of the window form leaves packed states; a backward of the same problem that also takes or returns gradient
     moments, or writes into rows the copy engine cannot, runs on the moment engines and must not read them (nor may the
-    window form read what a prompt's state left).  Same gradients with and without the hand-over."""
+    window form read what a prompt's state left).  Same gradients with and without the hand-over.  "entry point": the array is
+    passed whatever its size, and fastmax_backward itself leaves it unread."""
     import reproducing_fastmax_results_b200 as pkg
     from reproducing_fastmax_results_b200 import _lib as L
 
@@ -153,9 +154,11 @@ def test_key_moments_of_another_form_are_not_read(dtype, D, N, variant, binding)
         return [torch.zeros(B, H, N, D + 1, device="cuda", dtype=dtype)[..., :D] for _ in range(3)]
 
     def run(hand_over):
-        if binding == "ctypes":
+        if binding != "extension":
             km = L.KeyMoments()
             o, gg, _ = L.forward(q, k, v, True, it, *poly, want_state=want_state, flags=L.FLAG_PAIRWISE, key_moments=km)
+            if binding == "entry point":
+                monkeypatch.setattr(L.load(), "fastmax_backward_key_moments_bytes", lambda *_: km.buf.numel() * 4)
             res = L.backward(q, k, v, o, gg, do, True, it, *poly, dstate_in=dstate, want_dstate=want_dstate, grads_out=rows(),
                              flags=L.FLAG_PAIRWISE, key_moments=km if hand_over else None)
             buf = km.buf
