@@ -19,6 +19,7 @@
 
 namespace f32 {
 
+constexpr int EW = 8, ROLES = EW + 3, THREADS = (W_EW + EW) * 32;   // element-wise warps: TMEM lane quarters x 32-column halves
 constexpr int TF = 64;                       // streamed rows per tile
 constexpr int XF = TF * 128;                 // one piece of a streamed tile
 constexpr int AF = R * 128;                  // one piece of a held tile

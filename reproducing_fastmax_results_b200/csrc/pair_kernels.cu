@@ -16,10 +16,11 @@
 // control: it takes over a block that has not started), so the items' lengths may differ by any factor; the loads and
 // first products of the next item run under the last tiles and the stores of the current one.
 //
-// Bound by neither pipe alone: the tensor pipe is active in 64 to 72 % of the clocks at d = 64 (31 to 38 % at d = 32), the
-// schedulers issue in 40 to 47 % (ncu, 64 heads of 4096 x 64 and 128 heads of 2048 x 32).  Measured (us; the scans of the moment engine before): 128 heads of 4096 x 64, causal,
-// forward + backward 2930 -> 1080; 128 heads of 1024 x 64 570 -> 135; 128 heads of 2048 x 32 1533 -> 285.  Heads of 16 dims have
-// the kernels of pair_f32.cuh.
+// Bound by no pipe alone, and where the GPU is busy for long, by power.  ncu, 64 heads of 4096 x 64 (forward, dk / dv, dq): tensor
+// pipe active in 66, 69, 70 % of the clocks, issue slots 59, 61, 38 %.  128 heads of 4096 x 64 back to back draw 1000 W and run at
+// 1.55 to 1.65 GHz (1.24 ms for forward and backward, 1.06 at 1.9 GHz).  Measured (us, forward and backward; the scans of the moment
+// engine before): 128 heads of 4096 x 64, causal 2930 -> 1060; of 1024 x 64 570 -> 122; of 2048 x 32 1533 -> 258.  Heads of 16 dims
+// have the kernels of pair_f32.cuh.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -46,13 +47,19 @@ __device__ int g_wait_hist[256];
 constexpr long long WAIT_CYCLES = 4000000000ll;   // ~2 s at 2 GHz
 constexpr int R = 128;                  // held rows of one accumulator (the TMEM lanes)
 constexpr int T = 128;                  // streamed rows per tile
-constexpr int EW = 8;                   // element-wise warps: two per TMEM lane quarter (FWD: one per held tile; else 64-column halves)
 constexpr int W_SCORE = 0, W_ACC = 1, W_LOAD = 2, W_EW = 4;   // warp roles: two issuers, loader, (spare), element-wise warps
-constexpr int ROLES = EW + 3;           // warps that follow the items
-constexpr int THREADS = (W_EW + EW) * 32;
 constexpr int X_BYTES = T * 128;        // operand tile: 128-byte rows whatever the head dim (narrow heads zero-filled by the copy engine)
 constexpr int STAGES = 4;               // ring of streamed tile pairs
 enum Kind { FWD = 0, DQ = 1, DKV = 2 };
+// Element-wise warps: sixteen, four per TMEM lane quarter (FWD: two 64-column halves of each held tile; else 32 columns).  A tile is a
+// chain of waits and TMEM accesses around some hundred instructions; with two warps per scheduler nothing ran beside it for half
+// of the time.  Eight -> sixteen (us): 128 heads of 2048 x 32 forward 68 -> 62, dq 84 -> 79, dk / dv 124 -> 111; 192 of 577 x 64
+// without a mask dk / dv 47 -> 44.  dq with 64 dims has three operations per score and keeps eight: 343 with sixteen, 335 with
+// eight (128 heads of 4096).
+template <int D, int KIND>
+constexpr int EW = KIND == DQ && D == 64 ? 8 : 16;
+template <int D, int KIND>
+constexpr int THREADS = (W_EW + EW<D, KIND>) * 32;
 
 struct Params {
   View out0, out1;            // FWD: o, g; DQ: dq; DKV: dk, dv
@@ -163,25 +170,28 @@ constexpr int OFF_X = 4 * X_BYTES;
 constexpr int STAGE = 2 * X_BYTES;
 constexpr int OFF_ND = OFF_X + STAGES * STAGE;           // DKV: -delta of the streamed queries, T floats per stage
 constexpr int OFF_H = OFF_ND + STAGES * T * 4;              // SQ: two constant 128 x 16 operands whose product is h everywhere
-constexpr int OFF_CLC = OFF_H + 2 * R * 32;         // ring of 16-byte answers of the scheduler
+constexpr int OFF_SUM = OFF_H + 2 * R * 32;         // FWD: row sums of the second halves, of the last four items
+constexpr int OFF_CLC = OFF_SUM + 4 * 2 * R * 4;    // ring of 16-byte answers of the scheduler
 constexpr int CLC = 4;
 constexpr int OFF_BAR = OFF_CLC + 16 * CLC;
 constexpr int SMEM_BYTES = OFF_BAR + 512 + 1024;
 static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 // barrier slots
-constexpr int B_FULL = 0, B_EMPTY = 4, B_HFULL = 8, B_HEMPTY = 10, B_S = 12, B_READS = 14, B_READD = 16, B_P = 17, B_SFREE = 19, B_ACC = 21,
-              B_AFREE = 23, B_CFULL = 25, B_CEMPTY = B_CFULL + CLC, B_DRAIN = B_CEMPTY + CLC, B_COUNT = B_DRAIN + 2;
+constexpr int B_FULL = 0, B_EMPTY = 4, B_HFULL = 8, B_HEMPTY = 10, B_S = 12, B_READD = 18, B_P = 19, B_SFREE = 22, B_ACC = 25,
+              B_AFREE = 27, B_CFULL = 29, B_CEMPTY = B_CFULL + CLC, B_DRAIN = B_CEMPTY + CLC, B_COUNT = B_DRAIN + 2;
 static_assert(B_COUNT * 8 <= 384, "barriers and flags share 512 bytes");
-// TMEM columns.  FWD: O' of the two held tiles, their scores, their bf16 tiles P.  DQ: dq, dS, two score buffers, dP.
-// DKV: dv, dk, scores, dP, P, dS.  The bf16 tiles have columns of their own: scores and dP are free as soon as the
-// element-wise warps have READ them, so the next tile's first products run under this tile's arithmetic.
-constexpr uint32_t C_ACC = 0, C_ACC1 = 64, C_S = 128;
+// TMEM columns.  Accumulators (FWD: O' of the two held tiles; DQ: dq; DKV: dv, dk), then score buffers of 128 columns that take
+// turns (FWD three, else two) and DQ, DKV: one of dP.  The bf16 A operands of the second products replace the scores that their
+// warp has read, 32 columns by 32 columns (FWD: 64 by 64): no two warps touch the same columns, and a buffer is free again when the
+// second products are done.  dP is free as soon as it has been read.
+constexpr uint32_t C_ACC = 0, C_ACC1 = 64, C_S = 128, C_DP = 384;
 template <int KIND>
-struct Cols {
-  static constexpr uint32_t DP = KIND == DQ ? 384 : 256;
-  static constexpr uint32_t P = 384;                         // FWD: + 64 for the second held tile
-  static constexpr uint32_t DS = KIND == DQ ? 64 : 448;
-};
+constexpr uint32_t NBUF = KIND == FWD ? 3u : 2u;
+// where K step kk (16 streamed rows) of P (FWD, DKV) or dS lies in its buffer
+template <int KIND>
+__device__ __forceinline__ constexpr uint32_t weights_at(int kk, bool ds) {
+  return KIND == FWD ? 64u * (kk >> 2) + 8u * (kk & 3) : 32u * (kk >> 1) + 8u * (kk & 1) + (KIND == DKV && ds ? 16u : 0u);
+}
 
 struct Item {
   int head, b, h;
@@ -238,9 +248,11 @@ struct Maps {
 };
 
 template <int D, int KIND, bool SQ>
-__global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant__ Maps M, const Params P) {
+__global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_constant__ Maps M, const Params P) {
   constexpr int KS = D / 16;                    // K steps of the first products
   constexpr int HELD_ROWS = KIND == FWD ? 2 * R : R;
+  constexpr int EWN = EW<D, KIND>, ROLES = EWN + 3;   // ROLES: warps that follow the items
+  constexpr int W = KIND == FWD ? 64 : 512 / EWN;     // columns of an element-wise warp
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* sm = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
@@ -253,9 +265,9 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
   if (tid == 0) {
     for (int i = 0; i < B_COUNT; ++i) {
       uint32_t n = 1;
-      if (i >= B_READS && i < B_SFREE) n = KIND == FWD ? EW / 2 : EW;                          // READS, READD, P
-      if (i == B_AFREE || i == B_AFREE + 1) n = KIND == DKV ? EW : EW / 2;
-      if (i == B_HEMPTY || i == B_HEMPTY + 1) n = 1 + EW;                       // products done, output rows staged there copied
+      if (i >= B_READD && i < B_SFREE) n = KIND == FWD ? EWN / 2 : EWN;           // READD, P
+      if (i == B_AFREE || i == B_AFREE + 1) n = KIND == DKV ? 8 : 4;
+      if (i == B_HEMPTY || i == B_HEMPTY + 1) n = 1 + (KIND == DQ ? 4 : 8);     // products done, output rows staged there copied
       if (i >= B_CEMPTY && i < B_CEMPTY + CLC) n = ROLES;                       // every role has read the answer
       mbar_init(&bars[i], n);
     }
@@ -343,8 +355,8 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
     const uint64_t dHeld = make_smem_desc(smem_u32(sm + OFF_HELD), 16, 1024, 2);
     const uint64_t dXk = make_smem_desc(smem_u32(sm + OFF_X), 16, 1024, 2);          // streamed tile, K-major
     const uint64_t dHa = make_smem_desc(smem_u32(sm + OFF_H), 128, 256, 0), dHb = make_smem_desc(smem_u32(sm + OFF_H + R * 32), 128, 256, 0);
-    uint32_t cnt[2] = {0, 0};     // tiles so far (FWD: of each held tile)
     uint32_t tile = 0;            // streamed tiles so far
+    uint32_t buf = 0, use = 0;    // score buffer, times that it has been used
     int idx = blockIdx.x;
     for (int n = 0; idx >= 0; ++n) {
       const Item it = decode<KIND, T, HELD_ROWS>(idx, P);
@@ -358,25 +370,23 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
 #pragma unroll
         for (int m = 0; m < (KIND == FWD ? 2 : 1); ++m) {
           if (i < (m ? it.n1 : it.n0)) {
-            const uint32_t k = cnt[m];
-            const uint32_t buf = KIND == FWD ? (uint32_t)m : KIND == DQ ? (k & 1u) : 0u;
-            if (KIND == DQ) { if (k >= 2) WAIT(B_READS + buf, (k >> 1) - 1u, 80); }   // the buffer's last scores have been read
-            else if (k > 0) WAIT(B_READS + buf, k - 1u, 80);
+            if (use > 0) WAIT(B_SFREE + (int)buf, use - 1u, 80);   // the second products that read this buffer are done
             tc_fence_after_sync();
+            const uint32_t c = tmem + C_S + buf * 128u;
             const bool add_h = SQ && !first_rows(P, it.r0 + m * R);
-            if (add_h) mma_ss_elect(tmem + C_S + buf * 128u, dHa, dHb, ID_S, 0u);
+            if (add_h) mma_ss_elect(c, dHa, dHb, ID_S, 0u);
 #pragma unroll
             for (int ks = 0; ks < KS; ++ks)
-              mma_ss_elect(tmem + C_S + buf * 128u, dH + (uint64_t)(m * (X_BYTES >> 4) + 2 * ks), dX + (uint64_t)(2 * ks), ID_S, (add_h || ks > 0) ? 1u : 0u);
+              mma_ss_elect(c, dH + (uint64_t)(m * (X_BYTES >> 4) + 2 * ks), dX + (uint64_t)(2 * ks), ID_S, (add_h || ks > 0) ? 1u : 0u);
             if (KIND != FWD) {
-              if (k > 0) WAIT(B_READD, k - 1u, 82);
+              if (tile > 0) WAIT(B_READD, tile - 1u, 82);
               tc_fence_after_sync();
 #pragma unroll
               for (int ks = 0; ks < KS; ++ks)
-                mma_ss_elect(tmem + Cols<KIND>::DP, dH + (uint64_t)((X_BYTES >> 4) + 2 * ks), dY + (uint64_t)(2 * ks), ID_S, ks > 0);
+                mma_ss_elect(tmem + C_DP, dH + (uint64_t)((X_BYTES >> 4) + 2 * ks), dY + (uint64_t)(2 * ks), ID_S, ks > 0);
             }
-            mma_commit_elect(&bars[B_S + buf]);
-            cnt[m] = k + 1;
+            mma_commit_elect(&bars[B_S + 3 * m + (int)buf]);
+            if (++buf == NBUF<KIND>) { buf = 0; ++use; }
           }
         }
         ++tile;
@@ -392,7 +402,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
     // ================= issuer of the second products =================
     constexpr uint32_t ID_ACC = make_idesc_bf16(R, D, 0, 1);
     const uint64_t dXm = make_smem_desc(smem_u32(sm + OFF_X), X_BYTES, 1024, 2);     // streamed tile, MN-major
-    uint32_t cnt[2] = {0, 0}, tile = 0;
+    uint32_t tile = 0, buf = 0, use = 0;   // as above
     uint32_t nfree[2] = {0, 0};   // items that have started on each accumulator
     int idx = blockIdx.x;
     for (int n = 0; idx >= 0; ++n) {
@@ -409,19 +419,20 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
               if (nfree[m] > 0) WAIT(B_AFREE + m, nfree[m] - 1u, 79);
               nfree[m]++;
             }
-            WAIT(B_P + m, cnt[m]++, 72);   // the bf16 tiles of the element-wise warps
+            WAIT(B_P + (int)buf, use, 72);   // the bf16 tiles of the element-wise warps
             tc_fence_after_sync();
             const uint32_t keep = i > 0 ? 1u : 0u;
-            const uint32_t a = tmem + (KIND == DQ ? Cols<KIND>::DS : Cols<KIND>::P + 64u * m);
+            const uint32_t a = tmem + C_S + buf * 128u;
 #pragma unroll
             for (int kk = 0; kk < T / 16; ++kk)
-              mma_ts_elect(tmem + C_ACC + 64u * m, a + 8u * kk, (KIND == DQ ? dX : dY) + (uint64_t)(128 * kk), ID_ACC, kk > 0 ? 1u : keep);
+              mma_ts_elect(tmem + C_ACC + 64u * m, a + weights_at<KIND>(kk, false), (KIND == DQ ? dX : dY) + (uint64_t)(128 * kk), ID_ACC, kk > 0 ? 1u : keep);
             if (KIND == DKV) {
 #pragma unroll
               for (int kk = 0; kk < T / 16; ++kk)
-                mma_ts_elect(tmem + C_ACC1, tmem + Cols<KIND>::DS + 8u * kk, dX + (uint64_t)(128 * kk), ID_ACC, kk > 0 ? 1u : keep);
+                mma_ts_elect(tmem + C_ACC1, a + weights_at<KIND>(kk, true), dX + (uint64_t)(128 * kk), ID_ACC, kk > 0 ? 1u : keep);
             }
-            mma_commit_elect(&bars[B_SFREE + m]);
+            mma_commit_elect(&bars[B_SFREE + (int)buf]);
+            if (++buf == NBUF<KIND>) { buf = 0; ++use; }
             if (KIND != FWD || m == 1 || i >= it.n1) mma_commit_elect(&bars[B_EMPTY + s]);
             if (i == nm - 1) mma_commit_elect(&bars[B_ACC + m]);
           }
@@ -437,34 +448,37 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
   } else if (w >= W_EW) {
     // ================= element-wise warps =================
     const int we = w - W_EW, quarter = w & 3;
-    const int grp = KIND == FWD ? we >> 2 : 0;    // FWD: held tile
-    const int half = KIND == FWD ? 0 : we >> 2;   // else: 64-column half of the tile
-    constexpr int W = KIND == FWD ? 128 : 64;     // columns of a warp
+    const int grp = KIND == FWD ? we >> 3 : 0;                  // FWD: held tile
+    const int part = KIND == FWD ? (we >> 2) & 1 : we >> 2;     // columns of the tile: halves, or quarters
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
     const uint64_t C0 = pack2(P.c0, P.c0), C1 = pack2(P.c1, P.c1), C2 = pack2(P.c2, P.c2), C22 = pack2(2.f * P.c2, 2.f * P.c2),
                    K = pack2(P.k, P.k);   // what a mode does not use is not computed
-    // which rows this warp writes out: FWD O' of its tile, DKV dv (half 0) and dk (half 1), DQ dq (half 0)
-    const bool writes = KIND != DQ || half == 0;
+    // which rows this warp writes out: FWD O' of its tile (part 0), DKV dv (part 0) and dk (part 1), DQ dq (part 0)
+    const bool writes = part < (KIND == DKV ? 2 : 1);
+    float* const sums = reinterpret_cast<float*>(sm + OFF_SUM) + grp * R + quarter * 32 + lane;   // [item & 3][held tile][row]
     uint64_t sum[4] = {0ull, 0ull, 0ull, 0ull};   // FWD: four chains, one would serialise the additions
     uint64_t ND = 0ull;                           // DQ: -delta of this row
-    uint32_t k = 0;          // tiles of this warp's group so far
+    uint32_t tile = 0;       // streamed tiles so far
+    uint32_t buf = 0;        // score buffer of the next tile (FWD: of either group)
+    uint32_t phases = 0;     // per buffer: the phase that this group's next scores there complete
     uint32_t done = 0;       // items whose results this warp has written
     // Results of an item are written after the next item's first tile, whose products run meanwhile.
     auto results = [&](int n, const Item& it, float total) {
       const int row = it.r0 + grp * R + quarter * 32 + lane;
       WAIT(B_ACC + grp, done, 75);
       ++done;
-      if (!writes) return;
       tc_fence_after_sync();
+      // (written before the last second product was started)
+      if (KIND == FWD) total += sums[(n & 3) * 2 * R];
       constexpr int CH = 32;
       uint32_t r[D / CH][CH];
 #pragma unroll
-      for (int c = 0; c < D / CH; ++c) tmem_ld<CH>(lane_addr + (KIND == FWD ? 64u * grp : 64u * half) + (uint32_t)(CH * c), r[c]);
+      for (int c = 0; c < D / CH; ++c) tmem_ld<CH>(lane_addr + 64u * (KIND == FWD ? grp : part) + (uint32_t)(CH * c), r[c]);
       tmem_ld_wait();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars[B_AFREE + grp]);
-      const bool second = KIND == DKV && half == 0;   // dv
+      const bool second = KIND == DKV && part == 0;   // dv
       const bool first = first_rows(P, it.r0 + grp * R);
       const float w1 = first ? 1.f : P.w1;
       float wgt = second ? w1 : first ? 1.f : P.w0;
@@ -476,7 +490,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
           reinterpret_cast<float*>(const_cast<void*>(P.out1.ptr))[(long long)it.b * P.out1.sb + (long long)it.h * P.out1.sh + (long long)row * P.out1.sn] = total * w1;
       }
       if (partial) {
-        uint8_t* stage = sm + OFF_HELD + (n & 1) * STAGE + (KIND == FWD ? grp : half) * X_BYTES + quarter * 4096;
+        uint8_t* stage = sm + OFF_HELD + (n & 1) * STAGE + (KIND == FWD ? grp : part) * X_BYTES + quarter * 4096;
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
           if (c > 0) {   // one box of space per warp
@@ -498,7 +512,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
       } else if (second ? P.vec1 : P.vec0) {
         // rows -> the item's held set (its products are done), 128-byte swizzle -> the copy engine, which writes whole lines
         // and clips what lies outside; stored by the threads, 32 lines per instruction, this took 1200 to 3000 clocks
-        uint8_t* stage = sm + OFF_HELD + (n & 1) * STAGE + (KIND == FWD ? grp : half) * X_BYTES + quarter * 4096;
+        uint8_t* stage = sm + OFF_HELD + (n & 1) * STAGE + (KIND == FWD ? grp : part) * X_BYTES + quarter * 4096;
 #pragma unroll
         for (int c = 0; c < D / 8; ++c) {
           const uint32_t(&x)[CH] = r[8 * c / CH];
@@ -531,6 +545,7 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
       }
     };
     bool pend = false;   // the last item's results are still to be written
+    float total = 0.f;   // FWD: this half's row sum of the last item
     Item last{};
     int idx = blockIdx.x, n = 0;
     for (; idx >= 0; ++n) {
@@ -538,23 +553,25 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
       const int nt = (KIND == FWD && grp) ? it.n1 : it.n0;
       const int row = it.r0 + grp * R + quarter * 32 + lane;
       const bool first = first_rows(P, it.r0 + grp * R);
-      float total = 0.f;
-      if (KIND == FWD) {
-        float a, b;
-        unpack2(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])), a, b);
-        total = a + b;
-        sum[0] = sum[1] = sum[2] = sum[3] = 0ull;
-      }
+      float next_total = 0.f;
       if (KIND == DQ) {
         const float nd = row < P.nr ? __ldg(P.ndelta + (long long)it.head * P.nd_ld + row) : 0.f;
         ND = pack2(nd, nd);
       }
-      for (int i = 0; i < nt; ++i) {
-        const int buf = KIND == FWD ? grp : KIND == DQ ? (int)(k & 1u) : 0;
-        WAIT(B_S + buf, KIND == DQ ? k >> 1 : k, 74);
-        if (KIND == DKV) WAIT(B_FULL + (int)(k & (STAGES - 1)), k / STAGES, 81);
+      const int tiles = it.n0 > it.n1 ? it.n0 : it.n1;
+      for (int i = 0; i < tiles; ++i, ++tile) {
+        if (KIND == FWD) {   // buffers go to the held tiles in turn
+          if (grp == 1 && i < it.n0) buf = buf == 2 ? 0 : buf + 1;
+          if (i >= nt) {
+            if (grp == 0) buf = buf == 2 ? 0 : buf + 1;
+            continue;
+          }
+        }
+        WAIT(B_S + 3 * grp + (int)buf, phases >> buf, 74);
+        phases ^= 1u << buf;
+        if (KIND == DKV) WAIT(B_FULL + (int)(tile & (STAGES - 1)), tile / STAGES, 81);
         tc_fence_after_sync();
-        const int x0 = (it.t0 + i) * T + half * W;   // streamed row of this warp's first column
+        const int x0 = (it.t0 + i) * T + part * W;   // streamed row of this warp's first column
         // columns [lo, hi) of this row are visible
         int lo = 0, hi = W;
         if (KIND == DKV) {
@@ -564,13 +581,11 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
           if (KIND == FWD && P.nx - x0 < hi) hi = P.nx - x0;   // rows past the last key would count f(0) in the sum
         }
         const bool whole = __all_sync(0xffffffffu, lo <= 0 && hi >= W);
-        const uint32_t sa = lane_addr + C_S + (uint32_t)(buf * 128 + W * half);
+        const uint32_t sa = lane_addr + C_S + buf * 128u + (uint32_t)(W * part);
         if (KIND == FWD) {
           if (first) {   // general form, the sum of the rounded weights
-            if (k > 0) WAIT(B_SFREE + grp, k - 1u, 83);
-            tc_fence_after_sync();
 #pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < 2; ++c) {
               uint32_t x32[32], pr[16];
               tmem_ld32(sa + 32u * c, x32);
               tmem_ld_wait();
@@ -582,65 +597,63 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
                 pr[j] = bf16x2(32 * c + 2 * j < hi ? p0 : 0.f, 32 * c + 2 * j + 1 < hi ? p1 : 0.f);
                 sum[j & 3] = add2(sum[j & 3], pack2u(pr[j] << 16, pr[j] & 0xffff0000u));
               }
-              tmem_st16(lane_addr + Cols<KIND>::P + 64u * grp + 16u * c, pr);
+              tmem_st16(sa + 16u * c, pr);
             }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars[B_READS + grp]);
           } else {
-          uint32_t s[4][32];
+            uint32_t s[2][32];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) tmem_ld32(sa + 32u * c, s[c]);
-          tmem_ld_wait();
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars[B_READS + grp]);
-          if (k > 0) WAIT(B_SFREE + grp, k - 1u, 83);   // the last tile's second product has read P
-          tc_fence_after_sync();
+            for (int c = 0; c < 2; ++c) tmem_ld32(sa + 32u * c, s[c]);
+            tmem_ld_wait();
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t pr[16];
-            if (whole) {
+            for (int c = 0; c < 2; ++c) {
+              uint32_t pr[16];
+              if (whole) {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const uint64_t x = pack2u(s[c][2 * j], s[c][2 * j + 1]);
-                const uint64_t p = SQ ? fma2(x, x, K) : fma2(fma2(C2, x, C1), x, C0);
-                sum[j & 3] = add2(sum[j & 3], p);
-                pr[j] = bf16x2(p);
+                for (int j = 0; j < 16; ++j) {
+                  const uint64_t x = pack2u(s[c][2 * j], s[c][2 * j + 1]);
+                  const uint64_t p = SQ ? fma2(x, x, K) : fma2(fma2(C2, x, C1), x, C0);
+                  sum[j & 3] = add2(sum[j & 3], p);
+                  pr[j] = bf16x2(p);
+                }
+              } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                  const uint64_t x = pack2u(s[c][2 * j], s[c][2 * j + 1]);
+                  float p0, p1;
+                  unpack2(SQ ? fma2(x, x, K) : fma2(fma2(C2, x, C1), x, C0), p0, p1);
+                  if (32 * c + 2 * j >= hi) p0 = 0.f;
+                  if (32 * c + 2 * j + 1 >= hi) p1 = 0.f;
+                  sum[j & 3] = add2(sum[j & 3], pack2(p0, p1));
+                  pr[j] = bf16x2(p0, p1);
+                }
               }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const uint64_t x = pack2u(s[c][2 * j], s[c][2 * j + 1]);
-                float p0, p1;
-                unpack2(SQ ? fma2(x, x, K) : fma2(fma2(C2, x, C1), x, C0), p0, p1);
-                if (32 * c + 2 * j >= hi) p0 = 0.f;
-                if (32 * c + 2 * j + 1 >= hi) p1 = 0.f;
-                sum[j & 3] = add2(sum[j & 3], pack2(p0, p1));
-                pr[j] = bf16x2(p0, p1);
-              }
+              tmem_st16(sa + 16u * c, pr);
             }
-            tmem_st16(lane_addr + Cols<KIND>::P + 64u * grp + 16u * c, pr);
           }
+          if (i == nt - 1) {
+            float a, b;
+            unpack2(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])), a, b);
+            sum[0] = sum[1] = sum[2] = sum[3] = 0ull;
+            if (part == 0) next_total = a + b;
+            else sums[(n & 3) * 2 * R] = a + b;
           }
         } else {
-          uint32_t d[2][32], s[2][32], pr[2][16], dr[2][16];
-          tmem_ld32(lane_addr + Cols<KIND>::DP + 64u * half, d[0]);
-          tmem_ld32(lane_addr + Cols<KIND>::DP + 64u * half + 32u, d[1]);
-          tmem_ld32(sa, s[0]);
-          tmem_ld32(sa + 32u, s[1]);
+          constexpr int CW = W / 32;
+          uint32_t d[CW][32], s[CW][32], pr[CW][16], dr[CW][16];
+#pragma unroll
+          for (int c = 0; c < CW; ++c) {
+            tmem_ld32(lane_addr + C_DP + (uint32_t)(W * part + 32 * c), d[c]);
+            tmem_ld32(sa + 32u * c, s[c]);
+          }
           tmem_ld_wait();
           tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) {
-            mbar_arrive(&bars[B_READS + buf]);
-            mbar_arrive(&bars[B_READD]);
-          }
+          if (lane == 0) mbar_arrive(&bars[B_READD]);
           auto weights = [&](auto square) {   // the element-wise part: f and f' (dP - delta), in bf16
             constexpr bool Q = decltype(square)::value;
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const ulonglong2* ndp = reinterpret_cast<const ulonglong2*>(sm + OFF_ND + (k & (STAGES - 1)) * T * 4 + half * 256 + c * 128);
+            for (int c = 0; c < CW; ++c) {
+              const ulonglong2* ndp = reinterpret_cast<const ulonglong2*>(sm + OFF_ND + ((tile & (STAGES - 1)) * T + W * part + 32 * c) * 4);
 #pragma unroll
               for (int j2 = 0; j2 < 8; ++j2) {
                 ulonglong2 n2;
@@ -662,25 +675,28 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
           else weights(std::false_type{});
           if (!whole) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
+            for (int j = 0; j < W / 2; ++j) {
               const uint32_t keep = ((2 * j >= lo && 2 * j < hi) ? 0x0000ffffu : 0u) | ((2 * j + 1 >= lo && 2 * j + 1 < hi) ? 0xffff0000u : 0u);
               dr[j >> 4][j & 15] &= keep;
               if (KIND == DKV) pr[j >> 4][j & 15] &= keep;
             }
           }
-          if (k > 0) WAIT(B_SFREE, k - 1u, 83);   // the last tile's second products have read theirs
-          tc_fence_after_sync();
 #pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            if (KIND == DKV) tmem_st16(lane_addr + Cols<KIND>::P + 32u * half + 16u * c, pr[c]);
-            tmem_st16(lane_addr + Cols<KIND>::DS + 32u * half + 16u * c, dr[c]);
+          for (int c = 0; c < CW; ++c) {
+            if (KIND == DKV) tmem_st16(sa + 32u * c, pr[c]);
+            tmem_st16(sa + 32u * c + (KIND == DKV ? 16u : 0u), dr[c]);
           }
         }
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[B_P + grp]);
-        ++k;
+        if (lane == 0) mbar_arrive(&bars[B_P + (int)buf]);
+        if (KIND == FWD) {   // (the second held tile's turn)
+          buf = buf == 2 ? 0 : buf + 1;
+          if (grp == 0 && i < it.n1) buf = buf == 2 ? 0 : buf + 1;
+        } else {
+          buf ^= 1u;
+        }
         if (i == 0 && pend) results(n - 1, last, total);
         if (i == 1 && pend) give_back(n - 1);
       }
@@ -689,20 +705,19 @@ __global__ void __launch_bounds__(THREADS, 1) pair_kernel(const __grid_constant_
           results(n - 1, last, total);
           give_back(n - 1);
         }
-        WAIT(B_HFULL + (n & 1), (uint32_t)(n >> 1), 84);   // (not before the set's last phase is over)
-        if (lane == 0) mbar_arrive(&bars[B_HEMPTY + (n & 1)]);
+        if (writes) {
+          WAIT(B_HFULL + (n & 1), (uint32_t)(n >> 1), 84);   // (not before the set's last phase is over)
+          if (lane == 0) mbar_arrive(&bars[B_HEMPTY + (n & 1)]);
+        }
       } else if (nt == 1 && pend) {
         give_back(n - 1);
       }
-      pend = nt > 0;
+      pend = writes && nt > 0;
       last = it;
+      total = next_total;
       idx = next_item(n);
     }
-    if (pend) {
-      float a, b;
-      unpack2(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])), a, b);
-      results(n - 1, last, a + b);
-    }
+    if (pend) results(n - 1, last, total);
     if (lane == 0) bulk_wait_read_all();   // before the block's shared memory goes
   }
   tc_fence_before_sync();
@@ -794,7 +809,7 @@ cudaError_t launch(const pair::Maps& M, const pair::Params& P, int bh, cudaStrea
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
   }
-  kernel<<<dim3((unsigned)(P.ntiles * bh)), pair::THREADS, pair::SMEM_BYTES, st>>>(M, P);
+  kernel<<<dim3((unsigned)(P.ntiles * bh)), pair::THREADS<D, KIND>, pair::SMEM_BYTES, st>>>(M, P);
   return cudaGetLastError();
 }
 // Heads per group of the item order (decode).  With a mask, items differ in length: as many heads as have their streamed tiles in

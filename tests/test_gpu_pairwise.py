@@ -180,3 +180,33 @@ def test_bf16_heads_of_16_dims_keep_float32_weights(nq, nk, causal, order):
     assert {"pair_f32_fwd", "pair_f32_bwd_q", "pair_f32_bwd_kv"} <= kinds and "scan_fwd" in kinds_engine
     for name, a, b in zip(("o", "dq", "dk", "dv"), got, engine):
         assert a < 1.05 * b, (name, a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("case", [(12, 40, 320, 320, 64, True), (12, 40, 320, 60, 32, False), (20, 40, 60, 60, 64, True), (8, 40, 130, 300, 32, True)])
+def test_items_of_different_lengths_follow_one_another_on_a_block(case, dtype):
+    """Several items per block, some of one tile, some without a second held tile: the rings of score buffers, row sums and held
+    tiles go round with every alignment.  Every head is checked, against float64."""
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    B, H, nq, nk, D, causal = case
+    g = torch.Generator(device="cuda").manual_seed(nq + nk)
+    q, do = (torch.randn(B, H, nq, D, device="cuda", generator=g).to(dtype) for _ in range(2))
+    k, v = (torch.randn(B, H, nk, D, device="cuda", generator=g).to(dtype) for _ in range(2))
+    it = 1.0 / (8.0 * math.sqrt(D))
+    o, gg, _ = L.forward(q, k, v, causal, it, flags=L.FLAG_PAIRWISE)
+    dq, dk, dv, _ = L.backward(q, k, v, o, gg, do, causal, it, flags=L.FLAG_PAIRWISE)
+    L.check_status()
+    assert L.wait_histogram() == {}
+    qd, kd, vd = (t.double().requires_grad_(True) for t in (q, k, v))
+    s = qd @ kd.transpose(-1, -2) * it
+    f = 1.0 + s + 0.5 * s * s
+    if causal:
+        f = f * torch.ones(nq, nk, device="cuda", dtype=torch.float64).tril(nk - nq)
+    ref = (f @ vd) / f.sum(-1, keepdim=True)
+    grads = torch.autograd.grad(ref, (qd, kd, vd), do.double())
+    # bf16: operands and results of 8 bits (2^-9 each, five roundings in a row); float32: 2e-7 measured in every size
+    tol = 1e-2 if dtype == torch.bfloat16 else 2e-6
+    for name, x, r in (("o", o, ref.detach()), ("dq", dq, grads[0]), ("dk", dk, grads[1]), ("dv", dv, grads[2])):
+        err = (x.double() - r).norm(dim=(-1, -2)) / r.norm(dim=(-1, -2))
+        assert float(err.max()) < tol, (name, float(err.max()), int(err.argmax()))
