@@ -10,8 +10,14 @@
 // for every streamed tile (64 rows: four additions of hi hi behind the twenty small ones, which go first) and the
 // element-wise warps add the tile's result to float32 totals in registers, rounding to nearest.
 //
-// Measured: 128 heads of 1024 x 64, causal, forward + backward with splitting 13400 us in the CUDA-core engine (FFMA), 600 here;
-// bf16, 128 heads of 1024 x 16 (q, k, v are one piece each: 1 or 3 products instead of 6, no pass that splits) 771 and 233.
+// Measured: 128 heads of 1024 x 64, causal, forward + backward with splitting 13400 us in the CUDA-core engine (FFMA), 528 here
+// (forward 114, dq 138, dk / dv 190, splitting 77, dO' 25); bf16, 128 heads of 1024 x 16 (q, k, v are one piece each: 1 or 3
+// products instead of 6, no pass that splits) 771 and 216.  Bound by the chain scores -> element-wise -> second products
+// between few warps (tensor pipe active in 51 to 65 % of the clocks at 64 dims, issue slots 30 %).  What took the forward from 131
+// to 114, dq from 156 to 138 and dk / dv from 216 to 190: scores in two blocks (product2), the results of a tile added up behind
+// the next tile's P instead of before it (dq: before its arithmetic, when its products have ended), rows written 16 bytes a
+// thread (one row per instruction, the warps that write dk and dv held up the next item for 7000 clocks), and the forward's held
+// tile of the next item loaded early.
 //
 // Roles and hand-offs are those of the bf16 kernels; the streamed pair's two tiles have barriers of their own, because with
 // three pieces each only two or three stages fit and each tile can be let go at a different time.
@@ -25,21 +31,30 @@ constexpr int XF = TF * 128;                 // one piece of a streamed tile
 constexpr int AF = R * 128;                  // one piece of a held tile
 template <int KIND>
 struct Lay {
-  static constexpr int STAGES = KIND == FWD ? 3 : 2;
+  static constexpr int SETS = KIND == FWD ? 2 : 1;                    // held sets
   static constexpr int HELD = (KIND == FWD ? 3 : 6) * AF;
+  static constexpr int STAGES = 2;
   static constexpr int STAGE = 6 * XF;       // X pieces, then Y pieces
-  static constexpr int OFF_X = HELD;
-  static constexpr int OFF_OUT = OFF_X + STAGES * STAGE;   // 4 KB of output staging per element-wise warp
-  static constexpr int OFF_ND = OFF_OUT + EW * 4096;       // DKV: -delta of the streamed queries per stage; FWD: row sums of the halves
-  static constexpr int OFF_CLC = OFF_ND + 1024;
+  static constexpr int OFF_X = SETS * HELD;
+  static constexpr int OFF_OUT = OFF_X + STAGES * STAGE;   // 4 KB of output staging per warp that writes rows
+  static constexpr int OFF_ND = OFF_OUT + (KIND == DKV ? 4 : EW) * 4096;   // DKV: -delta of the streamed queries per stage
+  static constexpr int OFF_CLC = OFF_ND + STAGES * TF * 4;
   static constexpr int OFF_BAR = OFF_CLC + 16 * CLC;
   static constexpr int BYTES = OFF_BAR + 512 + 1024;
 };
-static_assert(Lay<FWD>::BYTES <= 232448 && Lay<DKV>::BYTES <= 232448, "shared memory budget");
-constexpr int B_FX = 0, B_FY = 3, B_EX = 6, B_EY = 9, B_HFULL = 12, B_HEMPTY = 13, B_S = 14, B_READ = 15, B_P = 16, B_ACC = 17, B_AFREE = 18,
-              B_CFULL = 19, B_CEMPTY = B_CFULL + CLC, B_DRAIN = B_CEMPTY + CLC, B_COUNT = B_DRAIN + 2;
-// TMEM columns: accumulators (dv, dk / dq / O'), scores, dP, pieces of P and of dS (32 columns each)
-constexpr uint32_t C_ACC = 0, C_ACC1 = 64, C_S = 128, C_DP = 192, C_P = 256, C_DS = 352;
+static_assert(Lay<FWD>::BYTES <= 232448 && Lay<DQ>::BYTES <= 232448 && Lay<DKV>::BYTES <= 232448, "shared memory budget");
+constexpr int B_FX = 0, B_FY = 2, B_EX = 4, B_EY = 6, B_HFULL = 8, B_HEMPTY = 10, B_S = 12, B_READ = 14, B_P = 15, B_ACC = 17, B_AFREE = 19,
+              B_CFULL = 21, B_CEMPTY = B_CFULL + CLC, B_DRAIN = B_CEMPTY + CLC, B_COUNT = B_DRAIN + 2;
+// TMEM columns.  S (and DQ: dP) in two blocks of 64 columns, the small piece products in the second; P and dS in three pieces of
+// 32 columns.  What a tile leaves (P or dS, its results) is doubled where there is room, so that the element-wise warps go on
+// with the next tile while its second products run.
+template <int KIND>
+struct Cols {
+  static constexpr uint32_t NACC = KIND == FWD ? 2 : 1, NP = KIND == DKV ? 1 : 2;   // results, P / dS
+  static constexpr uint32_t ACC = 0, ACC1 = 64, S = KIND == DQ ? 64 : 128, DP = KIND == DQ ? 192 : 256;   // DKV: dv, dk
+  static constexpr uint32_t P = KIND == FWD ? 256 : 320, DS = KIND == DKV ? 416 : 320;
+  static constexpr uint32_t SUM = 448;   // FWD: row sums of the two halves, of the last four items
+};
 // dk / dv: a warpgroup of its own adds up the accumulators (128 totals per thread: beside a tile they do not fit into the
 // element-wise warps' registers; spilled, the kernel took four times as long).  Registers are moved between the warpgroups.
 constexpr int W_SUM = W_EW + EW;
@@ -94,8 +109,8 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
   if (tid == 0) {
     for (int i = 0; i < B_COUNT; ++i) {
       uint32_t n = 1;
-      if (i == B_READ || i == B_P) n = EW;
-      if (i == B_AFREE) n = KIND == DKV ? 4 : EW;
+      if (i == B_READ || i == B_P || i == B_P + 1) n = EW;
+      if (i == B_AFREE || i == B_AFREE + 1) n = KIND == DKV ? 4 : EW;
       if (i >= B_CEMPTY && i < B_CEMPTY + CLC) n = KIND == DKV ? ROLES + 4 : ROLES;
       mbar_init(&bars[i], n);
     }
@@ -158,17 +173,18 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
       }
       asked = n + 1;
       const Item it = decode<KIND, TF, R>(idx, P);
-      if (n >= 1) WAIT(B_HEMPTY, (uint32_t)n - 1u, 78);
+      const int hs = n % L::SETS;
+      if (n >= L::SETS) WAIT(B_HEMPTY + hs, (uint32_t)(n / L::SETS) - 1u, 78);
       if (*abort_flag != 0) break;
       if (lane == 0) {
-        mbar_arrive_expect_tx(&bars[B_HFULL], (IN + (KIND == FWD ? 0 : PB)) * AF);
+        mbar_arrive_expect_tx(&bars[B_HFULL + hs], (IN + (KIND == FWD ? 0 : PB)) * AF);
         auto load_held = [&](uint8_t* dst, const CUtensorMap* m, int pieces) {
-          if (pieces == 1) tma_load_4d(dst, m, &bars[B_HFULL], 0, it.r0, it.h, it.b);
+          if (pieces == 1) tma_load_4d(dst, m, &bars[B_HFULL + hs], 0, it.r0, it.h, it.b);
           else
 #pragma unroll
-            for (int p = 0; p < 3; ++p) tma_load_4d(dst + p * AF, m, &bars[B_HFULL], 0, it.r0, it.head, p);
+            for (int p = 0; p < 3; ++p) tma_load_4d(dst + p * AF, m, &bars[B_HFULL + hs], 0, it.r0, it.head, p);
         };
-        load_held(sm, &M.a, IN);
+        load_held(sm + hs * L::HELD, &M.a, IN);
         if (KIND != FWD) load_held(sm + 3 * AF, &M.b, PB);
       }
       helds = n + 1;
@@ -181,8 +197,8 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
   } else if (w == W_SCORE) {
     FM_REG_DEC();
     // ================= issuer of the first products =================
-    constexpr uint32_t ID_S = make_idesc_bf16(R, TF, 0, 0);
-    const uint64_t dH = make_smem_desc(smem_u32(sm), 16, 1024, 2);
+    constexpr uint32_t ID_S = make_idesc_bf16(R, TF, 0, 0), ID_S2 = make_idesc_bf16(R, 2 * TF, 0, 0);
+    const uint64_t dH0 = make_smem_desc(smem_u32(sm), 16, 1024, 2);
     const uint64_t dX0 = make_smem_desc(smem_u32(sm + L::OFF_X), 16, 1024, 2);
     // sum over the piece products of a held tile with `na` pieces and a streamed one with `nb`, the smallest first
     auto product = [&](uint32_t acc, uint64_t a, int na, uint64_t b, int nb) {
@@ -197,11 +213,25 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
         }
       }
     };
+    // The same of three pieces each, in two blocks: the streamed tile's hi and mid pieces lie one behind the other and enter as one
+    // operand of 128 rows.  A product of 64 columns keeps the pipe for 48 clocks, one of 128 for 64: 896 instead of 1152 a tile.
+    auto product2 = [&](uint32_t acc, uint64_t a, uint64_t b) {
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) mma_ss_elect(acc, a + (uint64_t)((AF >> 4) + 2 * ks), b + (uint64_t)(2 * ks), ID_S2, ks > 0);   // mid hi, mid mid
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) mma_ss_elect(acc + 64u, a + (uint64_t)(2 * (AF >> 4) + 2 * ks), b + (uint64_t)(2 * ks), ID_S, 1u);   // lo hi
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) mma_ss_elect(acc + 64u, a + (uint64_t)(2 * ks), b + (uint64_t)(2 * (XF >> 4) + 2 * ks), ID_S, 1u);   // hi lo
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) mma_ss_elect(acc, a + (uint64_t)(2 * ks), b + (uint64_t)(2 * ks), ID_S2, 1u);                      // hi hi, hi mid
+    };
     uint32_t k = 0;
     int idx = blockIdx.x;
     for (int n = 0; idx >= 0; ++n) {
       const Item it = decode<KIND, TF, R>(idx, P);
-      WAIT(B_HFULL, (uint32_t)n, 72);
+      const int hs = n % L::SETS;
+      const uint64_t dH = dH0 + (uint64_t)(hs * (L::HELD >> 4));
+      WAIT(B_HFULL + hs, (uint32_t)(n / L::SETS), 72);
       for (int i = 0; i < it.n0; ++i) {
         const uint32_t s = k % STAGES;
         const uint64_t dX = dX0 + (uint64_t)(s * (L::STAGE >> 4)), dY = dX + (uint64_t)(3 * XF >> 4);
@@ -209,22 +239,24 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
         if (KIND == DQ) {   // v is needed here only: it can go before k, which the second product reads too
           WAIT(B_FY + (int)s, k / STAGES, 74);
           tc_fence_after_sync();
-          product(tmem + C_DP, dH + (uint64_t)(3 * AF >> 4), PB, dY, PY);
+          if constexpr (IN == 3) product2(tmem + Cols<KIND>::DP, dH + (uint64_t)(3 * AF >> 4), dY);
+          else product(tmem + Cols<KIND>::DP, dH + (uint64_t)(3 * AF >> 4), PB, dY, PY);
           mma_commit_elect(&bars[B_EY + s]);
         }
         WAIT(B_FX + (int)s, k / STAGES, 73);
         tc_fence_after_sync();
-        product(tmem + C_S, dH, IN, dX, IN);
+        if constexpr (IN == 3) product2(tmem + Cols<KIND>::S, dH, dX);
+        else product(tmem + Cols<KIND>::S, dH, IN, dX, IN);
         if (KIND == FWD) mma_commit_elect(&bars[B_EX + s]);
         if (KIND == DKV) {
           WAIT(B_FY + (int)s, k / STAGES, 74);
           tc_fence_after_sync();
-          product(tmem + C_DP, dH + (uint64_t)(3 * AF >> 4), PB, dY, PY);
+          product(tmem + Cols<KIND>::DP, dH + (uint64_t)(3 * AF >> 4), PB, dY, PY);
         }
-        mma_commit_elect(&bars[B_S]);
+        mma_commit_elect(&bars[B_S + (k & 1u)]);
         ++k;
       }
-      mma_commit_elect(&bars[B_HEMPTY]);
+      mma_commit_elect(&bars[B_HEMPTY + hs]);
       idx = next_item(n);
     }
     if (*abort_flag != 0) {
@@ -248,6 +280,7 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
         }
       }
     };
+    using C = Cols<KIND>;
     uint32_t k = 0;
     int idx = blockIdx.x;
     for (int n = 0; idx >= 0; ++n) {
@@ -256,18 +289,18 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
         const uint32_t s = k % STAGES;
         const uint64_t dX = dX0 + (uint64_t)(s * (L::STAGE >> 4)), dY = dX + (uint64_t)(3 * XF >> 4);
         if (KIND == FWD) WAIT(B_FY + (int)s, k / STAGES, 75);
-        WAIT(B_P, k, 79);
-        if (k > 0) WAIT(B_AFREE, k - 1u, 82);   // the last tile's results are in the totals
+        WAIT(B_P + (int)(k % C::NP), k / C::NP, 79);
+        if (k >= C::NACC) WAIT(B_AFREE + (int)(k % C::NACC), k / C::NACC - 1u, 82);   // the results there have been added up
         tc_fence_after_sync();
         if (KIND != FWD) {
-          product(tmem + (KIND == DKV ? C_ACC1 : C_ACC), tmem + C_DS, dX, IN);
+          product(tmem + (KIND == DKV ? C::ACC1 : C::ACC), tmem + C::DS + 96u * (k % C::NP), dX, IN);
           mma_commit_elect(&bars[B_EX + s]);
         }
         if (KIND != DQ) {
-          product(tmem + C_ACC, tmem + C_P, dY, PY);
+          product(tmem + C::ACC + 64u * (k % C::NACC), tmem + C::P + 96u * (k % C::NP), dY, PY);
           mma_commit_elect(&bars[B_EY + s]);
         }
-        mma_commit_elect(&bars[B_ACC]);
+        mma_commit_elect(&bars[B_ACC + (int)(k % C::NACC)]);
         ++k;
       }
       idx = next_item(n);
@@ -284,36 +317,59 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
     // Totals of this warp: half a row of dq or O'; dv and dk (two rows of D) in the warps that add up
     constexpr int NA = KIND == DKV ? 2 * D : D / 2;
+    constexpr uint32_t NACC = Cols<KIND>::NACC, NP = Cols<KIND>::NP;
     constexpr int CH = KIND == DKV ? (D < 32 ? D : 32) : (NA < 32 ? NA : 32);
     auto clear = [&](uint64_t (&tot)[NA / 2]) {
 #pragma unroll
       for (int j = 0; j < NA / 2; ++j) tot[j] = 0ull;
     };
     auto drain = [&](uint64_t (&tot)[NA / 2], uint32_t tile) {   // adds the results of a tile's second products
-      WAIT(B_ACC, tile, 83);
+      WAIT(B_ACC + (int)(tile % NACC), tile / NACC, 83);
       tc_fence_after_sync();
 #pragma unroll
       for (int c = 0; c < NA / CH; ++c) {
         uint32_t r[CH];
         // DKV: chunks of dv, then of dk
-        tmem_ld<CH>(lane_addr + (KIND == DKV ? (uint32_t)(64 * (c * CH / D) + c * CH % D) : (uint32_t)(half * NA + CH * c)), r);
+        tmem_ld<CH>(lane_addr + (KIND == DKV ? (uint32_t)(64 * (c * CH / D) + c * CH % D) : 64u * (tile % NACC) + (uint32_t)(half * NA + CH * c)), r);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < CH / 2; ++j) tot[c * (CH / 2) + j] = add2(tot[c * (CH / 2) + j], pack2u(r[2 * j], r[2 * j + 1]));
       }
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[B_AFREE]);
+      if (lane == 0) mbar_arrive(&bars[B_AFREE + (int)(tile % NACC)]);
     };
-    // rows -> shared memory (column xor row: no bank conflicts either way) -> one row per store instruction, any strides
+    // rows -> shared memory -> whole rows in global memory: 16 bytes a thread where the rows allow it (P.vec0, P.vec1), else element
+    // by element (one row per store instruction).  The exchange is free of bank conflicts either way.
     auto write_rows = [&](const Item& it, const uint64_t (&tot)[NA / 2], float wgt) {
       float* stage = reinterpret_cast<float*>(sm + L::OFF_OUT + (KIND == DKV ? quarter : w - W_EW) * 4096);
 #pragma unroll
       for (int c = 0; c < NA / CH; ++c) {
-        const View& out = KIND == DKV && c * CH < D ? P.out1 : P.out0;
+        const bool second = KIND == DKV && c * CH < D;
+        const View& out = second ? P.out1 : P.out0;
         Out* base = reinterpret_cast<Out*>(const_cast<void*>(out.ptr)) + (long long)it.b * out.sb + (long long)it.h * out.sh +
                     (KIND == DKV ? c * CH % D : half * NA + CH * c);
         __syncwarp();
+        if (sizeof(Out) == 4 && CH >= 8 && (second ? P.vec1 : P.vec0)) {
+          constexpr int Q = CH / 4;   // 16-byte pieces of a row
+#pragma unroll
+          for (int j = 0; j < Q; ++j) {
+            float4 v;
+            unpack2(tot[c * (CH / 2) + 2 * j], v.x, v.y);
+            unpack2(tot[c * (CH / 2) + 2 * j + 1], v.z, v.w);
+            v.x *= wgt; v.y *= wgt; v.z *= wgt; v.w *= wgt;
+            reinterpret_cast<float4*>(stage)[lane * Q + (j ^ (lane & (Q - 1)))] = v;
+          }
+          __syncwarp();
+          const int rr = lane / Q, cc = lane % Q;
+#pragma unroll
+          for (int r = 0; r < 32; r += 32 / Q) {
+            const int g = it.r0 + quarter * 32 + r + rr;
+            const float4 v = reinterpret_cast<const float4*>(stage)[(r + rr) * Q + (cc ^ ((r + rr) & (Q - 1)))];
+            if (g < P.nr) reinterpret_cast<float4*>(base + (long long)g * out.sn)[cc] = v;
+          }
+          continue;
+        }
 #pragma unroll
         for (int j = 0; j < CH / 2; ++j) {
           float a, b;
@@ -347,6 +403,26 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
     } else {
       FM_REG_INC(REG_EW);
       const uint64_t C0 = pack2(P.c0, P.c0), C1 = pack2(P.c1, P.c1), C2 = pack2(P.c2, P.c2);
+      uint64_t tot[NA / 2];
+      bool pend = false;       // the last item's rows are still to be written: they are behind the next item's first tile
+      Item last{};
+      int last_n = 0;
+      auto results = [&] {
+        drain(tot, k - 1u);
+        float wgt = 1.f;
+        if (KIND == FWD) {   // (each half's sum was there before its last P of the item)
+          uint32_t h[2];
+          tmem_ld2(lane_addr + Cols<KIND>::SUM + 2u * ((uint32_t)last_n & 3u), h);
+          tmem_ld_wait();
+          const float g = __uint_as_float(h[0]) + __uint_as_float(h[1]);
+          wgt = last.r0 >= P.part_lo && last.r0 < P.part_hi ? 1.f : 1.f / g;   // partial rows: not divided yet
+          const int row = last.r0 + quarter * 32 + lane;
+          if (half == 0 && row < P.nr)
+            reinterpret_cast<float*>(const_cast<void*>(P.out1.ptr))[(long long)last.b * P.out1.sb + (long long)last.h * P.out1.sh + (long long)row * P.out1.sn] = g;
+        }
+        write_rows(last, tot, wgt);
+      };
+      if (KIND != DKV) clear(tot);
       for (int n = 0; idx >= 0; ++n) {
         const Item it = decode<KIND, TF, R>(idx, P);
         const int row = it.r0 + quarter * 32 + lane;
@@ -355,11 +431,9 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
           const float nd = row < P.nr ? __ldg(P.ndelta + (long long)it.head * P.nd_ld + row) : 0.f;
           ND = pack2(nd, nd);
         }
-        uint64_t tot[NA / 2];
-        if (KIND != DKV) clear(tot);
-        float total = 0.f;
+        float total = 0.f;   // FWD: this half's row sum
         for (int i = 0; i < it.n0; ++i) {
-          WAIT(B_S, k, 84);
+          WAIT(B_S + (int)(k & 1u), k >> 1, 84);
           const int s_ = (int)(k % STAGES);
           if (KIND == DKV) WAIT(B_FY + s_, k / STAGES, 81);
           tc_fence_after_sync();
@@ -373,90 +447,100 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
           }
           const bool whole = __all_sync(0xffffffffu, lo <= 0 && hi >= 32);
           uint32_t s[32], d[32];
-          tmem_ld32(lane_addr + C_S + 32u * half, s);
-          if (KIND != FWD) tmem_ld32(lane_addr + C_DP + 32u * half, d);
-          tmem_ld_wait();
+          auto load = [&](uint32_t (&v)[32], uint32_t col, bool both) {   // both blocks of S or dP
+            uint32_t small[32];
+            tmem_ld32(lane_addr + col + 32u * half, v);
+            if (both) tmem_ld32(lane_addr + col + 64u + 32u * half, small);
+            if (KIND == DKV) tmem_ld32(lane_addr + Cols<KIND>::DP + 32u * half, d);
+            tmem_ld_wait();
+            if (both)
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const uint64_t x = add2(pack2u(v[2 * j], v[2 * j + 1]), pack2u(small[2 * j], small[2 * j + 1]));
+                v[2 * j] = (uint32_t)x;
+                v[2 * j + 1] = (uint32_t)(x >> 32);
+              }
+          };
+          load(s, Cols<KIND>::S, IN == 3);
+          if (KIND == DQ) load(d, Cols<KIND>::DP, IN == 3);
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars[B_READ]);
-          // the last tile's second products are done: P and dS may be overwritten, and their results are added up
-          if (KIND == DKV) {
-            if (k > 0) WAIT(B_ACC, k - 1u, 85);
-            tc_fence_after_sync();
-          } else if (i > 0) {
-            drain(tot, k - 1u);
-          }
+          if (KIND == DQ && i > 0) drain(tot, k - 1u);   // (its products ended under the first ones of this tile)
+          // values: P in s, dS in d
           const ulonglong2* ndp = reinterpret_cast<const ulonglong2*>(sm + L::OFF_ND + s_ * TF * 4 + half * 128);
           uint64_t sum = 0ull;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t pp[3][4], dd[3][4];
+          for (int j2 = 0; j2 < 8; ++j2) {
+            ulonglong2 n2;
+            n2.x = n2.y = ND;
+            if (KIND == DKV) n2 = ndp[j2];
 #pragma unroll
-            for (int j2 = 0; j2 < 2; ++j2) {
-              ulonglong2 n2;
-              n2.x = n2.y = ND;
-              if (KIND == DKV) n2 = ndp[2 * c + j2];
-#pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const int j = 2 * j2 + e, col = 8 * c + 2 * j;
-                const bool v0 = whole || (col >= lo && col < hi), v1 = whole || (col + 1 >= lo && col + 1 < hi);
-                const uint64_t x = pack2u(s[col], s[col + 1]);
-                const uint64_t t = fma2(C2, x, C1);
-                if (KIND != DQ) {
-                  uint64_t p = fma2(t, x, C0);
-                  if (!whole) {
-                    float a, b;
-                    unpack2(p, a, b);
-                    p = pack2(v0 ? a : 0.f, v1 ? b : 0.f);
-                  }
-                  if (KIND == FWD) sum = add2(sum, p);
-                  split3(p, pp[0][j], pp[1][j], pp[2][j]);
-                }
-                if (KIND != FWD) {
-                  uint64_t ds = mul2(fma2(C2, x, t), add2(pack2u(d[col], d[col + 1]), e ? n2.y : n2.x));
-                  if (!whole) {
-                    float a, b;
-                    unpack2(ds, a, b);
-                    ds = pack2(v0 ? a : 0.f, v1 ? b : 0.f);
-                  }
-                  split3(ds, dd[0][j], dd[1][j], dd[2][j]);
-                }
+            for (int e = 0; e < 2; ++e) {
+              const int col = 4 * j2 + 2 * e;
+              const bool v0 = whole || (col >= lo && col < hi), v1 = whole || (col + 1 >= lo && col + 1 < hi);
+              const uint64_t x = pack2u(s[col], s[col + 1]);
+              const uint64_t t = fma2(C2, x, C1);
+              if (KIND != DQ) {
+                float a, b;
+                unpack2(fma2(t, x, C0), a, b);
+                if (!whole) { a = v0 ? a : 0.f; b = v1 ? b : 0.f; }
+                if (KIND == FWD) sum = add2(sum, pack2(a, b));
+                s[col] = __float_as_uint(a);
+                s[col + 1] = __float_as_uint(b);
+              }
+              if (KIND != FWD) {
+                float a, b;
+                unpack2(mul2(fma2(C2, x, t), add2(pack2u(d[col], d[col + 1]), e ? n2.y : n2.x)), a, b);
+                if (!whole) { a = v0 ? a : 0.f; b = v1 ? b : 0.f; }
+                d[col] = __float_as_uint(a);
+                d[col + 1] = __float_as_uint(b);
               }
             }
-#pragma unroll
-            for (int p = 0; p < 3; ++p) {
-              if (KIND != DQ) tmem_st4(lane_addr + C_P + 32u * p + 16u * half + 4u * c, pp[p]);
-              if (KIND != FWD) tmem_st4(lane_addr + C_DS + 32u * p + 16u * half + 4u * c, dd[p]);
-            }
           }
-          tmem_st_wait();
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars[B_P]);
           if (KIND == FWD) {
             float a, b;
             unpack2(sum, a, b);
             total += a + b;
+            if (i == it.n0 - 1) tmem_st1(lane_addr + Cols<KIND>::SUM + 2u * ((uint32_t)n & 3u) + (uint32_t)half, __float_as_uint(total));
+          }
+          if (KIND == DKV && k > 0) {   // the last tile's second products are done: P and dS may be overwritten
+            WAIT(B_ACC, k - 1u, 85);
+            tc_fence_after_sync();
+          }
+          // in pieces.  (FWD, DQ: the tile before the last one is added up, so these columns are free)
+          auto put = [&](const uint32_t (&v)[32], uint32_t addr) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              uint32_t pp[3][8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) split3(pack2u(v[16 * c + 2 * j], v[16 * c + 2 * j + 1]), pp[0][j], pp[1][j], pp[2][j]);
+#pragma unroll
+              for (int p = 0; p < 3; ++p) tmem_st8(addr + 32u * p + 16u * half + 8u * c, pp[p]);
+            }
+          };
+          if (KIND != DQ) put(s, lane_addr + Cols<KIND>::P + 96u * (k % NP));
+          if (KIND != FWD) put(d, lane_addr + Cols<KIND>::DS + 96u * (k % NP));
+          tmem_st_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars[B_P + (int)(k % NP)]);
+          if (KIND != DKV) {
+            if (KIND == FWD && i > 0) {
+              drain(tot, k - 1u);
+            } else if (i == 0 && pend) {
+              results();
+              clear(tot);
+            }
           }
           ++k;
         }
-        if (KIND != DKV) {
-          drain(tot, k - 1u);
-          float wgt = 1.f;
-          if (KIND == FWD) {   // the two halves' row sums
-            float* sums = reinterpret_cast<float*>(sm + L::OFF_ND);
-            sums[half * R + quarter * 32 + lane] = total;
-            named_bar_sync(1 + quarter, 64);
-            const float g = sums[quarter * 32 + lane] + sums[R + quarter * 32 + lane];
-            named_bar_sync(1 + quarter, 64);
-            wgt = it.r0 >= P.part_lo && it.r0 < P.part_hi ? 1.f : 1.f / g;   // partial rows: not divided yet
-            if (half == 0 && row < P.nr)
-              reinterpret_cast<float*>(const_cast<void*>(P.out1.ptr))[(long long)it.b * P.out1.sb + (long long)it.h * P.out1.sh + (long long)row * P.out1.sn] = g;
-          }
-          write_rows(it, tot, wgt);
-        }
+        pend = KIND != DKV;
+        last = it;
+        last_n = n;
         idx = next_item(n);
       }
+      if (pend) results();
     }
   }
   tc_fence_before_sync();
@@ -467,7 +551,8 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
         mbar_wait_bounded(&bars[B_FX + i % STAGES], (uint32_t)(i / STAGES) & 1u, WAIT_CYCLES);
       for (int i = issued_y > STAGES ? issued_y - STAGES : 0; i < issued_y; ++i)
         mbar_wait_bounded(&bars[B_FY + i % STAGES], (uint32_t)(i / STAGES) & 1u, WAIT_CYCLES);
-      if (helds > 0) mbar_wait_bounded(&bars[B_HFULL], (uint32_t)(helds - 1) & 1u, WAIT_CYCLES);
+      for (int i = helds > L::SETS ? helds - L::SETS : 0; i < helds; ++i)
+        mbar_wait_bounded(&bars[B_HFULL + i % L::SETS], (uint32_t)(i / L::SETS) & 1u, WAIT_CYCLES);
       for (int i = asked > CLC ? asked - CLC : 0; i < asked; ++i)
         mbar_wait_bounded(&bars[B_CFULL + (i & (CLC - 1))], (uint32_t)(i / CLC) & 1u, WAIT_CYCLES);
     }

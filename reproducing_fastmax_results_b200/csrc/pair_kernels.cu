@@ -813,12 +813,14 @@ cudaError_t launch(const pair::Maps& M, const pair::Params& P, int bh, cudaStrea
   return cudaGetLastError();
 }
 // Heads per group of the item order (decode).  With a mask, items differ in length: as many heads as have their streamed tiles in
-// a quarter of L2 (us forward / backward, one head at a time, 32, 128: 128 heads of 4096 x 64 252/862, 241/838, 262/939; 128 heads
-// of 2048 x 32 78/237, 70/218, 66/214; of 1024 x 64 44/105, 42/98, 42/92).  Without one (and within windows) the items are alike, and the order of the heads is best for L2.
+// 32 MB (pieces: 64 MB) of L2.  us forward / dq / dk, dv for 16, 32, 64, 128 MB: 128 heads of 4096 x 64 253 / 335 / 445,
+// 247 / 335 / 444, 248 / 341 / 445, 273 / 385 / 500; of 1024 x 64 33 / 38 / 47, then 31 / 37 / 46; float32, of 1024 x 64
+// 121 / 176 / 198, 114 / 166 / 190, 111 / 160 / 185, 110 / 156 / 188 (few items per block: the last group's long ones decide).
+// Without a mask (and within windows) the items are alike, and the order of the heads is best for L2.
 void order_items(int d, int es, pair::Params& P, int bh) {
   long long group = 1;
   if (P.causal && !P.window) {
-    group = (32ll << 20) / ((long long)P.nx * d * 2 * es);
+    group = ((es > 2 ? 64ll : 32ll) << 20) / ((long long)P.nx * d * 2 * es);
     group = group < 1 ? 1 : group > bh ? bh : group;
     const long long n = (bh + group - 1) / group;
     group = (bh + n - 1) / n;
@@ -1089,6 +1091,7 @@ static int pair_f32_forward(const fastmax_problem* pb, const fastmax_forward_arg
   P.nr = pb->nq;
   P.nx = pb->nk;
   P.ntiles = tiles(pb->nq);
+  P.vec0 = rows_f32(a->o, pb, pb->nq);
   LaunchScope ls(KK_PAIR_F32_FWD, st);
   e = launch_f32_d<pair::FWD>(pb, M, P, st);
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
@@ -1142,6 +1145,8 @@ static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   K.nr = pb->nk;
   K.nx = pb->nq;
   K.ntiles = tiles(pb->nk);
+  K.vec0 = rows_f32(a->dk, pb, pb->nk);
+  K.vec1 = rows_f32(a->dv, pb, pb->nk);
   {
     LaunchScope ls(KK_PAIR_F32_BWD_KV, st);
     e = launch_f32_d<pair::DKV>(pb, N, K, st);
@@ -1151,6 +1156,7 @@ static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   P.nr = pb->nq;
   P.nx = pb->nk;
   P.ntiles = tiles(pb->nq);
+  P.vec0 = rows_f32(a->dq, pb, pb->nq);
   {
     LaunchScope ls(KK_PAIR_F32_BWD_Q, st);
     e = launch_f32_d<pair::DQ>(pb, M, P, st);
@@ -1517,6 +1523,7 @@ static int long_f32_forward(const fastmax_problem* pb, const fastmax_forward_arg
     P.out1 = view_of(a->g);
     P.nr = P.nx = n;
     P.ntiles = tiles(n);
+    P.vec0 = 1;   // (see forward_form)
     LaunchScope ls(KK_PAIR_F32_FWD, st);
     e = launch_f32_d<pair::FWD>(pb, M, P, st);
   }
@@ -1567,6 +1574,7 @@ static int long_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   P.nd_ld = nd_ld(n);
   P.nr = P.nx = n;
   P.ntiles = tiles(n);
+  P.vec0 = P.vec1 = 1;   // (see backward_form)
   pair::Params B = P;
   B.out0 = view_of(a->dk);
   B.out1 = view_of(a->dv);

@@ -172,3 +172,20 @@ def test_key_moments_of_another_form_are_not_read(dtype, D, N, variant, binding,
 
     for a, b in zip(run(True), run(False)):
         assert orc.max_norm_err(host(a), host(b)) < (1e-2 if dtype == torch.bfloat16 else 2e-6)
+
+
+@pytest.mark.parametrize("order", [2, 1])
+def test_float32_windows_with_many_items_per_block(order):
+    """Several items per block in the moments, apply and chain kernels, whose producers take slabs in turn."""
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    g = torch.Generator(device="cuda").manual_seed(order)
+    q, k, v, do = (torch.randn(1, 40, 4100, 32, device="cuda", generator=g) for _ in range(4))
+    res = []
+    for flags in (L.FLAG_PAIRWISE, L.FLAG_NO_TENSOR_CORES):
+        o, gg, _ = L.forward(q, k, v, True, 0.02, order=order, flags=flags)
+        res.append((o, gg) + tuple(L.backward(q, k, v, o, gg, do, True, 0.02, order=order, flags=flags)[:3]))
+    L.check_status()
+    assert L.wait_histogram() == {}
+    for name, a, b in zip(("o", "g", "dq", "dk", "dv"), *res):   # both at 1e-7 to 3e-7 against float64
+        assert float((a - b).norm() / b.norm()) < 3e-6, name
