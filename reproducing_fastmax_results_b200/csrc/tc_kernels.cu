@@ -937,7 +937,7 @@ cudaError_t tc_moments(const fastmax_problem* pb, const fastmax_tensor& x, const
   CUtensorMap tmxt, tmy, tmt;
   if (!make_map_t(&tmxt, xt, bh, n, tokens_padded(n), d) || !make_map(&tmy, y, pb->batch, pb->heads, n, 64, tc::CH, true, d)) return cudaErrorInvalidValue;
   tmt = tmy;
-  if (dop && !make_map(&tmt, y, pb->batch, pb->heads, n, 8, tc::CH, false, d + 16)) return cudaErrorInvalidValue;
+  if (dop && !make_map(&tmt, y, pb->batch, pb->heads, n, 64, tc::CH, true, d + 16)) return cudaErrorInvalidValue;
   cudaError_t e = launch_transpose(x, pb->batch, pb->heads, n, 0, (__nv_bfloat16*)xt, st, d);
   if (e != cudaSuccess) return e;
   const int npair = (d / 8) * (d / 8 + 1) / 2;

@@ -3,14 +3,14 @@
 //
 // Without an output there is no order between the chunks, so the tokens of a head may be cut over several thread blocks and
 // no copy of the state is needed.  A block takes up to four feature tiles (the accumulators) of one head and a range of
-// 128-token chunks.  Four producer warpgroups, one per 32-token quarter of a chunk, form the products in registers and store
-// them to tensor memory as the A operand; thread = feature, tokens from the transposed copy.  The row of the feature's first
-// factor is kept in registers across the tiles that share it: 1.25 rows read per feature instead of two (a 128-bit load of a
-// warp takes four wavefronts whatever its lanes share).
+// 128-token chunks.  Two groups of eight producer warps form the slabs (a tile's features of a chunk) in turn, in registers, and
+// store them to tensor memory as the A operand; thread = feature, tokens from the transposed copy.  The row of the feature's
+// first factor is kept in registers across a group's tiles that share it.
 // TMEM: four 80-column accumulators, three 64-column slots.
 //
-// 620 clocks per tile and chunk.  No unit is full: 64 heads of 4096 x 64 (130 us) keep the shared-memory pipe busy for 58 % of the
-// time, the tensor pipe for 43 % (two products per K step, N = D and N = 16), the schedulers for 48 %.
+// No unit is full: 8 heads of 32768 x 64 keep the shared-memory pipe busy for 52 % of the clocks, the tensor pipe for 36 %, the
+// schedulers for 39 %.  One product of 80 columns per K step instead of one of 64 and one of 16, and slabs in turn instead of every
+// warp at every slab (half as many hand-overs): 72.6 -> 69.6 us for 64 heads of 1999 x 64, 578 -> 572 for the segments of 8 heads of 131072.
 #pragma once
 
 namespace mo {
@@ -24,12 +24,10 @@ struct Lay {
   static constexpr int NB = D / 8;
   static constexpr int PAIR_TILES = NB * (NB + 1) / 4;
   static constexpr int TILES = PAIR_TILES + 1;
-  static constexpr int NC = D + 16;                       // accumulator columns of a tile: Y and its tail column
   static constexpr int KT_BOX = D * s2::KT_ROW;           // D dims x 72 tokens
-  // Y: 128 tokens, 128-byte swizzled rows; tail (-delta of dO'): one 8-column block (8 columns used as 16: zeros follow)
-  static constexpr int OFF_T = REGION, OFF_XT = REGION + BLK, STAGE = (OFF_XT + 2 * KT_BOX + 1023) / 1024 * 1024;
-  static constexpr int OFF_ONES = STAGES * STAGE;         // the tail of [v | 1]: one constant block of ones, then a block of zeros
-  static constexpr int OFF_BAR = OFF_ONES + 2 * BLK;
+  // Y and its tail (ones or -delta, then zeros): 128 tokens, 128-byte swizzled rows, one 64-column group behind the other
+  static constexpr int OFF_T = REGION, OFF_XT = 2 * REGION, STAGE = (OFF_XT + 2 * KT_BOX + 1023) / 1024 * 1024;
+  static constexpr int OFF_BAR = STAGES * STAGE;
   static constexpr int SMEM_BYTES = OFF_BAR + 512 + 1024;
   static constexpr int LD = D + 4;
   static_assert((NB * (NB + 1) / 2) % 2 == 0, "whole tiles of two pair units");
@@ -37,8 +35,9 @@ struct Lay {
   static_assert(4 * CH * LD * 4 <= STAGES * STAGE, "the output rows are staged over the tiles");
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 };
-constexpr int B_FULL = 0, B_EMPTY = STAGES, B_SLOT = 2 * STAGES, B_FREE = B_SLOT + 3, B_DONE = B_FREE + 3, B_COUNT = B_DONE + 1;
-constexpr uint32_t COL_A = 320;   // behind four accumulators of 80 columns
+constexpr int B_FULL = 0, B_EMPTY = STAGES, B_SLOT = 2 * STAGES, B_FREE = B_SLOT + 3, B_DONE = B_FREE + 6, B_COUNT = B_DONE + 1;
+constexpr int NC = 80;            // accumulator columns of a tile: 64 of Y (narrow heads: zeros behind them), the tail, zeros
+constexpr uint32_t COL_A = 4 * NC;
 
 struct Params {
   float* out;          // [BH][state_rows][D + 4]; per_split: [BH][nsplit][state_rows][D + 4]
@@ -74,12 +73,15 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
   const int nc = c1 - c0;
 
   if (tid == 0) {
-    for (int i = 0; i < B_COUNT; ++i) mbar_init(&bars[i], (i >= B_SLOT && i < B_FREE) ? 16 : 1);
+    for (int i = 0; i < B_COUNT; ++i) mbar_init(&bars[i], (i >= B_SLOT && i < B_FREE) ? 8 : 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
-  for (int i = tid; i < 2 * CH; i += THREADS)   // (features of tokens past the last one are zero)
-    *reinterpret_cast<uint4*>(sm + L::OFF_ONES + i * 16) = make_uint4(i < CH ? 0x00003F80u : 0u, 0u, 0u, 0u);
+  if (!P.dop)   // the tail of [v | 1], the same in every stage (features of tokens past the last one are zero)
+    for (int i = tid; i < STAGES * CH * 8; i += THREADS) {
+      const int row = (i >> 3) % CH;
+      *reinterpret_cast<uint4*>(sm + i / (8 * CH) * STAGE + L::OFF_T + row * 128 + (i & 7) * 16) = make_uint4((i & 7) == (row & 7) ? 0x00003F80u : 0u, 0u, 0u, 0u);
+    }
   fence_proxy_async_smem();
   if (w == W_MMA) tmem_alloc(tmem_slot, 512);
   tc_fence_before_sync();
@@ -99,7 +101,7 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
       if (lane == 0) {
         uint8_t* st = sm + s * STAGE;
         const int tok = (c0 + i) * CH;
-        mbar_arrive_expect_tx(&bars[B_FULL + s], 2 * KT_BOX + REGION + (P.dop ? BLK : 0));
+        mbar_arrive_expect_tx(&bars[B_FULL + s], 2 * KT_BOX + (P.dop ? 2 : 1) * REGION);
         tma_load_4d(st, &tmy, &bars[B_FULL + s], 0, tok, h_idx, b_idx);
         if (P.dop) tma_load_4d(st + L::OFF_T, &tmt, &bars[B_FULL + s], D, tok, h_idx, b_idx);
         tma_load_3d(st + OFF_XT, &tmxt, &bars[B_FULL + s], tok, 0, head);
@@ -108,34 +110,28 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
       loaded = i + 1;
     }
   } else if (w == W_MMA) {
-    constexpr uint32_t ID = make_idesc_bf16(128, D, 0, 1), ID_T = make_idesc_bf16(128, 16, 0, 1);
-    const uint64_t dY = make_smem_desc(smem_u32(sm), REGION, 1024, 2);
-    const uint32_t zeros = smem_u32(sm + L::OFF_ONES + BLK);
+    constexpr uint32_t ID = make_idesc_bf16(128, NC, 0, 1);
+    const uint64_t dY = make_smem_desc(smem_u32(sm), L::OFF_T, 1024, 2);
     uint32_t k = 0;   // slabs so far
     for (int i = 0; i < nc; ++i) {
       const uint32_t s = (uint32_t)i % STAGES;
       WAIT(B_FULL + (int)s, (uint32_t)(i / STAGES), 111);
-      // tail operand: its block of eight columns, and the zeros a fixed distance behind it
-      const uint32_t tail = P.dop ? smem_u32(sm + s * STAGE + L::OFF_T) : smem_u32(sm + L::OFF_ONES);
-      const uint64_t dT = make_smem_desc(tail, 128, zeros - tail, 0);
       for (int t = 0; t < ntl; ++t, ++k) {
         const uint32_t slot = k % 3u;
         WAIT(B_SLOT + (int)slot, k / 3u, 112);
         tc_fence_after_sync();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t a = tmem + COL_A + 64u * slot + 8u * kk, acc = (i > 0 || kk > 0) ? 1u : 0u;
-          mma_ts_elect(tmem + L::NC * t, a, dY + (uint64_t)(s * (STAGE >> 4) + 128 * kk), ID, acc);
-          mma_ts_elect(tmem + L::NC * t + D, a, dT + (uint64_t)(16 * kk), ID_T, acc);
-        }
-        mma_commit_elect(&bars[B_FREE + slot]);
+        for (int kk = 0; kk < 8; ++kk)
+          mma_ts_elect(tmem + NC * t, tmem + COL_A + 64u * slot + 8u * kk, dY + (uint64_t)(s * (STAGE >> 4) + 128 * kk), ID, (i > 0 || kk > 0) ? 1u : 0u);
+        mma_commit_elect(&bars[B_FREE + (k + 3u) % 6u]);   // to the group that fills the slot next
       }
       mma_commit_elect(&bars[B_EMPTY + s]);
     }
     mma_commit_elect(&bars[B_DONE]);
     mbar_wait_bounded(&bars[B_DONE], 0, WAIT_CYCLES);   // (also after a failure: leave only after the products in flight)
   } else {
-    const int g = w >> 2, row = (w & 3) * 32 + lane;    // producer group = quarter of the chunk; feature row of a tile
+    const uint32_t group = (uint32_t)w >> 3;            // slabs take turns between the two groups
+    const int half = (w >> 2) & 1, row = (w & 3) * 32 + lane;   // 64 tokens of the chunk; feature row of a tile
     const uint32_t lane_addr = tmem + ((uint32_t)((w & 3) * 32) << 16);
     // byte offsets of the two factor rows of each tile's feature (16 bits each); b0 < 0: the linear tile
     const int f = row & 63;
@@ -147,50 +143,55 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
       rows[t] = (uint32_t)((8 * a + (f >> 3)) * s2::KT_ROW) | (uint32_t)((8 * b + (f & 7)) * s2::KT_ROW) << 16;
       if (tile0 + t == LIN) rows[t] = (uint32_t)((f & (D - 1)) * s2::KT_ROW) | (uint32_t)((f & (D - 1)) * s2::KT_ROW) << 16;
     }
-    uint32_t k = 0;
+    uint32_t k = 0;   // slabs so far, of both groups
     for (int i = 0; i < nc; ++i) {
       const int s = i % STAGES;
-      WAIT(B_FULL + s, (uint32_t)(i / STAGES), 113);
-      const uint8_t* box = sm + s * STAGE + OFF_XT + (g >> 1) * KT_BOX + (g & 1) * 64;
-      uint4 xa[4], xb[4];
-      auto load = [&](uint4 (&x)[4], uint32_t off) {
+      const uint8_t* box = sm + s * STAGE + OFF_XT + half * KT_BOX;
+      auto load = [&](uint4 (&x)[8], uint32_t off) {
         const uint4* p = reinterpret_cast<const uint4*>(box + off);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) x[c] = p[c];
+        for (int c = 0; c < 8; ++c) x[c] = p[c];
       };
-      load(xb, rows[0] >> 16);
+      uint4 xa[8];
+      uint32_t have = ~0u;   // the row in xa
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        if (t < ntl) {
-          uint32_t r[16];
-          if (tile0 + t < LIN) {
-            if (t == 0 || (rows[t] & 0xffffu) != (rows[t > 0 ? t - 1 : 0] & 0xffffu)) load(xa, rows[t] & 0xffffu);
+      for (int t = 0; t < 4; ++t, ++k) {
+        if (t >= ntl) break;
+        if ((k & 1u) != group) continue;
+        // (a group without a slab in this chunk does not wait for it: the stage may be filled again before it would look)
+        if (t < 2) WAIT(B_FULL + s, (uint32_t)(i / STAGES), 113);
+        uint32_t r[32];
+        {
+          uint4 xb[8];
+          load(xb, rows[t] >> 16);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              r[4 * c] = hmul2_u32(xa[c].x, xb[c].x);
-              r[4 * c + 1] = hmul2_u32(xa[c].y, xb[c].y);
-              r[4 * c + 2] = hmul2_u32(xa[c].z, xb[c].z);
-              r[4 * c + 3] = hmul2_u32(xa[c].w, xb[c].w);
-            }
-          } else if (row < D) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) { r[4 * c] = xb[c].x; r[4 * c + 1] = xb[c].y; r[4 * c + 2] = xb[c].z; r[4 * c + 3] = xb[c].w; }
-          } else {   // the constant feature (row D), zero for tokens past the last one, and nothing
-            const int left = row == D ? P.n - ((c0 + i) * CH + 32 * g) : 0;
-#pragma unroll
-            for (int c = 0; c < 16; ++c) r[c] = (2 * c < left ? 0x00003F80u : 0u) | (2 * c + 1 < left ? 0x3F800000u : 0u);
-          }
-          if (t + 1 < ntl) load(xb, rows[t < 3 ? t + 1 : 3] >> 16);   // in flight while this slab is handed over
-          const uint32_t slot = k % 3u;
-          if (k >= 3) WAIT(B_FREE + (int)slot, k / 3u - 1u, 114);
-          tc_fence_after_sync();
-          tmem_st16(lane_addr + COL_A + 64u * slot + 16u * g, r);
-          tmem_st_wait();
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars[B_SLOT + slot]);
-          ++k;
+          for (int c = 0; c < 8; ++c) { r[4 * c] = xb[c].x; r[4 * c + 1] = xb[c].y; r[4 * c + 2] = xb[c].z; r[4 * c + 3] = xb[c].w; }
         }
+        if (tile0 + t < LIN) {
+          if ((rows[t] & 0xffffu) != have) {
+            have = rows[t] & 0xffffu;
+            load(xa, have);
+          }
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            r[4 * c] = hmul2_u32(xa[c].x, r[4 * c]);
+            r[4 * c + 1] = hmul2_u32(xa[c].y, r[4 * c + 1]);
+            r[4 * c + 2] = hmul2_u32(xa[c].z, r[4 * c + 2]);
+            r[4 * c + 3] = hmul2_u32(xa[c].w, r[4 * c + 3]);
+          }
+        } else if (row >= D) {   // the constant feature (row D), zero for tokens past the last one, and nothing
+          const int left = row == D ? P.n - ((c0 + i) * CH + 64 * half) : 0;
+#pragma unroll
+          for (int c = 0; c < 32; ++c) r[c] = (2 * c < left ? 0x00003F80u : 0u) | (2 * c + 1 < left ? 0x3F800000u : 0u);
+        }
+        const uint32_t slot = k % 3u;
+        if (k >= 3) WAIT(B_FREE + (int)(k % 6u), k / 6u - (k % 6u < 3u ? 1u : 0u), 114);
+        tc_fence_after_sync();
+        tmem_st32(lane_addr + COL_A + 64u * slot + 32u * half, r);
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[B_SLOT + slot]);
       }
     }
     WAIT(B_DONE, 0, 115);
@@ -204,10 +205,10 @@ moments_kernel(const __grid_constant__ CUtensorMap tmxt, const __grid_constant__
     if (g < ntl) {
       float* stage = reinterpret_cast<float*>(sm) + g * CH * L::LD;
       const int row = (w & 3) * 32 + lane;
-      const uint32_t a = tmem + ((uint32_t)((w & 3) * 32) << 16) + (uint32_t)(L::NC * g);
+      const uint32_t a = tmem + ((uint32_t)((w & 3) * 32) << 16) + (uint32_t)(NC * g);
       float4* dst = reinterpret_cast<float4*>(stage + row * L::LD);
       uint32_t r[32], r8[8];
-      tmem_ld8(a + (uint32_t)D, r8);
+      tmem_ld8(a + 64u, r8);
 #pragma unroll
       for (int half = 0; half < D / 32; ++half) {
         tmem_ld32(a + 32u * half, r);

@@ -14,7 +14,7 @@ def host(t):
 
 
 @pytest.mark.parametrize("order,B,H,N", [(2, 1, 13, 1), (2, 1, 13, 129), (2, 2, 16, 640), (2, 1, 16, 4097), (2, 4, 40, 300),
-                                         (1, 1, 64, 1000), (1, 2, 100, 127)])
+                                         (1, 1, 64, 1000), (1, 2, 100, 127), (1, 1, 64, 40), (2, 1, 150, 1700)])
 @pytest.mark.parametrize("carried", [False, True])
 def test_state_only_calls_match_the_cuda_core_engine(order, B, H, N, carried):
     from reproducing_fastmax_results_b200 import _lib as L
