@@ -424,15 +424,16 @@ __global__ void norm_bwd_apply_vec_kernel(View y, View dy, View dx, int n, int h
 }
 
 // ---- one-launch variants: a thread-block cluster per (batch, head) ---------------------------------------------
-// gridDim = (CL, batch*heads, tensors) with CL blocks of 256 threads per cluster; q and k of a call go in one launch (two of
-// 1024 blocks each were 31 us for 128 heads of 1024 tokens, most of it the start and the end of a launch).  Pass 1: every block walks its share of the
+// gridDim = (CL, batch*heads, tensors) with CL blocks of 256 threads per cluster (norm_cluster_size); q and k of a call go in one
+// launch.  Bound by waves of short blocks up to some thousand tokens a head, beyond by memory (128 heads of 4096 x 64 bf16, backward:
+// 302 MB in 90 us; in two passes, which read 503 MB, 115).  Pass 1: every block walks its share of the
 // head's tokens and reduces (max squared norm / sum dy.y); the CL partial results meet through distributed shared
 // memory (each block reads its peers' partial after a cluster barrier, in rank order, so the sum does not depend on
-// timing).  Pass 2 walks the same tokens in the opposite order and writes the result; what it reads again comes from
-// L2 as far as the tensors in flight fit there.  No atomics, no zeroed scratch, one launch per direction.
-// (Measured against this form on B8 H16 N4096 D64 bf16, forward + backward, 0.113 ms: blocks of 1024 threads, one
-// per SM, that keep their loads in registers between the passes took 0.156 ms, since with one block per SM nothing
-// overlaps the barrier between the passes; fewer resident blocks of this form, for more L2 hits, took 0.119 ms.)
+// timing).  Forward, pass 2 walks the same tokens in the opposite order and writes the result; what it reads again comes from
+// L2 as far as the tensors in flight fit there.  Backward there is no second pass.  No atomics, no zeroed scratch, one launch per
+// direction.
+// (Measured on B8 H16 N4096 D64 bf16: blocks of 1024 threads, one per SM, that keep their loads in registers between the passes were
+// slower, since with one block per SM nothing overlaps the barrier; so were fewer resident blocks, for more L2 hits.)
 struct NormArgs {
   View x[2], y[2];
   int n[2];
@@ -544,16 +545,41 @@ __global__ void __launch_bounds__(256) norm_bwd_fused_vec_kernel(const NormBwdAr
   T* ob = reinterpret_cast<T*>(const_cast<void*>(dx.ptr)) + (long long)b * dx.sb + (long long)h * dx.sh;
   const int iters = (n + RPI * cl - 1) / (RPI * cl);
   const int lrow = (int)threadIdx.x / LPR, c = ((int)threadIdx.x - lrow * LPR) * 8;
+  const unsigned long long st = stats[head];
+  const float m = sqrtf(__uint_as_float((unsigned)(st >> 32)));
+  const int am = (int)(0xffffffffu - (unsigned)(st & 0xffffffffu));
+  const float sc = lim / m;
+  // One pass: the sum over the head enters the row of the maximum alone, so every other row is written as soon as it is read, and
+  // that one waits in the registers of the threads that met it.
+  bool mine_am = false;
+  float ka[8], kg[8];
   float q = 0.f;
 #pragma unroll 4
   for (int it = 0; it < iters; ++it) {
     const int l = (it * cl + rank) * RPI + lrow;
-    if (l < n) {
-      float a[8], g[8];
+    const bool valid = l < n;
+    float a[8], g[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = g[i] = 0.f;
+    if (valid) {
       load8<T>(yb + (long long)l * y.sn + c, a);
       load8<T>(gb + (long long)l * dy.sn + c, g);
 #pragma unroll
       for (int i = 0; i < 8; ++i) q += a[i] * g[i];
+    }
+    float sg = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sg += g[i];
+    const float gmean = row_sum<LPR>(sg) / (float)D;
+    if (valid && l == am) {
+      mine_am = true;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { ka[i] = a[i]; kg[i] = g[i] - gmean; }
+    } else if (valid) {
+      float o[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o[i] = sc * (g[i] - gmean) + 0.f * a[i];   // (a NaN of y stays one)
+      store8<T>(ob + (long long)l * dx.sn + c, o);
     }
   }
 #pragma unroll
@@ -571,33 +597,12 @@ __global__ void __launch_bounds__(256) norm_bwd_fused_vec_kernel(const NormBwdAr
     total = t;
   }
   __syncthreads();
-  const unsigned long long st = stats[head];
-  const float m = sqrtf(__uint_as_float((unsigned)(st >> 32)));
-  const int am = (int)(0xffffffffu - (unsigned)(st & 0xffffffffu));
-  const float sc = lim / m;
-  const float extra_am = -total / (lim * m);
-#pragma unroll 4
-  for (int it = iters - 1; it >= 0; --it) {
-    const int l = (it * cl + rank) * RPI + lrow;
-    const bool valid = l < n;
-    float a[8], g[8];
+  if (mine_am) {
+    const float extra = -total / (lim * m);
+    float o[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) a[i] = g[i] = 0.f;
-    if (valid) {
-      load8<T>(yb + (long long)l * y.sn + c, a);
-      load8<T>(gb + (long long)l * dy.sn + c, g);
-    }
-    float sg = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) sg += g[i];
-    const float gmean = row_sum<LPR>(sg) / (float)D;
-    if (valid) {
-      const float extra = (l == am) ? extra_am : 0.f;
-      float o[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = sc * (g[i] - gmean) + extra * a[i];
-      store8<T>(ob + (long long)l * dx.sn + c, o);
-    }
+    for (int i = 0; i < 8; ++i) o[i] = sc * kg[i] + extra * ka[i];
+    store8<T>(ob + (long long)am * dx.sn + c, o);
   }
   cluster.sync();
 }

@@ -905,15 +905,20 @@ static bool norm_vec_ok(int d, int dtype, std::initializer_list<const fastmax_te
     }                                                                                                   \
   } while (0)
 
-// One launch with a thread-block cluster per (batch, head).  Used when there are enough heads to fill the device
-// with such clusters; a few long heads keep the two-launch form, whose blocks spread over all tokens.
-static int norm_cluster_size(int batch, int heads, int n, int d) {
-  const long long bh = (long long)batch * heads;
-  const int rows_per_iter = 256 / (d / 8);
-  int cl = 8;
-  while (cl > 1 && n < cl * rows_per_iter * 2) cl /= 2;
-  if (bh * cl < 2LL * sm_count()) return 0;
-  return cl;
+// Blocks per (batch, head) of the one-launch form, or 0 for the two-launch form, whose blocks spread over all tokens.  heads: of all
+// the call's tensors.  Blocks of at least 256 rows at d = 64 in the forward, which reads them twice, and as few blocks as fill the
+// device in the backward, which is one pass and a barrier; more where heads are few.  us, forward / backward of two tensors for 1, 2,
+// 4, 8 blocks a head: 128 heads of 1024 x 64 bf16 24 / 35, 21 / 23, 21 / 27, 21 / 33; of 4096 x 64 159 / 138, 101 / 90, 78 / 92,
+// 72 / 97; 192 of 577 x 64 19 / 22, 19 / 24, 19 / 25, 25 / 35; 24 of 512 x 64 12 / 12, 9 / 8, 7 / 8, 7 / 7 (two launches a tensor 25 / 24).
+// Few long heads: a block walks up to 32 steps of 256 threads in less time than two more launches a tensor take.
+static int norm_cluster_size(long long heads, int n, int d, bool backward) {
+  const int rows = 256 / (d / 8);   // per step
+  const long long fill = 5LL * sm_count() / 2;
+  int cl = 1;
+  if (!backward)
+    while (cl < 8 && n >= 2 * cl * rows * 8) cl *= 2;
+  while (cl < 8 && heads * cl < fill && n >= 2 * cl * rows * 2) cl *= 2;
+  return heads * cl >= 2LL * sm_count() || n <= 32 * cl * rows ? cl : 0;
 }
 #define FM_NORM_FUSED(KERNEL, CL, COUNT, ...)                                                                  \
   do {                                                                                                  \
@@ -948,7 +953,7 @@ int32_t fastmax_normalize_forward(int32_t batch, int32_t heads, int32_t n, int32
   if (dtype != FASTMAX_F32 && dtype != FASTMAX_BF16) return FASTMAX_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   long long nrows = (long long)batch * heads * n;
-  const int cl = nrows > 0 && norm_vec_ok(d, dtype, {x, y}) && (long long)batch * heads <= 65535 ? norm_cluster_size(batch, heads, n, d) : 0;
+  const int cl = nrows > 0 && norm_vec_ok(d, dtype, {x, y}) && (long long)batch * heads <= 65535 ? norm_cluster_size((long long)batch * heads, n, d, false) : 0;
   if (cl == 0) FM_CUDA(cudaMemsetAsync(stats, 0, (size_t)batch * heads * sizeof(uint64_t), st));   // (the cluster kernel writes all of it)
   if (nrows == 0) return FASTMAX_OK;
   int threads = 256;
@@ -999,7 +1004,7 @@ int32_t fastmax_normalize_backward(int32_t batch, int32_t heads, int32_t n, int3
   if (dtype != FASTMAX_F32 && dtype != FASTMAX_BF16) return FASTMAX_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   long long nrows = (long long)batch * heads * n;
-  const int cl = nrows > 0 && norm_vec_ok(d, dtype, {y, dy, dx}) && (long long)batch * heads <= 65535 ? norm_cluster_size(batch, heads, n, d) : 0;
+  const int cl = nrows > 0 && norm_vec_ok(d, dtype, {y, dy, dx}) && (long long)batch * heads <= 65535 ? norm_cluster_size((long long)batch * heads, n, d, true) : 0;
   if (cl == 0) FM_CUDA(cudaMemsetAsync(scratch, 0, (size_t)batch * heads * sizeof(float), st));
   if (nrows == 0) return FASTMAX_OK;
   int threads = 256;
@@ -1048,7 +1053,7 @@ int32_t fastmax_normalize_forward_qk(int32_t batch, int32_t heads, int32_t nq, i
   const int most = nq > nk ? nq : nk;
   if (q && yq && k && yk && q->ptr && yq->ptr && k->ptr && yk->ptr && stats_q && stats_k && batch > 0 && heads > 0 && nq > 0 && nk > 0 && lim > 0.f &&
       (dtype == FASTMAX_F32 || dtype == FASTMAX_BF16) && norm_vec_ok(d, dtype, {q, yq, k, yk}) && (long long)batch * heads <= 65535) {
-    if (const int cl = norm_cluster_size(batch, heads, most, d)) {
+    if (const int cl = norm_cluster_size(2LL * batch * heads, most, d, false)) {
       cudaStream_t st = (cudaStream_t)stream;
       const NormArgs A{{to_view(*q), to_view(*k)}, {to_view(*yq), to_view(*yk)}, {(int)nq, (int)nk},
                        {reinterpret_cast<unsigned long long*>(stats_q), reinterpret_cast<unsigned long long*>(stats_k)}};
@@ -1068,7 +1073,7 @@ int32_t fastmax_normalize_backward_qk(int32_t batch, int32_t heads, int32_t nq, 
   if (yq && dyq && dxq && yk && dyk && dxk && yq->ptr && dyq->ptr && dxq->ptr && yk->ptr && dyk->ptr && dxk->ptr && stats_q && stats_k && batch > 0 &&
       heads > 0 && nq > 0 && nk > 0 && lim > 0.f && (dtype == FASTMAX_F32 || dtype == FASTMAX_BF16) &&
       norm_vec_ok(d, dtype, {yq, dyq, dxq, yk, dyk, dxk}) && (long long)batch * heads <= 65535) {
-    if (const int cl = norm_cluster_size(batch, heads, most, d)) {
+    if (const int cl = norm_cluster_size(2LL * batch * heads, most, d, true)) {
       cudaStream_t st = (cudaStream_t)stream;
       const NormBwdArgs A{{to_view(*yq), to_view(*yk)}, {to_view(*dyq), to_view(*dyk)}, {to_view(*dxq), to_view(*dxk)}, {(int)nq, (int)nk},
                           {reinterpret_cast<const unsigned long long*>(stats_q), reinterpret_cast<const unsigned long long*>(stats_k)}};
