@@ -122,6 +122,8 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  grid_wait();
+  grid_trigger();
   auto WAIT = [&](int bar, uint32_t phase, int code) { wait_inline(&bars[bar], phase & 1u, code, abort_flag); };
   auto next_item = [&](int n) -> int {
     const int c = n & (CLC - 1);
@@ -589,6 +591,8 @@ __device__ __forceinline__ void store_tail(__nv_bfloat16* out, long long plane, 
 template <int D>
 __global__ void __launch_bounds__(256) split_kernel(const SplitArgs A, int heads) {
   constexpr int TPR = D / 8;
+  grid_wait();
+  grid_trigger();
   const int t = blockIdx.z, head = blockIdx.y, b = head / heads, h = head - b * heads;
   const int row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, c = (threadIdx.x % TPR) * 8;
   if (row >= A.n[t]) return;
@@ -607,6 +611,8 @@ template <typename T, int D, bool VEC>
 __global__ void __launch_bounds__(256) prologue_f32_kernel(View dout, View o, View g, __nv_bfloat16* __restrict__ dop, float* __restrict__ ndelta,
                                                            int nq, int nd_ld, int heads, int ld) {
   constexpr int TPR = D / 8;
+  grid_wait();
+  grid_trigger();
   const int head = blockIdx.y, b = head / heads, h = head - b * heads;
   const int row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, c = (threadIdx.x % TPR) * 8;
   float v[8], dot = 0.f;

@@ -285,6 +285,8 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  grid_wait();
+  grid_trigger();
   auto WAIT = [&](int bar, uint32_t phase, int code) { wait_fast(&bars[bar], phase & 1u, code, abort_flag); };
   // item n + 1 of this block, for every role: -1 at the end (or when a wait ran out)
   auto next_item = [&](int n) -> int {
@@ -741,6 +743,8 @@ template <int D, bool VEC>
 __global__ void __launch_bounds__(256) prologue_kernel(View dout, View o, View g, __nv_bfloat16* __restrict__ dop, float* __restrict__ ndelta,
                                                        int nq, int nd_ld, int heads, int ld) {
   constexpr int TPR = D / 8;
+  grid_wait();
+  grid_trigger();
   const int head = blockIdx.y, b = head / heads, h = head - b * heads;
   const int row = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, c = (threadIdx.x % TPR) * 8;
   float dv[8], dot = 0.f;
@@ -797,6 +801,21 @@ void quotient(int d, uint32_t& mul, int& shift) {
   mul = (uint32_t)(((1ull << shift) + d - 1) / d);
 }
 
+// Launches `kernel`, which calls grid_wait() before it touches global memory, so that its blocks start while the kernel before it ends.
+template <typename... P, typename... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int threads, int bytes, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)bytes;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
 template <int D, int KIND, bool SQ>
 cudaError_t launch(const pair::Maps& M, const pair::Params& P, int bh, cudaStream_t st) {
   auto kernel = pair::pair_kernel<D, KIND, SQ>;
@@ -809,8 +828,7 @@ cudaError_t launch(const pair::Maps& M, const pair::Params& P, int bh, cudaStrea
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
   }
-  kernel<<<dim3((unsigned)(P.ntiles * bh)), pair::THREADS<D, KIND>, pair::SMEM_BYTES, st>>>(M, P);
-  return cudaGetLastError();
+  return launch_after(kernel, dim3((unsigned)(P.ntiles * bh)), pair::THREADS<D, KIND>, pair::SMEM_BYTES, st, M, P);
 }
 // Heads per group of the item order (decode).  With a mask, items differ in length: as many heads as have their streamed tiles in
 // 32 MB (pieces: 64 MB) of L2.  us forward / dq / dk, dv for 16, 32, 64, 128 MB: 128 heads of 4096 x 64 253 / 335 / 445,
@@ -1017,9 +1035,9 @@ static void launch_split(const fastmax_problem* pb, const pair::f32::SplitArgs& 
   const dim3 grid((unsigned)((n + rows - 1) / rows), (unsigned)(pb->batch * pb->heads), (unsigned)count);
   LaunchScope ls(KK_PAIR_SPLIT, st);
   switch (pb->d) {
-    case 16: pair::f32::split_kernel<16><<<grid, 256, 0, st>>>(A, pb->heads); break;
-    case 32: pair::f32::split_kernel<32><<<grid, 256, 0, st>>>(A, pb->heads); break;
-    default: pair::f32::split_kernel<64><<<grid, 256, 0, st>>>(A, pb->heads); break;
+    case 16: launch_after(pair::f32::split_kernel<16>, grid, 256, 0, st, A, pb->heads); break;
+    case 32: launch_after(pair::f32::split_kernel<32>, grid, 256, 0, st, A, pb->heads); break;
+    default: launch_after(pair::f32::split_kernel<64>, grid, 256, 0, st, A, pb->heads); break;
   }
 }
 template <int D, int KIND, int IN>
@@ -1035,8 +1053,7 @@ static cudaError_t launch_f32(const pair::Maps& M, const pair::Params& P, int bh
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
   }
-  kernel<<<dim3((unsigned)(P.ntiles * bh)), pair::f32::THREADS_F<KIND>, bytes, st>>>(M, P);
-  return cudaGetLastError();
+  return launch_after(kernel, dim3((unsigned)(P.ntiles * bh)), pair::f32::THREADS_F<KIND>, bytes, st, M, P);
 }
 template <int KIND>
 static cudaError_t launch_f32_d(const fastmax_problem* pb, const pair::Maps& M, pair::Params& P, cudaStream_t st) {
@@ -1106,9 +1123,9 @@ static void launch_prologue_f32(const fastmax_problem* pb, const fastmax_backwar
     return ((uintptr_t)t.ptr & 15) == 0 && (t.stride_b & odd) == 0 && (t.stride_h & odd) == 0 && (t.stride_n & odd) == 0;
   };
   if (vec(a->o) && vec(a->d_out))
-    pair::f32::prologue_f32_kernel<T, D, true><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+    launch_after(pair::f32::prologue_f32_kernel<T, D, true>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
   else
-    pair::f32::prologue_f32_kernel<T, D, false><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+    launch_after(pair::f32::prologue_f32_kernel<T, D, false>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
 }
 
 static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
@@ -1175,9 +1192,9 @@ static void launch_prologue(const fastmax_problem* pb, const fastmax_backward_ar
   const int ld = nd_ld(pb->nq), rows = 256 / (D / 8);
   const dim3 grid((unsigned)((ld + rows - 1) / rows), (unsigned)(pb->batch * pb->heads));
   if (rows16(a->o) && rows16(a->d_out))
-    pair::prologue_kernel<D, true><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+    launch_after(pair::prologue_kernel<D, true>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
   else
-    pair::prologue_kernel<D, false><<<grid, 256, 0, st>>>(view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+    launch_after(pair::prologue_kernel<D, false>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
 }
 static void launch_prologue_any(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
   LaunchScope ls(KK_PROLOGUE, st);
