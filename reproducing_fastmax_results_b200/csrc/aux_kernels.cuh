@@ -449,6 +449,8 @@ __global__ void __launch_bounds__(256) norm_fused_vec_kernel(const NormArgs A, i
   const View x = A.x[blockIdx.z], y = A.y[blockIdx.z];
   const int n = A.n[blockIdx.z];
   unsigned long long* stats = A.stats[blockIdx.z];
+  grid_wait();
+  grid_trigger();
   constexpr int D = 8 * LPR, RPI = 256 / LPR;
   namespace cgx = cooperative_groups;
   cgx::cluster_group cluster = cgx::this_cluster();
@@ -532,6 +534,8 @@ __global__ void __launch_bounds__(256) norm_bwd_fused_vec_kernel(const NormBwdAr
   const View y = A.y[blockIdx.z], dy = A.dy[blockIdx.z], dx = A.dx[blockIdx.z];
   const int n = A.n[blockIdx.z];
   const unsigned long long* stats = A.stats[blockIdx.z];
+  grid_wait();
+  grid_trigger();
   constexpr int D = 8 * LPR, RPI = 256 / LPR;
   namespace cgx = cooperative_groups;
   cgx::cluster_group cluster = cgx::this_cluster();

@@ -28,8 +28,10 @@ int report_cuda_error(cudaError_t e);
 namespace dec {
 
 constexpr int MAX_CL = 8;   // largest cluster: thread blocks that share one head
-constexpr int RG = 16;      // rows a block works on at a time
 constexpr int UNROLL = 4;   // rows a thread has in flight
+// RG: rows a block works on at a time.  Sixteen, or 48 where all blocks are on the SMs at once: a thread's rows are then one memory
+// latency per UNROLL of them behind one another (8 heads of 64 dims, 296 rows a block: five of them with 16). With the launch
+// behind the step before (grid_wait) 8 heads take 8.2 -> 6.4 us a step, where the host's call ends up; 512 heads 119.0 -> 117.3.
 
 struct DecodeParams {
   View q, k, v, o, g;
@@ -51,7 +53,7 @@ __device__ __forceinline__ float from_f<float>(float x) { return x; }
 template <>
 __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
 
-template <typename T, int D, int ORDER>
+template <typename T, int D, int ORDER, int RG>
 __global__ void __launch_bounds__(((D + 4) / 4) * RG)
 decode_step_kernel(const DecodeParams P) {
   using G = Geo<D>;
@@ -72,6 +74,14 @@ decode_step_kernel(const DecodeParams P) {
   const int head = blockIdx.y;
   const int bi = head / P.heads, hi = head - bi * P.heads;
 
+  if (ORDER == 2 && tid < G::NPAIRS) {
+    int a, b;
+    pair_decode(tid, G::NB, a, b);
+    tab_a[tid] = (unsigned char)a;
+    tab_b[tid] = (unsigned char)b;
+  }
+  grid_wait();   // the step before this one wrote the state
+  grid_trigger();
   if (tid < D) {
     const long long off_q = (long long)bi * P.q.sb + (long long)hi * P.q.sh;
     const long long off_k = (long long)bi * P.k.sb + (long long)hi * P.k.sh;
@@ -83,12 +93,6 @@ decode_step_kernel(const DecodeParams P) {
     float4 x = make_float4(1.f, 0.f, 0.f, 0.f);   // the ones column of [v | 1] and the padding
     if (tid < D / 4) x = make_float4(to_f<T>(vp[4 * tid]), to_f<T>(vp[4 * tid + 1]), to_f<T>(vp[4 * tid + 2]), to_f<T>(vp[4 * tid + 3]));
     sv[tid] = x;
-  }
-  if (ORDER == 2 && tid < G::NPAIRS) {
-    int a, b;
-    pair_decode(tid, G::NB, a, b);
-    tab_a[tid] = (unsigned char)a;
-    tab_b[tid] = (unsigned char)b;
   }
   __syncthreads();
 
@@ -186,25 +190,29 @@ decode_step_kernel(const DecodeParams P) {
   }
 }
 
-template <typename T, int D>
-static cudaError_t launch(int order, const DecodeParams& P, int bh, cudaStream_t st) {
-  constexpr int NT = ((D + 4) / 4) * RG;
-  int cl = 1;
-  while (cl < MAX_CL && (long long)cl * bh < 1024) cl *= 2;
+template <typename T, int D, int RG>
+static cudaError_t launch(int order, const DecodeParams& P, int bh, int cl, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cl, bh);
-  cfg.blockDim = dim3(NT);
+  cfg.blockDim = dim3(((D + 4) / 4) * RG);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = cl;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1] = launch_attribute_after();
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (order == 2) return cudaLaunchKernelEx(&cfg, decode_step_kernel<T, D, 2>, P);
-  return cudaLaunchKernelEx(&cfg, decode_step_kernel<T, D, 1>, P);
+  cfg.numAttrs = 2;
+  if (order == 2) return cudaLaunchKernelEx(&cfg, decode_step_kernel<T, D, 2, RG>, P);
+  return cudaLaunchKernelEx(&cfg, decode_step_kernel<T, D, 1, RG>, P);
+}
+template <typename T, int D>
+static cudaError_t launch(int order, const DecodeParams& P, int bh, cudaStream_t st) {
+  int cl = 1;
+  while (cl < MAX_CL && (long long)cl * bh < 1024) cl *= 2;
+  return (long long)cl * bh <= 148 ? launch<T, D, 48>(order, P, bh, cl, st) : launch<T, D, 16>(order, P, bh, cl, st);
 }
 
 template <typename T>

@@ -926,13 +926,14 @@ static int norm_cluster_size(long long heads, int n, int d, bool backward) {
     cfg.gridDim = dim3((unsigned)(CL), (unsigned)(batch * heads), (unsigned)(COUNT));                                      \
     cfg.blockDim = dim3(256);                                                                           \
     cfg.stream = st;                                                                                    \
-    cudaLaunchAttribute attr[1];                                                                        \
+    cudaLaunchAttribute attr[2];                                                                        \
     attr[0].id = cudaLaunchAttributeClusterDimension;                                                   \
     attr[0].val.clusterDim.x = (unsigned)(CL);                                                          \
     attr[0].val.clusterDim.y = 1;                                                                       \
     attr[0].val.clusterDim.z = 1;                                                                       \
+    attr[1] = launch_attribute_after();                                                                 \
     cfg.attrs = attr;                                                                                   \
-    cfg.numAttrs = 1;                                                                                   \
+    cfg.numAttrs = 2;                                                                                   \
     cudaError_t fe;                                                                                     \
     if (dtype == FASTMAX_F32) {                                                                         \
       if (d == 64) fe = cudaLaunchKernelEx(&cfg, KERNEL<float, 8>, __VA_ARGS__);                        \

@@ -801,21 +801,6 @@ void quotient(int d, uint32_t& mul, int& shift) {
   mul = (uint32_t)(((1ull << shift) + d - 1) / d);
 }
 
-// Launches `kernel`, which calls grid_wait() before it touches global memory, so that its blocks start while the kernel before it ends.
-template <typename... P, typename... A>
-cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int threads, int bytes, cudaStream_t st, const A&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = (size_t)bytes;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
 template <int D, int KIND, bool SQ>
 cudaError_t launch(const pair::Maps& M, const pair::Params& P, int bh, cudaStream_t st) {
   auto kernel = pair::pair_kernel<D, KIND, SQ>;

@@ -830,9 +830,8 @@ static int tc_p1_forward(const fastmax_problem* pb, const fastmax_forward_args* 
                      pb->heads, pb->nq, pb->nk, pb->a0, pb->a1 * pb->inv_temperature};
   {
     LaunchScope ls(KK_P1_FWD, st);
-    tc::p1::p1_forward_kernel<<<dim3(pb->batch * pb->heads), tc::p1::THREADS, tc::p1::SMEM_BYTES, st>>>(tmq, tmk, tmv, tmo, P);
+    e = launch_after(tc::p1::p1_forward_kernel, dim3(pb->batch * pb->heads), tc::p1::THREADS, tc::p1::SMEM_BYTES, st, tmq, tmk, tmv, tmo, P);
   }
-  e = cudaGetLastError();
   return e == cudaSuccess ? FASTMAX_OK : report_cuda_error(e);
 }
 

@@ -78,6 +78,8 @@ p1_forward_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  grid_wait();
+  grid_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
   auto WAIT = [&](int bar, uint32_t n) -> bool { return mbar_wait_abortable(&bars[bar], n & 1u, WAIT_CYCLES, abort_flag); };

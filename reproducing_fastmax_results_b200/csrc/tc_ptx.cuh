@@ -128,13 +128,6 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// ---- programmatic launches (pair_launchers.cuh, launch_after) ---------------------------------------------------------------
-// A kernel that is launched so starts while the one before it in the stream ends: nothing that one may have written is read, and
-// nothing that it may read is written, before grid_wait(), which returns when it is complete and its results are visible.
-// grid_trigger(): the next kernel's blocks may come as soon as every block of this one has started.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // ---- fences ------------------------------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
