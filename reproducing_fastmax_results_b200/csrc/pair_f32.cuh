@@ -10,11 +10,11 @@
 // for every streamed tile (64 rows: four additions of hi hi behind the twenty small ones, which go first) and the
 // element-wise warps add the tile's result to float32 totals in registers, rounding to nearest.
 //
-// Measured: 128 heads of 1024 x 64, causal, forward + backward with splitting 13400 us in the CUDA-core engine (FFMA), 528 here
-// (forward 114, dq 138, dk / dv 190, splitting 77, dO' 25); bf16, 128 heads of 1024 x 16 (q, k, v are one piece each: 1 or 3
+// Measured: 128 heads of 1024 x 64, causal, forward + backward with splitting 13400 us in the CUDA-core engine (FFMA), 520 here
+// (forward 110, dq 135, dk / dv 185, splitting 77, dO' 25); bf16, 128 heads of 1024 x 16 (q, k, v are one piece each: 1 or 3
 // products instead of 6, no pass that splits) 771 and 216.  Bound by the chain scores -> element-wise -> second products
 // between few warps (tensor pipe active in 51 to 65 % of the clocks at 64 dims, issue slots 30 %).  What took the forward from 131
-// to 114, dq from 156 to 138 and dk / dv from 216 to 190: scores in two blocks (product2), the results of a tile added up behind
+// to 110, dq from 156 to 135 and dk / dv from 216 to 185: scores in two blocks (product2), the results of a tile added up behind
 // the next tile's P instead of before it (dq: before its arithmetic, when its products have ended), rows written 16 bytes a
 // thread (one row per instruction, the warps that write dk and dv held up the next item for 7000 clocks), and the forward's held
 // tile of the next item loaded early.
