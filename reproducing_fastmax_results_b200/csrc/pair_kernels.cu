@@ -51,13 +51,16 @@ constexpr int W_SCORE = 0, W_ACC = 1, W_LOAD = 2, W_EW = 4;   // warp roles: two
 constexpr int X_BYTES = T * 128;        // operand tile: 128-byte rows whatever the head dim (narrow heads zero-filled by the copy engine)
 constexpr int STAGES = 4;               // ring of streamed tile pairs
 enum Kind { FWD = 0, DQ = 1, DKV = 2 };
-// Element-wise warps: sixteen, four per TMEM lane quarter (FWD: two 64-column halves of each held tile; else 32 columns).  A tile is a
-// chain of waits and TMEM accesses around some hundred instructions; with two warps per scheduler nothing ran beside it for half
-// of the time.  Eight -> sixteen (us): 128 heads of 2048 x 32 forward 68 -> 62, dq 84 -> 79, dk / dv 124 -> 111; 192 of 577 x 64
-// without a mask dk / dv 47 -> 44.  dq with 64 dims has three operations per score and keeps eight: 343 with sixteen, 335 with
-// eight (128 heads of 4096).
+// Element-wise warps: sixteen, four per TMEM lane quarter (32 columns each), in the backward kernels.  A tile is a chain of waits and
+// TMEM accesses around some hundred instructions; with two warps per scheduler nothing ran beside it for half of the time.  Eight ->
+// sixteen (us): 128 heads of 2048 x 32 dq 84 -> 79, dk / dv 124 -> 111; 192 of 577 x 64 without a mask dk / dv 47 -> 44.  dq with 64
+// dims has three operations per score and keeps eight: 343 with sixteen, 335 with eight (128 heads of 4096).  The forward has eight,
+// two per quarter, one per held tile, because a row's weights are added up there: one thread does it, in the order of the columns,
+// and every bit of g, which the outputs and gradients are divided by, stays what it is.  Sixteen warps with a row in two parts gave
+// other bits (240 -> 246, 31 -> 31, 33 -> 31, 68 -> 62 us: 128 heads of 4096 x 64, of 1024 x 64, 192 of 577 x 64, 128 of 2048 x 32);
+// sixteen with the same bits were no faster: four threads a row (16-lane loads) 261, 32, 33, 67; chains handed on 294, 36, 37, 80.
 template <int D, int KIND>
-constexpr int EW = KIND == DQ && D == 64 ? 8 : 16;
+constexpr int EW = KIND == FWD || (KIND == DQ && D == 64) ? 8 : 16;
 template <int D, int KIND>
 constexpr int THREADS = (W_EW + EW<D, KIND>) * 32;
 
@@ -170,27 +173,25 @@ constexpr int OFF_X = 4 * X_BYTES;
 constexpr int STAGE = 2 * X_BYTES;
 constexpr int OFF_ND = OFF_X + STAGES * STAGE;           // DKV: -delta of the streamed queries, T floats per stage
 constexpr int OFF_H = OFF_ND + STAGES * T * 4;              // SQ: two constant 128 x 16 operands whose product is h everywhere
-constexpr int OFF_SUM = OFF_H + 2 * R * 32;         // FWD: row sums of the second halves, of the last four items
-constexpr int OFF_CLC = OFF_SUM + 4 * 2 * R * 4;    // ring of 16-byte answers of the scheduler
+constexpr int OFF_CLC = OFF_H + 2 * R * 32;         // ring of 16-byte answers of the scheduler
 constexpr int CLC = 4;
 constexpr int OFF_BAR = OFF_CLC + 16 * CLC;
 constexpr int SMEM_BYTES = OFF_BAR + 512 + 1024;
 static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 // barrier slots
-constexpr int B_FULL = 0, B_EMPTY = 4, B_HFULL = 8, B_HEMPTY = 10, B_S = 12, B_READD = 18, B_P = 19, B_SFREE = 22, B_ACC = 25,
-              B_AFREE = 27, B_CFULL = 29, B_CEMPTY = B_CFULL + CLC, B_DRAIN = B_CEMPTY + CLC, B_COUNT = B_DRAIN + 2;
+constexpr int B_FULL = 0, B_EMPTY = 4, B_HFULL = 8, B_HEMPTY = 10, B_S = 12, B_READS = 14, B_READD = 16, B_P = 17, B_SFREE = 19, B_ACC = 21,
+              B_AFREE = 23, B_CFULL = 25, B_CEMPTY = B_CFULL + CLC, B_DRAIN = B_CEMPTY + CLC, B_COUNT = B_DRAIN + 2;
 static_assert(B_COUNT * 8 <= 384, "barriers and flags share 512 bytes");
-// TMEM columns.  Accumulators (FWD: O' of the two held tiles; DQ: dq; DKV: dv, dk), then score buffers of 128 columns that take
-// turns (FWD three, else two) and DQ, DKV: one of dP.  The bf16 A operands of the second products replace the scores that their
-// warp has read, 32 columns by 32 columns (FWD: 64 by 64): no two warps touch the same columns, and a buffer is free again when the
-// second products are done.  dP is free as soon as it has been read.
-constexpr uint32_t C_ACC = 0, C_ACC1 = 64, C_S = 128, C_DP = 384;
-template <int KIND>
-constexpr uint32_t NBUF = KIND == FWD ? 3u : 2u;
-// where K step kk (16 streamed rows) of P (FWD, DKV) or dS lies in its buffer
+// TMEM columns.  FWD: O' of the two held tiles, their scores, their bf16 tiles P, which have columns of their own: the scores are free
+// as soon as they have been read, and the next tile's first products run under this tile's arithmetic.  DQ, DKV: accumulators (dq; dv,
+// dk), two score buffers that take turns, dP.  The bf16 A operands of the second products replace the scores that their warp has
+// read, 32 columns by 32 columns: no two warps touch the same columns, and a buffer is free again when the second products are
+// done.  dP is free as soon as it has been read.
+constexpr uint32_t C_ACC = 0, C_ACC1 = 64, C_S = 128, C_DP = 384, C_P = 384;
+// where K step kk (16 streamed rows) of P (FWD, DKV) or dS lies
 template <int KIND>
 __device__ __forceinline__ constexpr uint32_t weights_at(int kk, bool ds) {
-  return KIND == FWD ? 64u * (kk >> 2) + 8u * (kk & 3) : 32u * (kk >> 1) + 8u * (kk & 1) + (KIND == DKV && ds ? 16u : 0u);
+  return KIND == FWD ? 8u * kk : 32u * (kk >> 1) + 8u * (kk & 1) + (KIND == DKV && ds ? 16u : 0u);
 }
 
 struct Item {
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
   constexpr int KS = D / 16;                    // K steps of the first products
   constexpr int HELD_ROWS = KIND == FWD ? 2 * R : R;
   constexpr int EWN = EW<D, KIND>, ROLES = EWN + 3;   // ROLES: warps that follow the items
-  constexpr int W = KIND == FWD ? 64 : 512 / EWN;     // columns of an element-wise warp
+  constexpr int W = KIND == FWD ? T : 512 / EWN;      // columns of an element-wise warp
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* sm = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
@@ -265,7 +266,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
   if (tid == 0) {
     for (int i = 0; i < B_COUNT; ++i) {
       uint32_t n = 1;
-      if (i >= B_READD && i < B_SFREE) n = KIND == FWD ? EWN / 2 : EWN;           // READD, P
+      if (i >= B_READS && i < B_SFREE) n = KIND == FWD ? EWN / 2 : EWN;           // READS, READD, P
       if (i == B_AFREE || i == B_AFREE + 1) n = KIND == DKV ? 8 : 4;
       if (i == B_HEMPTY || i == B_HEMPTY + 1) n = 1 + (KIND == DQ ? 4 : 8);     // products done, output rows staged there copied
       if (i >= B_CEMPTY && i < B_CEMPTY + CLC) n = ROLES;                       // every role has read the answer
@@ -358,7 +359,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
     const uint64_t dXk = make_smem_desc(smem_u32(sm + OFF_X), 16, 1024, 2);          // streamed tile, K-major
     const uint64_t dHa = make_smem_desc(smem_u32(sm + OFF_H), 128, 256, 0), dHb = make_smem_desc(smem_u32(sm + OFF_H + R * 32), 128, 256, 0);
     uint32_t tile = 0;            // streamed tiles so far
-    uint32_t buf = 0, use = 0;    // score buffer, times that it has been used
+    uint32_t cnt[2] = {0, 0};     // FWD: of each held tile
     int idx = blockIdx.x;
     for (int n = 0; idx >= 0; ++n) {
       const Item it = decode<KIND, T, HELD_ROWS>(idx, P);
@@ -372,7 +373,9 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
 #pragma unroll
         for (int m = 0; m < (KIND == FWD ? 2 : 1); ++m) {
           if (i < (m ? it.n1 : it.n0)) {
-            if (use > 0) WAIT(B_SFREE + (int)buf, use - 1u, 80);   // the second products that read this buffer are done
+            const uint32_t k = KIND == FWD ? cnt[m]++ : tile, buf = KIND == FWD ? (uint32_t)m : k & 1u;
+            if (KIND == FWD) { if (k > 0) WAIT(B_READS + m, k - 1u, 80); }               // the last scores have been read
+            else if (k >= 2) WAIT(B_SFREE + (int)buf, (k >> 1) - 1u, 80);   // the second products that read this buffer are done
             tc_fence_after_sync();
             const uint32_t c = tmem + C_S + buf * 128u;
             const bool add_h = SQ && !first_rows(P, it.r0 + m * R);
@@ -387,8 +390,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
               for (int ks = 0; ks < KS; ++ks)
                 mma_ss_elect(tmem + C_DP, dH + (uint64_t)((X_BYTES >> 4) + 2 * ks), dY + (uint64_t)(2 * ks), ID_S, ks > 0);
             }
-            mma_commit_elect(&bars[B_S + 3 * m + (int)buf]);
-            if (++buf == NBUF<KIND>) { buf = 0; ++use; }
+            mma_commit_elect(&bars[B_S + (int)buf]);
           }
         }
         ++tile;
@@ -404,7 +406,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
     // ================= issuer of the second products =================
     constexpr uint32_t ID_ACC = make_idesc_bf16(R, D, 0, 1);
     const uint64_t dXm = make_smem_desc(smem_u32(sm + OFF_X), X_BYTES, 1024, 2);     // streamed tile, MN-major
-    uint32_t tile = 0, buf = 0, use = 0;   // as above
+    uint32_t tile = 0, cnt[2] = {0, 0};   // as above
     uint32_t nfree[2] = {0, 0};   // items that have started on each accumulator
     int idx = blockIdx.x;
     for (int n = 0; idx >= 0; ++n) {
@@ -421,10 +423,11 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
               if (nfree[m] > 0) WAIT(B_AFREE + m, nfree[m] - 1u, 79);
               nfree[m]++;
             }
-            WAIT(B_P + (int)buf, use, 72);   // the bf16 tiles of the element-wise warps
+            const uint32_t k = KIND == FWD ? cnt[m]++ : tile, buf = KIND == FWD ? (uint32_t)m : k & 1u;
+            WAIT(B_P + (int)buf, KIND == FWD ? k : k >> 1, 72);   // the bf16 tiles of the element-wise warps
             tc_fence_after_sync();
             const uint32_t keep = i > 0 ? 1u : 0u;
-            const uint32_t a = tmem + C_S + buf * 128u;
+            const uint32_t a = tmem + (KIND == FWD ? C_P + buf * 64u : C_S + buf * 128u);
 #pragma unroll
             for (int kk = 0; kk < T / 16; ++kk)
               mma_ts_elect(tmem + C_ACC + 64u * m, a + weights_at<KIND>(kk, false), (KIND == DQ ? dX : dY) + (uint64_t)(128 * kk), ID_ACC, kk > 0 ? 1u : keep);
@@ -434,7 +437,6 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
                 mma_ts_elect(tmem + C_ACC1, a + weights_at<KIND>(kk, true), dX + (uint64_t)(128 * kk), ID_ACC, kk > 0 ? 1u : keep);
             }
             mma_commit_elect(&bars[B_SFREE + (int)buf]);
-            if (++buf == NBUF<KIND>) { buf = 0; ++use; }
             if (KIND != FWD || m == 1 || i >= it.n1) mma_commit_elect(&bars[B_EMPTY + s]);
             if (i == nm - 1) mma_commit_elect(&bars[B_ACC + m]);
           }
@@ -450,19 +452,16 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
   } else if (w >= W_EW) {
     // ================= element-wise warps =================
     const int we = w - W_EW, quarter = w & 3;
-    const int grp = KIND == FWD ? we >> 3 : 0;                  // FWD: held tile
-    const int part = KIND == FWD ? (we >> 2) & 1 : we >> 2;     // columns of the tile: halves, or quarters
+    const int grp = KIND == FWD ? we >> 2 : 0;    // FWD: held tile
+    const int part = KIND == FWD ? 0 : we >> 2;   // else: columns of the tile, in quarters or halves
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
     const uint64_t C0 = pack2(P.c0, P.c0), C1 = pack2(P.c1, P.c1), C2 = pack2(P.c2, P.c2), C22 = pack2(2.f * P.c2, 2.f * P.c2),
                    K = pack2(P.k, P.k);   // what a mode does not use is not computed
-    // which rows this warp writes out: FWD O' of its tile (part 0), DKV dv (part 0) and dk (part 1), DQ dq (part 0)
+    // which rows this warp writes out: FWD O' of its tile, DKV dv (part 0) and dk (part 1), DQ dq (part 0)
     const bool writes = part < (KIND == DKV ? 2 : 1);
-    float* const sums = reinterpret_cast<float*>(sm + OFF_SUM) + grp * R + quarter * 32 + lane;   // [item & 3][held tile][row]
     uint64_t sum[4] = {0ull, 0ull, 0ull, 0ull};   // FWD: four chains, one would serialise the additions
     uint64_t ND = 0ull;                           // DQ: -delta of this row
-    uint32_t tile = 0;       // streamed tiles so far
-    uint32_t buf = 0;        // score buffer of the next tile (FWD: of either group)
-    uint32_t phases = 0;     // per buffer: the phase that this group's next scores there complete
+    uint32_t k = 0;          // tiles of this warp's group so far
     uint32_t done = 0;       // items whose results this warp has written
     // Results of an item are written after the next item's first tile, whose products run meanwhile.
     auto results = [&](int n, const Item& it, float total) {
@@ -470,8 +469,6 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
       WAIT(B_ACC + grp, done, 75);
       ++done;
       tc_fence_after_sync();
-      // (written before the last second product was started)
-      if (KIND == FWD) total += sums[(n & 3) * 2 * R];
       constexpr int CH = 32;
       uint32_t r[D / CH][CH];
 #pragma unroll
@@ -547,7 +544,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
       }
     };
     bool pend = false;   // the last item's results are still to be written
-    float total = 0.f;   // FWD: this half's row sum of the last item
+    float total = 0.f;   // FWD: this row's sum of the last item
     Item last{};
     int idx = blockIdx.x, n = 0;
     for (; idx >= 0; ++n) {
@@ -560,18 +557,10 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
         const float nd = row < P.nr ? __ldg(P.ndelta + (long long)it.head * P.nd_ld + row) : 0.f;
         ND = pack2(nd, nd);
       }
-      const int tiles = it.n0 > it.n1 ? it.n0 : it.n1;
-      for (int i = 0; i < tiles; ++i, ++tile) {
-        if (KIND == FWD) {   // buffers go to the held tiles in turn
-          if (grp == 1 && i < it.n0) buf = buf == 2 ? 0 : buf + 1;
-          if (i >= nt) {
-            if (grp == 0) buf = buf == 2 ? 0 : buf + 1;
-            continue;
-          }
-        }
-        WAIT(B_S + 3 * grp + (int)buf, phases >> buf, 74);
-        phases ^= 1u << buf;
-        if (KIND == DKV) WAIT(B_FULL + (int)(tile & (STAGES - 1)), tile / STAGES, 81);
+      for (int i = 0; i < nt; ++i, ++k) {
+        const uint32_t buf = KIND == FWD ? (uint32_t)grp : k & 1u;
+        WAIT(B_S + (int)buf, KIND == FWD ? k : k >> 1, 74);
+        if (KIND == DKV) WAIT(B_FULL + (int)(k & (STAGES - 1)), k / STAGES, 81);
         tc_fence_after_sync();
         const int x0 = (it.t0 + i) * T + part * W;   // streamed row of this warp's first column
         // columns [lo, hi) of this row are visible
@@ -585,9 +574,12 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
         const bool whole = __all_sync(0xffffffffu, lo <= 0 && hi >= W);
         const uint32_t sa = lane_addr + C_S + buf * 128u + (uint32_t)(W * part);
         if (KIND == FWD) {
+          const uint32_t pa = lane_addr + C_P + 64u * grp;
           if (first) {   // general form, the sum of the rounded weights
+            if (k > 0) WAIT(B_SFREE + grp, k - 1u, 83);
+            tc_fence_after_sync();
 #pragma unroll 1
-            for (int c = 0; c < 2; ++c) {
+            for (int c = 0; c < 4; ++c) {
               uint32_t x32[32], pr[16];
               tmem_ld32(sa + 32u * c, x32);
               tmem_ld_wait();
@@ -599,15 +591,23 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
                 pr[j] = bf16x2(32 * c + 2 * j < hi ? p0 : 0.f, 32 * c + 2 * j + 1 < hi ? p1 : 0.f);
                 sum[j & 3] = add2(sum[j & 3], pack2u(pr[j] << 16, pr[j] & 0xffff0000u));
               }
-              tmem_st16(sa + 16u * c, pr);
+              tmem_st16(pa + 16u * c, pr);
             }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars[B_READS + grp]);
           } else {
-            uint32_t s[2][32];
+            uint32_t s[4][32];
 #pragma unroll
-            for (int c = 0; c < 2; ++c) tmem_ld32(sa + 32u * c, s[c]);
+            for (int c = 0; c < 4; ++c) tmem_ld32(sa + 32u * c, s[c]);
             tmem_ld_wait();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars[B_READS + grp]);
+            if (k > 0) WAIT(B_SFREE + grp, k - 1u, 83);   // the last tile's second product has read P
+            tc_fence_after_sync();
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            for (int c = 0; c < 4; ++c) {
               uint32_t pr[16];
               if (whole) {
 #pragma unroll
@@ -629,15 +629,14 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
                   pr[j] = bf16x2(p0, p1);
                 }
               }
-              tmem_st16(sa + 16u * c, pr);
+              tmem_st16(pa + 16u * c, pr);
             }
           }
           if (i == nt - 1) {
             float a, b;
             unpack2(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])), a, b);
             sum[0] = sum[1] = sum[2] = sum[3] = 0ull;
-            if (part == 0) next_total = a + b;
-            else sums[(n & 3) * 2 * R] = a + b;
+            next_total = a + b;
           }
         } else {
           constexpr int CW = W / 32;
@@ -655,7 +654,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
             constexpr bool Q = decltype(square)::value;
 #pragma unroll
             for (int c = 0; c < CW; ++c) {
-              const ulonglong2* ndp = reinterpret_cast<const ulonglong2*>(sm + OFF_ND + ((tile & (STAGES - 1)) * T + W * part + 32 * c) * 4);
+              const ulonglong2* ndp = reinterpret_cast<const ulonglong2*>(sm + OFF_ND + ((k & (STAGES - 1)) * T + W * part + 32 * c) * 4);
 #pragma unroll
               for (int j2 = 0; j2 < 8; ++j2) {
                 ulonglong2 n2;
@@ -693,12 +692,6 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[B_P + (int)buf]);
-        if (KIND == FWD) {   // (the second held tile's turn)
-          buf = buf == 2 ? 0 : buf + 1;
-          if (grp == 0 && i < it.n1) buf = buf == 2 ? 0 : buf + 1;
-        } else {
-          buf ^= 1u;
-        }
         if (i == 0 && pend) results(n - 1, last, total);
         if (i == 1 && pend) give_back(n - 1);
       }

@@ -210,3 +210,35 @@ def test_items_of_different_lengths_follow_one_another_on_a_block(case, dtype):
     for name, x, r in (("o", o, ref.detach()), ("dq", dq, grads[0]), ("dk", dk, grads[1]), ("dv", dv, grads[2])):
         err = (x.double() - r).norm(dim=(-1, -2)) / r.norm(dim=(-1, -2))
         assert float(err.max()) < tol, (name, float(err.max()), int(err.argmax()))
+
+
+@pytest.mark.parametrize("case", [(2, 70, 333, 333, 64, False, 2), (1, 3, 700, 700, 64, True, 2), (1, 2, 260, 1031, 32, False, 2),
+                                  (2, 90, 513, 513, 32, True, 2), (1, 4, 300, 300, 64, False, 1)])
+def test_row_sums_of_bf16_heads_are_added_in_a_fixed_order(case):
+    """g, which every gradient is divided by, does not depend on how many warps share a tile: a row's weights are added in four
+    chains of column pairs, whose two lanes meet last.  With scores of few bits all that is rounded is each weight and each
+    addition, so the bits of g are those of the same additions here."""
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    B, H, nq, nk, D, causal, order = case
+    g = torch.Generator(device="cuda").manual_seed(nq + nk)
+    mk = lambda n: (torch.randint(-64, 65, (B, H, n, D), device="cuda", generator=g) / 32.0).to(torch.bfloat16)
+    q, k, v = mk(nq), mk(nk), mk(nk)
+    it = 1.0 / 8.0
+    _, gg, _ = L.forward(q, k, v, causal, it, order=order, flags=L.FLAG_PAIRWISE)
+    L.check_status()
+    s = q.double() @ k.double().transpose(-1, -2)   # exact
+    if order == 2:   # 1 + s / 8 + s^2 / 128 = ((s + 8)^2 + 64) / 128: one rounding
+        p, scale = ((s + 8.0) ** 2 + 64.0).float(), 1.0 / 128.0
+    else:
+        p, scale = (1.0 + s * it).float(), 1.0
+    if causal:
+        p = p * torch.ones(nq, nk, device="cuda").tril(nk - nq)
+    p = torch.nn.functional.pad(p, (0, -nk % 8)).cpu().unflatten(-1, (-1, 4, 2)).numpy()   # [..., 8 columns, chain, lane]
+    sums = np.zeros(p.shape[:3] + (4, 2), np.float32)
+    for m in range(p.shape[3]):
+        sums += p[:, :, :, m]
+    total = (sums[..., 0, :] + sums[..., 1, :]) + (sums[..., 2, :] + sums[..., 3, :])
+    want = (total[..., 0] + total[..., 1]) * np.float32(scale)
+    first = 128 if causal else 0   # the first rows of a causal sequence sum rounded weights
+    assert np.array_equal(gg[:, :, first:].cpu().numpy(), want[:, :, first:])
