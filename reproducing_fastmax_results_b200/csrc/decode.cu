@@ -15,6 +15,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "../../include/fastmax_b200.h"
 #include "common.cuh"
 #include "launchers.cuh"
@@ -24,14 +26,19 @@ namespace cg = cooperative_groups;
 namespace fm {
 
 int report_cuda_error(cudaError_t e);
+int sm_count();
 
 namespace dec {
 
 constexpr int MAX_CL = 8;   // largest cluster: thread blocks that share one head
 constexpr int UNROLL = 4;   // rows a thread has in flight
-// RG: rows a block works on at a time.  Sixteen, or 48 where all blocks are on the SMs at once: a thread's rows are then one memory
-// latency per UNROLL of them behind one another (8 heads of 64 dims, 296 rows a block: five of them with 16). With the launch
-// behind the step before (grid_wait) 8 heads take 8.2 -> 6.4 us a step, where the host's call ends up; 512 heads 119.0 -> 117.3.
+// RG: rows a block works on at a time.  Sixteen, or 48 where a thread's rows are then fewer memory latencies behind one another (more
+// than 16 UNROLL rows a block) and all blocks run at once, one to an SM: 816 threads leave room for no more, and a cluster of eight
+// needs eight SMs of one GPC (fifteen such clusters fit).  us a step with 16 / 48 rows, order 2: d = 64, 8 heads 6.4 / 5.8, 15 heads
+// 6.5 / 5.9, 16 heads 7.7 / 10.7, 18 heads 7.7 / 10.9; d = 32, 8 heads 3.80 / 3.52, 18 heads 4.05 / 3.97, 32 heads 4.24 / 5.03; few
+// rows a block: d = 16, 8 heads 3.13 / 3.11, order 1, d = 64, 8 heads 3.25 / 3.84, 16 heads 3.3 / 6.3.  The partial sums of either are
+// added in an order of their own: float32 outputs may differ in their last bits between a call that takes 48 and one that takes 16.
+// Launched behind the step before (grid_wait), 8 heads take 8.2 -> 6.2 us a step, where the host's call ends up; 512 heads 117.8 -> 116.0.
 
 struct DecodeParams {
   View q, k, v, o, g;
@@ -190,14 +197,12 @@ decode_step_kernel(const DecodeParams P) {
   }
 }
 
-template <typename T, int D, int RG>
-static cudaError_t launch(int order, const DecodeParams& P, int bh, int cl, cudaStream_t st) {
-  cudaLaunchConfig_t cfg = {};
+template <int D, int RG>
+static void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int bh, int cl, cudaStream_t st) {
   cfg.gridDim = dim3(cl, bh);
   cfg.blockDim = dim3(((D + 4) / 4) * RG);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
-  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = cl;
   attr[0].val.clusterDim.y = 1;
@@ -205,14 +210,43 @@ static cudaError_t launch(int order, const DecodeParams& P, int bh, int cl, cuda
   attr[1] = launch_attribute_after();
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  if (order == 2) return cudaLaunchKernelEx(&cfg, decode_step_kernel<T, D, 2, RG>, P);
-  return cudaLaunchKernelEx(&cfg, decode_step_kernel<T, D, 1, RG>, P);
+}
+template <typename T, int D, int ORDER, int RG>
+static cudaError_t launch(const DecodeParams& P, int bh, int cl, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  configure<D, RG>(cfg, attr, bh, cl, st);
+  return cudaLaunchKernelEx(&cfg, decode_step_kernel<T, D, ORDER, RG>, P);
+}
+// clusters of MAX_CL blocks of the 48-row kernel that the current device runs at once
+template <typename T, int D>
+static int clusters_at_once() {
+  static std::atomic<int> cached[64];   // + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = cached[dev].load(std::memory_order_relaxed) - 1;
+  if (n < 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    configure<D, 48>(cfg, attr, 1, MAX_CL, nullptr);
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, decode_step_kernel<T, D, 2, 48>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    cached[dev].store(n + 1, std::memory_order_relaxed);
+  }
+  return n;
 }
 template <typename T, int D>
 static cudaError_t launch(int order, const DecodeParams& P, int bh, cudaStream_t st) {
   int cl = 1;
   while (cl < MAX_CL && (long long)cl * bh < 1024) cl *= 2;
-  return (long long)cl * bh <= 148 ? launch<T, D, 48>(order, P, bh, cl, st) : launch<T, D, 16>(order, P, bh, cl, st);
+  // (order 1 and D = 16 have at most 9 and 27 rows a block where the cluster is that large)
+  if constexpr (D > 16)
+    if (order == 2 && cl == MAX_CL && (P.rows + cl - 1) / cl > 16 * UNROLL && cl * bh <= sm_count() && bh <= clusters_at_once<T, D>())
+      return launch<T, D, 2, 48>(P, bh, cl, st);
+  return order == 2 ? launch<T, D, 2, 16>(P, bh, cl, st) : launch<T, D, 1, 16>(P, bh, cl, st);
 }
 
 template <typename T>

@@ -57,7 +57,7 @@ static const char* kKindNames[KK_COUNT] = {
     "pair_fwd", "pair_bwd_q", "pair_bwd_kv", "pair_f32_fwd", "pair_f32_bwd_q", "pair_f32_bwd_kv", "pair_split",
     "window_pack", "window_fwd", "window_bwd_q", "window_bwd_k", "window_bwd_v"};
 
-static int sm_count() {
+int sm_count() {
   static int cached[64] = {0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;

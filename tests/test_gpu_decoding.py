@@ -219,3 +219,29 @@ def test_step_into_an_output_of_either_rank():
         assert dec.step(*token, out=out) is out
         outs.append(out.reshape(2, 4, 32))
     assert float(outs[0].abs().max()) > 0 and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", [16, 32, 64])
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("heads", [4, 15, 19, 300, 600, 1030])   # 48 and 16 rows at a time; clusters of 8, 8, 8, 4, 2 and 1 blocks
+def test_decode_at_every_cluster_size(heads, order, D, dtype):
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    T = 3
+    g = torch.Generator(device="cuda").manual_seed(heads + D)
+    q, k, v = (torch.randn(1, heads, T, D, device="cuda", generator=g).to(dtype) for _ in range(3))
+    poly = orc.Poly(0.9, 1.1, 0.45, 1.0 / (2.0 * math.sqrt(D)), order)
+    state = L.new_state(1, heads, D, order)
+    outs, gs = [], []
+    for t in range(T):
+        o, gg = L.decode_step(q[:, :, t], k[:, :, t], v[:, :, t], state, poly.inv_temp, poly.a0, poly.a1, poly.a2, order)
+        outs.append(o)
+        gs.append(gg)
+    some = sorted({0, 1, heads // 2, heads - 1})
+    o_ref, g_ref = orc.fastmax_naive(*(host(t[:, some]) for t in (q, k, v)), True, poly)
+    # float32 sums of up to 2369 terms in at least 16 partial sums a block; bf16: one rounding of the output (2^-9)
+    assert orc.max_norm_err(host(torch.stack(outs, 2)[:, some]), o_ref) < (1e-5 if dtype == torch.float32 else 4e-3)
+    assert orc.max_norm_err(host(torch.stack(gs, 2)[:, some]), g_ref) < 1e-5
+    for h in some:
+        assert orc.max_norm_err(host(state[0, h, :, : D + 1]), exchange_state(host(k[0, h]), host(v[0, h]), order)) < 1e-6
