@@ -26,6 +26,11 @@ inline cudaLaunchAttribute launch_attribute_after() {
   a.val.programmaticStreamSerializationAllowed = 1;
   return a;
 }
+// The code of a refused launch also stays in the runtime's last-error slot, where the next check would take it for its own: out with it.
+inline cudaError_t launched(cudaError_t e) {
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
 // Launches `kernel`, which calls grid_wait() before it touches global memory, so that its blocks start while the kernel before it ends.
 template <typename... P, typename... A>
 inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int threads, int bytes, cudaStream_t st, const A&... args) {
@@ -37,7 +42,7 @@ inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int threads, in
   cudaLaunchAttribute attr = launch_attribute_after();
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+  return launched(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
 template <int D>

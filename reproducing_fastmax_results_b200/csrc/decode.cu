@@ -216,7 +216,7 @@ static cudaError_t launch(const DecodeParams& P, int bh, int cl, cudaStream_t st
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   configure<D, RG>(cfg, attr, bh, cl, st);
-  return cudaLaunchKernelEx(&cfg, decode_step_kernel<T, D, ORDER, RG>, P);
+  return launched(cudaLaunchKernelEx(&cfg, decode_step_kernel<T, D, ORDER, RG>, P));
 }
 // clusters of MAX_CL blocks of the 48-row kernel that the current device runs at once
 template <typename T, int D>

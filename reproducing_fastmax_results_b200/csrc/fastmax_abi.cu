@@ -944,7 +944,7 @@ static int norm_cluster_size(long long heads, int n, int d, bool backward) {
       else if (d == 32) fe = cudaLaunchKernelEx(&cfg, KERNEL<__nv_bfloat16, 4>, __VA_ARGS__);           \
       else fe = cudaLaunchKernelEx(&cfg, KERNEL<__nv_bfloat16, 2>, __VA_ARGS__);                        \
     }                                                                                                   \
-    FM_CUDA(fe);                                                                                        \
+    FM_CUDA(launched(fe));                                                                                        \
   } while (0)
 
 int32_t fastmax_normalize_forward(int32_t batch, int32_t heads, int32_t n, int32_t d, int32_t dtype, float lim,

@@ -1006,16 +1006,16 @@ static bool pieces_map(CUtensorMap* m, void* p, const fastmax_problem* pb, int n
   const fastmax_tensor t{(__nv_bfloat16*)p + (int64_t)first * ld, bh * n * ld, (int64_t)n * ld, ld};
   return tc_make_map(m, t, 3, (int)bh, n - first, 64, rows, true, cols > 0 ? cols : pb->d);
 }
-static void launch_split(const fastmax_problem* pb, const pair::f32::SplitArgs& A, int count, cudaStream_t st) {
+static cudaError_t launch_split(const fastmax_problem* pb, const pair::f32::SplitArgs& A, int count, cudaStream_t st) {
   int n = A.n[0];
   for (int i = 1; i < count; ++i) n = A.n[i] > n ? A.n[i] : n;
   const int rows = 256 / (pb->d / 8);
   const dim3 grid((unsigned)((n + rows - 1) / rows), (unsigned)(pb->batch * pb->heads), (unsigned)count);
   LaunchScope ls(KK_PAIR_SPLIT, st);
   switch (pb->d) {
-    case 16: launch_after(pair::f32::split_kernel<16>, grid, 256, 0, st, A, pb->heads); break;
-    case 32: launch_after(pair::f32::split_kernel<32>, grid, 256, 0, st, A, pb->heads); break;
-    default: launch_after(pair::f32::split_kernel<64>, grid, 256, 0, st, A, pb->heads); break;
+    case 16: return launch_after(pair::f32::split_kernel<16>, grid, 256, 0, st, A, pb->heads);
+    case 32: return launch_after(pair::f32::split_kernel<32>, grid, 256, 0, st, A, pb->heads);
+    default: return launch_after(pair::f32::split_kernel<64>, grid, 256, 0, st, A, pb->heads);
   }
 }
 template <int D, int KIND, int IN>
@@ -1065,9 +1065,8 @@ static bool input_map(CUtensorMap* m, const fastmax_tensor& t, void* pieces, con
 static cudaError_t split_inputs(const fastmax_problem* pb, const fastmax_tensor& q, const fastmax_tensor& k, const fastmax_tensor& v, void* qp, void* kp, void* vp,
                                 cudaStream_t st) {
   if (pb->dtype != FASTMAX_F32) return cudaSuccess;
-  launch_split(pb, pair::f32::SplitArgs{{view_of(q), view_of(k), view_of(v)}, {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp},
-                                        {pb->nq, pb->nk, pb->nk}, {pb->d, pb->d, pb->d}}, 3, st);
-  return cudaGetLastError();
+  return launch_split(pb, pair::f32::SplitArgs{{view_of(q), view_of(k), view_of(v)}, {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp},
+                                               {pb->nq, pb->nk, pb->nk}, {pb->d, pb->d, pb->d}}, 3, st);
 }
 static int pair_f32_forward(const fastmax_problem* pb, const fastmax_forward_args* a, void* ws, cudaStream_t st) {
   char* base = (char*)ws;
@@ -1093,7 +1092,7 @@ static int pair_f32_forward(const fastmax_problem* pb, const fastmax_forward_arg
 }
 
 template <typename T, int D>
-static void launch_prologue_f32(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
+static cudaError_t launch_prologue_f32(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
   const int ld = nd_ld(pb->nq), rows = 256 / (D / 8);
   const dim3 grid((unsigned)((ld + rows - 1) / rows), (unsigned)(pb->batch * pb->heads));
   auto vec = [](const fastmax_tensor& t) {
@@ -1101,9 +1100,8 @@ static void launch_prologue_f32(const fastmax_problem* pb, const fastmax_backwar
     return ((uintptr_t)t.ptr & 15) == 0 && (t.stride_b & odd) == 0 && (t.stride_h & odd) == 0 && (t.stride_n & odd) == 0;
   };
   if (vec(a->o) && vec(a->d_out))
-    launch_after(pair::f32::prologue_f32_kernel<T, D, true>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
-  else
-    launch_after(pair::f32::prologue_f32_kernel<T, D, false>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+    return launch_after(pair::f32::prologue_f32_kernel<T, D, true>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+  return launch_after(pair::f32::prologue_f32_kernel<T, D, false>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
 }
 
 static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_args* a, void* ws, cudaStream_t st) {
@@ -1123,12 +1121,11 @@ static int pair_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   {
     LaunchScope ls(KK_PROLOGUE, st);
     __nv_bfloat16* dop = (__nv_bfloat16*)dp;
-    if (pb->dtype == FASTMAX_BF16) launch_prologue_f32<__nv_bfloat16, 16>(pb, a, dop, nd, pb->d, st);
-    else if (pb->d == 16) launch_prologue_f32<float, 16>(pb, a, dop, nd, pb->d, st);
-    else if (pb->d == 32) launch_prologue_f32<float, 32>(pb, a, dop, nd, pb->d, st);
-    else launch_prologue_f32<float, 64>(pb, a, dop, nd, pb->d, st);
+    if (pb->dtype == FASTMAX_BF16) e = launch_prologue_f32<__nv_bfloat16, 16>(pb, a, dop, nd, pb->d, st);
+    else if (pb->d == 16) e = launch_prologue_f32<float, 16>(pb, a, dop, nd, pb->d, st);
+    else if (pb->d == 32) e = launch_prologue_f32<float, 32>(pb, a, dop, nd, pb->d, st);
+    else e = launch_prologue_f32<float, 64>(pb, a, dop, nd, pb->d, st);
   }
-  e = cudaGetLastError();
   if (e != cudaSuccess) return report_cuda_error(e);
   pair::Params P{};
   fill(pb, P);
@@ -1166,18 +1163,16 @@ static int out_map(CUtensorMap* m, const fastmax_tensor& t, const fastmax_proble
 }
 
 template <int D>
-static void launch_prologue(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
+static cudaError_t launch_prologue(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
   const int ld = nd_ld(pb->nq), rows = 256 / (D / 8);
   const dim3 grid((unsigned)((ld + rows - 1) / rows), (unsigned)(pb->batch * pb->heads));
   if (rows16(a->o) && rows16(a->d_out))
-    launch_after(pair::prologue_kernel<D, true>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
-  else
-    launch_after(pair::prologue_kernel<D, false>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+    return launch_after(pair::prologue_kernel<D, true>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
+  return launch_after(pair::prologue_kernel<D, false>, grid, 256, 0, st, view_of(a->d_out), view_of(a->o), view_of(a->g), dop, nd, pb->nq, ld, pb->heads, dld);
 }
-static void launch_prologue_any(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
+static cudaError_t launch_prologue_any(const fastmax_problem* pb, const fastmax_backward_args* a, __nv_bfloat16* dop, float* nd, int dld, cudaStream_t st) {
   LaunchScope ls(KK_PROLOGUE, st);
-  if (pb->d == 32) launch_prologue<32>(pb, a, dop, nd, dld, st);
-  else launch_prologue<64>(pb, a, dop, nd, dld, st);
+  return pb->d == 32 ? launch_prologue<32>(pb, a, dop, nd, dld, st) : launch_prologue<64>(pb, a, dop, nd, dld, st);
 }
 
 // ---- long bf16 sequences (long_kernels.cuh) -----------------------------------------------------------------------------
@@ -1374,8 +1369,7 @@ static int long_backward(const fastmax_problem* pb, const fastmax_backward_args*
   if (pb->causal && (!f32_map(&M.p0, pq, pb, pb->nq, 32) || !f32_map(&N.p0, pk, pb, pb->nk, 32) || !f32_map(&N.p1, pv, pb, pb->nk, 32) ||
                      !f32_map(&Q.part, pq, pb, pb->nq, 128) || !f32_map(&K.part, pk, pb, pb->nk, 128) || !f32_map(&V.part, pv, pb, pb->nk, 128)))
     return FASTMAX_ERR_UNSUPPORTED;
-  launch_prologue_any(pb, a, dop, nd, ld, st);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_prologue_any(pb, a, dop, nd, ld, st);
   if (e != cudaSuccess) return report_cuda_error(e);
   if (pb->causal) {
     pair::Params P{};
@@ -1505,9 +1499,8 @@ static int long_f32_forward(const fastmax_problem* pb, const fastmax_forward_arg
     return FASTMAX_ERR_UNSUPPORTED;
   M.b = M.o0 = M.o1 = M.p0 = M.p1 = M.a;
   A.y = A.x;
-  launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
-                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {n, n, n}, {pb->d, pb->d, lng::f32::NC}}, 3, st);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
+                                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {n, n, n}, {pb->d, pb->d, lng::f32::NC}}, 3, st);
   if (e != cudaSuccess) return report_cuda_error(e);
   {
     pair::Params P{};
@@ -1554,13 +1547,12 @@ static int long_f32_backward(const fastmax_problem* pb, const fastmax_backward_a
   M.o0 = M.o1 = M.p0 = M.p1 = N.o0 = N.o1 = N.p0 = N.p1 = M.a;
   V.x = K.x;
   V.y = K.y;
-  launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
-                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {n, n, n}, {pb->d, pb->d, NC}}, 3, st);
-  {
+  cudaError_t e = launch_split(pb, pair::f32::SplitArgs{{view_of(a->q), view_of(a->k), view_of(a->v)},
+                                                        {(__nv_bfloat16*)qp, (__nv_bfloat16*)kp, (__nv_bfloat16*)vp}, {n, n, n}, {pb->d, pb->d, NC}}, 3, st);
+  if (e == cudaSuccess) {
     LaunchScope ls(KK_PROLOGUE, st);
-    launch_prologue_f32<float, 32>(pb, a, (__nv_bfloat16*)dp, nd, NC, st);
+    e = launch_prologue_f32<float, 32>(pb, a, (__nv_bfloat16*)dp, nd, NC, st);
   }
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return report_cuda_error(e);
   pair::Params P{};
   fill(pb, P);
@@ -1646,8 +1638,7 @@ int pair_backward(const fastmax_problem* pb, const fastmax_backward_args* a, voi
   M.o0 = M.o1 = M.a;
   pair::Maps N;   // dk, dv: the other way round (held and streamed tiles have the same 128-row box)
   N.x = M.a; N.y = M.b; N.a = M.x; N.b = M.y; N.o0 = N.o1 = M.a;
-  launch_prologue_any(pb, a, dop, nd, pb->d, st);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_prologue_any(pb, a, dop, nd, pb->d, st);
   if (e != cudaSuccess) return report_cuda_error(e);
   pair::Params P{};
   const bool sq = fill(pb, P);

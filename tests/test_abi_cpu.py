@@ -203,3 +203,31 @@ def test_ctypes_structures_match_the_c_header(tmp_path):
             _lib.BackwardArgs.dstate_out.offset, _lib.BackwardArgs.grad_moments_out.offset,
             _lib.Problem.inv_temperature.offset, _lib.DecodeArgs.state.offset]
     assert got == want
+
+
+def test_a_refused_launch_leaves_no_error_for_the_next_call(tmp_path):
+    """launch_after() reports a launch that the runtime refuses (here a stand-in, which keeps the code as the runtime does) and
+    leaves nothing in the last-error slot, which the checks behind other launches read."""
+    import subprocess
+
+    from reproducing_fastmax_results_b200 import build
+
+    if not os.path.exists(build.NVCC):
+        pytest.skip("no nvcc")
+    src = tmp_path / "refused.cu"
+    src.write_text(
+        "#include <cuda_bf16.h>\n#include <cuda_runtime.h>\n#include <stdio.h>\n"
+        "static cudaError_t slot = cudaSuccess;\n"
+        "template <typename... A> static cudaError_t refuse(A...) { return slot = cudaErrorInvalidConfiguration; }\n"
+        "static cudaError_t last_error() { const cudaError_t e = slot; slot = cudaSuccess; return e; }\n"
+        "#define cudaLaunchKernelEx refuse\n#define cudaGetLastError last_error\n"
+        '#include "common.cuh"\n'
+        "__global__ void kernel(int) {}\n"
+        "int main() {\n"
+        "  const cudaError_t e = fm::launch_after(kernel, dim3(1), 32, 0, nullptr, 1);\n"
+        '  printf("%d %d\\n", (int)e, (int)slot);\n'
+        "  return 0;\n}\n")
+    exe = tmp_path / "refused"
+    subprocess.run([build.NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-I", build.CSRC, str(src), "-o", str(exe)], check=True,
+                   capture_output=True)
+    assert subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split() == ["9", "0"]
