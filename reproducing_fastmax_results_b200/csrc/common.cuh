@@ -16,6 +16,8 @@ namespace fm {
 // ---- programmatic launches ------------------------------------------------------------------------------------------------
 // A kernel that is launched so starts while the one before it in the stream ends: nothing that one may have written is read, and
 // nothing that it may read is written, before grid_wait(), which returns when it is complete and its results are visible.
+// Behind it, too, such a kernel reads by ordinary loads or the copy engine, not through the read-only path (__ldg): that takes memory
+// which nothing writes while the kernel runs, and the kernel before may still write when this one's first blocks start.
 // grid_trigger(): the next kernel's blocks may come as soon as every block of this one has got so far; it stands behind a block's
 // allocation of tensor memory, so no block of this kernel waits for one of the next.  About 3 us between two dependent kernels.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

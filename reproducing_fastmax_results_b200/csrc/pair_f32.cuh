@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(THREADS_F<KIND>, 1) pair_f32_kernel(const __gr
         const int row = it.r0 + quarter * 32 + lane;
         uint64_t ND = 0ull;
         if (KIND == DQ) {
-          const float nd = row < P.nr ? __ldg(P.ndelta + (long long)it.head * P.nd_ld + row) : 0.f;
+          const float nd = row < P.nr ? P.ndelta[(long long)it.head * P.nd_ld + row] : 0.f;
           ND = pack2(nd, nd);
         }
         float total = 0.f;   // FWD: this half's row sum

@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
       const bool first = first_rows(P, it.r0 + grp * R);
       float next_total = 0.f;
       if (KIND == DQ) {
-        const float nd = row < P.nr ? __ldg(P.ndelta + (long long)it.head * P.nd_ld + row) : 0.f;
+        const float nd = row < P.nr ? P.ndelta[(long long)it.head * P.nd_ld + row] : 0.f;
         ND = pack2(nd, nd);
       }
       for (int i = 0; i < nt; ++i, ++k) {

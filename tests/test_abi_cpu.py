@@ -231,3 +231,23 @@ def test_a_refused_launch_leaves_no_error_for_the_next_call(tmp_path):
     subprocess.run([build.NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-I", build.CSRC, str(src), "-o", str(exe)], check=True,
                    capture_output=True)
     assert subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split() == ["9", "0"]
+
+
+def test_kernels_that_start_early_do_not_read_through_the_read_only_path():
+    """A kernel that waits for the one before it (grid_wait) runs while that one still writes: loads that assume memory nothing
+    writes during the kernel (__ldg, ld.global.nc, const __restrict__ parameters) are not for it."""
+    from reproducing_fastmax_results_b200 import build
+
+    found = 0
+    for name in sorted(os.listdir(build.CSRC)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(build.CSRC, name)).read())
+        for start in (m.start() for m in re.finditer(r"__global__", text)):
+            end = text.find("\n}\n", start)
+            kernel = text[start:end]
+            if "grid_wait();" not in kernel:
+                continue
+            found += 1
+            assert not re.search(r"__ldg\(|ld\.global\.nc|const [\w ]+\*\s*__restrict__", kernel), (name, kernel[:200])
+    assert found >= 9
