@@ -229,7 +229,8 @@ int32_t fastmax_normalize_backward(int32_t batch, int32_t heads, int32_t n, int3
                                    const fastmax_tensor* dx, const uint64_t* stats, float* scratch_bh,
                                    void* cuda_stream);
 
-/* The same for the queries and the keys of a call, in one launch where both are large enough. */
+/* The same for the queries and the keys of a call, in one launch where their shapes allow it; one after the other, the queries
+ * first, where they do not or where one's result lies in the other's memory. */
 int32_t fastmax_normalize_forward_qk(int32_t batch, int32_t heads, int32_t nq, int32_t nk, int32_t d, int32_t dtype,
                                      float lim, const fastmax_tensor* q, const fastmax_tensor* yq,
                                      const fastmax_tensor* k, const fastmax_tensor* yk,

@@ -1047,13 +1047,30 @@ int32_t fastmax_normalize_backward(int32_t batch, int32_t heads, int32_t n, int3
   return FASTMAX_OK;
 }
 
-// Queries and keys of a call: one launch where both take the cluster kernel, else one after the other.
+// Whether the memory that two views span has bytes in common.
+static bool share_memory(const fastmax_tensor* a, int na, const fastmax_tensor* b, int nb, int batch, int heads, int d, int dtype) {
+  const int64_t es = dtype == FASTMAX_F32 ? 4 : 2;
+  int64_t lo[2], hi[2];
+  for (int i = 0; i < 2; ++i) {
+    const fastmax_tensor* t = i ? b : a;
+    const int64_t steps[3] = {(batch - 1) * t->stride_b, (heads - 1) * t->stride_h, ((i ? nb : na) - 1) * t->stride_n};
+    lo[i] = hi[i] = 0;
+    for (int64_t s : steps) (s < 0 ? lo[i] : hi[i]) += s;
+    lo[i] = (int64_t)(intptr_t)t->ptr + es * lo[i];
+    hi[i] = (int64_t)(intptr_t)t->ptr + es * (hi[i] + d);
+  }
+  return lo[0] < hi[1] && lo[1] < hi[0];
+}
+// Queries and keys of a call: one launch where both take the cluster kernel, else one after the other: so too where one of them is
+// written into the other's memory (in place, as windows of one buffer).
 int32_t fastmax_normalize_forward_qk(int32_t batch, int32_t heads, int32_t nq, int32_t nk, int32_t d, int32_t dtype, float lim,
                                      const fastmax_tensor* q, const fastmax_tensor* yq, const fastmax_tensor* k, const fastmax_tensor* yk,
                                      uint64_t* stats_q, uint64_t* stats_k, void* stream) {
   const int most = nq > nk ? nq : nk;
   if (q && yq && k && yk && q->ptr && yq->ptr && k->ptr && yk->ptr && stats_q && stats_k && batch > 0 && heads > 0 && nq > 0 && nk > 0 && lim > 0.f &&
-      (dtype == FASTMAX_F32 || dtype == FASTMAX_BF16) && norm_vec_ok(d, dtype, {q, yq, k, yk}) && (long long)batch * heads <= 65535) {
+      (dtype == FASTMAX_F32 || dtype == FASTMAX_BF16) && norm_vec_ok(d, dtype, {q, yq, k, yk}) && (long long)batch * heads <= 65535 &&
+      !share_memory(yq, nq, k, nk, batch, heads, d, dtype) && !share_memory(yq, nq, yk, nk, batch, heads, d, dtype) &&
+      !share_memory(q, nq, yk, nk, batch, heads, d, dtype)) {
     if (const int cl = norm_cluster_size(2LL * batch * heads, most, d, false)) {
       cudaStream_t st = (cudaStream_t)stream;
       const NormArgs A{{to_view(*q), to_view(*k)}, {to_view(*yq), to_view(*yk)}, {(int)nq, (int)nk},
@@ -1073,7 +1090,10 @@ int32_t fastmax_normalize_backward_qk(int32_t batch, int32_t heads, int32_t nq, 
   const int most = nq > nk ? nq : nk;
   if (yq && dyq && dxq && yk && dyk && dxk && yq->ptr && dyq->ptr && dxq->ptr && yk->ptr && dyk->ptr && dxk->ptr && stats_q && stats_k && batch > 0 &&
       heads > 0 && nq > 0 && nk > 0 && lim > 0.f && (dtype == FASTMAX_F32 || dtype == FASTMAX_BF16) &&
-      norm_vec_ok(d, dtype, {yq, dyq, dxq, yk, dyk, dxk}) && (long long)batch * heads <= 65535) {
+      norm_vec_ok(d, dtype, {yq, dyq, dxq, yk, dyk, dxk}) && (long long)batch * heads <= 65535 &&
+      !share_memory(dxq, nq, yk, nk, batch, heads, d, dtype) && !share_memory(dxq, nq, dyk, nk, batch, heads, d, dtype) &&
+      !share_memory(dxq, nq, dxk, nk, batch, heads, d, dtype) && !share_memory(yq, nq, dxk, nk, batch, heads, d, dtype) &&
+      !share_memory(dyq, nq, dxk, nk, batch, heads, d, dtype)) {
     if (const int cl = norm_cluster_size(2LL * batch * heads, most, d, true)) {
       cudaStream_t st = (cudaStream_t)stream;
       const NormBwdArgs A{{to_view(*yq), to_view(*yk)}, {to_view(*dyq), to_view(*dyk)}, {to_view(*dxq), to_view(*dxk)}, {(int)nq, (int)nk},

@@ -87,13 +87,7 @@ torch::Tensor forwardpass(torch::Tensor q, torch::Tensor k, torch::Tensor v, tor
     auto stats = torch::empty({2 * bh}, q.options().dtype(torch::kInt64));
     uint64_t* sp = (uint64_t*)stats.data_ptr();
     fastmax_tensor qv = view_nbd(q), kv = view_nbd(k);
-    const char *q0 = (const char*)q.data_ptr(), *k0 = (const char*)k.data_ptr();
-    if (q0 < k0 + k.nbytes() && k0 < q0 + q.nbytes()) {   // they share memory and are written in place: one after the other
-      check_status(fastmax_normalize_forward(1, bh, nq, d, FASTMAX_F32, lim, &qv, &qv, sp, stream), "fastmax normalize(q)");
-      check_status(fastmax_normalize_forward(1, bh, nk, d, FASTMAX_F32, lim, &kv, &kv, sp, stream), "fastmax normalize(k)");
-    } else {
-      check_status(fastmax_normalize_forward_qk(1, bh, nq, nk, d, FASTMAX_F32, lim, &qv, &qv, &kv, &kv, sp, sp + bh, stream), "fastmax normalize");
-    }
+    check_status(fastmax_normalize_forward_qk(1, bh, nq, nk, d, FASTMAX_F32, lim, &qv, &qv, &kv, &kv, sp, sp + bh, stream), "fastmax normalize");
   }
   if (temperature != 1.0f) {   // k <- k / temperature in place, as apply_rpe_and_temp does (fwd.cu:282-292)
     fastmax_tensor kv = view_nbd(k);

@@ -459,3 +459,42 @@ def test_forwardpass_normalises_overlapping_tensors_one_after_the_other(shift):
         ref[window] = L.normalize_forward(x, 1.0)[0][0].permute(1, 0, 2)
     ext.forwardpass(buf[:n], buf[shift:], v, noise, rpe, True, 0.0, True, 1.0, 1.0, 1.0, 0.5, 1.0, 2)
     assert torch.allclose(buf, ref, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("bh", [6, 24, 160])
+@pytest.mark.parametrize("shift", [0, 1, 37])
+def test_normalising_windows_of_one_buffer_in_place(bh, shift):
+    """fastmax_normalize_forward_qk and its backward on views that overlap, whatever the number of heads: queries first, then keys
+    on what the queries left."""
+    import ctypes as C
+
+    from reproducing_fastmax_results_b200 import _lib as L
+
+    lib = L.load()
+    fwd, bwd = lib.fastmax_normalize_forward_qk, lib.fastmax_normalize_backward_qk
+    p, i32 = C.c_void_p, C.c_int32
+    fwd.argtypes = [i32] * 6 + [C.c_float] + [p] * 7
+    bwd.argtypes = [i32] * 6 + [C.c_float] + [p] * 10
+    n, d = 400, 32
+    g = torch.Generator(device="cuda").manual_seed(shift)
+    buf = torch.randn(1, bh, n + shift, d, device="cuda", generator=g)
+    grads = torch.randn(1, bh, n + shift, d, device="cuda", generator=g)
+    ref, gref = buf.clone(), grads.clone()
+    stats = []
+    for window in (slice(0, n), slice(shift, n + shift)):
+        y, st = L.normalize_forward(ref[:, :, window], 1.0)
+        ref[:, :, window] = y
+        stats.append(st)
+    for window, st in zip((slice(0, n), slice(shift, n + shift)), stats):
+        gref[:, :, window] = L.normalize_backward(ref[:, :, window], gref[:, :, window], st, 1.0)
+    q, k = buf[:, :, :n], buf[:, :, shift:]
+    st = torch.empty(2, bh, dtype=torch.int64, device="cuda")
+    qv, kv = L.view_bhnd(q), L.view_bhnd(k)
+    stream = torch.cuda.current_stream().cuda_stream
+    assert fwd(1, bh, n, n, d, L.dtype_code(q), 1.0, C.byref(qv), C.byref(qv), C.byref(kv), C.byref(kv), st[0].data_ptr(), st[1].data_ptr(), stream) == 0
+    assert torch.allclose(buf, ref, rtol=1e-5, atol=1e-6)
+    scratch = torch.empty(bh, device="cuda")
+    gq, gk = L.view_bhnd(grads[:, :, :n]), L.view_bhnd(grads[:, :, shift:])
+    assert bwd(1, bh, n, n, d, L.dtype_code(q), 1.0, C.byref(qv), C.byref(gq), C.byref(gq), C.byref(kv), C.byref(gk), C.byref(gk), st[0].data_ptr(),
+               st[1].data_ptr(), scratch.data_ptr(), stream) == 0
+    assert torch.allclose(grads, gref, rtol=1e-4, atol=1e-4 * float(gref.abs().max()))
