@@ -498,3 +498,51 @@ def test_normalising_windows_of_one_buffer_in_place(bh, shift):
     assert bwd(1, bh, n, n, d, L.dtype_code(q), 1.0, C.byref(qv), C.byref(gq), C.byref(gq), C.byref(kv), C.byref(gk), C.byref(gk), st[0].data_ptr(),
                st[1].data_ptr(), scratch.data_ptr(), stream) == 0
     assert torch.allclose(grads, gref, rtol=1e-4, atol=1e-4 * float(gref.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,d,normalize", [(384, 64, True), (130, 32, False), (2304, 32, False)])
+def test_kernels_that_start_early_follow_one_another(n, d, normalize, dtype):
+    """Training calls of the pairwise and window forms, and decoding steps, whose kernels start while the one before them ends: back
+    to back, in memory that the call before has just used, and replayed from a graph, they give the bits of calls that run alone."""
+    from reproducing_fastmax_results_b200 import _lib as L, fastmax_custom
+    from reproducing_fastmax_results_b200.decoding import FastmaxDecoder
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    sets = [[torch.randn(2, 8, n, d, device="cuda", generator=g).to(dtype).requires_grad_(i < 3) for i in range(4)] for _ in range(3)]
+
+    def call(q, k, v, do):
+        o = fastmax_custom(q, k, v, None, None, True, 0.0, normalize, 1.0 if normalize else 8.0 * math.sqrt(d), 1.0, 1.0, 0.5, 1.0, 2)
+        return (o.detach(),) + torch.autograd.grad(o, (q, k, v), do)
+
+    def steps(q, k, v, do):
+        dec = FastmaxDecoder(2, 8, d, p=2, temperature=8.0)
+        return [dec.step(*(x[:, :, t].detach() for x in (q, k, v))).clone() for t in range(4)] + [dec.state]
+
+    alone = []
+    for s in sets:
+        alone.append([list(call(*s)), steps(*s)])
+        torch.cuda.synchronize()
+    for _ in range(3):
+        together = [[list(call(*s)), steps(*s)] for s in sets]   # no synchronisation between them
+        for a, b in zip(alone, together):
+            assert all(torch.equal(x, y) for x, y in zip(a[0] + a[1], b[0] + b[1]))
+        del together
+    q, k, v, do = ([x.detach().clone().requires_grad_(i < 3) for i, x in enumerate(sets[0])])
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call(q, k, v, do)
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs = call(q, k, v, do)
+    for s, want in list(zip(sets, alone)) * 3:
+        with torch.no_grad():
+            for mine, theirs in zip((q, k, v, do), s):
+                mine.copy_(theirs)
+        graph.replay()
+        assert all(torch.equal(x, y) for x, y in zip(outs, want[0]))
+    L.check_status()
+    assert L.wait_histogram() == {}
