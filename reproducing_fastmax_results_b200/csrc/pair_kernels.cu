@@ -56,9 +56,9 @@ enum Kind { FWD = 0, DQ = 1, DKV = 2 };
 // sixteen (us): 128 heads of 2048 x 32 dq 84 -> 79, dk / dv 124 -> 111; 192 of 577 x 64 without a mask dk / dv 47 -> 44.  dq with 64
 // dims has three operations per score and keeps eight: 343 with sixteen, 335 with eight (128 heads of 4096).  The forward has eight,
 // two per quarter, one per held tile, because a row's weights are added up there: one thread does it, in the order of the columns,
-// and every bit of g, which the outputs and gradients are divided by, stays what it is.  Sixteen warps with a row in two parts gave
-// other bits (240 -> 246, 31 -> 31, 33 -> 31, 68 -> 62 us: 128 heads of 4096 x 64, of 1024 x 64, 192 of 577 x 64, 128 of 2048 x 32);
-// sixteen with the same bits were no faster: four threads a row (16-lane loads) 261, 32, 33, 67; chains handed on 294, 36, 37, 80.
+// and every bit of g, which the outputs and gradients are divided by, stays what it is.  us forward, 128 heads of 4096 x 64, of 1024 x
+// 64, 192 of 577 x 64, 128 of 2048 x 32: eight 247, 31, 33, 68; sixteen with a row in two parts 247, 31, 31, 62, but other bits; sixteen
+// with the same bits: four threads a row (16-lane loads) 261, 32, 33, 67; the chains handed from warp to warp 296, 36, 37, 80.
 template <int D, int KIND>
 constexpr int EW = KIND == FWD || (KIND == DQ && D == 64) ? 8 : 16;
 template <int D, int KIND>
@@ -360,6 +360,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
     const uint64_t dHa = make_smem_desc(smem_u32(sm + OFF_H), 128, 256, 0), dHb = make_smem_desc(smem_u32(sm + OFF_H + R * 32), 128, 256, 0);
     uint32_t tile = 0;            // streamed tiles so far
     uint32_t cnt[2] = {0, 0};     // FWD: of each held tile
+    uint32_t buf = 0, use = 0;    // else: score buffer, times that it has been used
     int idx = blockIdx.x;
     for (int n = 0; idx >= 0; ++n) {
       const Item it = decode<KIND, T, HELD_ROWS>(idx, P);
@@ -373,9 +374,13 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
 #pragma unroll
         for (int m = 0; m < (KIND == FWD ? 2 : 1); ++m) {
           if (i < (m ? it.n1 : it.n0)) {
-            const uint32_t k = KIND == FWD ? cnt[m]++ : tile, buf = KIND == FWD ? (uint32_t)m : k & 1u;
-            if (KIND == FWD) { if (k > 0) WAIT(B_READS + m, k - 1u, 80); }               // the last scores have been read
-            else if (k >= 2) WAIT(B_SFREE + (int)buf, (k >> 1) - 1u, 80);   // the second products that read this buffer are done
+            if (KIND == FWD) {
+              buf = (uint32_t)m;
+              if (cnt[m] > 0) WAIT(B_READS + m, cnt[m] - 1u, 80);      // the last scores have been read
+              cnt[m]++;
+            } else if (use > 0) {
+              WAIT(B_SFREE + (int)buf, use - 1u, 80);                  // the second products that read this buffer are done
+            }
             tc_fence_after_sync();
             const uint32_t c = tmem + C_S + buf * 128u;
             const bool add_h = SQ && !first_rows(P, it.r0 + m * R);
@@ -391,6 +396,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
                 mma_ss_elect(tmem + C_DP, dH + (uint64_t)((X_BYTES >> 4) + 2 * ks), dY + (uint64_t)(2 * ks), ID_S, ks > 0);
             }
             mma_commit_elect(&bars[B_S + (int)buf]);
+            if (KIND != FWD && ++buf == 2) { buf = 0; ++use; }
           }
         }
         ++tile;
@@ -406,7 +412,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
     // ================= issuer of the second products =================
     constexpr uint32_t ID_ACC = make_idesc_bf16(R, D, 0, 1);
     const uint64_t dXm = make_smem_desc(smem_u32(sm + OFF_X), X_BYTES, 1024, 2);     // streamed tile, MN-major
-    uint32_t tile = 0, cnt[2] = {0, 0};   // as above
+    uint32_t tile = 0, cnt[2] = {0, 0}, buf = 0, use = 0;   // as above
     uint32_t nfree[2] = {0, 0};   // items that have started on each accumulator
     int idx = blockIdx.x;
     for (int n = 0; idx >= 0; ++n) {
@@ -423,8 +429,8 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
               if (nfree[m] > 0) WAIT(B_AFREE + m, nfree[m] - 1u, 79);
               nfree[m]++;
             }
-            const uint32_t k = KIND == FWD ? cnt[m]++ : tile, buf = KIND == FWD ? (uint32_t)m : k & 1u;
-            WAIT(B_P + (int)buf, KIND == FWD ? k : k >> 1, 72);   // the bf16 tiles of the element-wise warps
+            if (KIND == FWD) { buf = (uint32_t)m; use = cnt[m]++; }
+            WAIT(B_P + (int)buf, use, 72);   // the bf16 tiles of the element-wise warps
             tc_fence_after_sync();
             const uint32_t keep = i > 0 ? 1u : 0u;
             const uint32_t a = tmem + (KIND == FWD ? C_P + buf * 64u : C_S + buf * 128u);
@@ -437,6 +443,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
                 mma_ts_elect(tmem + C_ACC1, a + weights_at<KIND>(kk, true), dX + (uint64_t)(128 * kk), ID_ACC, kk > 0 ? 1u : keep);
             }
             mma_commit_elect(&bars[B_SFREE + (int)buf]);
+            if (KIND != FWD && ++buf == 2) { buf = 0; ++use; }
             if (KIND != FWD || m == 1 || i >= it.n1) mma_commit_elect(&bars[B_EMPTY + s]);
             if (i == nm - 1) mma_commit_elect(&bars[B_ACC + m]);
           }
@@ -462,6 +469,8 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
     uint64_t sum[4] = {0ull, 0ull, 0ull, 0ull};   // FWD: four chains, one would serialise the additions
     uint64_t ND = 0ull;                           // DQ: -delta of this row
     uint32_t k = 0;          // tiles of this warp's group so far
+    uint32_t buf = KIND == FWD ? (uint32_t)grp : 0u;   // score buffer of the next tile
+    uint32_t phases = 0;     // per buffer: the phase that the next scores there complete
     uint32_t done = 0;       // items whose results this warp has written
     // Results of an item are written after the next item's first tile, whose products run meanwhile.
     auto results = [&](int n, const Item& it, float total) {
@@ -558,8 +567,8 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
         ND = pack2(nd, nd);
       }
       for (int i = 0; i < nt; ++i, ++k) {
-        const uint32_t buf = KIND == FWD ? (uint32_t)grp : k & 1u;
-        WAIT(B_S + (int)buf, KIND == FWD ? k : k >> 1, 74);
+        WAIT(B_S + (int)buf, KIND == FWD ? k : phases >> buf, 74);
+        if (KIND != FWD) phases ^= 1u << buf;
         if (KIND == DKV) WAIT(B_FULL + (int)(k & (STAGES - 1)), k / STAGES, 81);
         tc_fence_after_sync();
         const int x0 = (it.t0 + i) * T + part * W;   // streamed row of this warp's first column
@@ -692,6 +701,7 @@ __global__ void __launch_bounds__(THREADS<D, KIND>, 1) pair_kernel(const __grid_
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[B_P + (int)buf]);
+        if (KIND != FWD) buf ^= 1u;
         if (i == 0 && pend) results(n - 1, last, total);
         if (i == 1 && pend) give_back(n - 1);
       }
