@@ -905,22 +905,34 @@ static bool norm_vec_ok(int d, int dtype, std::initializer_list<const fastmax_te
     }                                                                                                   \
   } while (0)
 
-// Blocks per (batch, head) of the one-launch form, or 0 for the two-launch form, whose blocks spread over all tokens.  heads: of all
+// Blocks per (batch, head) of the one-launch form, or 0 for the two-launch form, whose blocks spread over all tokens.  heads: of one of
 // the call's tensors.  Blocks of at least 256 rows at d = 64 in the forward, which reads them twice, and as few blocks as fill the
 // device in the backward, which is one pass and a barrier; more where heads are few.  us, forward / backward of two tensors for 1, 2,
 // 4, 8 blocks a head: 128 heads of 1024 x 64 bf16 24 / 35, 21 / 23, 21 / 27, 21 / 33; of 4096 x 64 159 / 138, 101 / 90, 78 / 92,
 // 72 / 97; 192 of 577 x 64 19 / 22, 19 / 24, 19 / 25, 25 / 35; 24 of 512 x 64 12 / 12, 9 / 8, 7 / 8, 7 / 7 (two launches a tensor 25 / 24).
-// Few long heads: a block walks up to 32 steps of 256 threads in less time than two more launches a tensor take.
-static int norm_cluster_size(long long heads, int n, int d, bool backward) {
+// Few long heads: two launches take 12.6 a tensor, a block 0.55 to 0.7 for a step of 256 threads (2 heads of 4096 x 64 float32, 16 steps:
+// one tensor 13.1, two 13.4; of 8192, 32 steps: 22.6 and 22.9).
+static int norm_cluster_size(int tensors, long long heads, int n, int d, bool backward) {
   const int rows = 256 / (d / 8);   // per step
   const long long fill = 5LL * sm_count() / 2;
+  heads *= tensors;
   int cl = 1;
   if (!backward)
     while (cl < 8 && n >= 2 * cl * rows * 8) cl *= 2;
   while (cl < 8 && heads * cl < fill && n >= 2 * cl * rows * 2) cl *= 2;
-  return heads * cl >= 2LL * sm_count() || n <= 32 * cl * rows ? cl : 0;
+  return heads * cl >= 2LL * sm_count() || n <= 16 * tensors * cl * rows ? cl : 0;
 }
-#define FM_NORM_FUSED(KERNEL, CL, COUNT, ...)                                                                  \
+// Whether the blocks start while the kernel before them ends (grid_wait).  Those of a launch that is all at work at once are then placed
+// where that kernel leaves room first, several to one SM and none to another: fine where a block is short (some steps of 256
+// threads), where every block finds an SM of its own and where the launch has many rounds of blocks.  us, back to back, without / with:
+// 48 heads of 4096 x 64 float32, two tensors, 768 blocks of 16 steps 49.6 / 59.5, 96 of 2048 x 64 24.9 / 30.5; 12 of 8192 x 64, 192
+// blocks of 32 steps 31.2 / 38.4; but 8 of 1024 x 64, one tensor, 64 blocks of 4 steps 8.4 / 5.8.
+static bool norm_early(int cl, long long blocks, int n, int d) {
+  const int steps = (n + cl * (256 / (d / 8)) - 1) / (cl * (256 / (d / 8)));
+  const long long sms = sm_count();
+  return steps <= 4 || blocks <= (steps <= 8 ? 4 : 1) * sms || blocks > 8 * sms;
+}
+#define FM_NORM_FUSED(KERNEL, CL, COUNT, N, ...)                                                                  \
   do {                                                                                                  \
     cudaLaunchConfig_t cfg = {};                                                                        \
     cfg.gridDim = dim3((unsigned)(CL), (unsigned)(batch * heads), (unsigned)(COUNT));                                      \
@@ -933,7 +945,7 @@ static int norm_cluster_size(long long heads, int n, int d, bool backward) {
     attr[0].val.clusterDim.z = 1;                                                                       \
     attr[1] = launch_attribute_after();                                                                 \
     cfg.attrs = attr;                                                                                   \
-    cfg.numAttrs = 2;                                                                                   \
+    cfg.numAttrs = norm_early(CL, (long long)(CL) * batch * heads * (COUNT), N, d) ? 2 : 1;             \
     cudaError_t fe;                                                                                     \
     if (dtype == FASTMAX_F32) {                                                                         \
       if (d == 64) fe = cudaLaunchKernelEx(&cfg, KERNEL<float, 8>, __VA_ARGS__);                        \
@@ -954,7 +966,7 @@ int32_t fastmax_normalize_forward(int32_t batch, int32_t heads, int32_t n, int32
   if (dtype != FASTMAX_F32 && dtype != FASTMAX_BF16) return FASTMAX_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   long long nrows = (long long)batch * heads * n;
-  const int cl = nrows > 0 && norm_vec_ok(d, dtype, {x, y}) && (long long)batch * heads <= 65535 ? norm_cluster_size((long long)batch * heads, n, d, false) : 0;
+  const int cl = nrows > 0 && norm_vec_ok(d, dtype, {x, y}) && (long long)batch * heads <= 65535 ? norm_cluster_size(1, (long long)batch * heads, n, d, false) : 0;
   if (cl == 0) FM_CUDA(cudaMemsetAsync(stats, 0, (size_t)batch * heads * sizeof(uint64_t), st));   // (the cluster kernel writes all of it)
   if (nrows == 0) return FASTMAX_OK;
   int threads = 256;
@@ -964,7 +976,7 @@ int32_t fastmax_normalize_forward(int32_t batch, int32_t heads, int32_t n, int32
     if (cl > 0) {
       const NormArgs A{{to_view(*x)}, {to_view(*y)}, {(int)n}, {sp}};
       LaunchScope ls(KK_NORMALIZE, st);
-      FM_NORM_FUSED(norm_fused_vec_kernel, cl, 1, A, (int)heads, lim);
+      FM_NORM_FUSED(norm_fused_vec_kernel, cl, 1, n, A, (int)heads, lim);
       return FASTMAX_OK;
     }
     {
@@ -1005,7 +1017,7 @@ int32_t fastmax_normalize_backward(int32_t batch, int32_t heads, int32_t n, int3
   if (dtype != FASTMAX_F32 && dtype != FASTMAX_BF16) return FASTMAX_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   long long nrows = (long long)batch * heads * n;
-  const int cl = nrows > 0 && norm_vec_ok(d, dtype, {y, dy, dx}) && (long long)batch * heads <= 65535 ? norm_cluster_size((long long)batch * heads, n, d, true) : 0;
+  const int cl = nrows > 0 && norm_vec_ok(d, dtype, {y, dy, dx}) && (long long)batch * heads <= 65535 ? norm_cluster_size(1, (long long)batch * heads, n, d, true) : 0;
   if (cl == 0) FM_CUDA(cudaMemsetAsync(scratch, 0, (size_t)batch * heads * sizeof(float), st));
   if (nrows == 0) return FASTMAX_OK;
   int threads = 256;
@@ -1015,7 +1027,7 @@ int32_t fastmax_normalize_backward(int32_t batch, int32_t heads, int32_t n, int3
     if (cl > 0) {
       const NormBwdArgs A{{to_view(*y)}, {to_view(*dy)}, {to_view(*dx)}, {(int)n}, {sp}};
       LaunchScope ls(KK_NORMALIZE, st);
-      FM_NORM_FUSED(norm_bwd_fused_vec_kernel, cl, 1, A, (int)heads, lim);
+      FM_NORM_FUSED(norm_bwd_fused_vec_kernel, cl, 1, n, A, (int)heads, lim);
       return FASTMAX_OK;
     }
     {
@@ -1071,12 +1083,12 @@ int32_t fastmax_normalize_forward_qk(int32_t batch, int32_t heads, int32_t nq, i
       (dtype == FASTMAX_F32 || dtype == FASTMAX_BF16) && norm_vec_ok(d, dtype, {q, yq, k, yk}) && (long long)batch * heads <= 65535 &&
       !share_memory(yq, nq, k, nk, batch, heads, d, dtype) && !share_memory(yq, nq, yk, nk, batch, heads, d, dtype) &&
       !share_memory(q, nq, yk, nk, batch, heads, d, dtype)) {
-    if (const int cl = norm_cluster_size(2LL * batch * heads, most, d, false)) {
+    if (const int cl = norm_cluster_size(2, (long long)batch * heads, most, d, false)) {
       cudaStream_t st = (cudaStream_t)stream;
       const NormArgs A{{to_view(*q), to_view(*k)}, {to_view(*yq), to_view(*yk)}, {(int)nq, (int)nk},
                        {reinterpret_cast<unsigned long long*>(stats_q), reinterpret_cast<unsigned long long*>(stats_k)}};
       LaunchScope ls(KK_NORMALIZE, st);
-      FM_NORM_FUSED(norm_fused_vec_kernel, cl, 2, A, (int)heads, lim);
+      FM_NORM_FUSED(norm_fused_vec_kernel, cl, 2, most, A, (int)heads, lim);
       return FASTMAX_OK;
     }
   }
@@ -1094,12 +1106,12 @@ int32_t fastmax_normalize_backward_qk(int32_t batch, int32_t heads, int32_t nq, 
       !share_memory(dxq, nq, yk, nk, batch, heads, d, dtype) && !share_memory(dxq, nq, dyk, nk, batch, heads, d, dtype) &&
       !share_memory(dxq, nq, dxk, nk, batch, heads, d, dtype) && !share_memory(yq, nq, dxk, nk, batch, heads, d, dtype) &&
       !share_memory(dyq, nq, dxk, nk, batch, heads, d, dtype)) {
-    if (const int cl = norm_cluster_size(2LL * batch * heads, most, d, true)) {
+    if (const int cl = norm_cluster_size(2, (long long)batch * heads, most, d, true)) {
       cudaStream_t st = (cudaStream_t)stream;
       const NormBwdArgs A{{to_view(*yq), to_view(*yk)}, {to_view(*dyq), to_view(*dyk)}, {to_view(*dxq), to_view(*dxk)}, {(int)nq, (int)nk},
                           {reinterpret_cast<const unsigned long long*>(stats_q), reinterpret_cast<const unsigned long long*>(stats_k)}};
       LaunchScope ls(KK_NORMALIZE, st);
-      FM_NORM_FUSED(norm_bwd_fused_vec_kernel, cl, 2, A, (int)heads, lim);
+      FM_NORM_FUSED(norm_bwd_fused_vec_kernel, cl, 2, most, A, (int)heads, lim);
       return FASTMAX_OK;
     }
   }

@@ -205,7 +205,7 @@ def test_normalize_forward_backward(dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("shape", [(8, 40, 333, 64), (4, 80, 333, 32), (8, 40, 1000, 16), (8, 16, 4096, 64), (1, 1, 1, 32), (1, 3, 200, 64), (1, 2, 8192, 64), (2, 4, 1100, 16)])
+@pytest.mark.parametrize("shape", [(8, 40, 333, 64), (4, 80, 333, 32), (8, 40, 1000, 16), (8, 16, 4096, 64), (1, 1, 1, 32), (1, 3, 200, 64), (1, 2, 4096, 64), (2, 4, 1100, 16)])
 def test_normalize_one_launch_per_direction(shape, dtype):
     """Many heads or short ones: one launch per direction (a thread-block cluster per head), ragged token
     counts, every cluster size; the argmax token sits in the middle of the sequence."""
@@ -230,6 +230,25 @@ def test_normalize_one_launch_per_direction(shape, dtype):
     y2, stats2 = L.normalize_forward(xd, 1.5)
     dx2 = L.normalize_backward(y2, dyd, stats2, 1.5)
     assert torch.equal(y, y2) and torch.equal(dx, dx2) and torch.equal(stats, stats2)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_normalize_one_tensor_of_few_long_heads(dtype):
+    """32 steps of a block take longer than the two launches whose blocks spread over all tokens: two launches per direction."""
+    rng = np.random.default_rng(8)
+    x, dy = (rng.standard_normal((1, 2, 8192, 64)).astype(np.float32) for _ in range(2))
+    x[:, :, 5000] *= 3.0
+    L = lib()
+    xd, dyd = dev(x, dtype), dev(dy, dtype)
+    L.profile_collect()
+    L.profile(True)
+    y, stats = L.normalize_forward(xd, 1.5)
+    dx = L.normalize_backward(y, dyd, stats, 1.5)
+    torch.cuda.synchronize()
+    L.profile(False)
+    assert L.profile_collect()["normalize"][1] == 4
+    assert orc.max_norm_err(host(y), orc.normalize(host(xd), 1.5)) < TOL[dtype]
+    assert orc.max_norm_err(host(dx), orc.normalize_grad(host(xd), host(dyd), 1.5)) < TOL[dtype]
 
 
 def test_normalize_golden_vectors():
