@@ -218,7 +218,7 @@ static cudaError_t launch(const DecodeParams& P, int bh, int cl, cudaStream_t st
   configure<D, RG>(cfg, attr, bh, cl, st);
   return launched(cudaLaunchKernelEx(&cfg, decode_step_kernel<T, D, ORDER, RG>, P));
 }
-// clusters of MAX_CL blocks of the 48-row kernel that the current device runs at once
+// clusters of MAX_CL blocks of the 48-row kernel that the current device runs at once with a block to an SM
 template <typename T, int D>
 static int clusters_at_once() {
   static std::atomic<int> cached[64];   // + 1
@@ -234,6 +234,7 @@ static int clusters_at_once() {
       cudaGetLastError();
       n = 0;
     }
+    if (n > sm_count() / MAX_CL) n = sm_count() / MAX_CL;
     cached[dev].store(n + 1, std::memory_order_relaxed);
   }
   return n;
@@ -244,8 +245,7 @@ static cudaError_t launch(int order, const DecodeParams& P, int bh, cudaStream_t
   while (cl < MAX_CL && (long long)cl * bh < 1024) cl *= 2;
   // (order 1 and D = 16 have at most 9 and 27 rows a block where the cluster is that large)
   if constexpr (D > 16)
-    if (order == 2 && cl == MAX_CL && (P.rows + cl - 1) / cl > 16 * UNROLL && cl * bh <= sm_count() && bh <= clusters_at_once<T, D>())
-      return launch<T, D, 2, 48>(P, bh, cl, st);
+    if (order == 2 && cl == MAX_CL && (P.rows + cl - 1) / cl > 16 * UNROLL && bh <= clusters_at_once<T, D>()) return launch<T, D, 2, 48>(P, bh, cl, st);
   return order == 2 ? launch<T, D, 2, 16>(P, bh, cl, st) : launch<T, D, 1, 16>(P, bh, cl, st);
 }
 
