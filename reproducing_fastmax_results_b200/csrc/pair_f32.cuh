@@ -11,7 +11,7 @@
 // element-wise warps add the tile's result to float32 totals in registers, rounding to nearest.
 //
 // Measured: 128 heads of 1024 x 64, causal, forward + backward with splitting 13400 us in the CUDA-core engine (FFMA), 520 here
-// (forward 110, dq 135, dk / dv 185, splitting 77, dO' 25); bf16, 128 heads of 1024 x 16 (q, k, v are one piece each: 1 or 3
+// (each launch by itself: forward 110, dq 135, dk / dv 185, splitting 78 in two passes, dO' 25; back to back they overlap); bf16, 128 heads of 1024 x 16 (q, k, v are one piece each: 1 or 3
 // products instead of 6, no pass that splits) 771 and 216.  Bound by the chain scores -> element-wise -> second products
 // between few warps (tensor pipe active in 51 to 65 % of the clocks at 64 dims, issue slots 30 %).  What took the forward from 131
 // to 110, dq from 156 to 135 and dk / dv from 216 to 185: scores in two blocks (product2), the results of a tile added up behind

@@ -16,11 +16,11 @@
 // control: it takes over a block that has not started), so the items' lengths may differ by any factor; the loads and
 // first products of the next item run under the last tiles and the stores of the current one.
 //
-// Bound by no pipe alone, and where the GPU is busy for long, by power.  ncu, 64 heads of 4096 x 64 (forward, dk / dv, dq): tensor
-// pipe active in 66, 69, 70 % of the clocks, issue slots 59, 61, 38 %.  128 heads of 4096 x 64 back to back draw 1000 W and run at
-// 1.55 to 1.65 GHz (1.24 ms for forward and backward, 1.06 at 1.9 GHz).  Measured (us, forward and backward; the scans of the moment
-// engine before): 128 heads of 4096 x 64, causal 2930 -> 1060; of 1024 x 64 570 -> 122; of 2048 x 32 1533 -> 258.  Heads of 16 dims
-// have the kernels of pair_f32.cuh.
+// Bound by no pipe alone, and where the GPU is busy for long, by power.  ncu (forward, dk / dv, dq), 64 heads of 4096 x 64: tensor
+// pipe active in 67, 69, 70 % of the clocks, issue slots 47, 61, 38 %; 128 heads of 2048 x 32: 33, 35, 40 % and 46, 65, 57 %.  128 heads
+// of 4096 x 64 back to back draw 1000 W and run at 1.55 to 1.65 GHz (1.23 ms for forward and backward, 1.07 at 1.9 GHz).  Measured (us,
+// forward and backward; the scans of the moment engine before): 128 heads of 4096 x 64, causal 2930 -> 1070; of 1024 x 64 570 -> 114;
+// of 2048 x 32 1533 -> 255.  Heads of 16 dims have the kernels of pair_f32.cuh.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -819,9 +819,9 @@ cudaError_t launch(const pair::Maps& M, const pair::Params& P, int bh, cudaStrea
   return launch_after(kernel, dim3((unsigned)(P.ntiles * bh)), pair::THREADS<D, KIND>, pair::SMEM_BYTES, st, M, P);
 }
 // Heads per group of the item order (decode).  With a mask, items differ in length: as many heads as have their streamed tiles in
-// 32 MB (pieces: 64 MB) of L2.  us forward / dq / dk, dv for 16, 32, 64, 128 MB: 128 heads of 4096 x 64 253 / 335 / 445,
-// 247 / 335 / 444, 248 / 341 / 445, 273 / 385 / 500; of 1024 x 64 33 / 38 / 47, then 31 / 37 / 46; float32, of 1024 x 64
-// 121 / 176 / 198, 114 / 166 / 190, 111 / 160 / 185, 110 / 156 / 188 (few items per block: the last group's long ones decide).
+// 32 MB (pieces: 64 MB) of L2.  us forward / dq / dk, dv for 16, 32, 64, 128 MB: 128 heads of 4096 x 64 252 / 337 / 453,
+// 245 / 337 / 452, 248 / 342 / 457, 273 / 395 / 518; of 1024 x 64 34 / 39 / 48, then 31 / 37 / 47; float32, of 1024 x 64
+// 120 / 144 / 198, 113 / 138 / 190, 110 / 135 / 185, 111 / 136 / 189 (few items per block: the last group's long ones decide).
 // Without a mask (and within windows) the items are alike, and the order of the heads is best for L2.
 void order_items(int d, int es, pair::Params& P, int bh) {
   long long group = 1;
@@ -880,14 +880,20 @@ bool rows_f32(const fastmax_tensor& t, const fastmax_problem* pb, int n) {
 // Which form takes a call.  USE_OUT: output alone; USE_TRAIN: forward and backward of a training call (the states of the forward
 // are handed on, so both take the same form); USE_PROMPT: output and final state.
 enum Use { USE_OUT, USE_TRAIN, USE_PROMPT };
-// The pairwise kernels cost about 1e-6 us per visible pair forward and backward (d = 64; narrower heads are bound by the
-// element-wise warps and cost the same), windows and states a time per token.  `per_token`, the keys a token sees on average,
-// at which both cost the same, from measurements at 64 to 128 heads (us, forward + backward, pairs / windows):
-//   order 2, mask:    d = 64 6144 tokens 1117 / 1240, 8192 1952 / 1790; d = 32 2048 358 / 433, 4096 1094 / 832
-//   order 2, no mask: d = 64 2048 302 / 473, 4096 1006 / 758;           d = 32 1024 108 / 118, 2048 272 / 163
-//   order 1, mask:    d = 64 1024 180 / 219, 2048 457 / 430;            d = 32 2048 371 / 323
-//   order 1, no mask: d = 64 512 89 / 107, 2048 568 / 192;              d = 32 1024 168 / 109
-// The forward alone crosses later (order 2, mask, d = 64: 8192 424 / 576, 16384 919 / 645), with a state to be returned earlier.
+// The pairwise kernels cost about 1e-6 us per visible pair forward and backward (d = 64; d = 32: 1.2e-6 to 0.9e-6, it is bound by the
+// same number of scores), windows and states a time per token.  `per_token`: the keys a token sees on average at which both cost the
+// same.  us at 128 heads, forward + backward, pairs / windows:
+//   order 2, mask:    d = 64 6144 tokens 2375 / 2536, 7168 3326 / 3057; d = 32 2048 349 / 492, 3072 690 / 659
+//   order 2, no mask: d = 64 2048 519 / 717, 3072 1106 / 989;           d = 32 1024 167 / 195, 1536 324 / 251
+//   order 1, mask:    d = 64 1536 256 / 330, 2048 358 / 425;            d = 32 1536 205 / 240, 2048 313 / 312
+//   order 1, no mask: d = 64 768 105 / 110, 1024 148 / 130;             d = 32 768 104 / 110, 1024 150 / 111
+// and forward alone: order 2, mask, d = 64 8192 874 / 1103, 11264 1628 / 1535, d = 32 4096 269 / 336, 6144 551 / 475; no mask, d = 64
+// 4096 448 / 436, d = 32 1536 82 / 81; order 1, mask, d = 64 2048 101 / 140, 3072 198 / 193, d = 32 2048 96 / 106; no mask, d = 32 1024
+// 51 / 42.  Prompts (pairs with the moments beside them / windows): order 2, d = 64 4096 479 / 596, 6144 872 / 925, d = 32 2048 302 /
+// 182; order 1, d = 64 1024 78 / 85, d = 32 1024 93 / 70.  At 60 heads training calls cross a little later (order 2, mask, d = 64
+// 7168 1425 / 1447; d = 32 4096 505 / 496).  The lines stand where the kernels before the present ones crossed: pairs are now the
+// faster form somewhat beyond those of order 1 with a mask (up to some 2500 tokens, 2000 with 32 dims) and of prompts of 64 dims (up to
+// some 6500), and windows below that of prompts of 32 dims.
 double window_line(const fastmax_problem* pb, Use use) {
   const bool wide = pb->d == 64;
   if (pb->order == 2) {
@@ -906,24 +912,23 @@ int chosen(const fastmax_problem* pb, bool backward, Use use) {   // 0: neither,
   const double per_token = pairs / (0.5 * (nq + nk));
   if (pb->dtype == FASTMAX_F32) {
     // against the CUDA-core engine, whose cost per token goes with d^3 (order 2) or d^2, while six piece products on half-empty
-    // tiles hardly get cheaper for narrow heads.  Measured ratios near the line (x = pairs faster, forward / backward):
-    // order 2: d = 64 12000 keys 2.0 / 1.9, d = 32 4096 keys 1.2-1.45 / 1.3-1.4, d = 16 2048 keys 1.05 / 1.2;
-    // order 1, mask: d = 64 2048 keys 1.2 / 1.2, d = 32 1024 keys 1.0 / 1.2; no mask: d = 64 1024 keys 1.3 / 1.3.
+    // tiles hardly get cheaper for narrow heads.  us, forward + backward, pairs / engine: order 2, no mask, d = 64 16 heads 12288 tokens
+    // 12900 / 22700, d = 32 32 heads 4096 2110 / 2570, 5120 3180 / 2440, d = 16 64 heads 1536 554 / 576, 2048 796 / 742; mask, d = 16 64
+    // heads 4096 1540 / 1983; order 1, mask, d = 64 64 heads 4096 2900 / 3710, d = 16 64 heads 1536 291 / 452, 2048 475 / 474; no mask, 64
+    // heads, d = 64 1024 544 / 513, 1280 793 / 633, d = 32 768 190 / 174, d = 16 512 89 / 135, 768 151 / 134.
     const double most = pb->order == 2 ? (pb->d == 64 ? 16000.0 : pb->d == 32 ? 5000.0 : 2000.0)
                         : pb->causal   ? (pb->d == 64 ? 2300.0 : pb->d == 32 ? 1050.0 : 900.0)
                                        : (pb->d == 64 ? 1300.0 : pb->d == 32 ? 800.0 : 600.0);
-    // d = 32 with a mask: windows and states (us, forward + backward, pairs / windows: order 2 64 heads 2048 tokens 724 / 589,
-    // 128 heads 1024 tokens 434 / 512; order 1 128 heads 1024 tokens 436 / 377)
+    // d = 32 with a mask: windows and states (us, forward + backward, pairs / windows: order 2 64 heads 1536 tokens 350 / 433, 2048
+    // 557 / 554; order 1 128 heads 768 tokens 232 / 268, 1024 351 / 342)
     if (pb->d == 32 && pb->causal && pb->nq == pb->nk && pb->nq < (1 << 30) && f32_registers_ok() && per_token > (pb->order == 2 ? 900. : 450.)) return 2;
     return per_token <= most && f32_registers_ok() ? 1 : 0;
   }
   // order 1 without a mask: one pass over the tensors (p1_forward_kernel), always the cheapest where it fills the GPU
   if (!backward && pb->order == 1 && !pb->causal && pb->d == 64 && (long long)pb->batch * pb->heads >= 64) return 0;
-  // d = 16: float32 weights (float32_weights) against the CUDA-core engine; there is no states kernel.  us, forward / backward,
-  // pairs against engine: order 2, mask, 64 heads 4096 tokens 359 / 1041 against 574 / 1565, 32 heads 8192 687 / 1996 against
-  // 543 / 1495; no mask, 64 heads 2048 182 / 521 against 202 / 602, 4096 680 / 1987 against 384 / 1175; order 1, mask, 64 heads
-  // 2048 103 / 295 against 122 / 350, 4096 359 / 1041 against 229 / 705; no mask, 64 heads 256 31 / 49 against 45 / 74, 128
-  // heads 1024 97 / 278 against 67 / 188.
+  // d = 16: float32 weights (float32_weights) against the CUDA-core engine; there is no states kernel.  us, forward + backward of 64
+  // heads, pairs / engine: order 2, mask, 4096 tokens 1261 / 1973, 6144 2737 / 2639; no mask, 2048 629 / 736, 4096 2420 / 1388; order 1,
+  // mask, 2048 357 / 453, 4096 1260 / 888; no mask, 256 81 / 133, 768 124 / 135, 128 heads 1024 336 / 233.
   if (pb->d == 16)
     return per_token <= (pb->order == 2 ? (pb->causal ? 3000.0 : 2300.0) : pb->causal ? 1200.0 : 700.0) && f32_registers_ok() ? 1 : 0;
   if (per_token <= window_line(pb, use)) return 1;

@@ -952,9 +952,11 @@ cudaError_t tc_moments(const fastmax_problem* pb, const fastmax_tensor& x, const
   P.per_split = seg_tokens > 0;
   // Tiles per block and cuts of the token axis: the combination that ends first when the SMs take the blocks in order (full
   // slices, then the shorter last ones), in clocks: 620 per tile and chunk, 12000 to start a block and write its rows, 20000 to
-  // add them, and 12000 for the memset that adding needs.  16 heads of 8192 tokens: 74 us with three tiles a block, 89 with
-  // four, 92 with four and two cuts; 128 heads of 4096: 220 us with four, 239 with three.  No more cuts than give the same bits
-  // whatever order they end in: two that add to zeros, one that adds to a carried state.
+  // add them, and 12000 for the memset that adding needs.  148 heads of 512 / 1024 / 2048 / 4096 tokens take 62.9 / 86.8 / 135.4 /
+  // 232.2 us, five blocks to an SM: 625 per tile and chunk and 15300 per block.  (With 15300 for the 12000, 1.6 % of the sizes from 4 to
+  // 1024 heads and 64 to 16384 tokens would be cut in another way, and the estimate gains 5 % at most.)  16 heads of 8192 tokens: 74 us
+  // with three tiles a block; 128 heads of 4096: 215 us with four.  No more cuts than give the same bits whatever order they end in:
+  // two that add to zeros, one that adds to a carried state.
   const int ntiles = pb->order == 2 ? npair / 2 + 1 : 1, sms = device_sms();
   const int segs = seg_tokens > 0 ? (n + seg_tokens - 1) / seg_tokens : 0, most = segs > 0 ? segs : init != nullptr ? 1 : 2;
   long long best = -1;

@@ -176,7 +176,7 @@ def test_key_moments_of_another_form_are_not_read(dtype, D, N, variant, binding,
 
 @pytest.mark.parametrize("order", [2, 1])
 def test_float32_windows_with_many_items_per_block(order):
-    """Several items per block in the moments, apply and chain kernels, whose producers take slabs in turn."""
+    """Several items per block in the moments, apply and chain kernels: their rings go on from one item to the next."""
     from reproducing_fastmax_results_b200 import _lib as L
 
     g = torch.Generator(device="cuda").manual_seed(order)
